@@ -9,7 +9,7 @@ short (7-tap FIR), medium (128-tap FIR) and long (implicit, pole/residue) Hyena 
 kernels for the same pieces: evo2/opt/evo2_opt/kit/base.py:55 ``_fir3_kernel``, :160 ``_hcs7_kernel_s``,
 :219/:242 FFT-convolution epilogues, gen/hyenafuse for the decode-step state update).
 
-Prefill runs the medium / long operators as FFT convolutions; decoding keeps per-layer state (FIR
+Prefill runs the medium operator as a direct convolution and the long one as its recurrence over chunks; decoding keeps per-layer state (FIR
 tails, pole states, attention KV cache) and advances one token per step.  Tensor parallelism shards
 the channel dimension of every operator (``parallel.tp``): column-parallel input projections, row-parallel
 output projections whose reduce-scatter is done by the GEMM epilogue over peer memory.  The causal attention
@@ -193,13 +193,19 @@ class HyenaOperator(nn.Module):
             self._taps = (seq.taps_major(self.fir), None if self.kind == "hcl" else seq.taps_major(self.h))
         return self._taps
 
-    def _fused_inner(self, u, x2, tail):
-        """x2 * (conv(u) + D u) with the gate folded into the convolution's epilogue."""
+    def _fused_inner(self, u, x2, state: Optional[dict] = None):
+        """x2 * (conv(u) + D u) with the gate folded into the convolution's epilogue.  The recurrence form of the long
+        operator ends with the pole state, which goes into ``state``."""
         from ..ops import seq
+        if self.kind == "hcl" and self.log_poles.shape[1] <= 16:
+            gated, poles = seq.pole_conv_gate(u, self._lam(), self.residues, self.D, x2)
+            if state is not None:
+                state["poles"] = poles
+            return gated
         if self.kind in ("hcs", "hcm") and self.h.shape[1] <= 512:
             # short filters from a register window, the medium filter (128 taps) as a tiled direct convolution:
             # 17 G multiply-adds per operator at the 7B shape against three FFT-sized fp32 passes
-            return seq.fir_inner_gate(u, self._kernel_taps()[1], self.D, x2, tail)
+            return seq.fir_inner_gate(u, self._kernel_taps()[1], self.D, x2)
         Hf, n = self.filter_spectrum(u.shape[1])
         X = torch.fft.rfft(seq.fft_pad_transpose(u, n))          # channel-major fp32, zero-padded to the transform size
         y = torch.fft.irfft(seq.spectrum_mul_(X, Hf.contiguous()), n=n)                   # [B, d, n] fp32
@@ -217,7 +223,7 @@ class HyenaOperator(nn.Module):
         if fused:
             from ..ops import seq
             u, x2 = seq.fir_gate3(z, self._kernel_taps()[0])
-            gated = self._fused_inner(u, x2, None)
+            gated = self._fused_inner(u, x2, state)
         else:
             zf = causal_fir(z, self.fir)
             x1, x2, v = zf.chunk(3, dim=-1)
@@ -228,10 +234,7 @@ class HyenaOperator(nn.Module):
             state["fir_tail"] = _last(z, K - 1)
             if self.kind in ("hcs", "hcm"):
                 state["inner_tail"] = _last(u, self.h.shape[1] - 1)
-            elif fused and self.log_poles.shape[1] <= 16:
-                from ..ops import seq
-                state["poles"] = seq.pole_prefill_state(u, self._lam())           # sum_t lam^(L-1-t) u_t
-            else:
+            elif not (fused and self.log_poles.shape[1] <= 16):                   # else set by the scan above
                 lam = torch.exp(self.log_poles.float())                           # [d, S]
                 L = u.shape[1]
                 w = lam.unsqueeze(0) ** torch.arange(L - 1, -1, -1, device=u.device, dtype=torch.float32).view(L, 1, 1)

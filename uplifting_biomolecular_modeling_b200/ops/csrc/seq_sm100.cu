@@ -653,61 +653,6 @@ __global__ void __launch_bounds__(256) pole_step_kernel(float* __restrict__ stat
   }
 }
 
-// ------------------------------------------------------------------------------------------ hcl prefill state
-// The pole state a prefill of L tokens leaves for decoding: state[b][c][k] = sum_t lam[c][k]^(L-1-t) u[b][t][c].
-// The sequence is split into chunks; a thread owns one channel and all S poles of it and runs the recurrence
-// s = s * lam + u over its chunk (the u loads of a CTA are 256 contiguous bytes per position); a second kernel
-// weights the chunk results by lam^(L - end of chunk) and adds them.  Writing the powers out as a [L][d][S]
-// tensor and contracting it - the plain statement - moves 8.6 GB per operator at the 7B shape.
-constexpr int kPoleMaxS = 16;
-
-__global__ void __launch_bounds__(128) pole_scan_kernel(const __nv_bfloat16* __restrict__ u,
-                                                        const float* __restrict__ lam, float* __restrict__ part,
-                                                        int L, int d, int S, int chunk) {
-  const int c = blockIdx.x * 128 + threadIdx.x;
-  const int ch = blockIdx.y, nch = gridDim.y, b = blockIdx.z;
-  if (c >= d) return;
-  const int t0 = ch * chunk;
-  const int t1 = min(L, t0 + chunk);
-  float lm[kPoleMaxS], st[kPoleMaxS];
-#pragma unroll
-  for (int k = 0; k < kPoleMaxS; ++k) {
-    lm[k] = k < S ? lam[static_cast<long long>(c) * S + k] : 0.f;
-    st[k] = 0.f;
-  }
-  const __nv_bfloat16* ub = u + static_cast<long long>(b) * L * d + c;
-#pragma unroll 8
-  for (int t = t0; t < t1; ++t) {
-    const float uv = __bfloat162float(ub[static_cast<long long>(t) * d]);
-#pragma unroll
-    for (int k = 0; k < kPoleMaxS; ++k) st[k] = fmaf(st[k], lm[k], uv);
-  }
-  float* o = part + ((static_cast<long long>(b) * nch + ch) * d + c) * S;
-#pragma unroll
-  for (int k = 0; k < kPoleMaxS; ++k)
-    if (k < S) o[k] = st[k];
-}
-
-__global__ void __launch_bounds__(256) pole_combine_kernel(const float* __restrict__ part,
-                                                           const float* __restrict__ lam, float* __restrict__ state,
-                                                           int B, int L, int d, int S, int chunk, int nch) {
-  const long long total = static_cast<long long>(B) * d * S;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long cs = i % (static_cast<long long>(d) * S);
-    const int b = static_cast<int>(i / (static_cast<long long>(d) * S));
-    const float lm = lam[cs];
-    float acc = 0.f;
-    for (int ch = 0; ch < nch; ++ch) {
-      const int t1 = min(L, (ch + 1) * chunk);
-      if (t1 <= ch * chunk) break;
-      const float w = powf(lm, static_cast<float>(L - t1));           // 1 for the last chunk
-      acc = fmaf(w, part[(static_cast<long long>(b) * nch + ch) * d * S + cs], acc);
-    }
-    state[i] = acc;
-  }
-}
-
 // ------------------------------------------------------------------------------------------ FFT-conv prologue
 // u: bf16 [B][L][d] -> out: fp32 [B][d][n], zero from position L on: the channel-major, zero-padded input the
 // real FFT of the long convolution reads (a cast, a strided copy and the transform's own padding otherwise).
@@ -1100,23 +1045,6 @@ extern "C" int ubm_fftconv_epilogue(const void* y, int n, const void* u, const v
       static_cast<const float*>(y), n, static_cast<const __nv_bfloat16*>(u), static_cast<const float*>(D),
       static_cast<const __nv_bfloat16*>(x2), static_cast<__nv_bfloat16*>(out), B, L, d);
   UBM_CHECK_LAUNCH("fftconv_epilogue_kernel");
-  return UBM_OK;
-}
-
-// u: bf16 [B][L][d]; lam: fp32 [d][S] (S <= 16); part: fp32 [B][chunks][d][S] scratch; state: fp32 [B][d][S]
-extern "C" int ubm_pole_prefill_state(const void* u, const void* lam, void* part, void* state, int B, int L, int d,
-                                      int S, int chunks, void* stream) {
-  if (B <= 0 || B > 65535 || L <= 0 || d <= 0 || S <= 0 || S > kPoleMaxS || chunks < 1 || chunks > 65535)
-    return UBM_ERR_ARGUMENT;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int chunk = (L + chunks - 1) / chunks;
-  pole_scan_kernel<<<dim3((d + 127) / 128, chunks, B), 128, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(u), static_cast<const float*>(lam), static_cast<float*>(part), L, d, S, chunk);
-  UBM_CHECK_LAUNCH("pole_scan_kernel");
-  pole_combine_kernel<<<seq_grid(static_cast<long long>(B) * d * S, 256), 256, 0, st>>>(
-      static_cast<const float*>(part), static_cast<const float*>(lam), static_cast<float*>(state), B, L, d, S, chunk,
-      chunks);
-  UBM_CHECK_LAUNCH("pole_combine_kernel");
   return UBM_OK;
 }
 

@@ -29,7 +29,7 @@ native.declare("ubm_residual_ln", [c_void_p] * 6 + [c_ll, c_int, c_float, c_void
 native.declare("ubm_gemv_fused", [c_void_p] * 2 + [c_float] + [c_void_p] * 5 + [c_int] * 3 + [c_void_p])
 native.declare("ubm_gemv_fused_w8", [c_void_p] * 2 + [c_float, c_void_p, c_float] + [c_void_p] * 3 + [c_int] * 3 + [c_void_p])
 native.declare("ubm_rmsnorm_fp8", [c_void_p] * 5 + [c_ll, c_int, c_float, c_void_p])
-native.declare("ubm_pole_prefill_state", [c_void_p] * 4 + [c_int] * 5 + [c_void_p])
+native.declare("ubm_pole_conv_gate", [c_void_p] * 8 + [c_int] * 5 + [c_void_p])
 native.declare("ubm_fft_pad_transpose", [c_void_p] * 2 + [c_int] * 4 + [c_void_p])
 native.declare("ubm_spectrum_mul", [c_void_p] * 2 + [c_int, c_ll, c_void_p])
 native.declare("ubm_decode_attention", [c_void_p] * 7 + [c_int] * 4 + [c_float] * 2 + [c_void_p] * 2)
@@ -183,19 +183,48 @@ def pole_step(state: torch.Tensor, lam: torch.Tensor, res: torch.Tensor, u: torc
     return out
 
 
+def _pole_chunk(B: int, L: int, d: int) -> int:
+    """Positions per chunk of :func:`pole_conv_gate`: about 16 CTAs of 128 channels per SM (148 of them), between 32
+    (below that the chunk states outweigh the sequence) and 1024, in whole batches of 32; long sequences take longer
+    chunks so that the chunk count fits a grid."""
+    per = B * L * d // (128 * 148 * 16)
+    return max(32, min(1024, (per + 31) // 32 * 32), (L + 65534) // 65535)
+
+
+def pole_conv_gate(u: torch.Tensor, lam: torch.Tensor, res: torch.Tensor, D: torch.Tensor,
+                   x2: Optional[torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Long operator of a prefill: (x2 * (sum_s res_s * state_s + D * u), state after the last position) with
+    state_t = state_(t-1) * lam + u_t from zero, the causal convolution with h[t] = sum_s res_s lam_s^t.
+    u, x2: bf16 [B, L, d]; lam, res: [d, S], S <= 16.  Returns (bf16 [B, L, d], fp32 [B, d, S])."""
+    u = _bf16c(u)
+    B, L, d = u.shape
+    lamf, resf, Df = _f32(lam), _f32(res), _f32(D)
+    S = lamf.shape[1]
+    chunk = _pole_chunk(B, L, d)
+    part = torch.empty((B, (L + chunk - 1) // chunk, d, S), dtype=torch.float32, device=u.device)
+    state = torch.empty((B, d, S), dtype=torch.float32, device=u.device)
+    out = torch.empty_like(u)
+    x2c = None if x2 is None else _bf16c(x2)
+    rc = native.lib().ubm_pole_conv_gate(native.ptr(u), native.ptr(lamf), native.ptr(resf), native.ptr(Df),
+                                         native.ptr(x2c), native.ptr(part), native.ptr(state), native.ptr(out), B, L, d,
+                                         S, chunk, _stream(u))
+    native.check(rc, "ubm_pole_conv_gate")
+    return out, state
+
+
 def pole_prefill_state(u: torch.Tensor, lam: torch.Tensor) -> torch.Tensor:
-    """The pole state a prefill leaves for decoding: fp32 [B, d, S] with state[b, c, k] = sum_t lam[c, k]^(L-1-t)
-    u[b, t, c].  u: bf16 [B, L, d]; lam: [d, S], S <= 16."""
+    """The state of :func:`pole_conv_gate` alone: fp32 [B, d, S] with state[b, c, k] = sum_t lam[c, k]^(L-1-t)
+    u[b, t, c]."""
     u = _bf16c(u)
     B, L, d = u.shape
     lamf = _f32(lam)
     S = lamf.shape[1]
-    chunks = max(1, min(64, (L + 1023) // 1024))
-    part = torch.empty((B, chunks, d, S), dtype=torch.float32, device=u.device)
+    chunk = _pole_chunk(B, L, d)
+    part = torch.empty((B, (L + chunk - 1) // chunk, d, S), dtype=torch.float32, device=u.device)
     state = torch.empty((B, d, S), dtype=torch.float32, device=u.device)
-    rc = native.lib().ubm_pole_prefill_state(native.ptr(u), native.ptr(lamf), native.ptr(part), native.ptr(state),
-                                             B, L, d, S, chunks, _stream(u))
-    native.check(rc, "ubm_pole_prefill_state")
+    rc = native.lib().ubm_pole_conv_gate(native.ptr(u), native.ptr(lamf), 0, 0, 0, native.ptr(part), native.ptr(state),
+                                         0, B, L, d, S, chunk, _stream(u))
+    native.check(rc, "ubm_pole_conv_gate")
     return state
 
 
