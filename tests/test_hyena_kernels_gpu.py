@@ -55,7 +55,39 @@ def test_pole_chunks_fit_a_grid_and_cover_the_sequence():
         assert 32 <= c and (L + c - 1) // c <= 65535
 
 
-@pytest.mark.parametrize("kind", ["hcl"])
+@pytest.mark.parametrize("K,L,d", [(65, 64, 8), (128, 64, 40), (100, 511, 72), (127, 513, 32), (128, 1300, 136)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_medium_filter_on_the_tensor_cores(K, L, d, gated):
+    from uplifting_biomolecular_modeling_b200.ops import seq
+    g = _gen(K + L)
+    u = torch.randn(2, L, d, device="cuda", generator=g).bfloat16()
+    x2 = torch.randn(2, L, d, device="cuda", generator=g).bfloat16() if gated else None
+    h = (torch.randn(d, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    D = torch.randn(d, device="cuda", generator=g)
+    out = seq.fir_inner_gate(u, seq.taps_major(h), D, x2, taps_bf16=True)
+    y = _conv(u.double(), h.double())
+    ref = (y + u.double() * D.double()) * (1.0 if x2 is None else x2.double())
+    assert ((out.double() - ref).abs() <= _bound(y, u, D, x2)).all()
+
+
+def test_medium_filter_keeps_infinities_where_the_multiply_adds_keep_them():
+    from uplifting_biomolecular_modeling_b200.ops import seq
+    g = _gen(5)
+    L, d, K = 1200, 40, 128
+    u = torch.randn(1, L, d, device="cuda", generator=g).bfloat16()
+    u[0, 300, 3], u[0, 700, 9], u[0, 1199, 0] = float("inf"), float("nan"), float("-inf")
+    x2 = torch.ones_like(u)
+    h = torch.randn(d, K, device="cuda", generator=g).bfloat16()
+    D = torch.zeros(d, device="cuda")
+    ht = seq.taps_major(h)
+    a = seq.fir_inner_gate(u, ht, D, x2, taps_bf16=True)
+    b = seq.fir_inner_gate(u, ht, D, x2)
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    ok = b.isfinite()
+    assert (a[ok].double() - b[ok].double()).abs().max() <= 2.0 ** -7 * b[ok].double().abs().max()
+
+
+@pytest.mark.parametrize("kind", ["hcm", "hcl"])
 def test_operator_prefill_matches_its_plain_statement(kind):
     from uplifting_biomolecular_modeling_b200.models import evo2
     torch.manual_seed(3)

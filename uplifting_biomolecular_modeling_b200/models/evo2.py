@@ -205,7 +205,7 @@ class HyenaOperator(nn.Module):
         if self.kind in ("hcs", "hcm") and self.h.shape[1] <= 512:
             # short filters from a register window, the medium filter (128 taps) as a tiled direct convolution:
             # 17 G multiply-adds per operator at the 7B shape against three FFT-sized fp32 passes
-            return seq.fir_inner_gate(u, self._kernel_taps()[1], self.D, x2)
+            return seq.fir_inner_gate(u, self._kernel_taps()[1], self.D, x2, taps_bf16=self.h.dtype == torch.bfloat16)
         Hf, n = self.filter_spectrum(u.shape[1])
         X = torch.fft.rfft(seq.fft_pad_transpose(u, n))          # channel-major fp32, zero-padded to the transform size
         y = torch.fft.irfft(seq.spectrum_mul_(X, Hf.contiguous()), n=n)                   # [B, d, n] fp32

@@ -1,4 +1,4 @@
-// Prefill kernels of the genomic decoder's long convolution operator.
+// Prefill kernels of the genomic decoder's long and medium convolution operators.
 //
 // Long operator (pole / residue filter h[t] = sum_s res_s lam_s^t): the convolution is run as the recurrence it
 // came from, s_k <- s_k lam_k + u, y = sum_k res_k s_k, over chunks of the sequence.  Three passes:
@@ -12,6 +12,10 @@
 // state for decoding included) against 0.75 ms of transform kernels, their epilogue and a separate state scan, and
 // 0.16 ms of copies around them.  Bound by the 48 multiply-adds per position and channel (45 us) and the waits of the
 // 2-byte accesses of a thread per channel.
+//
+// Medium operator (up to 128 taps): a depthwise convolution as one Toeplitz product per channel on mma.sync
+// m16n8k16 (see fir_toeplitz_kernel).  tcgen05 has no use here: a channel's operand is 16 x 144, its 128 x 64 tiles
+// would be mostly zero.
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -141,6 +145,167 @@ __global__ void __launch_bounds__(kPcThreads) pole_apply_kernel(
   }
 }
 
+// ------------------------------------------------------------------------------------------ medium operator
+// out = x2 * (bf16(fir(u)) + D u) for 64 < K <= 128 taps whose values are bf16 (a bf16 parameter), no tail.
+//
+// Per channel, positions are taken in blocks of 16: y[16 n + i] = sum_m sum_k T_m[i][k] u[16 (n - m) + k] with
+// T_m[i][k] = h[16 m + i - k], m = 0..8: nine m16n8k16 products give 128 positions.  Products of bf16 values are
+// exact and the sums are fp32, as on the FMA pipes.  T_m is Toeplitz, so a lane's A fragments of all nine products are
+// 36 registers, loaded once per channel and used for four groups of 128 positions.  The k index of a fragment is
+// permuted (a lane's four k values are four consecutive positions) so that a B fragment is one 8-byte shared load.
+//
+// A CTA owns 32 channels x 512 positions (+ 128 of halo), transposed into shared memory as [channel][position];
+// a warp owns four channels.  Results replace the inputs of their channel in place (the skip term is added there)
+// and leave through the same transpose, 16 bytes (8 channels) per access.
+// 8192 x 4096, 128 taps: 133 us against 248 us on the FMA pipes (17 G multiply-adds); what is left is the two
+// transposes through shared memory around 31 us of traffic.
+constexpr int kTpCh = 32;
+constexpr int kTpPos = 512;
+constexpr int kTpHalo = 128;
+constexpr int kTpThreads = 256;
+constexpr int kTpW = (kTpPos + kTpHalo) / 2 + 2;      // 32-bit words per channel row; 2 mod 4: two-way conflicts at most
+constexpr int kTpTapW = 84;                           // words per channel of one tap copy (168 taps)
+constexpr int kTpSmem = kTpCh * kTpW * 4 + 2 * kTpCh * kTpTapW * 4;
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__global__ void __launch_bounds__(kTpThreads, 2) fir_toeplitz_kernel(const __nv_bfloat16* __restrict__ u,
+                                                                     const float* __restrict__ ht, int K,
+                                                                     const float* __restrict__ D,
+                                                                     const __nv_bfloat16* __restrict__ x2,
+                                                                     __nv_bfloat16* __restrict__ out, int L, int d) {
+  extern __shared__ __align__(16) uint32_t tp_smem[];
+  uint32_t* su = tp_smem;                                   // [32][kTpW]: word p = positions t0 - 128 + 2p, + 1
+  // reversed taps, twice: r[x] = h[kTpTap0 - x], in copy 1 shifted by one so that odd pairs are aligned as well
+  constexpr int kTap0 = 143;                                // r[0] = h[143] = 0; r[143] = h[0]; r[159] = h[-16] = 0
+  __nv_bfloat16* st0 = reinterpret_cast<__nv_bfloat16*>(su + kTpCh * kTpW);
+  __nv_bfloat16* st1 = st0 + 2 * kTpCh * kTpTapW;
+  const int c0 = blockIdx.x * kTpCh, t0 = blockIdx.y * kTpPos;
+  const long long base = static_cast<long long>(blockIdx.z) * L * d;
+  for (int i = threadIdx.x; i < kTpCh * 2 * kTpTapW; i += kTpThreads) {
+    const int ch = i % kTpCh, x = i / kTpCh;                // lanes over channels: the tap rows are read coalesced
+    auto tap = [&](int k) { return k >= 0 && k < K && c0 + ch < d ? ht[static_cast<long long>(k) * d + c0 + ch] : 0.f; };
+    st0[ch * 2 * kTpTapW + x] = __float2bfloat16(tap(kTap0 - x));
+    st1[ch * 2 * kTpTapW + x] = __float2bfloat16(tap(kTap0 - x - 1));
+  }
+  uint32_t odd = 0;                                         // a word with an infinite or NaN half was seen
+  for (int i = threadIdx.x; i < (kTpPos + kTpHalo) / 2 * (kTpCh / 8); i += kTpThreads) {
+    const int g8 = (i & 3) * 8, p = i >> 2;                 // eight channels, two positions
+    const int l = t0 - kTpHalo + 2 * p;
+    uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0;
+    if (c0 + g8 < d) {
+      const __nv_bfloat16* src = u + base + static_cast<long long>(l) * d + c0 + g8;
+      if (l >= 0 && l < L) v0 = *reinterpret_cast<const uint4*>(src);
+      if (l + 1 >= 0 && l + 1 < L) v1 = *reinterpret_cast<const uint4*>(src + d);
+    }
+    const uint32_t a[4] = {v0.x, v0.y, v0.z, v0.w}, b[4] = {v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      odd |= (__vcmpeq2(a[e] & 0x7F807F80u, 0x7F807F80u) | __vcmpeq2(b[e] & 0x7F807F80u, 0x7F807F80u));
+      su[(g8 + 2 * e) * kTpW + p] = __byte_perm(a[e], b[e], 0x5410);
+      su[(g8 + 2 * e + 1) * kTpW + p] = __byte_perm(a[e], b[e], 0x7632);
+    }
+  }
+  // The zeros of T_m would turn an infinity or NaN into NaN at positions whose window does not hold it (up to 15
+  // before it and behind it): a tile with such a value is summed tap by tap instead.
+  const bool finite = __syncthreads_or(odd != 0) == 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  for (int cc = 0; cc < kTpCh / 8; ++cc) {
+    const int ch = warp * (kTpCh / 8) + cc;
+    if (c0 + ch >= d) break;
+    uint32_t* row = su + ch * kTpW;
+    const float dv = D[c0 + ch];
+    __nv_bfloat16* rowb = reinterpret_cast<__nv_bfloat16*>(row) + kTpHalo;
+    if (!finite) {
+      float y[kTpPos / 32];
+#pragma unroll
+      for (int j = 0; j < kTpPos / 32; ++j) {
+        y[j] = 0.f;
+        const int pos = 32 * j + lane;
+        for (int k = 0; k < K; ++k)
+          y[j] = fmaf(__bfloat162float(st0[ch * 2 * kTpTapW + kTap0 - k]), __bfloat162float(rowb[pos - k]), y[j]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < kTpPos / 32; ++j) {
+        __nv_bfloat16* at = rowb + 32 * j + lane;
+        const float conv = __bfloat162float(__float2bfloat16(y[j]));
+        *at = __float2bfloat16(conv + __bfloat162float(*at) * dv);
+      }
+      continue;
+    }
+    // pairs (h[n], h[n - 1]) = (r[143 - n], r[144 - n]) for n = 8 j + g - 4 t (x) and n - 2 (y), j = 0..17
+    uint32_t ax[18], ay[18];
+    {
+      const int x0 = kTap0 - g + 4 * t;                     // r index of n at j = 0; parity picks the aligned copy
+      const uint32_t* r = reinterpret_cast<const uint32_t*>((x0 & 1) ? st1 : st0) + ch * kTpTapW + (x0 >> 1);
+#pragma unroll
+      for (int j = 0; j < 18; ++j) {
+        ax[j] = r[-4 * j];
+        ay[j] = r[-4 * j + 1];
+      }
+    }
+    float acc[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[q][e] = 0.f;
+    // block of column n = g of group q at lag m: positions 16 (8 q + g - m) .. + 15 of the tile
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint2 bv = *reinterpret_cast<const uint2*>(row + kTpHalo / 2 + 8 * (8 * q + g - m) + 2 * t);
+        mma_16816(acc[q], ax[2 * m], ax[2 * m + 1], ay[2 * m], ay[2 * m + 1], bv.x, bv.y);
+      }
+    }
+    __syncwarp();
+    // accumulator (row i = g, g + 8; column n = 2 t, 2 t + 1) -> position 16 (8 q + n) + i; in place over the input
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        __nv_bfloat16* at = rowb + 16 * (8 * q + 2 * t + (e & 1)) + g + 8 * (e >> 1);
+        const float conv = __bfloat162float(__float2bfloat16(acc[q][e]));
+        *at = __float2bfloat16(conv + __bfloat162float(*at) * dv);
+      }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kTpPos / 2 * (kTpCh / 8); i += kTpThreads) {
+    const int g8 = (i & 3) * 8, p = i >> 2;
+    const int l = t0 + 2 * p;
+    if (l >= L || c0 + g8 >= d) continue;
+    uint32_t a[4], b[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t w0 = su[(g8 + 2 * e) * kTpW + kTpHalo / 2 + p], w1 = su[(g8 + 2 * e + 1) * kTpW + kTpHalo / 2 + p];
+      a[e] = __byte_perm(w0, w1, 0x5410);
+      b[e] = __byte_perm(w0, w1, 0x7632);
+    }
+    const long long o = base + static_cast<long long>(l) * d + c0 + g8;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      if (l + r >= L) break;
+      uint32_t* v = r ? b : a;
+      if (x2 != nullptr) {
+        const uint4 gv = *reinterpret_cast<const uint4*>(x2 + o + static_cast<long long>(r) * d);
+        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = pack_bf16x2(bf16_lo(gw[e]) * bf16_lo(v[e]), bf16_hi(gw[e]) * bf16_hi(v[e]));
+      }
+      *reinterpret_cast<uint4*>(out + o + static_cast<long long>(r) * d) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
 }  // namespace ubm
 
 // u, x2 (or null), out (or null: the state alone): bf16 [B][L][d]; lam, res: fp32 [d][S] (S <= 16); D: fp32 [d]; part: fp32
@@ -174,5 +339,21 @@ extern "C" int ubm_pole_conv_gate(const void* u, const void* lam, const void* re
   else UBM_POLE_CONV(16);
 #undef UBM_POLE_CONV
   UBM_CHECK_LAUNCH("pole_conv kernels");
+  return UBM_OK;
+}
+
+// u, x2 (or null), out: bf16 [B][L][d], d a multiple of 8; ht: fp32 [K][d] whose values are bf16, K <= 128.
+extern "C" int ubm_fir_toeplitz(const void* u, const void* ht, const void* D, const void* x2, void* out, int B, int L,
+                                int d, int K, void* stream) {
+  using namespace ubm;
+  if (B <= 0 || B > 65535 || L <= 0 || (L - 1) / kTpPos + 1 > 65535 || d <= 0 || (d & 7) || K < 1 || K > kTpHalo)
+    return UBM_ERR_ARGUMENT;
+  int rc = set_smem(fir_toeplitz_kernel, kTpSmem);
+  if (rc) return rc;
+  const dim3 grid((d + kTpCh - 1) / kTpCh, (L - 1) / kTpPos + 1, B);
+  fir_toeplitz_kernel<<<grid, kTpThreads, kTpSmem, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(u), static_cast<const float*>(ht), K, static_cast<const float*>(D),
+      static_cast<const __nv_bfloat16*>(x2), static_cast<__nv_bfloat16*>(out), L, d);
+  UBM_CHECK_LAUNCH("fir_toeplitz_kernel");
   return UBM_OK;
 }

@@ -30,6 +30,7 @@ native.declare("ubm_gemv_fused", [c_void_p] * 2 + [c_float] + [c_void_p] * 5 + [
 native.declare("ubm_gemv_fused_w8", [c_void_p] * 2 + [c_float, c_void_p, c_float] + [c_void_p] * 3 + [c_int] * 3 + [c_void_p])
 native.declare("ubm_rmsnorm_fp8", [c_void_p] * 5 + [c_ll, c_int, c_float, c_void_p])
 native.declare("ubm_pole_conv_gate", [c_void_p] * 8 + [c_int] * 5 + [c_void_p])
+native.declare("ubm_fir_toeplitz", [c_void_p] * 5 + [c_int] * 4 + [c_void_p])
 native.declare("ubm_fft_pad_transpose", [c_void_p] * 2 + [c_int] * 4 + [c_void_p])
 native.declare("ubm_spectrum_mul", [c_void_p] * 2 + [c_int, c_ll, c_void_p])
 native.declare("ubm_decode_attention", [c_void_p] * 7 + [c_int] * 4 + [c_float] * 2 + [c_void_p] * 2)
@@ -137,16 +138,26 @@ def fir_step(u: torch.Tensor, ht: torch.Tensor, D: torch.Tensor, x2: Optional[to
 
 
 def fir_inner_gate(u: torch.Tensor, ht: torch.Tensor, D: torch.Tensor, x2: Optional[torch.Tensor],
-                   tail: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x2 * (causal_fir(u, h) + D * u); u, x2: [B, L, d]; ht: fp32 [K, d]; tail: [B, K-1, d]."""
+                   tail: Optional[torch.Tensor] = None, taps_bf16: bool = False) -> torch.Tensor:
+    """x2 * (causal_fir(u, h) + D * u); u, x2: [B, L, d]; ht: fp32 [K, d]; tail: [B, K-1, d].  ``taps_bf16``: every
+    value of ``ht`` is a bf16 value (the filter is a bf16 parameter), so its products are exact on the tensor cores."""
     u = _bf16c(u)
     B, L, d = u.shape
+    K = ht.shape[0]
     out = torch.empty_like(u)
     x2c = None if x2 is None else _bf16c(x2)
     t = None if tail is None else _bf16c(tail)
     Df = _f32(D)
+    # one Toeplitz product per channel from 65 taps on (below, the multiply-adds it spends on zero taps outweigh the
+    # tensor cores); its accesses are 16 bytes wide
+    if taps_bf16 and t is None and 64 < K <= 128 and L >= 64 and d % 8 == 0 and u.data_ptr() % 16 == 0 and \
+            (x2c is None or x2c.data_ptr() % 16 == 0):
+        rc = native.lib().ubm_fir_toeplitz(native.ptr(u), native.ptr(ht), native.ptr(Df), native.ptr(x2c),
+                                           native.ptr(out), B, L, d, K, _stream(u))
+        native.check(rc, "ubm_fir_toeplitz")
+        return out
     rc = native.lib().ubm_fir_inner_gate(native.ptr(u), native.ptr(ht), native.ptr(Df), native.ptr(x2c),
-                                         native.ptr(t), native.ptr(out), B, L, d, ht.shape[0], _stream(u))
+                                         native.ptr(t), native.ptr(out), B, L, d, K, _stream(u))
     native.check(rc, "ubm_fir_inner_gate")
     return out
 
