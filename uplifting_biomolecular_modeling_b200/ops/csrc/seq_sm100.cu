@@ -188,118 +188,95 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_wide_kernel(const __nv_bfloa
 }
 
 // ------------------------------------------------------------------------------------------ causal FIR
-// Depthwise causal FIR over [B][L][C] with taps ht[k][c] (k = 0 multiplies the current sample).  A thread owns 8
-// channels and walks TL consecutive positions with the K-1 previous samples in registers, so each input element
-// is read once (plus K-1 per run of TL).  tail: [B][K-1][C] samples before position 0, or null (zeros).
-template <int K>
-struct FirWindow {
-  float h[K][8];
-  float w[K - 1][8];   // w[j] = sample at distance j+1 behind the current one
-  __device__ __forceinline__ void load_taps(const float* __restrict__ ht, int C, int c) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(ht + static_cast<long long>(k) * C + c));
-      const float4 b = __ldg(reinterpret_cast<const float4*>(ht + static_cast<long long>(k) * C + c + 4));
-      h[k][0] = a.x; h[k][1] = a.y; h[k][2] = a.z; h[k][3] = a.w;
-      h[k][4] = b.x; h[k][5] = b.y; h[k][6] = b.z; h[k][7] = b.w;
-    }
-  }
-  __device__ __forceinline__ void prime(const __nv_bfloat16* __restrict__ xb, const __nv_bfloat16* __restrict__ tb,
-                                        int l0, int C, int c) {
-#pragma unroll
-    for (int j = 0; j < K - 1; ++j) {
-      const int l = l0 - 1 - j;
-      if (l >= 0) {
-        unpack8(*reinterpret_cast<const uint4*>(xb + static_cast<long long>(l) * C + c), w[j]);
-      } else if (tb != nullptr) {
-        unpack8(*reinterpret_cast<const uint4*>(tb + static_cast<long long>(K - 1 + l) * C + c), w[j]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) w[j][e] = 0.f;
-      }
-    }
-  }
-  __device__ __forceinline__ void step(const float (&cur)[8], float (&y)[8]) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float a = h[0][e] * cur[e];
-#pragma unroll
-      for (int j = 0; j < K - 1; ++j) a = fmaf(h[j + 1][e], w[j][e], a);
-      y[e] = a;
-    }
-#pragma unroll
-    for (int j = K - 2; j > 0; --j)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) w[j][e] = w[j - 1][e];
-    if (K > 1) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) w[0][e] = cur[e];
-    }
-  }
-};
-
+// Depthwise causal FIR over [B][L][C] with taps ht[k][c] (k = 0 multiplies the current sample).  A thread walks TL
+// consecutive positions of its channels with the K-1 previous samples in registers, so each input element is read
+// once (plus K-1 per run of TL).  tail: [B][K-1][C] samples before position 0, or null (zeros).
 constexpr int kFirTL = 32;   // positions per thread run
 
 // Hyena input stage: z [B][L][3d] -> zf = fir(z) per channel; u = zf[0:d] * zf[2d:3d], x2 = zf[d:2d].
+// Bound by memory (three reads, two writes per position and channel), so what counts is bytes in flight: a thread owns
+// two neighbouring channels of the three thirds (a warp's access is one 128-byte line), which leaves registers for
+// many warps and for kFgBatch positions requested together.  With eight channels per thread
+// the three windows took 200 registers, two CTAs per SM, and one position's loads were in flight at a time: 107 us at
+// 8192 x 3 x 4096 against 76 us (335 MB, 4.4 TB/s).
+constexpr int kFgBatch = 8;
+
 template <int K>
 __global__ void __launch_bounds__(128) fir_gate3_kernel(const __nv_bfloat16* __restrict__ z,
                                                         const float* __restrict__ ht,     // [K][3d]
                                                         __nv_bfloat16* tail,  // [B][K-1][3d] or null
                                                         __nv_bfloat16* __restrict__ u, __nv_bfloat16* __restrict__ x2,
                                                         int B, int L, int d, int push) {
-  const int c8 = d / 8;
+  constexpr int KW = K > 1 ? K - 1 : 1;
+  const int c2 = d / 2;
   const int runs = (L + kFirTL - 1) / kFirTL;
-  const long long total = static_cast<long long>(B) * runs * c8;
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= static_cast<long long>(B) * runs * c2) return;
   const int C = 3 * d;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int cc = static_cast<int>(i % c8) * 8;
-    const long long br = i / c8;
-    const int run = static_cast<int>(br % runs);
-    const int b = static_cast<int>(br / runs);
-    const __nv_bfloat16* zb = z + static_cast<long long>(b) * L * C;
-    __nv_bfloat16* tb = tail == nullptr ? nullptr : tail + static_cast<long long>(b) * (K - 1) * C;
-    FirWindow<K> f1, f2, f3;
-    f1.load_taps(ht, C, cc);
-    f2.load_taps(ht, C, d + cc);
-    f3.load_taps(ht, C, 2 * d + cc);
-    const int l0 = run * kFirTL;
-    f1.prime(zb, tb, l0, C, cc);
-    f2.prime(zb, tb, l0, C, d + cc);
-    f3.prime(zb, tb, l0, C, 2 * d + cc);
-    const int l1 = min(L, l0 + kFirTL);
-    for (int l = l0; l < l1; ++l) {
-      float a[8], bb[8], cv[8], y1[8], y2[8], y3[8];
-      const __nv_bfloat16* row = zb + static_cast<long long>(l) * C;
-      unpack8(*reinterpret_cast<const uint4*>(row + cc), a);
-      unpack8(*reinterpret_cast<const uint4*>(row + d + cc), bb);
-      unpack8(*reinterpret_cast<const uint4*>(row + 2 * d + cc), cv);
-      f1.step(a, y1);
-      f2.step(bb, y2);
-      f3.step(cv, y3);
+  const int cc = static_cast<int>(i % c2) * 2;
+  const long long br = i / c2;
+  const int run = static_cast<int>(br % runs);
+  const int b = static_cast<int>(br / runs);
+  const __nv_bfloat16* zb = z + static_cast<long long>(b) * L * C + cc;
+  __nv_bfloat16* tb = tail == nullptr ? nullptr : tail + static_cast<long long>(b) * (K - 1) * C + cc;
+  float2 h[3][K], w[3][KW];   // w[j] = sample at distance j + 1 behind the current one
+  const int l0 = run * kFirTL;
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      h[p][k] = __ldg(reinterpret_cast<const float2*>(ht + static_cast<long long>(k) * C + p * d + cc));
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) {
+      const int l = l0 - 1 - j;
+      uint32_t v = 0u;
+      if (l >= 0) v = *reinterpret_cast<const uint32_t*>(zb + static_cast<long long>(l) * C + p * d);
+      else if (tb != nullptr) v = *reinterpret_cast<const uint32_t*>(tb + static_cast<long long>(K - 1 + l) * C + p * d);
+      w[p][j] = make_float2(bf16_lo(v), bf16_hi(v));
+    }
+  }
+  const int l1 = min(L, l0 + kFirTL);
+  for (int lb = l0; lb < l1; lb += kFgBatch) {
+    uint32_t raw[kFgBatch][3];
+#pragma unroll
+    for (int t = 0; t < kFgBatch; ++t)
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        raw[t][p] = lb + t < l1 ? *reinterpret_cast<const uint32_t*>(zb + static_cast<long long>(lb + t) * C + p * d) : 0u;
+#pragma unroll
+    for (int t = 0; t < kFgBatch; ++t) {
+      if (lb + t >= l1) break;
+      float2 y[3];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const float2 cur = make_float2(bf16_lo(raw[t][p]), bf16_hi(raw[t][p]));
+        y[p] = make_float2(h[p][0].x * cur.x, h[p][0].y * cur.y);
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) {
+          y[p].x = fmaf(h[p][j + 1].x, w[p][j].x, y[p].x);
+          y[p].y = fmaf(h[p][j + 1].y, w[p][j].y, y[p].y);
+        }
+#pragma unroll
+        for (int j = K - 2; j > 0; --j) w[p][j] = w[p][j - 1];
+        if (K > 1) w[p][0] = cur;
+      }
       // the plain statement rounds zf to the activation type before the gate product
-      float uo[8], xo[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        uo[e] = __bfloat162float(__float2bfloat16(y1[e])) * __bfloat162float(__float2bfloat16(y3[e]));
-        xo[e] = y2[e];
-      }
-      const long long o = (static_cast<long long>(b) * L + l) * d + cc;
-      *reinterpret_cast<uint4*>(u + o) = pack8(uo);
-      *reinterpret_cast<uint4*>(x2 + o) = pack8(xo);
+      const uint32_t r1 = pack_bf16x2(y[0].x, y[0].y), r3 = pack_bf16x2(y[2].x, y[2].y);
+      const long long o = (static_cast<long long>(b) * L + lb + t) * d + cc;
+      *reinterpret_cast<uint32_t*>(u + o) = pack_bf16x2(bf16_lo(r1) * bf16_lo(r3), bf16_hi(r1) * bf16_hi(r3));
+      *reinterpret_cast<uint32_t*>(x2 + o) = pack_bf16x2(y[1].x, y[1].y);
     }
-    // decode (one run per row of the batch): the tail is moved on in place - after the last step w[j] is the
-    // sample j + 1 positions behind the next one, i.e. row K - 2 - j of the new tail.  This thread is the only
-    // one that touches these channels of the tail.
-    if (push && K > 1) {
+  }
+  // decode (one run per row of the batch): the tail is moved on in place - after the last step w[j] is the
+  // sample j + 1 positions behind the next one, i.e. row K - 2 - j of the new tail.  This thread is the only
+  // one that touches these channels of the tail.
+  if (push && K > 1) {
 #pragma unroll
-      for (int j = 0; j < K - 1; ++j) {
-        __nv_bfloat16* row = tb + static_cast<long long>(K - 2 - j) * C;
-        *reinterpret_cast<uint4*>(row + cc) = pack8(f1.w[j]);
-        *reinterpret_cast<uint4*>(row + d + cc) = pack8(f2.w[j]);
-        *reinterpret_cast<uint4*>(row + 2 * d + cc) = pack8(f3.w[j]);
-      }
-    }
+    for (int j = 0; j < K - 1; ++j)
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        *reinterpret_cast<uint32_t*>(tb + static_cast<long long>(K - 2 - j) * C + p * d) =
+            pack_bf16x2(w[p][j].x, w[p][j].y);
   }
 }
 
@@ -386,7 +363,8 @@ __global__ void __launch_bounds__(256) fir_step_kernel(const __nv_bfloat16* __re
   }
 }
 
-// Inner operator of hcs / hcm: out = x2 * (fir(u, h) + D * u).  Short filters keep the window in registers;
+// Inner operator of hcs / hcm: out = x2 * (fir(u, h) + D * u).  Short filters keep the window in registers, two channels
+// per thread and kFgBatch positions requested together as in fir_gate3_kernel;
 // longer ones (the 128-tap medium filter) re-read the inputs through L1/L2 (generic kernel below).
 template <int K>
 __global__ void __launch_bounds__(128) fir_inner_gate_kernel(const __nv_bfloat16* __restrict__ u,
@@ -395,43 +373,57 @@ __global__ void __launch_bounds__(128) fir_inner_gate_kernel(const __nv_bfloat16
                                                              const __nv_bfloat16* __restrict__ x2,   // or null
                                                              const __nv_bfloat16* __restrict__ tail, // [B][K-1][d]
                                                              __nv_bfloat16* __restrict__ out, int B, int L, int d) {
-  const int c8 = d / 8;
+  constexpr int KW = K > 1 ? K - 1 : 1;
+  const int c2 = d / 2;
   const int runs = (L + kFirTL - 1) / kFirTL;
-  const long long total = static_cast<long long>(B) * runs * c8;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int cc = static_cast<int>(i % c8) * 8;
-    const long long br = i / c8;
-    const int run = static_cast<int>(br % runs);
-    const int b = static_cast<int>(br / runs);
-    const __nv_bfloat16* ub = u + static_cast<long long>(b) * L * d;
-    const __nv_bfloat16* tb = tail == nullptr ? nullptr : tail + static_cast<long long>(b) * (K - 1) * d;
-    FirWindow<K> f;
-    f.load_taps(ht, d, cc);
-    const int l0 = run * kFirTL;
-    f.prime(ub, tb, l0, d, cc);
-    const float4 d0 = __ldg(reinterpret_cast<const float4*>(D + cc));
-    const float4 d1 = __ldg(reinterpret_cast<const float4*>(D + cc + 4));
-    const float dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-    const int l1 = min(L, l0 + kFirTL);
-    for (int l = l0; l < l1; ++l) {
-      float cur[8], y[8], g[8];
-      const long long o = (static_cast<long long>(b) * L + l) * d + cc;
-      unpack8(*reinterpret_cast<const uint4*>(u + o), cur);
-      f.step(cur, y);
-      if (x2 != nullptr) {
-        unpack8(*reinterpret_cast<const uint4*>(x2 + o), g);
-      } else {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= static_cast<long long>(B) * runs * c2) return;
+  const int cc = static_cast<int>(i % c2) * 2;
+  const long long br = i / c2;
+  const int run = static_cast<int>(br % runs);
+  const int b = static_cast<int>(br / runs);
+  const long long base = static_cast<long long>(b) * L * d + cc;
+  const __nv_bfloat16* tb = tail == nullptr ? nullptr : tail + static_cast<long long>(b) * (K - 1) * d + cc;
+  const int l0 = run * kFirTL;
+  float2 h[K], w[KW];   // w[j] = sample at distance j + 1 behind the current one
 #pragma unroll
-        for (int e = 0; e < 8; ++e) g[e] = 1.f;
-      }
-      float r[8];
+  for (int k = 0; k < K; ++k) h[k] = __ldg(reinterpret_cast<const float2*>(ht + static_cast<long long>(k) * d + cc));
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float conv = __bfloat162float(__float2bfloat16(y[e]));     // the plain statement's bf16 conv output
-        r[e] = g[e] * __bfloat162float(__float2bfloat16(conv + cur[e] * dv[e]));
+  for (int j = 0; j < K - 1; ++j) {
+    const int l = l0 - 1 - j;
+    uint32_t v = 0u;
+    if (l >= 0) v = *reinterpret_cast<const uint32_t*>(u + base + static_cast<long long>(l) * d);
+    else if (tb != nullptr) v = *reinterpret_cast<const uint32_t*>(tb + static_cast<long long>(K - 1 + l) * d);
+    w[j] = make_float2(bf16_lo(v), bf16_hi(v));
+  }
+  const float2 dv = __ldg(reinterpret_cast<const float2*>(D + cc));
+  const int l1 = min(L, l0 + kFirTL);
+  for (int lb = l0; lb < l1; lb += kFgBatch) {
+    uint32_t raw[kFgBatch], gate[kFgBatch];
+#pragma unroll
+    for (int t = 0; t < kFgBatch; ++t) {
+      const long long o = base + static_cast<long long>(lb + t) * d;
+      raw[t] = lb + t < l1 ? *reinterpret_cast<const uint32_t*>(u + o) : 0u;
+      gate[t] = x2 != nullptr && lb + t < l1 ? *reinterpret_cast<const uint32_t*>(x2 + o) : 0x3F803F80u;   // 1, 1
+    }
+#pragma unroll
+    for (int t = 0; t < kFgBatch; ++t) {
+      if (lb + t >= l1) break;
+      const float2 cur = make_float2(bf16_lo(raw[t]), bf16_hi(raw[t]));
+      float2 y = make_float2(h[0].x * cur.x, h[0].y * cur.y);
+#pragma unroll
+      for (int j = 0; j < K - 1; ++j) {
+        y.x = fmaf(h[j + 1].x, w[j].x, y.x);
+        y.y = fmaf(h[j + 1].y, w[j].y, y.y);
       }
-      *reinterpret_cast<uint4*>(out + o) = pack8(r);
+#pragma unroll
+      for (int j = K - 2; j > 0; --j) w[j] = w[j - 1];
+      if (K > 1) w[0] = cur;
+      // rounded like the plain statement: the convolution, its sum with the skip term, the gated product
+      const uint32_t cv = pack_bf16x2(y.x, y.y);
+      const uint32_t sv = pack_bf16x2(bf16_lo(cv) + cur.x * dv.x, bf16_hi(cv) + cur.y * dv.y);
+      *reinterpret_cast<uint32_t*>(out + base + static_cast<long long>(lb + t) * d) =
+          pack_bf16x2(bf16_lo(gate[t]) * bf16_lo(sv), bf16_hi(gate[t]) * bf16_hi(sv));
     }
   }
 }
@@ -962,8 +954,9 @@ extern "C" int ubm_fir_gate3(const void* z, const void* ht, void* tail, void* u,
   if (B <= 0 || L <= 0 || d <= 0 || (d & 7) || K < 1 || K > 4) return UBM_ERR_ARGUMENT;
   if (push && (tail == nullptr || L > kFirTL)) return UBM_ERR_ARGUMENT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long total = static_cast<long long>(B) * ((L + kFirTL - 1) / kFirTL) * (d / 8);
-  const int grid = seq_grid(total, 128);
+  const long long total = static_cast<long long>(B) * ((L + kFirTL - 1) / kFirTL) * (d / 2);
+  if ((total + 127) / 128 > 0x7fffffffLL) return UBM_ERR_TOO_LARGE;
+  const unsigned grid = static_cast<unsigned>((total + 127) / 128);
 #define UBM_FG3(KK)                                                                                            \
   fir_gate3_kernel<KK><<<grid, 128, 0, st>>>(static_cast<const __nv_bfloat16*>(z), static_cast<const float*>(ht), \
                                              static_cast<__nv_bfloat16*>(tail),                                 \
@@ -992,8 +985,9 @@ extern "C" int ubm_fir_inner_gate(const void* u, const void* ht, const void* D, 
   const __nv_bfloat16* tt = static_cast<const __nv_bfloat16*>(tail);
   __nv_bfloat16* oo = static_cast<__nv_bfloat16*>(out);
   if (K <= 8) {
-    const long long total = static_cast<long long>(B) * ((L + kFirTL - 1) / kFirTL) * (d / 8);
-    const int grid = seq_grid(total, 128);
+    const long long total = static_cast<long long>(B) * ((L + kFirTL - 1) / kFirTL) * (d / 2);
+    if ((total + 127) / 128 > 0x7fffffffLL) return UBM_ERR_TOO_LARGE;
+    const unsigned grid = static_cast<unsigned>((total + 127) / 128);
 #define UBM_FIG(KK) fir_inner_gate_kernel<KK><<<grid, 128, 0, st>>>(uu, hh, dd, xx, tt, oo, B, L, d)
     switch (K) {
       case 1: UBM_FIG(1); break;
