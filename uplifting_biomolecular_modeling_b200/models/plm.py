@@ -173,14 +173,20 @@ class EncoderBlock(nn.Module):
         qkv = gemm.gemm(n, p["wqkv"])
         # the attention kernel takes q already multiplied by log2(e) / sqrt(D): folded into the q LayerNorm weight
         own = mask is None and Dh in (32, 64)
-        qkv[:, :d] = rows.layernorm_rows(qkv[:, :d].contiguous(), p["q_ln_scaled"] if own else p["q_ln"], None, cfg.eps)
-        qkv[:, d:2 * d] = rows.layernorm_rows(qkv[:, d:2 * d].contiguous(), self.k_ln.weight, None, cfg.eps)
-        q, k, v = seq.rotary_split_qkv(qkv, pos, H, cfg.rot)
+        q_gamma = p["q_ln_scaled"] if own else p["q_ln"]
+        if qkv.is_cuda and Dh in (32, 64) and d <= 2048:
+            # normalised and rotated where the projection wrote them; attention reads the three column slices
+            seq.qk_norm_rotary_(qkv, pos, q_gamma, self.k_ln.weight, H, cfg.rot, cfg.eps)
+            q, k, v = qkv.split(d, 1)
+        else:
+            qkv[:, :d] = rows.layernorm_rows(qkv[:, :d].contiguous(), q_gamma, None, cfg.eps)
+            qkv[:, d:2 * d] = rows.layernorm_rows(qkv[:, d:2 * d].contiguous(), self.k_ln.weight, None, cfg.eps)
+            q, k, v = (t.view(T, d) for t in seq.rotary_split_qkv(qkv, pos, H, cfg.rot))
         if own:
             o = torch.empty((T, d), dtype=x.dtype, device=x.device)
-            pair.attention(q.view(T, d), k.view(T, d), v.view(T, d), None, None, o, rows=B, Nq=L, Nk=L, H=H, D=Dh)
+            pair.attention(q, k, v, None, None, o, rows=B, Nq=L, Nk=L, H=H, D=Dh, ld_in=q.stride(0))
         else:
-            o = _sdpa(q, k, v, B, L, mask)
+            o = _sdpa(*(t.view(T, H, Dh) for t in (q, k, v)), B, L, mask)
         x2 = gemm.gemm(o, p["wo"], residual=x2)
         if cfg.family == "gpnstar":
             R = align.shape[1]

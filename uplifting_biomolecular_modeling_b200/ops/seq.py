@@ -29,6 +29,7 @@ native.declare("ubm_residual_ln", [c_void_p] * 6 + [c_ll, c_int, c_float, c_void
 native.declare("ubm_gemv_fused", [c_void_p] * 2 + [c_float] + [c_void_p] * 5 + [c_int] * 3 + [c_void_p])
 native.declare("ubm_gemv_fused_w8", [c_void_p] * 2 + [c_float, c_void_p, c_float] + [c_void_p] * 3 + [c_int] * 3 + [c_void_p])
 native.declare("ubm_rmsnorm_fp8", [c_void_p] * 5 + [c_ll, c_int, c_float, c_void_p])
+native.declare("ubm_qk_norm_rotary", [c_void_p] * 4 + [c_ll] + [c_int] * 3 + [c_float] * 2 + [c_void_p])
 native.declare("ubm_pole_conv_gate", [c_void_p] * 8 + [c_int] * 5 + [c_void_p])
 native.declare("ubm_fir_toeplitz", [c_void_p] * 5 + [c_int] * 4 + [c_void_p])
 native.declare("ubm_fft_pad_transpose", [c_void_p] * 2 + [c_int] * 4 + [c_void_p])
@@ -307,6 +308,21 @@ def rotary_split_qkv(qkv: torch.Tensor, pos: torch.Tensor, heads: int, rot: int,
                                            T, heads, Dh, rot, float(base), _stream(qkv))
     native.check(rc, "ubm_rotary_split_qkv")
     return q, k, v
+
+
+def qk_norm_rotary_(qkv: torch.Tensor, pos: torch.Tensor, q_gamma: torch.Tensor, k_gamma: torch.Tensor, heads: int,
+                    rot: int, eps: float = 1e-5, base: float = 10000.0) -> torch.Tensor:
+    """qkv: contiguous bf16 [T, 3 * heads * Dh] (Dh a power of two, 8 to 256; at most 2048 channels), its q and k thirds
+    replaced by rotary(LayerNorm(row) * gamma); the v third is left as it is."""
+    T, C3 = qkv.shape
+    C = C3 // 3
+    if qkv.dtype != torch.bfloat16 or not qkv.is_contiguous():
+        raise ValueError("qk_norm_rotary_ works in place on a contiguous bf16 projection")
+    p, qg, kg = pos.to(torch.int32).contiguous(), _f32(q_gamma), _f32(k_gamma)
+    rc = native.lib().ubm_qk_norm_rotary(native.ptr(qkv), native.ptr(p), native.ptr(qg), native.ptr(kg), T, C, C // heads,
+                                         rot, float(eps), float(base), _stream(qkv))
+    native.check(rc, "ubm_qk_norm_rotary")
+    return qkv
 
 
 def add2_softmax_rows(x: torch.Tensor, a: Optional[torch.Tensor] = None, b: Optional[torch.Tensor] = None):
