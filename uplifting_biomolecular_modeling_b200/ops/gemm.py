@@ -46,7 +46,7 @@ def _as3(t: torch.Tensor) -> torch.Tensor:
 def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Optional[torch.Tensor] = None,
          residual: Optional[torch.Tensor] = None, act: Optional[str] = None, alpha: float = 1.0,
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
-         c_blocked: Optional[tuple] = None, gate: Optional[torch.Tensor] = None, act_from: int = 0) -> torch.Tensor:
+         c_blocked: Optional[tuple] = None, c_batch: int = 0, gate: Optional[torch.Tensor] = None, act_from: int = 0) -> torch.Tensor:
     """C = act(alpha * A.B^T + bias) * gate + residual.
 
     ``act_from``: the activation applies to output columns >= act_from (a multiple of 32) only.
@@ -56,9 +56,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
     ``gate`` (bf16 [rows, N], rows dividing M, row stride free): row m is multiplied by gate row m % rows -
     a conditioning gate shared by the samples stacked along M.
 
-    ``c_blocked=(hi, lo, col)`` (with ``out`` given, N a multiple of 32, batch 1) stores element (m, n) at
+    ``c_blocked=(hi, lo, col)`` (with ``out`` given, N a multiple of 32) stores element (m, n) at
     ``out.data_ptr + (m // 32) * hi + (m % 32) * lo + (n // 32) * col + n % 32`` elements: the product of two
-    [(token, channel)] operands lands as [(i, j)][(c, d)] without a permuted copy.
+    [(token, channel)] operands lands as [(i, j)][(c, d)] without a permuted copy.  With a batch, entry b starts
+    ``c_batch`` elements after entry b - 1 (its elements may lie between the other entries').
 
     mn_major=False: a [.., M, K], b [.., N, K];  mn_major=True: a [.., K, M], b [.., K, N].
     The innermost dimension of a and b must be contiguous; other strides are free as long as
@@ -84,8 +85,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         if b3.shape[2] != K:
             raise ValueError("K mismatch")
     if c_blocked is not None:
-        if out is None or batch != 1 or N % 32 or residual is not None:
-            raise ValueError("c_blocked needs an output tensor, batch 1, N % 32 == 0 and no residual")
+        if out is None or (batch != 1 and c_batch <= 0) or N % 32 or residual is not None:
+            raise ValueError("c_blocked needs an output tensor, batch 1 or c_batch, N % 32 == 0 and no residual")
         out3 = out
     else:
         n_out = N
@@ -119,7 +120,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         a3.stride(1), b3.stride(1), 0 if c_blocked is not None else out3.stride(1),
         0 if res3 is None else res3.stride(1),
         a3.stride(0) if batch > 1 else 0, b3.stride(0) if batch > 1 else 0,
-        out3.stride(0) if batch > 1 and c_blocked is None else 0,
+        0 if batch == 1 else out3.stride(0) if c_blocked is None else c_batch,
         0 if res3 is None or batch == 1 else res3.stride(0),
         1 if mn_major else 0, 1 if out3.dtype == torch.float32 else 0, ACT[act], float(alpha),
         int(cb[0]), int(cb[1]), int(cb[2]), native.ptr(gate), 0 if gate is None else gate.stride(0),

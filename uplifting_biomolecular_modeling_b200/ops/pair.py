@@ -19,7 +19,7 @@ import torch
 
 from . import gemm as _gemm
 from . import native
-from .native import c_int, c_ll, c_void_p
+from .native import c_float, c_int, c_ll, c_void_p
 
 native.declare("ubm_trimul_proj", [c_void_p] * 7 + [c_int, c_int, c_void_p, c_void_p])
 native.declare("ubm_triatt_proj", [c_void_p] * 13 + [c_int, c_int, c_int, c_int, c_void_p, c_void_p])
@@ -431,6 +431,58 @@ def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, r
     z2 = z.view(N * N, 128)
     out = torch.empty_like(z) if out is None else out
     _gemm.gemm(og, w.wo, bias=w.bo, residual=z2 if residual else None, out=out.view(N * N, 128))
+    return out
+
+
+# ------------------------------------------------------------------------------------------
+native.declare("ubm_pwa_softmax", [c_void_p] * 2 + [c_int] * 4 + [c_void_p])
+native.declare("ubm_pwa_value", [c_void_p] * 5 + [c_int] * 3 + [c_float] + [c_void_p] * 2)
+native.declare("ubm_pwa_out", [c_void_p] * 7 + [c_int] * 2 + [c_float] + [c_void_p] * 2)
+
+
+@dataclass
+class PwaPacked:
+    wv: torch.Tensor         # bf16 [256, 64], gamma folded
+    v_colsum: torch.Tensor   # fp32 [256]
+    v_colbias: torch.Tensor
+    wg: torch.Tensor         # bf16 [256, 64], gamma folded
+    g_colsum: torch.Tensor
+    g_colbias: torch.Tensor
+    wo: torch.Tensor         # bf16 [64, 256]
+    eps: float
+
+    @classmethod
+    def pack(cls, norm_w, norm_b, w_m, w_g, w_o, eps: float) -> "PwaPacked":
+        if w_m.shape != (256, 64) or w_o.shape != (64, 256):
+            raise ValueError("fused pair-weighted averaging supports c_m = 64 and 8 heads of 32")
+        return cls(*fold_ln_linear(w_m, norm_w, norm_b), *fold_ln_linear(w_g, norm_w, norm_b),
+                   w_o.detach().to(torch.bfloat16).contiguous(), float(eps))
+
+
+def pair_weighted_averaging_fused(m: torch.Tensor, b: torch.Tensor, mask: Optional[torch.Tensor],
+                                  w: PwaPacked) -> torch.Tensor:
+    """m: bf16 [S, N, 64] contiguous; b: bf16 [8, N, N], a view of planes with row stride Np (from ``pair_head_bias``),
+    overwritten; mask: [N, N] (1 = keep) or None.  Returns proj_o(sigmoid(proj_g n) * softmax(b + mask) v), n = LN(m)."""
+    S, N, c = m.shape
+    Np = b.stride(1)
+    if m.dtype != torch.bfloat16 or c != 64 or not m.is_contiguous() or b.shape != (8, N, N) or b.stride(0) != N * Np:
+        raise ValueError("pair_weighted_averaging_fused expects contiguous bf16 [S, N, 64] and planes of 8 heads")
+    dev = m.device
+    if mask is not None and mask.dtype != torch.bfloat16:
+        mask = mask.float()
+    mk = None if mask is None else mask.expand(N, N).contiguous()
+    v = torch.empty((8, S * 32, Np), dtype=torch.bfloat16, device=dev)
+    o = torch.empty((N, S, 256), dtype=torch.bfloat16, device=dev)
+    out = torch.empty_like(m)
+    lib, stream, st = native.lib(), native.current_stream(dev), native.status_tensor(dev)
+    native.check(lib.ubm_pwa_softmax(native.ptr(b), native.ptr(mk), 1 if mk is not None and mk.dtype == torch.bfloat16
+                                     else 0, 8, N, Np, stream), "ubm_pwa_softmax")
+    native.check(lib.ubm_pwa_value(native.ptr(m), native.ptr(w.wv), native.ptr(w.v_colsum), native.ptr(w.v_colbias),
+                                   native.ptr(v), S, N, Np, w.eps, native.ptr(st), stream), "ubm_pwa_value")
+    _gemm.gemm(b, v[:, :, :N], out=o, c_blocked=(32 * S * 256, S * 256, 256), c_batch=32)
+    native.check(lib.ubm_pwa_out(native.ptr(m), native.ptr(o), native.ptr(w.wg), native.ptr(w.g_colsum),
+                                 native.ptr(w.g_colbias), native.ptr(w.wo), native.ptr(out), S, N, w.eps,
+                                 native.ptr(st), stream), "ubm_pwa_out")
     return out
 
 
