@@ -15,7 +15,10 @@
 // are computed thread-per-row from the shared-memory tile (as the row-major kernels do) and passed to all
 // threads of the epilogue group through a small shared array; the per-channel constants live in registers.
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer, 2-5 = epilogue group 0 (operand a), 6-9 = group 1 (operand b).
+// Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = four epilogue groups: operand (a, b) x half of the tile's columns.
+// The epilogue's arithmetic bounds the kernel (the tensor pipe is busy a fifth of the time): with eight warps, which
+// left half of the issue slots idle, and both operands' groups taking every row's statistics it took 314 us at 1021
+// tokens; sixteen warps that share the statistics take 265 us.
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -38,19 +41,18 @@ struct TrimulProjParams {
   const float* colsum;  // [512] rowsum(W') per output channel
   const float* colbias; // [512]
   const float* mask;    // [R] or null
-  __nv_bfloat16* planes;  // [2][128][plane_rows][Np]
   float* stats_out;       // optional [R][2]
   KernelStatus* status;
   PeerSrc src;            // src.n > 0: the input rows are columns of z fetched from their owners (see host_util.h)
-  // the planes leave through shared memory: every epilogue warp stages 32 channels x 32 entries (64-byte swizzle)
-  // and one lane stores the box {32 entries, 1 row, 32 planes} with a bulk tensor copy (map tmP over
-  // {Np, plane_rows, 256})
-  int out_tma;
 };
+// The planes leave through shared memory: every epilogue warp stages 32 channels x 32 entries (64-byte swizzle) and
+// one lane stores the box {32 entries, 1 row, 32 planes} with a bulk tensor copy (map tmP over {Np, plane_rows, 256}).
 constexpr int kTPOutWarpBytes = 32 * 64;
-constexpr int kTPOutBytes = 8 * kTPOutWarpBytes;
+constexpr int kTPEpiWarps = 16;
+constexpr int kTPOutBytes = kTPEpiWarps * kTPOutWarpBytes;
+constexpr int kTPThreads = 64 + 32 * kTPEpiWarps;
 
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kTPThreads, 1)
 trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                    const __grid_constant__ PeerSrcMaps peers, const __grid_constant__ CUtensorMap tmP,
                    TrimulProjParams p) {
@@ -58,9 +60,9 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sW = smem;                               // 128 KB
   uint8_t* sX = smem + kTPWBytes;                   // stages * 32 KB
-  uint8_t* sOut = sX + kTPStages * kTPXBytes;       // 8 warps x 2 KB of output staging
-  float* sStat = reinterpret_cast<float*>(sOut + kTPOutBytes);           // [2 groups][2 parities][3][128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 2 * 2 * 3 * 128);
+  uint8_t* sOut = sX + kTPStages * kTPXBytes;       // 16 warps x 2 KB of output staging
+  float* sStat = reinterpret_cast<float*>(sOut + kTPOutBytes);           // [3][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 3 * 128);
   uint64_t* x_full = bars;                 // [stages]
   uint64_t* x_empty = x_full + kTPStages;  // [stages]
   uint64_t* w_full = x_empty + kTPStages;  // [1]
@@ -77,12 +79,12 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     *abort_flag = 0;
     for (int s = 0; s < kTPStages; ++s) {
       mbar_init(&x_full[s], 1);
-      mbar_init(&x_empty[s], 1 + 8);  // MMA commit + one arrival per epilogue warp
+      mbar_init(&x_empty[s], 1 + kTPEpiWarps);  // MMA commit + one arrival per epilogue warp
     }
     mbar_init(w_full, 1);
     for (int h = 0; h < 2; ++h) {
       mbar_init(&acc_full[h], 1);
-      mbar_init(&acc_empty[h], 4);
+      mbar_init(&acc_empty[h], kTPEpiWarps / 2);
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmX);
@@ -175,30 +177,35 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     }
   } else {
     // ------------------------------------------------------------------ epilogue groups
-    const int grp = (warp - 2) >> 2;  // operand a or b
-    const int q = warp & 3;           // TMEM lane quadrant
-    const int ch = q * 32 + lane;     // output channel of this thread; also the tile row it takes statistics of
-    const float cs_v = p.colsum[grp * 256 + ch], cb_v = p.colbias[grp * 256 + ch];
-    const float cs_g = p.colsum[grp * 256 + 128 + ch], cb_g = p.colbias[grp * 256 + 128 + ch];
+    const int op = ((warp - 2) >> 2) & 1;   // operand a or b
+    const int half = (warp - 2) >> 3;       // columns 64 half .. 64 half + 63
+    const int q = warp & 3;                 // TMEM lane quadrant
+    const int ch = q * 32 + lane;           // output channel of this thread
+    const int et = threadIdx.x - 64;        // 0 .. 511: four threads take the statistics of one tile row
+    const int srow = et >> 2;
+    const float cs_v = p.colsum[op * 256 + ch], cb_v = p.colbias[op * 256 + ch];
+    const float cs_g = p.colsum[op * 256 + 128 + ch], cb_g = p.colbias[op * 256 + 128 + ch];
     const float2 csv2 = make_float2(cs_v, cs_v), cbv2 = make_float2(cb_v, cb_v);
     const float2 csg2 = make_float2(cs_g, cs_g), cbg2 = make_float2(cb_g, cb_g);
     int stage = 0;
     uint32_t phase = 0;
     uint32_t acc_phase = 0;
-    uint32_t par = 0;
-    const bool wide = (p.Np & 15) == 0;   // plane rows 32-byte aligned: 32-byte stores
-    const bool out_tma = p.out_tma != 0;  // warp-uniform
     uint8_t* stage_w = sOut + (warp - 2) * kTPOutWarpBytes;
-    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, par ^= 1u) {
+    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
       const int i = t / p.tiles_per_row;
       const int s0 = (t - i * p.tiles_per_row) * kTPRows;
-      // ---- statistics of tile row `ch` from the shared-memory tile
+      // ---- statistics of tile row `srow` from the shared-memory tile: 32 channels per thread
+      const int s = s0 + srow;
+      const bool valid = s < p.N;
+      const long long r = static_cast<long long>(i) * p.N + s;
+      float mval = valid ? 1.0f : 0.0f;            // entries past N are written as zeros (K padding of the contraction)
+      if (valid && p.mask != nullptr) mval = p.mask[r];
       mbar_wait(&x_full[stage], phase, ws, 15, stage);
-      const uint8_t* xs = sX + stage * kTPXBytes;
+      const uint8_t* xs = sX + stage * kTPXBytes + ((et & 3) >> 1) * 16384;
       float sum = 0.f, sumsq = 0.f;
-#pragma unroll 4
-      for (int c16 = 0; c16 < 16; ++c16) {
-        const uint4 u = *reinterpret_cast<const uint4*>(xs + (c16 >> 3) * 16384 + swz128_offset(ch, c16 & 7));
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint4 u = *reinterpret_cast<const uint4*>(xs + swz128_offset(srow, (et & 1) * 4 + c));
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -207,113 +214,86 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           sumsq += a * a + b * b;
         }
       }
-      __syncwarp();
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sumsq += __shfl_xor_sync(0xffffffffu, sumsq, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      sumsq += __shfl_xor_sync(0xffffffffu, sumsq, 2);
       if (lane == 0) mbar_arrive(&x_empty[stage]);
       const float mu = sum * (1.0f / kTPC);
       const float var = fmaxf(sumsq * (1.0f / kTPC) - mu * mu, 0.f);
       const float rstd = rsqrtf(var + 1e-5f);
-      const int s = s0 + ch;
-      const bool valid = s < p.N;
-      const long long r = static_cast<long long>(i) * p.N + s;
-      float mval = valid ? 1.0f : 0.0f;            // entries past N are written as zeros (K padding of the contraction)
-      if (valid && p.mask != nullptr) mval = p.mask[r];
-      if (p.stats_out != nullptr && grp == 0 && valid) {
+      if (p.stats_out != nullptr && (et & 3) == 0 && valid) {
         p.stats_out[2 * r] = mu;
         p.stats_out[2 * r + 1] = rstd;
       }
-      float* st = sStat + (grp * 2 + par) * 3 * 128;
-      st[ch] = rstd;
-      st[128 + ch] = -mu * rstd;
-      st[256 + ch] = mval;
-      // the 128 threads of this group exchange statistics; the array of the other parity is still being read
-      // by slower warps of the previous tile, which is why there are two
-      asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+      // all 512 threads exchange statistics: nobody reads the previous tile's any more, then nobody reads too early
+      asm volatile("bar.sync 1, 512;" ::: "memory");
+      if ((et & 3) == 0) {
+        sStat[srow] = rstd;
+        sStat[128 + srow] = -mu * rstd;
+        sStat[256 + srow] = mval;
+      }
+      asm volatile("bar.sync 1, 512;" ::: "memory");
 
       // ---- accumulators of this operand: value block at +0, gate block at +128
-      mbar_wait(&acc_full[grp], acc_phase, ws, 16, grp);
+      mbar_wait(&acc_full[op], acc_phase, ws, 16, op);
       tc_fence_after_sync();
-      const uint32_t tbase = tmem_addr(tmem_base, q, grp * 256);
-      __nv_bfloat16* dst =
-          p.planes + ((static_cast<long long>(grp) * 128 + ch) * p.plane_rows + i) * p.Np + s0;
-      const float4* st4 = reinterpret_cast<const float4*>(st);
-      uint32_t vv[2][16], gv[2][16];
-      tmem_ld16(tbase, vv[0]);
-      tmem_ld16(tbase + 128, gv[0]);
-#pragma unroll
-      for (int ci = 0; ci < 8; ++ci) {
+      const uint32_t tbase = tmem_addr(tmem_base, q, op * 256 + half * 64);
+      const float4* st4 = reinterpret_cast<const float4*>(sStat + half * 64);
+#pragma unroll 1
+      for (int c16 = 0; c16 < 4; ++c16) {
+        uint32_t v[16], g[16];
+        tmem_ld16(tbase + c16 * 16, v);
+        tmem_ld16(tbase + 128 + c16 * 16, g);
         tmem_ld_wait();
-        if (ci < 7) {
-          tmem_ld16(tbase + (ci + 1) * 16, vv[(ci + 1) & 1]);
-          tmem_ld16(tbase + 128 + (ci + 1) * 16, gv[(ci + 1) & 1]);
+        if (c16 == 3) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[op]);      // the accumulators are in registers
         }
-        const uint32_t* v = vv[ci & 1];
-        const uint32_t* g = gv[ci & 1];
-        float o[16];
+        if ((c16 & 1) == 0) {
+          if (lane == 0) tma_store_wait_read<0>();         // the previous box of this warp has left the staging rows
+          __syncwarp();
+        }
 #pragma unroll
-        for (int j4 = 0; j4 < 4; ++j4) {
-          const float4 rs = st4[ci * 4 + j4];
-          const float4 nm = st4[32 + ci * 4 + j4];
-          const float4 mk = st4[64 + ci * 4 + j4];
-          const float rsv[4] = {rs.x, rs.y, rs.z, rs.w};
-          const float nmv[4] = {nm.x, nm.y, nm.z, nm.w};
-          const float mkv[4] = {mk.x, mk.y, mk.z, mk.w};
+        for (int j8 = 0; j8 < 2; ++j8) {
+          uint32_t o[4];
 #pragma unroll
-          for (int e = 0; e < 4; e += 2) {
+          for (int h4 = 0; h4 < 2; ++h4) {
             // two adjacent s at a time in packed fp32 instructions
-            const int si = j4 * 4 + e;
-            const float2 rs2 = make_float2(rsv[e], rsv[e + 1]);
-            const float2 nm2 = make_float2(nmv[e], nmv[e + 1]);
-            const float2 val = __ffma2_rn(make_float2(__uint_as_float(v[si]), __uint_as_float(v[si + 1])), rs2,
-                                          __ffma2_rn(nm2, csv2, cbv2));
-            const float2 gt = __ffma2_rn(make_float2(__uint_as_float(g[si]), __uint_as_float(g[si + 1])), rs2,
-                                         __ffma2_rn(nm2, csg2, cbg2));
-            const float2 sg = make_float2(mkv[e] * sigmoidf_fast(gt.x), mkv[e + 1] * sigmoidf_fast(gt.y));
-            const float2 ov = __fmul2_rn(val, sg);
-            o[si] = ov.x;
-            o[si + 1] = ov.y;
+            const int f4 = c16 * 4 + j8 * 2 + h4, si = j8 * 8 + h4 * 4;
+            const float4 rs = st4[f4], nm = st4[32 + f4], mk = st4[64 + f4];
+            auto gated = [&](int k, float2 rs2, float2 nm2, float2 mk2) {
+              const float2 val = __ffma2_rn(make_float2(__uint_as_float(v[k]), __uint_as_float(v[k + 1])), rs2,
+                                            __ffma2_rn(nm2, csv2, cbv2));
+              const float2 gt = __ffma2_rn(make_float2(__uint_as_float(g[k]), __uint_as_float(g[k + 1])), rs2,
+                                           __ffma2_rn(nm2, csg2, cbg2));
+              const float2 ov = __fmul2_rn(
+                  val, __fmul2_rn(mk2, make_float2(sigmoidf_fast(gt.x), sigmoidf_fast(gt.y))));
+              return pack_bf16x2(ov.x, ov.y);
+            };
+            o[h4 * 2] = gated(si, make_float2(rs.x, rs.y), make_float2(nm.x, nm.y), make_float2(mk.x, mk.y));
+            o[h4 * 2 + 1] = gated(si + 2, make_float2(rs.z, rs.w), make_float2(nm.z, nm.w), make_float2(mk.z, mk.w));
           }
+          *reinterpret_cast<uint4*>(stage_w + swz64_offset(lane, (c16 & 1) * 2 + j8)) =
+              make_uint4(o[0], o[1], o[2], o[3]);
         }
-        uint4 u[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          u[j].x = pack_bf16x2(o[j * 8 + 0], o[j * 8 + 1]);
-          u[j].y = pack_bf16x2(o[j * 8 + 2], o[j * 8 + 3]);
-          u[j].z = pack_bf16x2(o[j * 8 + 4], o[j * 8 + 5]);
-          u[j].w = pack_bf16x2(o[j * 8 + 6], o[j * 8 + 7]);
-        }
-        const int sc = s0 + ci * 16;
-        if (out_tma) {
-          if ((ci & 1) == 0) {
-            if (lane == 0) tma_store_wait_read<0>();   // the previous box of this warp has left the staging rows
-            __syncwarp();
+        if (c16 & 1) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_3d(&tmP, stage_w, s0 + half * 64 + (c16 >> 1) * 32, i, op * 128 + q * 32);   // past Np: clipped
+            tma_store_commit();
           }
-          *reinterpret_cast<uint4*>(stage_w + swz64_offset(lane, (ci & 1) * 2)) = u[0];
-          *reinterpret_cast<uint4*>(stage_w + swz64_offset(lane, (ci & 1) * 2 + 1)) = u[1];
-          if (ci & 1) {
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_3d(&tmP, stage_w, s0 + (ci >> 1) * 32, i, grp * 128 + q * 32);   // entries past Np are clipped
-              tma_store_commit();
-            }
-          }
-        } else if (wide && sc + 16 <= p.Np) {
-          st_global_256(dst + ci * 16, u[0], u[1]);   // a whole 32-byte sector per lane
-        } else {
-          if (sc < p.Np) *reinterpret_cast<uint4*>(dst + ci * 16) = u[0];
-          if (sc + 8 < p.Np) *reinterpret_cast<uint4*>(dst + ci * 16 + 8) = u[1];
         }
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[grp]);
       if (++stage == kTPStages) {
         stage = 0;
         phase ^= 1u;
       }
       acc_phase ^= 1u;
     }
-    if (out_tma && lane == 0) tma_store_wait_all<0>();   // the staging rows are read and the boxes written
+    if (lane == 0) tma_store_wait_all<0>();   // the staging rows are read and the boxes written
   }
 
   tc_fence_before_sync();
@@ -324,7 +304,7 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   }
 }
 
-constexpr int kTPSmemBytes = kTPWBytes + kTPStages * kTPXBytes + kTPOutBytes + 2 * 2 * 3 * 128 * 4 + 256 + 1024;
+constexpr int kTPSmemBytes = kTPWBytes + kTPStages * kTPXBytes + kTPOutBytes + 3 * 128 * 4 + 256 + 1024;
 static_assert(kTPSmemBytes <= 232448, "shared memory of one CTA");
 
 }  // namespace ubm
@@ -351,7 +331,6 @@ static int trimul_proj_impl(const void* z, const void* w, const void* colsum, co
   p.colsum = static_cast<const float*>(colsum);
   p.colbias = static_cast<const float*>(colbias);
   p.mask = static_cast<const float*>(mask);
-  p.planes = static_cast<__nv_bfloat16*>(planes);
   p.stats_out = static_cast<float*>(stats_out);
   p.status = static_cast<KernelStatus*>(status);
   CUtensorMap tmX, tmW;
@@ -371,26 +350,16 @@ static int trimul_proj_impl(const void* z, const void* w, const void* colsum, co
     rc = make_peer_src(&maps, &p.src, z_ptrs, peer_rows, npeers, me, N, tmX);
     if (rc) return rc;
   }
-  CUtensorMap tmP = tmX;
-  p.out_tma = 0;
-  {
-    static const bool on = [] {
-      const char* e = getenv("UBM_PROJ_TMA_STORE");
-      return e == nullptr || e[0] != '0';
-    }();
-    if (on && (reinterpret_cast<uintptr_t>(planes) & 15) == 0) {
-      uint64_t dP[3] = {(uint64_t)Np, (uint64_t)plane_rows, 256};
-      uint64_t sP[2] = {(uint64_t)Np * 2, (uint64_t)plane_rows * Np * 2};
-      uint32_t bP[3] = {32, 1, 32};
-      rc = make_tmap(&tmP, planes, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dP, sP, bP, CU_TENSOR_MAP_SWIZZLE_64B);
-      if (rc) return rc;
-      p.out_tma = 1;
-    }
-  }
+  CUtensorMap tmP;
+  uint64_t dP[3] = {(uint64_t)Np, (uint64_t)plane_rows, 256};
+  uint64_t sP[2] = {(uint64_t)Np * 2, (uint64_t)plane_rows * Np * 2};
+  uint32_t bP[3] = {32, 1, 32};
+  rc = make_tmap(&tmP, planes, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dP, sP, bP, CU_TENSOR_MAP_SWIZZLE_64B);
+  if (rc) return rc;
   rc = set_smem(trimul_proj_kernel, kTPSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  trimul_proj_kernel<<<grid, 320, kTPSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmX, tmW, maps, tmP, p);
+  trimul_proj_kernel<<<grid, kTPThreads, kTPSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmX, tmW, maps, tmP, p);
   UBM_CHECK_LAUNCH("trimul_proj_kernel");
   return UBM_OK;
 }
