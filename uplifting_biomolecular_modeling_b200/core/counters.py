@@ -90,6 +90,10 @@ class LedgerBook:
             self._ledgers[lever] = lg
         return lg
 
+    def find(self, lever: str) -> Optional[Ledger]:
+        """The lever's ledger, or None before its first :meth:`get` (asked on every kernel call)."""
+        return self._ledgers.get(lever)
+
     def items(self):
         return self._ledgers.items()
 

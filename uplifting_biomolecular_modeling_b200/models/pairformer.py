@@ -245,7 +245,7 @@ class TriangleAttention(_Switchable):
         hb[:, :, :N] = (F.linear(n, self.linear.weight.to(n.dtype)).float() * pair.LOG2E).view(N, N, H).permute(2, 0, 1)
         km = None
         if mask is not None:
-            km = _cached_key_mask(self._workspace, mask[0], transposed=not self.starting)
+            km = pair.KeyMask.lay_out(mask[0] if self.starting else mask[0].t())
         o = torch.empty((N * N, HD), dtype=torch.bfloat16, device=z.device)
         pair.attention(qkvg[:, :HD], qkvg[:, HD:2 * HD], qkvg[:, 2 * HD:3 * HD], hb, qkvg[:, 3 * HD:], o, rows=N, Nq=N,
                        Nk=N, H=H, D=w.Dp, ldb=Np, ld_in=4 * HD, ld_gate=4 * HD, mask=km)
@@ -272,7 +272,7 @@ class TriangleAttention(_Switchable):
             from ..ops import pair
             km = None
             if mask is not None:
-                km = _cached_key_mask(self._workspace, mask[0], transposed=not self.starting)
+                km = pair.KeyMask.lay_out(mask[0] if self.starting else mask[0].t())
             if self._packed is None:
                 self._packed = pair.TriattPacked.pack(self.layer_norm.weight, self.layer_norm.bias,
                                                       self.linear.weight, m.linear_q.weight, m.linear_k.weight,
@@ -287,20 +287,6 @@ class TriangleAttention(_Switchable):
                                      m.linear_o.bias, self.heads, starting=self.starting, residual=residual)
                 for b in range(z.shape[0])]
         return torch.stack(outs, 0)
-
-
-def _cached_key_mask(workspace: Optional[dict], mask: torch.Tensor, transposed: bool = False):
-    """Key mask of the attention kernel for a [rows, keys] keep-mask, packed once per mask tensor: the same pair
-    mask reaches every triangle attention of a stack, so the packed form is kept in the stack's workspace under the
-    tensor's identity and version."""
-    from ..ops import pair
-    ws = workspace if workspace is not None else {}
-    key = ("keymask", mask.data_ptr(), mask._version, tuple(mask.shape), transposed)
-    if key not in ws:
-        for k in [k for k in ws if isinstance(k, tuple) and k and k[0] == "keymask" and k[1] != mask.data_ptr()]:
-            del ws[k]
-        ws[key] = pair.KeyMask.pack(mask.t() if transposed else mask)
-    return ws[key]
 
 
 class TriangleAttentionStartingNode(TriangleAttention):
@@ -358,9 +344,9 @@ class AttentionPairBias(_Switchable):
         from ..ops import pair
         km = None
         if mask is not None:
-            km = _cached_key_mask(self._workspace, mask if mask.shape[0] == s.shape[0] else
-                                  mask.expand(s.shape[0], -1) if mask.shape[0] == 1 else
-                                  mask.repeat_interleave(s.shape[0] // mask.shape[0], 0))
+            km = pair.KeyMask.lay_out(mask if mask.shape[0] == s.shape[0] else
+                                      mask.expand(s.shape[0], -1) if mask.shape[0] == 1 else
+                                      mask.repeat_interleave(s.shape[0] // mask.shape[0], 0))
         if self._packed is None:
             self._packed = pair.ApbPacked.pack(self.proj_q.weight, self.proj_q.bias, self.proj_k.weight,
                                                self.proj_v.weight, self.proj_g.weight, self.proj_o.weight,
@@ -431,9 +417,17 @@ class PairformerLayer(nn.Module):
             return s, z
         # single track in fp32, as upstream (pairformer.py:103-111)
         s32 = s.float()
-        sn = F.layer_norm(s32, (s32.shape[-1],), self.pre_norm_s.weight.float(), self.pre_norm_s.bias.float())
-        with torch.autocast(device_type=s.device.type, enabled=False):
-            upd = _run_fp32(self.attention, sn, z, mask)
+        norm = self.pre_norm_s
+        if self.attention.impl == "fused" and s.is_cuda and self.attention.proj_q.weight.dtype == torch.bfloat16 \
+                and s.shape[-1] % 8 == 0 and s.shape[-1] <= 1024:
+            # normalised in fp32 and rounded once to the projection's type, in one launch
+            from ..ops import rows
+            upd = self.attention(rows.layernorm_rows(s32.contiguous(), norm.weight, norm.bias, 1e-5, torch.bfloat16), z,
+                                 mask).float()
+        else:
+            sn = F.layer_norm(s32, (s32.shape[-1],), norm.weight.float(), norm.bias.float())
+            with torch.autocast(device_type=s.device.type, enabled=False):
+                upd = _run_fp32(self.attention, sn, z, mask)
         s32 = s32 + upd
         s32 = s32 + _run_fp32(self.transition_s, s32)
         return s32.to(s.dtype), z

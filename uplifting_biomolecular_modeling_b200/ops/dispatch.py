@@ -41,10 +41,11 @@ SIZE_REASONS = ("below_min_tokens", "above_max_tokens")
 
 
 def size_gate(lever: str):
-    import os
-    from . import provider
     g = _GATES.get(lever)
     if g is None:
+        import os
+        from . import provider
+
         def env(word):
             v = os.environ.get(f"UBM_{word}_TOKENS_{lever.upper()}") or os.environ.get(f"UBM_{word}_TOKENS")
             return int(v) if v else None
@@ -71,6 +72,9 @@ def _sm() -> str:
 
 
 def ledger(lever: str) -> counters.Ledger:
+    lg = counters.BOOK.find(lever)
+    if lg is not None:
+        return lg
     impl, _, declared = LEVERS.get(lever, ("unknown", lever, ()))
     return counters.BOOK.get(lever, impl, declared_fallbacks=tuple(declared) + SIZE_REASONS,
                              strategy="F1.kernel_fusion")
@@ -81,8 +85,10 @@ def decide(lever: str, reason: Optional[str], klass: Optional[str] = None, token
     """Record one call.  ``reason`` None = the kernel serves; otherwise the plain statement runs and the call is
     counted as ``fallback:<reason>``.  Returns True when the kernel serves."""
     lg = ledger(lever)
-    if reason is None and tokens is not None and not size_gate(lever).admit(int(tokens)):
-        reason = "below_min_tokens" if tokens < size_gate(lever).min_tokens else "above_max_tokens"
+    if reason is None and tokens is not None:
+        gate = size_gate(lever)
+        if not gate.admit(int(tokens)):
+            reason = "below_min_tokens" if tokens < gate.min_tokens else "above_max_tokens"
     if reason is None:
         lg.serve(klass)
     else:

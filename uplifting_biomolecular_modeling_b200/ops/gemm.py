@@ -7,6 +7,8 @@ multiplication (common/opt_core/opt_core/kernels/fpf_trimul_v4/DESIGN.md:21-37).
 """
 from __future__ import annotations
 
+import ctypes
+import struct
 from typing import Optional
 
 import torch
@@ -15,6 +17,9 @@ from . import native
 
 native.declare("ubm_gemm_fp8", [native.c_void_p] * 5 + [native.c_int] * 3 + [native.c_ll] * 4 +
                [native.c_int, native.c_float, native.c_void_p, native.c_void_p, native.c_void_p])
+
+native.declare("ubm_gemm_bf16_packed", [ctypes.c_char_p])
+_ARGS = struct.Struct("=29qd")       # the integer arguments of ubm_gemm_bf16_ex in order, then alpha
 
 ACT = {None: 0, "none": 0, "silu": 1, "sigmoid": 2, "gelu": 3, "relu": 4, "swiglu3": 5, "swiglu": 6}
 
@@ -37,10 +42,6 @@ def pack_swiglu(gate_w: torch.Tensor, value_w: torch.Tensor) -> torch.Tensor:
         raise ValueError("pack_swiglu expects two [H, K] weights with H a multiple of 32")
     w = torch.stack([gate_w.view(H // 32, 32, K), value_w.view(H // 32, 32, K)], 1)
     return w.reshape(2 * H, K).to(torch.bfloat16).contiguous()
-
-
-def _as3(t: torch.Tensor) -> torch.Tensor:
-    return t.unsqueeze(0) if t.dim() == 2 else t
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Optional[torch.Tensor] = None,
@@ -67,68 +68,66 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
     """
     if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
         raise TypeError("gemm expects bf16 operands")
-    squeeze = a.dim() == 2
-    a3, b3 = _as3(a), _as3(b)
-    if a3.stride(-1) != 1 or b3.stride(-1) != 1:
+    # shapes and strides are read once each and no views are made: this runs in front of every projection of a layer
+    sha, sta, shb, stb = a.shape, a.stride(), b.shape, b.stride()
+    batch = sha[0] if len(sha) == 3 else 1
+    if sta[-1] != 1 or stb[-1] != 1:
         raise ValueError("innermost dimension must be contiguous")
-    batch = a3.shape[0]
-    if b3.shape[0] != batch:
+    if (shb[0] if len(shb) == 3 else 1) != batch:
         raise ValueError("batch mismatch")
     if mn_major:
-        K, M = a3.shape[1], a3.shape[2]
-        N = b3.shape[2]
-        if b3.shape[1] != K:
-            raise ValueError("K mismatch")
+        K, M = sha[-2:]
+        kb, N = shb[-2:]
     else:
-        M, K = a3.shape[1], a3.shape[2]
-        N = b3.shape[1]
-        if b3.shape[2] != K:
-            raise ValueError("K mismatch")
+        M, K = sha[-2:]
+        N, kb = shb[-2:]
+    if kb != K:
+        raise ValueError("K mismatch")
+    n_out = N
     if c_blocked is not None:
         if out is None or (batch != 1 and c_batch <= 0) or N % 32 or residual is not None:
             raise ValueError("c_blocked needs an output tensor, batch 1 or c_batch, N % 32 == 0 and no residual")
-        out3 = out
+        ldc, stride_c = 0, c_batch
     else:
-        n_out = N
         if act in ("swiglu3", "swiglu"):
             group = 96 if act == "swiglu3" else 64
             if N % group or mn_major or bias is not None or gate is not None or residual is not None or act_from:
                 raise ValueError(f"{act} needs a K-major product with N % {group} == 0 and no bias / gate / residual")
             n_out = N // 3 if act == "swiglu3" else N // 2
         if out is None:
-            out = torch.empty((batch, M, n_out), dtype=torch.bfloat16 if n_out != N else out_dtype, device=a.device)
-        out3 = _as3(out)
-        if n_out != N and (out3.shape[-1] != n_out or out3.shape[-2] != M or out3.dtype != torch.bfloat16):
+            out = torch.empty((M, n_out) if len(sha) == 2 else (batch, M, n_out),
+                              dtype=torch.bfloat16 if n_out != N else out_dtype, device=a.device)
+        sho, sto = out.shape, out.stride()
+        if n_out != N and (sho[-1] != n_out or sho[-2] != M or out.dtype != torch.bfloat16):
             raise ValueError(f"{act} output must be bf16 [.., {M}, {n_out}]")
-        if out3.stride(-1) != 1:
+        if sto[-1] != 1:
             raise ValueError("output innermost dimension must be contiguous")
-    res3 = None
+        ldc, stride_c = (sto[1], sto[0]) if len(sho) == 3 else (sto[0], 0)
+    ldr = stride_r = 0
     if residual is not None:
-        res3 = _as3(residual)
-        if res3.dtype != torch.bfloat16 or res3.stride(-1) != 1:
+        str_ = residual.stride()
+        if residual.dtype != torch.bfloat16 or str_[-1] != 1:
             raise ValueError("residual must be bf16 with contiguous rows")
+        ldr, stride_r = (str_[1], str_[0]) if len(str_) == 3 else (str_[0], 0)
     if bias is not None and bias.dtype != torch.float32:
         bias = bias.float()
-    st = native.status_tensor(a.device)
+    gate_ptr = ld_gate = gate_rows = 0
     if gate is not None:
-        if gate.dtype != torch.bfloat16 or gate.dim() != 2 or gate.shape[1] != N or gate.stride(1) != 1 or batch != 1:
+        shg, stg = gate.shape, gate.stride()
+        if gate.dtype != torch.bfloat16 or len(shg) != 2 or shg[1] != N or stg[1] != 1 or batch != 1:
             raise ValueError("gate must be bf16 [rows, N] with contiguous rows (batch 1)")
-    cb = c_blocked if c_blocked is not None else (0, 0, 0)
-    rc = native.lib().ubm_gemm_bf16_ex(
-        native.ptr(a3), native.ptr(b3), native.ptr(out3), native.ptr(bias), native.ptr(res3),
-        M, N, K, batch,
-        a3.stride(1), b3.stride(1), 0 if c_blocked is not None else out3.stride(1),
-        0 if res3 is None else res3.stride(1),
-        a3.stride(0) if batch > 1 else 0, b3.stride(0) if batch > 1 else 0,
-        0 if batch == 1 else out3.stride(0) if c_blocked is None else c_batch,
-        0 if res3 is None or batch == 1 else res3.stride(0),
-        1 if mn_major else 0, 1 if out3.dtype == torch.float32 else 0, ACT[act], float(alpha),
-        int(cb[0]), int(cb[1]), int(cb[2]), native.ptr(gate), 0 if gate is None else gate.stride(0),
-        0 if gate is None else gate.shape[0], int(act_from), native.ptr(st), native.current_stream(a.device))
-    native.check(rc, "ubm_gemm_bf16_ex")
-    if c_blocked is not None:
-        return out
-    return out3[0] if squeeze and out.dim() == 3 else out
+        gate_ptr, ld_gate, gate_rows = gate.data_ptr(), stg[0], shg[0]
+    hi, lo, col = c_blocked if c_blocked is not None else (0, 0, 0)
+    dev = a.device
+    many = batch > 1
+    rc = native.lib().ubm_gemm_bf16_packed(_ARGS.pack(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), 0 if bias is None else bias.data_ptr(),
+        0 if residual is None else residual.data_ptr(), M, N, K, batch, sta[-2], stb[-2], ldc, ldr,
+        sta[0] if many else 0, stb[0] if many else 0, stride_c if many else 0, stride_r if many else 0,
+        1 if mn_major else 0, 1 if out.dtype == torch.float32 else 0, ACT[act], hi, lo, col, gate_ptr, ld_gate,
+        gate_rows, act_from, native.status_tensor(dev).data_ptr(), native.current_stream(dev), alpha))
+    native.check(rc, "ubm_gemm_bf16_packed")
+    return out[0] if len(sha) == 2 and c_blocked is None and out.dim() == 3 else out
 
 
 _E4M3 = (torch.uint8, torch.float8_e4m3fn)

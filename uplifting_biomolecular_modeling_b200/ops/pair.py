@@ -195,6 +195,7 @@ native.declare("ubm_attention_d32", _ATTN_SIG)
 native.declare("ubm_attention_d64", _ATTN_SIG)
 
 native.declare("ubm_attention_set_variant", [c_int])
+native.declare("ubm_key_mask", [c_void_p, c_int, c_ll, c_ll, c_void_p, c_void_p, c_int, c_int, c_void_p])
 
 LOG2E = 1.4426950408889634
 
@@ -230,6 +231,21 @@ class KeyMask:
         add = torch.zeros((rows, ld), dtype=torch.bfloat16, device=keep.device)
         add[:, :nk].masked_fill_(~keep, MASK_NEG)
         flags = (add.view(rows, ld // MASK_STEP, MASK_STEP) != 0).any(-1).to(torch.uint8).contiguous()
+        return cls(add, flags)
+
+    @classmethod
+    def lay_out(cls, keep: torch.Tensor) -> "KeyMask":
+        """:meth:`pack` of a mask on the GPU as one launch and without the host read: a mask that keeps everything gets
+        clear flags, with which the kernel runs its mask-free loop."""
+        rows, nk = keep.shape
+        steps = ceil_to(nk, MASK_STEP) // MASK_STEP
+        if keep.dtype not in (torch.float32, torch.bfloat16, torch.bool, torch.uint8):
+            keep = keep != 0
+        add = torch.empty((rows, steps * MASK_STEP), dtype=torch.bfloat16, device=keep.device)
+        flags = torch.empty((rows, steps), dtype=torch.uint8, device=keep.device)
+        rc = native.lib().ubm_key_mask(native.ptr(keep), keep.element_size(), keep.stride(0), keep.stride(1),
+                                       native.ptr(add), native.ptr(flags), rows, nk, native.current_stream(keep.device))
+        native.check(rc, "ubm_key_mask")
         return cls(add, flags)
 
 

@@ -32,7 +32,7 @@ def _f32_param(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     if t is None:
         return None
     if t.dtype == torch.float32 and t.is_contiguous():
-        return t.detach()
+        return t
     ent = _F32_CACHE.get(id(t))
     if ent is None or ent[0] is not t or ent[1] != t._version or ent[2].device != t.device:
         if len(_F32_CACHE) > 4096:
