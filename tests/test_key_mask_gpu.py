@@ -17,7 +17,7 @@ def test_lay_out_equals_pack(rows, nk, dtype, form):
     elif form == "expanded":
         keep = keep[:1].expand(rows, nk)
     elif form == "strided":
-        keep = torch.stack([keep, 1 - keep.to(torch.uint8).to(dtype)], -1)[..., 0]
+        keep = torch.stack([keep, (keep == 0).to(dtype)], -1)[..., 0]
     got, want = pair.KeyMask.lay_out(keep), pair.KeyMask.pack(keep)
     if want is None:
         assert not got.add.any() and not got.flags.any()
