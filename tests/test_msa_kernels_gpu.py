@@ -47,6 +47,24 @@ def test_pair_weighted_averaging(S, N, masked, mask_dtype):
     assert not m(x, z, mask).any()
 
 
+@pytest.mark.parametrize("S,N,full", [(1, 4, True), (7, 33, False), (64, 130, True), (40, 300, False)])
+def test_outer_product_mean(S, N, full):
+    from uplifting_biomolecular_modeling_b200.models import msa, pairformer
+    m = _module(msa.OuterProductMean, S)
+    pairformer.set_impl(m, "fused")
+    m.full_mask = full
+    x = torch.randn(1, S, N, 64, device="cuda").bfloat16()
+    mask = torch.ones(1, S, N, device="cuda", dtype=torch.bfloat16)
+    if not full:
+        mask = (torch.rand_like(mask, dtype=torch.float32) < 0.8).bfloat16()
+    got = m(x, mask)
+    d = lambda p: p.detach().double()  # noqa: E731
+    want = R.outer_product_mean(x.double(), mask.double(), d(m.norm.weight), d(m.norm.bias), d(m.proj_a.weight),
+                                d(m.proj_b.weight), d(m.proj_o.weight), d(m.proj_o.bias))
+    # normalised rows, both projections, the product, its projection and the rescaled result are bf16
+    assert _rel(got, want) <= 8 * 2.0 ** -9
+
+
 @pytest.mark.parametrize("M,N,batch", [(1, 32, 1), (33, 96, 3), (200, 320, 8)])
 def test_blocked_output_of_a_batch(M, N, batch):
     """Element (b, m, n) of the product at row m, block n // 32, entry b of the output."""

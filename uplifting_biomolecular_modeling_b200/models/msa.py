@@ -43,11 +43,18 @@ class OuterProductMean(_Switchable):
         B, S, N, _ = m.shape
         c = self.c_hidden
         n = rows.layernorm_rows(m.contiguous(), self.norm.weight, self.norm.bias, self.norm.eps)
-        mk = mask.unsqueeze(-1).to(n.dtype)
         # [S, N, c] seen as [S, N*c]: sequences (the contraction) along rows, (token, channel) contiguous - the
         # operand form of the MN-major GEMM, so no [N*c, S] transposed copies are made
-        a2 = (self.proj_a(n) * mk)[0].reshape(S, N * c)
-        b2 = (self.proj_b(n) * mk)[0].reshape(S, N * c)
+        wab = torch.cat([self.proj_a.weight, self.proj_b.weight], 0).to(torch.bfloat16)
+        if c == 32 and n.shape[-1] % 8 == 0:
+            # both projections from one product, its two 32-wide column blocks stored apart
+            ab = torch.empty((2, S * N, c), dtype=torch.bfloat16, device=m.device)
+            gemm.gemm(n.view(S * N, -1), wab, out=ab, c_blocked=(32 * c, c, S * N * c))
+        else:
+            ab = F.linear(n.view(S * N, -1), wab).view(S * N, 2, c).transpose(0, 1).contiguous()
+        if not self.full_mask:
+            ab *= mask.reshape(1, S * N, 1).to(ab.dtype)
+        a2, b2 = ab[0].view(S, N * c), ab[1].view(S, N * c)
         wo = self.proj_o.weight.to(torch.bfloat16).contiguous()
         bo = self.proj_o.bias.float()
         out = torch.empty((N, N, wo.shape[0]), dtype=torch.bfloat16, device=m.device)
