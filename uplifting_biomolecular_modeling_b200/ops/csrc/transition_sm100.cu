@@ -5,15 +5,17 @@
 // statistics, and as the residual.  LayerNorm is folded into the first GEMM (weights carry
 // gamma, the statistics scale the fp32 accumulator).  The hidden dimension is walked in chunks
 // of 64: GEMM1 produces [a | b] (128 TMEM columns), the SwiGLU warps turn them into a bf16
-// 128 x 64 tile in shared memory, GEMM2 accumulates it into the 128 x 128 output accumulator.
+// 128 x 64 tile that stays in tensor memory (the A operand of GEMM2), GEMM2 accumulates it into the 128 x 128 output accumulator.
 // The hidden activations never touch HBM.  Weight chunks stream from L2 through a 2-stage ring.
 //
 // Reference kernels with the same fusion boundary: fpf_transition_v2 (Triton, the fastest row on
 // B200: common/opt_core/opt_core/kernels/transition/TRANSITION_CELLS.json:2802), flash_sm90a and
 // ef2_t16 (wgmma, sm_90a only: common/opt_core/opt_core/kernels/transition/DESIGN.md:24-63).
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer, 2-5 / 6-9 = two SwiGLU/epilogue groups that take
-// alternate hidden chunks.
+// Warps: 0 = TMA producer, 1 = MMA issuer, 2-9 / 10-17 = two SwiGLU / epilogue groups that take alternate hidden
+// chunks; in a group two warps share each lane quadrant, 32 of the chunk's 64 columns each.  With the hidden tile in
+// shared memory and eight warps that wrote their rows directly: 1.479 ms at 1536 tokens against 1.438, 0.664 ms at 1021
+// against 0.648, 61 us at 256 against 57.  What holds it is not found: tensor pipe and issue slots are a third busy.
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -24,7 +26,6 @@ constexpr int kTRXBytes = 128 * 128 * 2;        // 32 KB
 constexpr int kTRWabBytes = 128 * 128 * 2;      // 32 KB: [a64|b64 rows][128 k] as two k-blocks
 constexpr int kTRWoBytes = 128 * 64 * 2;        // 16 KB: [128 out][64 k]
 constexpr int kTRWStage = kTRWabBytes + kTRWoBytes;
-constexpr int kTRHBytes = 128 * 64 * 2;         // 16 KB
 constexpr int kTRMaxHidden = 1024;
 
 struct TransitionParams {
@@ -34,35 +35,38 @@ struct TransitionParams {
   const float* ab_colbias;  // [hidden/64][128]
   const float* o_bias;      // [128] or null
   const float* mask;        // [R] or null: multiplies the update
-  __nv_bfloat16* out;       // [R][128]
   int add_residual;
   KernelStatus* status;
   int num_tiles;
 };
 
-__global__ void __launch_bounds__(320, 1)
+constexpr int kTREpiWarps = 16;
+constexpr int kTRThreads = 64 + 32 * kTREpiWarps;
+
+__global__ void __launch_bounds__(kTRThreads, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWab,
-                  const __grid_constant__ CUtensorMap tmWo, TransitionParams p) {
+                  const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmOut,
+                  TransitionParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sX = smem;                       // 2 x 32 KB
   uint8_t* sW = sX + 2 * kTRXBytes;         // 2 x 48 KB
-  uint8_t* sH = sW + 2 * kTRWStage;         // 2 x 16 KB
-  float* sColsum = reinterpret_cast<float*>(sH + 2 * kTRHBytes);  // [hidden*2]
+  float* sColsum = reinterpret_cast<float*>(sW + 2 * kTRWStage);  // [hidden*2]
   float* sColbias = sColsum + 2 * kTRMaxHidden;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sColbias + 2 * kTRMaxHidden);
+  float2* sPart = reinterpret_cast<float2*>(sColbias + 2 * kTRMaxHidden);   // [2 groups][2 halves][128] row sums
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sPart + 4 * 128);
   uint64_t* x_full = bars;            // [2]
-  uint64_t* x_empty = x_full + 2;     // [2] 8 arrivals
+  uint64_t* x_empty = x_full + 2;     // [2] 8 arrivals: one per box of output rows that has left the tile
   uint64_t* w_full = x_empty + 2;     // [2] first-GEMM weights (a|b rows) landed
   uint64_t* w_empty = w_full + 2;     // [2] commit after the first GEMM: its slot refills while SwiGLU runs
   uint64_t* wo_full = w_empty + 2;    // [2] second-GEMM weights landed
   uint64_t* wo_empty = wo_full + 2;   // [2] commit after the second GEMM
   uint64_t* ab_full = wo_empty + 2;   // [2] commit
-  uint64_t* ab_empty = ab_full + 2;   // [2] 4 arrivals
-  uint64_t* h_full = ab_empty + 2;    // [2] 4 arrivals
+  uint64_t* ab_empty = ab_full + 2;   // [2] 8 arrivals
+  uint64_t* h_full = ab_empty + 2;    // [2] 8 arrivals
   uint64_t* h_empty = h_full + 2;     // [2] commit
   uint64_t* y_full = h_empty + 2;     // [1] commit
-  uint64_t* y_empty = y_full + 1;     // [1] 8 arrivals
+  uint64_t* y_empty = y_full + 1;     // [1] 16 arrivals
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(y_empty + 1);   // 22 barriers before it: 176 of the 256 bytes
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -81,12 +85,12 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       mbar_init(&wo_full[s], 1);
       mbar_init(&wo_empty[s], 1);
       mbar_init(&ab_full[s], 1);
-      mbar_init(&ab_empty[s], 4);
-      mbar_init(&h_full[s], 4);
+      mbar_init(&ab_empty[s], kTREpiWarps / 2);
+      mbar_init(&h_full[s], kTREpiWarps / 2);
       mbar_init(&h_empty[s], 1);
     }
     mbar_init(y_full, 1);
-    mbar_init(y_empty, 8);
+    mbar_init(y_empty, kTREpiWarps);
     mbar_fence_init();
     tma_prefetch_desc(&tmX);
     tma_prefetch_desc(&tmWab);
@@ -106,6 +110,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tAB = tmem_base;        // two buffers of 128 columns
   const uint32_t tY = tmem_base + 256;   // 128 columns
+  const uint32_t tH = tmem_base + 384;   // two buffers of 32 columns (two bf16 each)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -170,14 +175,12 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         mbar_wait(&h_full[b], (c >> 1) & 1u, ws, 33, b);
         if (first_of_tile) mbar_wait(y_empty, (tl & 1u) ^ 1u, ws, 34);
         tc_fence_after_sync();
-        const uint32_t ha = smem_u32(sH + b * kTRHBytes);
         const uint32_t wo = smem_u32(sW + b * kTRWStage + kTRWabBytes);
-        const uint64_t ad0 = umma_smem_desc(ha, 16, 1024, kSwizzle128);
         const uint64_t bd0 = umma_smem_desc(wo, 16, 1024, kSwizzle128);
         if (leader) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_ss(tY, ad0 + static_cast<uint64_t>(k * 2), bd0 + static_cast<uint64_t>(k * 2), idesc,
+            umma_ts(tY, tH + b * 32 + k * 8, bd0 + static_cast<uint64_t>(k * 2), idesc,
                     (first_of_tile && k == 0) ? 0u : 1u);
           umma_commit(&h_empty[b]);
           umma_commit(&wo_empty[b]);
@@ -216,22 +219,23 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     }
   } else {
     // ------------------------------------------------------------------ SwiGLU / epilogue groups
-    const int grp = (warp - 2) >> 2;
+    const int grp = (warp - 2) >> 3;
+    const int half = ((warp - 2) >> 2) & 1;
     const int q = warp & 3;
     const int row = q * 32 + lane;
     uint32_t g = 0;
-    uint32_t xt = 0;
     uint32_t tile_cnt = 0;
-    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++xt, ++tile_cnt) {
+    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++tile_cnt) {
       const long long r = static_cast<long long>(t) * 128 + row;
-      const bool row_ok = r < p.R;
-      const int xs = xt & 1;
-      mbar_wait(&x_full[xs], (xt >> 1) & 1u, ws, 38, xs);
-      const uint8_t* xsm = sX + xs * kTRXBytes;
+      const int xs = tile_cnt & 1;
+      const float mval = (p.mask != nullptr && r < p.R) ? p.mask[r] : 1.0f;
+      mbar_wait(&x_full[xs], (tile_cnt >> 1) & 1u, ws, 38, xs);
+      uint8_t* xsm = sX + xs * kTRXBytes;
+      // row statistics: the two warps of a quadrant take 64 channels each and exchange their sums within the group
       float sum = 0.f, sumsq = 0.f;
-#pragma unroll 4
-      for (int c16 = 0; c16 < 16; ++c16) {
-        const uint4 u = *reinterpret_cast<const uint4*>(xsm + (c16 >> 3) * 16384 + swz128_offset(row, c16 & 7));
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint4 u = *reinterpret_cast<const uint4*>(xsm + half * 16384 + swz128_offset(row, c));
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
@@ -240,11 +244,21 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           sumsq += a * a + b * b;
         }
       }
+      sPart[(grp * 2 + half) * 128 + row] = make_float2(sum, sumsq);
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + grp * 4 + q) : "memory");
+      const float2 other = sPart[(grp * 2 + (half ^ 1)) * 128 + row];
+      sum += other.x;
+      sumsq += other.y;
       const float mu = sum * (1.f / kTRC);
       const float var = fmaxf(sumsq * (1.f / kTRC) - mu * mu, 0.f);
       const float rstd = rsqrtf(var + 1e-5f);
       const float2 a2 = make_float2(rstd, rstd);
       const float2 b2 = make_float2(-mu * rstd, -mu * rstd);
+      if (tile_cnt > 0 && half == 0 && lane == 0) {
+        // the boxes this thread stored from the previous tile have been read: its buffer may be loaded again
+        tma_store_wait_read<0>();
+        mbar_arrive(&x_empty[xs ^ 1]);
+      }
 
       for (int h = 0; h < nch; ++h, ++g) {
         const int b = g & 1;
@@ -252,84 +266,80 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const uint32_t ph = (g >> 1) & 1u;
         mbar_wait(&ab_full[b], ph, ws, 39, b);
         tc_fence_after_sync();
-        const uint32_t ta = tmem_addr(tAB, q, b * 128);
-        const float* cs = sColsum + h * 128;
-        const float* cb = sColbias + h * 128;
-        uint32_t packed[32];
+        const uint32_t ta = tmem_addr(tAB, q, b * 128 + half * 32);
+        uint32_t av[32], bv[32];
+        tmem_ld32(ta, av);
+        tmem_ld32(ta + 64, bv);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ab_empty[b]);
+        const float4* cs4 = reinterpret_cast<const float4*>(sColsum + h * 128 + half * 32);
+        const float4* cb4 = reinterpret_cast<const float4*>(sColbias + h * 128 + half * 32);
+        uint32_t packed[16];
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t av[32], bv[32];
-          tmem_ld32(ta + half * 32, av);
-          tmem_ld32(ta + 64 + half * 32, bv);
-          tmem_ld_wait();
-          if (half == 1) {
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ab_empty[b]);
-          }
-          float fa[32], fb[32];
-          ln_fold32(av, a2, b2, cs + half * 32, cb + half * 32, fa);
-          ln_fold32(bv, a2, b2, cs + 64 + half * 32, cb + 64 + half * 32, fb);
-#pragma unroll
-          for (int m = 0; m < 32; m += 2) {
-            const float2 hv = __fmul2_rn(make_float2(siluf_fast(fa[m]), siluf_fast(fa[m + 1])),
-                                         make_float2(fb[m], fb[m + 1]));
-            packed[half * 16 + (m >> 1)] = pack_bf16x2(hv.x, hv.y);
-          }
+        for (int j = 0; j < 8; ++j) {
+          const float4 sa = cs4[j], ba = cb4[j], sb = cs4[16 + j], bb = cb4[16 + j];
+          const float2 fa0 = ln_fold2(av[4 * j], av[4 * j + 1], a2, b2, sa.x, sa.y, ba.x, ba.y);
+          const float2 fa1 = ln_fold2(av[4 * j + 2], av[4 * j + 3], a2, b2, sa.z, sa.w, ba.z, ba.w);
+          const float2 fb0 = ln_fold2(bv[4 * j], bv[4 * j + 1], a2, b2, sb.x, sb.y, bb.x, bb.y);
+          const float2 fb1 = ln_fold2(bv[4 * j + 2], bv[4 * j + 3], a2, b2, sb.z, sb.w, bb.z, bb.w);
+          const float2 h0 = __fmul2_rn(make_float2(siluf_fast(fa0.x), siluf_fast(fa0.y)), fb0);
+          const float2 h1 = __fmul2_rn(make_float2(siluf_fast(fa1.x), siluf_fast(fa1.y)), fb1);
+          packed[2 * j] = pack_bf16x2(h0.x, h0.y);
+          packed[2 * j + 1] = pack_bf16x2(h1.x, h1.y);
         }
         mbar_wait(&h_empty[b], ph ^ 1u, ws, 40, b);
-        uint8_t* hs = sH + b * kTRHBytes;
-#pragma unroll
-        for (int c16 = 0; c16 < 8; ++c16) {
-          uint4 u = make_uint4(packed[c16 * 4], packed[c16 * 4 + 1], packed[c16 * 4 + 2], packed[c16 * 4 + 3]);
-          *reinterpret_cast<uint4*>(hs + swz128_offset(row, c16)) = u;
-        }
-        fence_proxy_async_smem();
+        tc_fence_after_sync();
+        tmem_st16(tmem_addr(tH, q, b * 32 + half * 16), packed);
+        tmem_st_wait();
+        tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&h_full[b]);
       }
 
-      // ---- output: columns grp*64 .. +63
+      // ---- output: columns grp * 64 + half * 32 .. + 31, over the tile's own rows (they are the residual)
       mbar_wait(y_full, tile_cnt & 1u, ws, 41);
       tc_fence_after_sync();
-      const float mval = (p.mask != nullptr && row_ok) ? p.mask[r] : 1.0f;
-#pragma unroll 1
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        uint32_t yv[32];
-        tmem_ld32(tmem_addr(tY, q, grp * 64 + c0), yv);
-        tmem_ld_wait();
-        float f[32];
+      const int c0 = half * 32;
+      uint32_t yv[32];
+      tmem_ld32(tmem_addr(tY, q, grp * 64 + c0), yv);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(y_empty);
 #pragma unroll
-        for (int m = 0; m < 32; ++m) {
-          float v = __uint_as_float(yv[m]);
-          if (p.o_bias != nullptr) v += __ldg(p.o_bias + grp * 64 + c0 + m);
+      for (int m8 = 0; m8 < 4; ++m8) {
+        uint4* at = reinterpret_cast<uint4*>(xsm + grp * 16384 + swz128_offset(row, half * 4 + m8));
+        float f[8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+          float v = __uint_as_float(yv[m8 * 8 + m]);
+          if (p.o_bias != nullptr) v += __ldg(p.o_bias + grp * 64 + c0 + m8 * 8 + m);
           f[m] = v * mval;
         }
         if (p.add_residual) {
+          const uint4 u = *at;
+          const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-          for (int m8 = 0; m8 < 4; ++m8) {
-            const uint4 u = *reinterpret_cast<const uint4*>(xsm + grp * 16384 + swz128_offset(row, (c0 >> 3) + m8));
-            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-              f[m8 * 8 + 2 * m] += bf16_lo(w[m]);
-              f[m8 * 8 + 2 * m + 1] += bf16_hi(w[m]);
-            }
+          for (int m = 0; m < 4; ++m) {
+            f[2 * m] += bf16_lo(w[m]);
+            f[2 * m + 1] += bf16_hi(w[m]);
           }
         }
-        if (row_ok) {
-          __nv_bfloat16* dst = p.out + r * 128 + grp * 64 + c0;
-          st_bf16x16(dst, f);
-          st_bf16x16(dst + 16, f + 16);
-        }
+        *at = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
+                         pack_bf16x2(f[6], f[7]));
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(y_empty);
-        mbar_arrive(&x_empty[xs]);
+      fence_proxy_async_smem();
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + grp * 4 + q) : "memory");
+      if (half == 0 && lane == 0) {
+        // 32 rows x 64 channels in the 128-byte swizzle, as the tile came in; rows past R are clipped
+        if (static_cast<long long>(t) * 128 + q * 32 < p.R)
+          tma_store_2d(&tmOut, xsm + grp * 16384 + q * 4096, grp * 64, t * 128 + q * 32);
+        tma_store_commit();
       }
     }
+    if (half == 0 && lane == 0) tma_store_wait_all<0>();
   }
 
   tc_fence_before_sync();
@@ -341,7 +351,8 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 }
 
 constexpr int kTRSmemBytes =
-    2 * kTRXBytes + 2 * kTRWStage + 2 * kTRHBytes + 4 * kTRMaxHidden * 4 + 256 + 1024;
+    2 * kTRXBytes + 2 * kTRWStage + 4 * kTRMaxHidden * 4 + 4 * 128 * 8 + 256 + 1024;
+static_assert(kTRSmemBytes <= 232448, "shared memory of one CTA");
 
 }  // namespace ubm
 
@@ -353,12 +364,15 @@ extern "C" int ubm_transition(const void* x, const void* wab, const void* wo, co
                               int hidden, int add_residual, void* status, void* stream) {
   using namespace ubm;
   if (R <= 0 || hidden <= 0 || (hidden % 64) || hidden > kTRMaxHidden) return UBM_ERR_ARGUMENT;
-  CUtensorMap tmX, tmWab, tmWo;
+  CUtensorMap tmX, tmWab, tmWo, tmOut;
   {
     uint64_t d[2] = {128, (uint64_t)R};
     uint64_t s[1] = {256};
     uint32_t b[2] = {64, 128};
     int rc = make_tmap(&tmX, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    uint32_t bo[2] = {64, 32};
+    rc = make_tmap(&tmOut, out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, d, s, bo, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
   }
   {
@@ -382,14 +396,13 @@ extern "C" int ubm_transition(const void* x, const void* wab, const void* wo, co
   p.ab_colbias = static_cast<const float*>(ab_colbias);
   p.o_bias = static_cast<const float*>(o_bias);
   p.mask = static_cast<const float*>(mask);
-  p.out = static_cast<__nv_bfloat16*>(out);
   p.add_residual = add_residual;
   p.status = static_cast<KernelStatus*>(status);
   p.num_tiles = static_cast<int>((R + 127) / 128);
   int rc = set_smem(transition_kernel, kTRSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  transition_kernel<<<grid, 320, kTRSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmX, tmWab, tmWo, p);
+  transition_kernel<<<grid, kTRThreads, kTRSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmX, tmWab, tmWo, tmOut, p);
   UBM_CHECK_LAUNCH("transition_kernel");
   return UBM_OK;
 }
