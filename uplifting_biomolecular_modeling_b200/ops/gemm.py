@@ -44,6 +44,20 @@ def pack_swiglu(gate_w: torch.Tensor, value_w: torch.Tensor) -> torch.Tensor:
     return w.reshape(2 * H, K).to(torch.bfloat16).contiguous()
 
 
+def _matrix(t: torch.Tensor, batch: int, M: int, N: int, what: str) -> tuple:
+    """(row stride, batch stride) of an output or residual that has to cover [batch, M, N]: the kernel addresses it by
+    these two numbers alone."""
+    sh, st = t.shape, t.stride()
+    if len(sh) == 2 and batch == 1 and sh[0] >= M and sh[1] >= N:
+        return st[0], 0
+    if len(sh) == 3 and sh[0] >= batch and sh[2] >= N:
+        # one product over rows that a 3-D tensor holds back to back may run on from one entry into the next
+        rows = sh[0] * sh[1] if batch == 1 and st[0] == sh[1] * st[1] else sh[1]
+        if rows >= M:
+            return st[1], st[0]
+    raise ValueError(f"{what} of shape {tuple(sh)} does not hold a [{batch}, {M}, {N}] product")
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Optional[torch.Tensor] = None,
          residual: Optional[torch.Tensor] = None, act: Optional[str] = None, alpha: float = 1.0,
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
@@ -62,7 +76,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
     [(token, channel)] operands lands as [(i, j)][(c, d)] without a permuted copy.  With a batch, entry b starts
     ``c_batch`` elements after entry b - 1 (its elements may lie between the other entries').
 
-    mn_major=False: a [.., M, K], b [.., N, K];  mn_major=True: a [.., K, M], b [.., K, N].
+    mn_major=False: a [M, K], b [N, K];  mn_major=True: a [K, M], b [K, N]; all of them, ``out`` and ``residual``
+    ([M, N] or larger) with one leading batch dimension or without.
     The innermost dimension of a and b must be contiguous; other strides are free as long as
     they are multiples of 8 elements.
     """
@@ -70,6 +85,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         raise TypeError("gemm expects bf16 operands")
     # shapes and strides are read once each and no views are made: this runs in front of every projection of a layer
     sha, sta, shb, stb = a.shape, a.stride(), b.shape, b.stride()
+    if not 2 <= len(sha) <= 3 or not 2 <= len(shb) <= 3:
+        raise ValueError("gemm takes matrices or one batch of them")
     batch = sha[0] if len(sha) == 3 else 1
     if sta[-1] != 1 or stb[-1] != 1:
         raise ValueError("innermost dimension must be contiguous")
@@ -97,18 +114,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         if out is None:
             out = torch.empty((M, n_out) if len(sha) == 2 else (batch, M, n_out),
                               dtype=torch.bfloat16 if n_out != N else out_dtype, device=a.device)
-        sho, sto = out.shape, out.stride()
-        if n_out != N and (sho[-1] != n_out or sho[-2] != M or out.dtype != torch.bfloat16):
+        sho = out.shape
+        if n_out != N and (sho[-1] != n_out or sho[-2:-1] != (M,) or out.dtype != torch.bfloat16):
             raise ValueError(f"{act} output must be bf16 [.., {M}, {n_out}]")
-        if sto[-1] != 1:
+        if out.stride(-1) != 1:
             raise ValueError("output innermost dimension must be contiguous")
-        ldc, stride_c = (sto[1], sto[0]) if len(sho) == 3 else (sto[0], 0)
+        ldc, stride_c = _matrix(out, batch, M, n_out, "output")
     ldr = stride_r = 0
     if residual is not None:
-        str_ = residual.stride()
-        if residual.dtype != torch.bfloat16 or str_[-1] != 1:
+        ldr, stride_r = _matrix(residual, batch, M, N, "residual")
+        if residual.dtype != torch.bfloat16 or residual.stride(-1) != 1:
             raise ValueError("residual must be bf16 with contiguous rows")
-        ldr, stride_r = (str_[1], str_[0]) if len(str_) == 3 else (str_[0], 0)
     if bias is not None and bias.dtype != torch.float32:
         bias = bias.float()
     gate_ptr = ld_gate = gate_rows = 0
@@ -117,7 +133,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         if gate.dtype != torch.bfloat16 or len(shg) != 2 or shg[1] != N or stg[1] != 1 or batch != 1:
             raise ValueError("gate must be bf16 [rows, N] with contiguous rows (batch 1)")
         gate_ptr, ld_gate, gate_rows = gate.data_ptr(), stg[0], shg[0]
-    hi, lo, col = c_blocked if c_blocked is not None else (0, 0, 0)
+    hi, lo, col = (0, 0, 0) if c_blocked is None else map(int, c_blocked)
     dev = a.device
     many = batch > 1
     rc = native.lib().ubm_gemm_bf16_packed(_ARGS.pack(
@@ -125,7 +141,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         0 if residual is None else residual.data_ptr(), M, N, K, batch, sta[-2], stb[-2], ldc, ldr,
         sta[0] if many else 0, stb[0] if many else 0, stride_c if many else 0, stride_r if many else 0,
         1 if mn_major else 0, 1 if out.dtype == torch.float32 else 0, ACT[act], hi, lo, col, gate_ptr, ld_gate,
-        gate_rows, act_from, native.status_tensor(dev).data_ptr(), native.current_stream(dev), alpha))
+        gate_rows, int(act_from), native.status_tensor(dev).data_ptr(), native.current_stream(dev), alpha))
     native.check(rc, "ubm_gemm_bf16_packed")
     return out[0] if len(sha) == 2 and c_blocked is None and out.dim() == 3 else out
 
