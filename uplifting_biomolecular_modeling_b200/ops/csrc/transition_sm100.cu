@@ -145,7 +145,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           tma_load_2d(dst + 16384, &tmWab, &w_full[s], 64, h * 128);
           if (g > 0) load_wo(g - 1, h == 0 ? nch - 1 : h - 1);
           if (*abort_flag) break;
-          if (h == 1 || nch == 1) {
+          if (h == 1) {
             const int tn = t + gridDim.x;
             if (tn < p.num_tiles) load_x(tn, xt++);
           }
@@ -363,7 +363,9 @@ extern "C" int ubm_transition(const void* x, const void* wab, const void* wo, co
                               const void* ab_colbias, const void* o_bias, const void* mask, void* out, long long R,
                               int hidden, int add_residual, void* status, void* stream) {
   using namespace ubm;
-  if (R <= 0 || hidden <= 0 || (hidden % 64) || hidden > kTRMaxHidden) return UBM_ERR_ARGUMENT;
+  // With one chunk per tile the second GEMM of a tile would be issued behind the first GEMM of the tile after next,
+  // whose rows wait for this tile's output: no CTA with three tiles would end.
+  if (R <= 0 || hidden < 128 || (hidden % 64) || hidden > kTRMaxHidden) return UBM_ERR_ARGUMENT;
   CUtensorMap tmX, tmWab, tmWo, tmOut;
   {
     uint64_t d[2] = {128, (uint64_t)R};

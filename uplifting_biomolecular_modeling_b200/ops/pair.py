@@ -16,6 +16,7 @@ from dataclasses import dataclass
 from typing import Optional
 
 import torch
+import torch.nn.functional as F
 
 from . import gemm as _gemm
 from . import native
@@ -67,11 +68,19 @@ class TransitionPacked:
             raise ValueError(f"fused transition supports c=128 and hidden%64==0, <=1024 (got c={c}, hidden={hidden})")
         a, a_sum, a_bias = fold_ln_linear(fc1, norm_w, norm_b)
         b, b_sum, b_bias = fold_ln_linear(fc2, norm_w, norm_b)
+        wo = fc3.detach().to(torch.bfloat16).contiguous()
+        if hidden == 64:
+            # the kernel's pipeline runs two chunks ahead of its output and takes two chunks of 64 or more; a chunk of
+            # zero weights adds silu(0) * 0 = 0
+            hidden = 128
+            a, b = F.pad(a, (0, 0, 0, 64)), F.pad(b, (0, 0, 0, 64))
+            a_sum, b_sum, a_bias, b_bias = (F.pad(t, (0, 64)) for t in (a_sum, b_sum, a_bias, b_bias))
+            wo = F.pad(wo, (0, 64))
         nch = hidden // 64
         wab = torch.stack([a.view(nch, 64, c), b.view(nch, 64, c)], dim=1).reshape(nch * 128, c).contiguous()
         colsum = torch.stack([a_sum.view(nch, 64), b_sum.view(nch, 64)], dim=1).reshape(-1).contiguous()
         colbias = torch.stack([a_bias.view(nch, 64), b_bias.view(nch, 64)], dim=1).reshape(-1).contiguous()
-        return cls(wab, fc3.detach().to(torch.bfloat16).contiguous(), colsum, colbias, hidden)
+        return cls(wab, wo, colsum, colbias, hidden)
 
 
 def transition_fused(x: torch.Tensor, w: TransitionPacked, residual: bool = True,
