@@ -35,3 +35,33 @@ def test_a_mask_that_keeps_everything_changes_nothing():
         pair.attention_d32(q, k, v, None, None, out, 5, 130, 130, 4, mask=mask)
         outs.append(out)
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bool])
+def test_a_mask_on_the_host_or_of_fewer_rows(dtype):
+    from uplifting_biomolecular_modeling_b200.ops import pair
+    keep = (torch.rand(90, 130, generator=torch.Generator().manual_seed(1)) < 0.9).to(dtype)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    want = pair.KeyMask.lay_out(keep.to(dev))
+    got = pair.KeyMask.lay_out(keep, device=dev)
+    assert got.add.device == dev and torch.equal(got.add, want.add) and torch.equal(got.flags, want.flags)
+    got = pair.KeyMask.lay_out(keep[:1], (90, 130), dev)
+    want = pair.KeyMask.lay_out(keep[:1].to(dev).repeat(90, 1))
+    assert torch.equal(got.add, want.add) and torch.equal(got.flags, want.flags)
+    with pytest.raises(ValueError):
+        pair.KeyMask.lay_out(keep)
+
+
+def test_triangle_attention_takes_the_mask_it_took():
+    """A pair mask on the host, and one that broadcasts over the attention rows, give what the expanded mask gives."""
+    from uplifting_biomolecular_modeling_b200.models import pairformer
+    torch.manual_seed(0)
+    n = 70
+    keys = torch.ones(1, 1, n)
+    keys[..., 60:] = 0
+    z = torch.randn(1, n, n, 128, device="cuda").bfloat16()
+    m = pairformer.TriangleAttention(starting=True).cuda().bfloat16().eval().requires_grad_(False)
+    pairformer.set_impl(m, "fused")
+    want = m(z, keys.expand(1, n, n).cuda().contiguous(), residual=True)
+    assert torch.equal(m(z, keys.cuda(), residual=True), want)
+    assert torch.equal(m(z, keys.expand(1, n, n), residual=True), want)

@@ -245,7 +245,7 @@ class TriangleAttention(_Switchable):
         hb[:, :, :N] = (F.linear(n, self.linear.weight.to(n.dtype)).float() * pair.LOG2E).view(N, N, H).permute(2, 0, 1)
         km = None
         if mask is not None:
-            km = pair.KeyMask.lay_out(mask[0] if self.starting else mask[0].t())
+            km = pair.KeyMask.lay_out(mask[0] if self.starting else mask[0].t(), (N, N), z.device)
         o = torch.empty((N * N, HD), dtype=torch.bfloat16, device=z.device)
         pair.attention(qkvg[:, :HD], qkvg[:, HD:2 * HD], qkvg[:, 2 * HD:3 * HD], hb, qkvg[:, 3 * HD:], o, rows=N, Nq=N,
                        Nk=N, H=H, D=w.Dp, ldb=Np, ld_in=4 * HD, ld_gate=4 * HD, mask=km)
@@ -272,7 +272,7 @@ class TriangleAttention(_Switchable):
             from ..ops import pair
             km = None
             if mask is not None:
-                km = pair.KeyMask.lay_out(mask[0] if self.starting else mask[0].t())
+                km = pair.KeyMask.lay_out(mask[0] if self.starting else mask[0].t(), z.shape[1:3], z.device)
             if self._packed is None:
                 self._packed = pair.TriattPacked.pack(self.layer_norm.weight, self.layer_norm.bias,
                                                       self.linear.weight, m.linear_q.weight, m.linear_k.weight,
@@ -346,7 +346,7 @@ class AttentionPairBias(_Switchable):
         if mask is not None:
             km = pair.KeyMask.lay_out(mask if mask.shape[0] == s.shape[0] else
                                       mask.expand(s.shape[0], -1) if mask.shape[0] == 1 else
-                                      mask.repeat_interleave(s.shape[0] // mask.shape[0], 0))
+                                      mask.repeat_interleave(s.shape[0] // mask.shape[0], 0), s.shape[:2], s.device)
         if self._packed is None:
             self._packed = pair.ApbPacked.pack(self.proj_q.weight, self.proj_q.bias, self.proj_k.weight,
                                                self.proj_v.weight, self.proj_g.weight, self.proj_o.weight,

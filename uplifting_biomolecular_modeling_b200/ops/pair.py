@@ -243,9 +243,17 @@ class KeyMask:
         return cls(add, flags)
 
     @classmethod
-    def lay_out(cls, keep: torch.Tensor) -> "KeyMask":
-        """:meth:`pack` of a mask on the GPU as one launch and without the host read: a mask that keeps everything gets
-        clear flags, with which the kernel runs its mask-free loop."""
+    def lay_out(cls, keep: torch.Tensor, shape: Optional[tuple] = None,
+                device: Optional[torch.device] = None) -> "KeyMask":
+        """:meth:`pack` of a mask as one launch and without the host read: a mask that keeps everything gets clear
+        flags, with which the kernel runs its mask-free loop.  ``shape`` = (rows, Nk) that sizes of one broadcast to, ``device`` = the
+        GPU it is wanted on (a mask made on the host is copied there)."""
+        if device is not None and keep.device != device:
+            keep = keep.to(device)
+        if not keep.is_cuda:
+            raise ValueError("a key mask is laid out on a GPU")
+        if shape is not None and 1 in keep.shape:
+            keep = keep.expand(*(to if n == 1 else -1 for n, to in zip(keep.shape, shape)))
         rows, nk = keep.shape
         steps = ceil_to(nk, MASK_STEP) // MASK_STEP
         if keep.dtype not in (torch.float32, torch.bfloat16, torch.bool, torch.uint8):
