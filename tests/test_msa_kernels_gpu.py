@@ -77,3 +77,42 @@ def test_blocked_output_of_a_batch(M, N, batch):
     want = torch.matmul(a.float(), b.float().transpose(1, 2)).view(batch, M, nb, 32).permute(1, 2, 0, 3)
     assert (out[:M].float() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
     assert (out[M] == 7).all()
+
+
+def _averaging(seed):
+    from uplifting_biomolecular_modeling_b200.models import msa, pairformer
+    m = _module(msa.PairWeightedAveraging, seed)
+    pairformer.set_impl(m, "fused")
+    return m
+
+
+def _averaging_exact(m, x, z, mask):
+    d = lambda p: p.detach().double()  # noqa: E731
+    return R.pair_weighted_averaging(x.double(), z.double(), mask.double(), d(m.norm_m.weight), d(m.norm_m.bias),
+                                     d(m.norm_z.weight), d(m.norm_z.bias), d(m.proj_m.weight), d(m.proj_g.weight),
+                                     d(m.proj_z.weight), d(m.proj_o.weight), m.heads)
+
+
+@pytest.mark.parametrize("logit", [-3.0, -9.0, -20.0])
+def test_pair_weighted_averaging_keeps_small_gates(logit):
+    """Gate logits around ``logit``: the gate's error is relative, so the bound is that of any other logits."""
+    m = _averaging(3)
+    m.norm_m.weight.fill_(1.0)                # folded weights are the weights themselves
+    m.norm_m.bias.fill_(0.5)
+    m.proj_g.weight.copy_(torch.randn_like(m.proj_g.weight) * 2.0 ** -6 + logit / 32)
+    x = torch.randn(1, 4, 50, 64, device="cuda").bfloat16()
+    z = torch.randn(1, 50, 50, 128, device="cuda").bfloat16()
+    mask = torch.ones(1, 50, 50, device="cuda")
+    assert _rel(m(x, z, mask), _averaging_exact(m, x, z, mask)) <= 12 * 2.0 ** -9
+
+
+def test_pair_weighted_averaging_of_rows_with_a_large_mean():
+    """Rows 1004 but for one channel of 1008: the mean is 2000 standard deviations.  Besides the bf16 roundings, fp32
+    sums of 64 products of 1004 and a weight below 1/2, divided by the deviation of 1/2: 64 * 2^-24 * 2000 < 2^-7."""
+    m = _averaging(4)
+    x = torch.full((1, 5, 60, 64), 1004.0, device="cuda")
+    x.scatter_(-1, torch.randint(0, 64, (1, 5, 60, 1), device="cuda"), 1008.0)
+    x = x.bfloat16()
+    z = torch.randn(1, 60, 60, 128, device="cuda").bfloat16()
+    mask = torch.ones(1, 60, 60, device="cuda")
+    assert _rel(m(x, z, mask), _averaging_exact(m, x, z, mask)) <= 12 * 2.0 ** -9 + 2.0 ** -7

@@ -20,6 +20,13 @@ constexpr int kPwC = 64;            // channels of m
 constexpr int kPwHC = 256;          // heads x head width
 constexpr int kPwTile = 128 * kPwC * 2;    // one [128 rows][64 channels] operand block, 16 KB
 
+// Variance of a row of 64 from its sum and its sum of squares.  bf16 values of one power of two have 16-bit squares (17
+// across two), so 64 of them add up without rounding in fp32, and the subtraction is one fused operation: what is left
+// of a variance far below the squared mean is exact.  Rows that span more have no such variance.
+__device__ __forceinline__ float row_rstd(float mu, float sumsq, float eps) {
+  return rsqrtf(fmaxf(fmaf(-mu, mu, sumsq * (1.f / kPwC)), 0.f) + eps);
+}
+
 // ------------------------------------------------------------------------------------------ softmax of the weights
 // b: bf16 [H][N][ld] in place, mask: [N][N] (bf16 or fp32; 1 = keep) added as (1 - mask) * -1e6; one warp per row.
 template <typename MT>
@@ -189,7 +196,7 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
       float* st = sStat + par * 256;
       if ((et & 1) == 0) {
         const float mu = sum * (1.f / kPwC);
-        const float rstd = rsqrtf(fmaxf(sumsq * (1.f / kPwC) - mu * mu, 0.f) + p.eps);
+        const float rstd = row_rstd(mu, sumsq, p.eps);
         st[et >> 1] = rstd;
         st[128 + (et >> 1)] = -mu * rstd;
       }
@@ -410,7 +417,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
         }
       }
       const float mu = sum * (1.f / kPwC);
-      const float rstd = rsqrtf(fmaxf(sumsq * (1.f / kPwC) - mu * mu, 0.f) + p.eps);
+      const float rstd = row_rstd(mu, sumsq, p.eps);
       const float2 a2 = make_float2(rstd, rstd), b2 = make_float2(-mu * rstd, -mu * rstd);
       mbar_wait(&g_full[team], ph, ws, 87, team);
       tc_fence_after_sync();
@@ -422,19 +429,28 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
         tmem_ld_wait();
         float f[32];
         ln_fold32(v, a2, b2, sConst + col, sConst + kPwHC + col, f);
+        float low = fminf(f[0], f[1]);
+#pragma unroll
+        for (int k = 2; k < 32; k += 2) low = min3f(low, f[k], f[k + 1]);
         uint8_t* ob = st + (1 + (col >> 6)) * kPwTile;
+        auto apply = [&](auto gate) {
 #pragma unroll
-        for (int j8 = 0; j8 < 4; ++j8) {
-          uint4* at = reinterpret_cast<uint4*>(ob + swz128_offset(row, ((col >> 5) & 1) * 4 + j8));
-          const uint4 u = *at;
-          const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-          uint32_t r[4];
+          for (int j8 = 0; j8 < 4; ++j8) {
+            uint4* at = reinterpret_cast<uint4*>(ob + swz128_offset(row, ((col >> 5) & 1) * 4 + j8));
+            const uint4 u = *at;
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+            uint32_t r[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            r[e] = pack_bf16x2(bf16_lo(w[e]) * sigmoidf_fast(f[j8 * 8 + 2 * e]),
-                               bf16_hi(w[e]) * sigmoidf_fast(f[j8 * 8 + 2 * e + 1]));
-          *at = make_uint4(r[0], r[1], r[2], r[3]);
-        }
+            for (int e = 0; e < 4; ++e)
+              r[e] = pack_bf16x2(bf16_lo(w[e]) * gate(f[j8 * 8 + 2 * e]), bf16_hi(w[e]) * gate(f[j8 * 8 + 2 * e + 1]));
+            *at = make_uint4(r[0], r[1], r[2], r[3]);
+          }
+        };
+        // nearly closed gates take the form that keeps their relative precision (for every gate it costs 27 us more)
+        if (__any_sync(0xffffffffu, low < kSigmoidTail))
+          apply([](float x) { return x < kSigmoidTail ? sigmoidf_rel(x) : sigmoidf_fast(x); });
+        else
+          apply([](float x) { return sigmoidf_fast(x); });
       }
       tc_fence_before_sync();
       fence_proxy_async_smem();
