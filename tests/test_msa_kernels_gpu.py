@@ -116,3 +116,10 @@ def test_pair_weighted_averaging_of_rows_with_a_large_mean():
     z = torch.randn(1, 60, 60, 128, device="cuda").bfloat16()
     mask = torch.ones(1, 60, 60, device="cuda")
     assert _rel(m(x, z, mask), _averaging_exact(m, x, z, mask)) <= 12 * 2.0 ** -9 + 2.0 ** -7
+
+
+def test_pair_weighted_averaging_refuses_a_mask_on_the_host():
+    m = _averaging(5)
+    x, z = torch.randn(1, 2, 20, 64, device="cuda").bfloat16(), torch.randn(1, 20, 20, 128, device="cuda").bfloat16()
+    with pytest.raises((ValueError, RuntimeError)):
+        m(x, z, torch.ones(1, 20, 20))

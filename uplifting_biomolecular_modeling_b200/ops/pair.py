@@ -501,6 +501,8 @@ def pair_weighted_averaging_fused(m: torch.Tensor, b: torch.Tensor, mask: Option
     if m.dtype != torch.bfloat16 or c != 64 or not m.is_contiguous() or b.shape != (8, N, N) or b.stride(0) != N * Np:
         raise ValueError("pair_weighted_averaging_fused expects contiguous bf16 [S, N, 64] and planes of 8 heads")
     dev = m.device
+    if b.device != dev or (mask is not None and mask.device != dev):
+        raise ValueError("pair_weighted_averaging_fused: rows, bias planes and mask live on one GPU")
     if mask is not None and mask.dtype != torch.bfloat16:
         mask = mask.float()
     mk = None if mask is None else mask.expand(N, N).contiguous()
