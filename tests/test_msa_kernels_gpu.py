@@ -123,3 +123,29 @@ def test_pair_weighted_averaging_refuses_a_mask_on_the_host():
     x, z = torch.randn(1, 2, 20, 64, device="cuda").bfloat16(), torch.randn(1, 20, 20, 128, device="cuda").bfloat16()
     with pytest.raises((ValueError, RuntimeError)):
         m(x, z, torch.ones(1, 20, 20))
+
+
+def test_pair_weighted_averaging_weights_count_however_written():
+    m = _averaging(6)
+    x, z = torch.randn(1, 3, 40, 64, device="cuda").bfloat16(), torch.randn(1, 40, 40, 128, device="cuda").bfloat16()
+    mask = torch.ones(1, 40, 40, device="cuda")
+    m(x, z, mask)
+    for p in (m.norm_m.weight, m.norm_m.bias, m.proj_m.weight, m.proj_g.weight, m.proj_o.weight):
+        p.data.mul_(0.5)                      # in place, without a new version of the parameter
+        assert _rel(m(x, z, mask), _averaging_exact(m, x, z, mask)) <= 12 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_folded_weights_of_pair_weighted_averaging(dtype):
+    from uplifting_biomolecular_modeling_b200.ops import pair
+    g = torch.Generator(device="cuda").manual_seed(7)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)  # noqa: E731
+    wm, wg, wo, nw, nb = r(256, 64), r(256, 64), r(64, 256), r(64), r(64)
+    for gamma, beta in ((nw, nb), (nw, None), (None, None)):
+        p = pair.PwaPacked.pack(gamma, beta, wm, wg, wo, 1e-5)
+        for w, (got, colsum, colbias) in ((wm, (p.wv, p.v_colsum, p.v_colbias)), (wg, (p.wg, p.g_colsum, p.g_colbias))):
+            want = pair.fold_ln_linear(w, gamma, beta)
+            assert torch.equal(got, want[0])
+            # sums of 64 fp32 values in another order
+            assert (colsum - want[1]).abs().max() <= 64 * 2.0 ** -24 * want[0].float().abs().sum(1).max()
+            assert (colbias - want[2]).abs().max() <= 64 * 2.0 ** -24 * 64 * w.float().abs().max() * nb.float().abs().max()

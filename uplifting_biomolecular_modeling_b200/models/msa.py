@@ -110,12 +110,10 @@ class PairWeightedAveraging(_Switchable):
         B, S, N, _ = m.shape
         H, c = self.heads, self.c_h
         if m.shape[-1] == 64 and (H, c) == (8, 32):
-            params = (self.norm_m.weight, self.norm_m.bias, self.proj_m.weight, self.proj_g.weight, self.proj_o.weight)
-            ver = tuple((p._version, p.data_ptr()) for p in params)
-            if self._packed is None or self._packed[0] != ver:       # weights written since the last call count
-                self._packed = (ver, pair.PwaPacked.pack(*params, self.norm_m.eps))
+            w = pair.PwaPacked.pack(self.norm_m.weight, self.norm_m.bias, self.proj_m.weight, self.proj_g.weight,
+                                    self.proj_o.weight, self.norm_m.eps)
             b = rows.pair_head_bias(z[0].contiguous(), self.norm_z.weight, self.norm_z.bias, self.proj_z.weight)
-            return pair.pair_weighted_averaging_fused(m[0].contiguous(), b, mask[0], self._packed[1]).unsqueeze(0)
+            return pair.pair_weighted_averaging_fused(m[0].contiguous(), b, mask[0], w).unsqueeze(0)
         mn = rows.layernorm_rows(m.contiguous(), self.norm_m.weight, self.norm_m.bias, self.norm_m.eps)
         b = rows.pair_head_bias(z[0].contiguous(), self.norm_z.weight, self.norm_z.bias, self.proj_z.weight).float()
         b = b + ((1.0 - mask[0].float()) * -1e6)[None]

@@ -1,7 +1,8 @@
 // Pair-weighted averaging of the MSA track (c_m = 64, 8 heads of 32): out[s][i] = W_o ( sigmoid(W_g n) * o ),
 // o[s][i][h] = sum_j softmax_j(b_h[i][j]) (W_m n)[s][j][h],  n = LayerNorm(m), b = W_z LayerNorm(z).
 //
-// Four launches around the batched GEMM (the softmax input comes from pair_head_bias_kernel):
+// Five launches around the batched GEMM (the softmax input comes from pair_head_bias_kernel):
+//   pwa_pack_kernel      LayerNorm folded into the two projections of m
 //   pwa_softmax_kernel   weights w[h][i][j], in place over the bias planes
 //   pwa_value_kernel     v[h][(s, c)][j]: the K-major operand of the contraction, straight from the rows of m
 //   (gemm)               o[i][s][(h, c)] = w[h] v[h]^T, stored token-major by the epilogue's blocked output
@@ -25,6 +26,36 @@ constexpr int kPwTile = 128 * kPwC * 2;    // one [128 rows][64 channels] operan
 // of a variance far below the squared mean is exact.  Rows that span more have no such variance.
 __device__ __forceinline__ float row_rstd(float mu, float sumsq, float eps) {
   return rsqrtf(fmaxf(fmaf(-mu, mu, sumsq * (1.f / kPwC)), 0.f) + eps);
+}
+
+// ------------------------------------------------------------------------------------------ weights
+// LayerNorm folded into the value and gate projections: w' = bf16(w gamma), its row sums and w beta.  On every call: it
+// reads 64 KB and takes about 3 us, and a weight written by any route counts.  One warp per output channel.
+__device__ __forceinline__ float param(const void* p, int fp32, int i) {
+  return fp32 ? static_cast<const float*>(p)[i] : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
+}
+__global__ void __launch_bounds__(256) pwa_pack_kernel(const void* __restrict__ wv, int wv_fp32,
+                                                       const void* __restrict__ wg, int wg_fp32,
+                                                       const void* __restrict__ gamma, int gamma_fp32,
+                                                       const void* __restrict__ beta, int beta_fp32,
+                                                       __nv_bfloat16* __restrict__ w, float* __restrict__ consts) {
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;     // 0 .. 511: values, then gates
+  const int ch = row & (kPwHC - 1), gate = row / kPwHC;
+  float sum = 0.f, bias = 0.f;
+#pragma unroll
+  for (int k = lane; k < kPwC; k += 32) {
+    const float v = gate ? param(wg, wg_fp32, ch * kPwC + k) : param(wv, wv_fp32, ch * kPwC + k);
+    const __nv_bfloat16 r = __float2bfloat16(gamma == nullptr ? v : v * param(gamma, gamma_fp32, k));
+    w[row * kPwC + k] = r;
+    sum += __bfloat162float(r);
+    if (beta != nullptr) bias += v * param(beta, beta_fp32, k);
+  }
+  sum = warp_sum(sum);
+  bias = warp_sum(bias);
+  if (lane == 0) {
+    consts[gate * 2 * kPwHC + ch] = sum;
+    consts[(gate * 2 + 1) * kPwHC + ch] = bias;
+  }
 }
 
 // ------------------------------------------------------------------------------------------ softmax of the weights
@@ -495,6 +526,19 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
 }
 
 }  // namespace ubm
+
+// wv, wg: [256][64], gamma, beta: [64] or null, each bf16 (its flag 0) or fp32 (1); w: bf16 [2][256][64];
+// consts: fp32 [4][256] = row sums and biases of the values, row sums and biases of the gates
+extern "C" int ubm_pwa_pack(const void* wv, int wv_fp32, const void* wg, int wg_fp32, const void* gamma, int gamma_fp32,
+                            const void* beta, int beta_fp32, void* w, void* consts, void* stream) {
+  using namespace ubm;
+  if (wv == nullptr || wg == nullptr || w == nullptr || consts == nullptr) return UBM_ERR_ARGUMENT;
+  pwa_pack_kernel<<<2 * kPwHC / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      wv, wv_fp32, wg, wg_fp32, gamma, gamma_fp32, beta, beta_fp32, static_cast<__nv_bfloat16*>(w),
+      static_cast<float*>(consts));
+  UBM_CHECK_LAUNCH("pwa_pack_kernel");
+  return UBM_OK;
+}
 
 // b: bf16 [H][N][ld] in place; mask: [N][N] fp32 (mask_bf16 = 0) or bf16 (1), or null
 extern "C" int ubm_pwa_softmax(void* b, const void* mask, int mask_bf16, int H, int N, int ld, void* stream) {

@@ -468,6 +468,7 @@ def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, r
 
 
 # ------------------------------------------------------------------------------------------
+native.declare("ubm_pwa_pack", [c_void_p, c_int] * 4 + [c_void_p] * 3)
 native.declare("ubm_pwa_softmax", [c_void_p] * 2 + [c_int] * 4 + [c_void_p])
 native.declare("ubm_pwa_value", [c_void_p] * 5 + [c_int] * 3 + [c_float] + [c_void_p] * 2)
 native.declare("ubm_pwa_out", [c_void_p] * 7 + [c_int] * 2 + [c_float] + [c_void_p] * 2)
@@ -486,10 +487,26 @@ class PwaPacked:
 
     @classmethod
     def pack(cls, norm_w, norm_b, w_m, w_g, w_o, eps: float) -> "PwaPacked":
-        if w_m.shape != (256, 64) or w_o.shape != (64, 256):
+        """Folded weights as they are now, in one launch.  Parameters bf16 or fp32; norm_w / norm_b may be None."""
+        if w_m.shape != (256, 64) or w_g.shape != (256, 64) or w_o.shape != (64, 256) or \
+                any(t is not None and t.shape != (64,) for t in (norm_w, norm_b)):
             raise ValueError("fused pair-weighted averaging supports c_m = 64 and 8 heads of 32")
-        return cls(*fold_ln_linear(w_m, norm_w, norm_b), *fold_ln_linear(w_g, norm_w, norm_b),
-                   w_o.detach().to(torch.bfloat16).contiguous(), float(eps))
+        dev = w_m.device
+        args, held = [], []                   # held: converted copies live until the launch is queued
+        for t in (w_m, w_g, norm_w, norm_b):
+            if t is not None:
+                if t.device != dev:
+                    raise ValueError("fused pair-weighted averaging: parameters on several devices")
+                t = t.detach().contiguous()
+                if t.dtype not in (torch.bfloat16, torch.float32):
+                    t = t.float()
+                held.append(t)
+            args += [native.ptr(t), 1 if t is not None and t.dtype == torch.float32 else 0]
+        w = torch.empty((2, 256, 64), dtype=torch.bfloat16, device=dev)
+        c = torch.empty((4, 256), dtype=torch.float32, device=dev)
+        native.check(native.lib().ubm_pwa_pack(*args, native.ptr(w), native.ptr(c), native.current_stream(dev)),
+                     "ubm_pwa_pack")
+        return cls(w[0], c[0], c[1], w[1], c[2], c[3], w_o.detach().to(torch.bfloat16).contiguous(), float(eps))
 
 
 def pair_weighted_averaging_fused(m: torch.Tensor, b: torch.Tensor, mask: Optional[torch.Tensor],
