@@ -149,3 +149,44 @@ def test_folded_weights_of_pair_weighted_averaging(dtype):
             # sums of 64 fp32 values in another order
             assert (colsum - want[1]).abs().max() <= 64 * 2.0 ** -24 * want[0].float().abs().sum(1).max()
             assert (colbias - want[2]).abs().max() <= 64 * 2.0 ** -24 * 64 * w.float().abs().max() * nb.float().abs().max()
+
+
+@pytest.mark.parametrize("name", ["proj_m", "proj_g", "proj_o"])
+def test_projections_of_pair_weighted_averaging_are_called(name):
+    """A hook on a projection, and another module in its place, take part in the call; gradients are recorded."""
+    m = _averaging(8)
+    x, z = torch.randn(1, 3, 40, 64, device="cuda").bfloat16(), torch.randn(1, 40, 40, 128, device="cuda").bfloat16()
+    mask = torch.ones(1, 40, 40, device="cuda")
+    lin = getattr(m, name)
+    handle = lin.register_forward_hook(lambda mod, args, y: y * 2)
+    hooked = m(x, z, mask)
+    handle.remove()
+    setattr(m, name, torch.nn.Sequential(lin))
+    replaced = m(x, z, mask)
+    setattr(m, name, lin)
+    plain = m(x, z, mask)
+    assert _rel(replaced, plain.double()) <= 12 * 2.0 ** -9
+    lin.weight.data.mul_(2)                   # what the hook did
+    assert _rel(hooked, m(x, z, mask).double()) <= 12 * 2.0 ** -9
+    assert _rel(hooked, plain.double()) > 0.1
+    if name != "proj_m":                      # its product is an operand of a kernel that records nothing
+        lin.weight.requires_grad_(True)
+        m(x, z, mask).float().sum().backward()
+        assert lin.weight.grad is not None and lin.weight.grad.abs().sum() > 0
+
+
+@pytest.mark.parametrize("name", ["proj_a", "proj_b"])
+def test_projections_of_the_outer_product_mean_are_called(name):
+    from uplifting_biomolecular_modeling_b200.models import msa, pairformer
+    m = _module(msa.OuterProductMean, 9)
+    pairformer.set_impl(m, "fused")
+    x = torch.randn(1, 6, 40, 64, device="cuda").bfloat16()
+    mask = torch.ones(1, 6, 40, device="cuda")
+    lin = getattr(m, name)
+    plain = m(x, mask)
+    handle = lin.register_forward_hook(lambda mod, args, y: y * 0)
+    # nothing is left but the bias, rounded to bf16 in the kernel's output
+    assert torch.equal(m(x, mask), m.proj_o.bias.expand_as(plain))
+    handle.remove()
+    setattr(m, name, torch.nn.Sequential(lin))
+    assert _rel(m(x, mask), plain.double()) <= 8 * 2.0 ** -9

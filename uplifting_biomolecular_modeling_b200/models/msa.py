@@ -15,10 +15,9 @@ from typing import Optional
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
 from ..ops import reference as R
-from .pairformer import PairformerLayer, Transition, _Switchable
+from .pairformer import PairformerLayer, Transition, _Switchable, plain_linears
 
 
 class OuterProductMean(_Switchable):
@@ -45,16 +44,18 @@ class OuterProductMean(_Switchable):
         n = rows.layernorm_rows(m.contiguous(), self.norm.weight, self.norm.bias, self.norm.eps)
         # [S, N, c] seen as [S, N*c]: sequences (the contraction) along rows, (token, channel) contiguous - the
         # operand form of the MN-major GEMM, so no [N*c, S] transposed copies are made
-        wab = torch.cat([self.proj_a.weight, self.proj_b.weight], 0).to(torch.bfloat16)
-        if c == 32 and n.shape[-1] % 8 == 0:
+        if c == 32 and n.shape[-1] % 8 == 0 and plain_linears(self.proj_a, self.proj_b):
             # both projections from one product, its two 32-wide column blocks stored apart
+            wab = torch.cat([self.proj_a.weight, self.proj_b.weight], 0)
             ab = torch.empty((2, S * N, c), dtype=torch.bfloat16, device=m.device)
             gemm.gemm(n.view(S * N, -1), wab, out=ab, c_blocked=(32 * c, c, S * N * c))
+            if not self.full_mask:
+                ab *= mask.reshape(1, S * N, 1).to(ab.dtype)
+            a2, b2 = ab[0].view(S, N * c), ab[1].view(S, N * c)
         else:
-            ab = F.linear(n.view(S * N, -1), wab).view(S * N, 2, c).transpose(0, 1).contiguous()
-        if not self.full_mask:
-            ab *= mask.reshape(1, S * N, 1).to(ab.dtype)
-        a2, b2 = ab[0].view(S, N * c), ab[1].view(S, N * c)
+            mk = mask.unsqueeze(-1).to(n.dtype)
+            a2 = (self.proj_a(n) * mk)[0].reshape(S, N * c)
+            b2 = (self.proj_b(n) * mk)[0].reshape(S, N * c)
         wo = self.proj_o.weight.to(torch.bfloat16).contiguous()
         bo = self.proj_o.bias.float()
         out = torch.empty((N, N, wo.shape[0]), dtype=torch.bfloat16, device=m.device)
@@ -109,7 +110,7 @@ class PairWeightedAveraging(_Switchable):
         from ..ops import gemm, pair, rows
         B, S, N, _ = m.shape
         H, c = self.heads, self.c_h
-        if m.shape[-1] == 64 and (H, c) == (8, 32):
+        if m.shape[-1] == 64 and (H, c) == (8, 32) and plain_linears(self.proj_m, self.proj_g, self.proj_o):
             w = pair.PwaPacked.pack(self.norm_m.weight, self.norm_m.bias, self.proj_m.weight, self.proj_g.weight,
                                     self.proj_o.weight, self.norm_m.eps)
             b = rows.pair_head_bias(z[0].contiguous(), self.norm_z.weight, self.norm_z.bias, self.proj_z.weight)

@@ -15,6 +15,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook as _any_global_hook
 
 from ..ops import reference as R
 
@@ -60,6 +61,16 @@ class _Switchable(nn.Module):
 
     def _fusable(self, z: torch.Tensor) -> bool:
         return (self.impl == "fused" and z.is_cuda and z.dtype == torch.bfloat16 and z.shape[-1] == 128)
+
+
+def plain_linears(*modules: nn.Module) -> bool:
+    """True where calling each of ``modules`` is one product with its bf16 weight and nothing else, so that a kernel may
+    read the weights instead: no other module in its place, no bias, no hook, no gradient to record."""
+    record = torch.is_grad_enabled()
+    return not _any_global_hook() and all(
+        type(m) is nn.Linear and m.bias is None and m.weight.dtype == torch.bfloat16 and "forward" not in m.__dict__ and
+        not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) and
+        not (record and m.weight.requires_grad) for m in modules)
 
 
 class Transition(_Switchable):
