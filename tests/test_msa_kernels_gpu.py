@@ -190,3 +190,12 @@ def test_projections_of_the_outer_product_mean_are_called(name):
     handle.remove()
     setattr(m, name, torch.nn.Sequential(lin))
     assert _rel(m(x, mask), plain.double()) <= 8 * 2.0 ** -9
+
+
+def test_outer_product_mean_with_a_mask_that_broadcasts_over_tokens():
+    from uplifting_biomolecular_modeling_b200.models import msa, pairformer
+    m = _module(msa.OuterProductMean, 10)
+    pairformer.set_impl(m, "fused")
+    x = torch.randn(1, 6, 40, 64, device="cuda").bfloat16()
+    rows = (torch.arange(6, device="cuda") < 4).float().view(1, 6, 1)
+    assert torch.equal(m(x, rows), m(x, rows.expand(1, 6, 40).contiguous()))

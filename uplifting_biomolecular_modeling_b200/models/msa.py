@@ -50,7 +50,7 @@ class OuterProductMean(_Switchable):
             ab = torch.empty((2, S * N, c), dtype=torch.bfloat16, device=m.device)
             gemm.gemm(n.view(S * N, -1), wab, out=ab, c_blocked=(32 * c, c, S * N * c))
             if not self.full_mask:
-                ab *= mask.reshape(1, S * N, 1).to(ab.dtype)
+                ab *= mask.expand(1, S, N).reshape(1, S * N, 1).to(ab.dtype)
             a2, b2 = ab[0].view(S, N * c), ab[1].view(S, N * c)
         else:
             mk = mask.unsqueeze(-1).to(n.dtype)
