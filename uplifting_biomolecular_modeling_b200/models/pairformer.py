@@ -430,7 +430,8 @@ class PairformerLayer(nn.Module):
         s32 = s.float()
         norm = self.pre_norm_s
         if self.attention.impl == "fused" and s.is_cuda and self.attention.proj_q.weight.dtype == torch.bfloat16 \
-                and s.shape[-1] % 8 == 0 and s.shape[-1] <= 1024:
+                and s.shape[-1] % 8 == 0 and s.shape[-1] <= 1024 and not torch.is_autocast_enabled("cuda") \
+                and not (torch.is_grad_enabled() and (s.requires_grad or norm.weight.requires_grad)):
             # normalised in fp32 and rounded once to the projection's type, in one launch
             from ..ops import rows
             upd = self.attention(rows.layernorm_rows(s32.contiguous(), norm.weight, norm.bias, 1e-5, torch.bfloat16), z,
