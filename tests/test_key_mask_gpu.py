@@ -65,3 +65,26 @@ def test_triangle_attention_takes_the_mask_it_took():
     want = m(z, keys.expand(1, n, n).cuda().contiguous(), residual=True)
     assert torch.equal(m(z, keys.cuda(), residual=True), want)
     assert torch.equal(m(z, keys.expand(1, n, n), residual=True), want)
+
+
+@pytest.mark.parametrize("rows,N,D,variant", [(1, 128, 32, 0), (3, 128, 32, 0), (5, 128, 32, 0x10), (5, 192, 64, 0x10),
+                                              (3, 200, 32, 0), (5, 200, 32, 0), (5, 128, 32, 0), (5, 200, 64, 0)])
+def test_a_row_without_keys_is_finite(rows, N, D, variant, request):
+    """The first row keeps no key.  No key count or form gives it a NaN (which would travel on through P.V of a later
+    attention over these rows); it is 0, give or take the 2^-125 that is the smallest polynomial exponential, except where
+    whole key steps leave those the only weights.  The other rows do not notice it."""
+    from uplifting_biomolecular_modeling_b200.ops import pair
+    pair.set_attention_variant(variant)
+    request.addfinalizer(lambda: pair.set_attention_variant(0))
+    q, k, v = (torch.randn(rows, N, 4 * D, device="cuda").bfloat16() for _ in range(3))
+    keep = torch.rand(rows, N, device="cuda") < 0.9
+    outs = []
+    for some in (0.0, 1.0):
+        keep[0] = bool(some)
+        out = torch.empty_like(q)
+        pair.attention(q, k, v, None, None, out, rows, N, N, 4, D, mask=pair.KeyMask.lay_out(keep))
+        outs.append(out)
+    assert outs[0].isfinite().all() and torch.equal(outs[0][1:], outs[1][1:])
+    poly = variant == 0 and (D == 64 or rows >= 4)
+    if not poly or N % 64:
+        assert outs[0][0].abs().max() <= 2.0 ** -100
