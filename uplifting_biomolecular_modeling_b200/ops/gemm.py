@@ -44,10 +44,9 @@ def pack_swiglu(gate_w: torch.Tensor, value_w: torch.Tensor) -> torch.Tensor:
     return w.reshape(2 * H, K).to(torch.bfloat16).contiguous()
 
 
-def _matrix(t: torch.Tensor, batch: int, M: int, N: int, what: str) -> tuple:
-    """(row stride, batch stride) of an output or residual that has to cover [batch, M, N]: the kernel addresses it by
-    these two numbers alone."""
-    sh, st = t.shape, t.stride()
+def _matrix(sh, st, batch: int, M: int, N: int, what: str) -> tuple:
+    """(row stride, batch stride) of an output or residual of shape ``sh`` and strides ``st`` that has to cover
+    [batch, M, N]: the kernel addresses it by these two numbers alone."""
     if len(sh) == 2 and batch == 1 and sh[0] >= M and sh[1] >= N:
         return st[0], 0
     if len(sh) == 3 and sh[0] >= batch and sh[2] >= N:
@@ -85,13 +84,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         raise TypeError("gemm expects bf16 operands")
     # shapes and strides are read once each and no views are made: this runs in front of every projection of a layer
     sha, sta, shb, stb = a.shape, a.stride(), b.shape, b.stride()
-    if not 2 <= len(sha) <= 3 or not 2 <= len(shb) <= 3:
+    da, db = len(sha), len(shb)
+    if da == 2 and db == 2:
+        batch = 1
+    elif 2 <= da <= 3 and 2 <= db <= 3:
+        batch = sha[0] if da == 3 else 1
+        if (shb[0] if db == 3 else 1) != batch:
+            raise ValueError("batch mismatch")
+    else:
         raise ValueError("gemm takes matrices or one batch of them")
-    batch = sha[0] if len(sha) == 3 else 1
     if sta[-1] != 1 or stb[-1] != 1:
         raise ValueError("innermost dimension must be contiguous")
-    if (shb[0] if len(shb) == 3 else 1) != batch:
-        raise ValueError("batch mismatch")
     if mn_major:
         K, M = sha[-2:]
         kb, N = shb[-2:]
@@ -112,19 +115,22 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
                 raise ValueError(f"{act} needs a K-major product with N % {group} == 0 and no bias / gate / residual")
             n_out = N // 3 if act == "swiglu3" else N // 2
         if out is None:
-            out = torch.empty((M, n_out) if len(sha) == 2 else (batch, M, n_out),
+            out = torch.empty((M, n_out) if da == 2 else (batch, M, n_out),
                               dtype=torch.bfloat16 if n_out != N else out_dtype, device=a.device)
-        sho = out.shape
-        if n_out != N and (sho[-1] != n_out or sho[-2:-1] != (M,) or out.dtype != torch.bfloat16):
-            raise ValueError(f"{act} output must be bf16 [.., {M}, {n_out}]")
-        if out.stride(-1) != 1:
-            raise ValueError("output innermost dimension must be contiguous")
-        ldc, stride_c = _matrix(out, batch, M, n_out, "output")
+            ldc, stride_c = n_out, M * n_out
+        else:
+            sho, sto = out.shape, out.stride()
+            if n_out != N and (sho[-1] != n_out or sho[-2:-1] != (M,) or out.dtype != torch.bfloat16):
+                raise ValueError(f"{act} output must be bf16 [.., {M}, {n_out}]")
+            if sto[-1] != 1:
+                raise ValueError("output innermost dimension must be contiguous")
+            ldc, stride_c = _matrix(sho, sto, batch, M, n_out, "output")
     ldr = stride_r = 0
     if residual is not None:
-        ldr, stride_r = _matrix(residual, batch, M, N, "residual")
-        if residual.dtype != torch.bfloat16 or residual.stride(-1) != 1:
+        str_ = residual.stride()
+        if residual.dtype != torch.bfloat16 or str_[-1] != 1:
             raise ValueError("residual must be bf16 with contiguous rows")
+        ldr, stride_r = _matrix(residual.shape, str_, batch, M, N, "residual")
     if bias is not None and bias.dtype != torch.float32:
         bias = bias.float()
     gate_ptr = ld_gate = gate_rows = 0
@@ -143,7 +149,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
         1 if mn_major else 0, 1 if out.dtype == torch.float32 else 0, ACT[act], hi, lo, col, gate_ptr, ld_gate,
         gate_rows, int(act_from), native.status_tensor(dev).data_ptr(), native.current_stream(dev), alpha))
     native.check(rc, "ubm_gemm_bf16_packed")
-    return out[0] if len(sha) == 2 and c_blocked is None and out.dim() == 3 else out
+    return out[0] if da == 2 and c_blocked is None and out.dim() == 3 else out
 
 
 _E4M3 = (torch.uint8, torch.float8_e4m3fn)
