@@ -180,12 +180,14 @@ class HyenaOperator(nn.Module):
         return y + u * self.D.to(u.dtype)
 
     def _lam(self) -> torch.Tensor:
-        """exp(log_poles) in fp32, kept until the parameter is written again (three launches per decode step)."""
-        ent = self._lam_cache
-        if ent is None or ent[0] != self.log_poles._version or ent[1].device != self.log_poles.device:
-            ent = (self.log_poles._version, torch.exp(self.log_poles.detach().float()).contiguous())
-            self._lam_cache = ent
-        return ent[1]
+        """exp(log_poles) in fp32, kept until the parameter is written again (three launches per decode step) or given
+        other storage (a sharded or converted copy swaps ``.data``, which leaves the version as it is; the entry holds
+        the storage it was made from, so that no other can have its address)."""
+        ent, p = self._lam_cache, self.log_poles
+        if ent is None or ent[0] != p._version or ent[1].data_ptr() != p.data_ptr() or ent[1].shape != p.shape:
+            src = p.detach()
+            ent = self._lam_cache = (p._version, src, torch.exp(src.float()).contiguous())
+        return ent[2]
 
     def _kernel_taps(self):
         if self._taps is None:
