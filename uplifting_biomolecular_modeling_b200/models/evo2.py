@@ -195,11 +195,16 @@ class HyenaOperator(nn.Module):
             self._taps = (seq.taps_major(self.fir), None if self.kind == "hcl" else seq.taps_major(self.h))
         return self._taps
 
+    def _scans(self, u) -> bool:
+        """Whether the kernel path runs this operator as the recurrence: up to 16 poles in registers, sequences in a grid
+        dimension.  Everything else takes the transform."""
+        return self.kind == "hcl" and self.log_poles.shape[1] <= 16 and u.shape[0] <= 65535
+
     def _fused_inner(self, u, x2, state: Optional[dict] = None):
         """x2 * (conv(u) + D u) with the gate folded into the convolution's epilogue.  The recurrence form of the long
         operator ends with the pole state, which goes into ``state``."""
         from ..ops import seq
-        if self.kind == "hcl" and self.log_poles.shape[1] <= 16:
+        if self._scans(u):
             gated, poles = seq.pole_conv_gate(u, self._lam(), self.residues, self.D, x2)
             if state is not None:
                 state["poles"] = poles
@@ -236,7 +241,7 @@ class HyenaOperator(nn.Module):
             state["fir_tail"] = _last(z, K - 1)
             if self.kind in ("hcs", "hcm"):
                 state["inner_tail"] = _last(u, self.h.shape[1] - 1)
-            elif not (fused and self.log_poles.shape[1] <= 16):                   # else set by the scan above
+            elif not (fused and self._scans(u)):                                  # else set by the scan above
                 lam = torch.exp(self.log_poles.float())                           # [d, S]
                 L = u.shape[1]
                 w = lam.unsqueeze(0) ** torch.arange(L - 1, -1, -1, device=u.device, dtype=torch.float32).view(L, 1, 1)

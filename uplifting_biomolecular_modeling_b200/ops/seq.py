@@ -150,8 +150,8 @@ def fir_inner_gate(u: torch.Tensor, ht: torch.Tensor, D: torch.Tensor, x2: Optio
     t = None if tail is None else _bf16c(tail)
     Df = _f32(D)
     # one Toeplitz product per channel from 65 taps on (below, the multiply-adds it spends on zero taps outweigh the
-    # tensor cores); its accesses are 16 bytes wide
-    if taps_bf16 and t is None and 64 < K <= 128 and L >= 64 and d % 8 == 0 and u.data_ptr() % 16 == 0 and \
+    # tensor cores); its accesses are 16 bytes wide and a batch entry is one layer of the grid
+    if taps_bf16 and t is None and 64 < K <= 128 and L >= 64 and B <= 65535 and d % 8 == 0 and u.data_ptr() % 16 == 0 and \
             (x2c is None or x2c.data_ptr() % 16 == 0):
         rc = native.lib().ubm_fir_toeplitz(native.ptr(u), native.ptr(ht), native.ptr(Df), native.ptr(x2c),
                                            native.ptr(out), B, L, d, K, _stream(u))
@@ -212,6 +212,8 @@ def pole_conv_gate(u: torch.Tensor, lam: torch.Tensor, res: torch.Tensor, D: tor
     B, L, d = u.shape
     lamf, resf, Df = _f32(lam), _f32(res), _f32(D)
     S = lamf.shape[1]
+    if lamf.shape != (d, S) or resf.shape != (d, S) or Df.numel() != d or (x2 is not None and x2.numel() != u.numel()):
+        raise ValueError(f"pole_conv_gate: poles, residues and skip of {d} channels and a gate like u are needed")
     chunk = _pole_chunk(B, L, d)
     part = torch.empty((B, (L + chunk - 1) // chunk, d, S), dtype=torch.float32, device=u.device)
     state = torch.empty((B, d, S), dtype=torch.float32, device=u.device)
