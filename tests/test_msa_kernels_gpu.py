@@ -199,3 +199,36 @@ def test_outer_product_mean_with_a_mask_that_broadcasts_over_tokens():
     x = torch.randn(1, 6, 40, 64, device="cuda").bfloat16()
     rows = (torch.arange(6, device="cuda") < 4).float().view(1, 6, 1)
     assert torch.equal(m(x, rows), m(x, rows.expand(1, 6, 40).contiguous()))
+
+
+@pytest.mark.parametrize("S,N", [(700, 129), (1000, 40)])
+def test_pair_weighted_averaging_with_many_tiles_per_cta(S, N):
+    """1400 and 1000 tiles of 128 tokens: both teams of the output stage, every buffer, ring slot and phase of the two
+    persistent kernels come round several times, with a ragged last tile in each sequence."""
+    from uplifting_biomolecular_modeling_b200.ops import native
+    m = _averaging(S)
+    x = torch.randn(1, S, N, 64, device="cuda").bfloat16()
+    z = torch.randn(1, N, N, 128, device="cuda").bfloat16()
+    mask = torch.ones(1, N, N, device="cuda")
+    mask[:, :, N - 3:] = 0
+    got, again = m(x, z, mask), m(x, z, mask)
+    native.raise_on_status("cuda", "pair-weighted averaging")
+    assert torch.equal(got, again)
+    want = _averaging_exact(m, x, z, mask)
+    assert _rel(got, want) <= 12 * 2.0 ** -9
+    # row by row, so that one wrong tile shows: a row's 64 values share the roundings above
+    assert ((got.double() - want).norm(dim=-1) <= 0.1 * want.norm(dim=-1) + 0.02 * want.norm(dim=-1).mean()).all()
+
+
+def test_blocked_output_of_a_batch_with_many_tiles():
+    """At least 384 output tiles: several per CTA, so that the staging of the stores is reused."""
+    from uplifting_biomolecular_modeling_b200.ops import gemm
+    batch, M, N = 8, 3003, 320
+    a = torch.randn(batch, M, 72, device="cuda").bfloat16()
+    b = torch.randn(batch, N, 72, device="cuda").bfloat16()
+    nb = N // 32
+    out = torch.full((M + 1, nb, batch, 32), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm.gemm(a, b, out=out, c_blocked=(32 * nb * batch * 32, nb * batch * 32, batch * 32), c_batch=32)
+    want = torch.matmul(a.float(), b.float().transpose(1, 2)).view(batch, M, nb, 32).permute(1, 2, 0, 3)
+    assert (out[:M].float() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+    assert (out[M] == 7).all()
