@@ -44,18 +44,11 @@ class OuterProductMean(_Switchable):
         n = rows.layernorm_rows(m.contiguous(), self.norm.weight, self.norm.bias, self.norm.eps)
         # [S, N, c] seen as [S, N*c]: sequences (the contraction) along rows, (token, channel) contiguous - the
         # operand form of the MN-major GEMM, so no [N*c, S] transposed copies are made
-        if c == 32 and n.shape[-1] % 8 == 0 and plain_linears(self.proj_a, self.proj_b):
-            # both projections from one product, its two 32-wide column blocks stored apart
-            wab = torch.cat([self.proj_a.weight, self.proj_b.weight], 0)
-            ab = torch.empty((2, S * N, c), dtype=torch.bfloat16, device=m.device)
-            gemm.gemm(n.view(S * N, -1), wab, out=ab, c_blocked=(32 * c, c, S * N * c))
-            if not self.full_mask:
-                ab *= mask.expand(1, S, N).reshape(1, S * N, 1).to(ab.dtype)
-            a2, b2 = ab[0].view(S, N * c), ab[1].view(S, N * c)
-        else:
+        a, b = self.proj_a(n), self.proj_b(n)
+        if not self.full_mask:
             mk = mask.unsqueeze(-1).to(n.dtype)
-            a2 = (self.proj_a(n) * mk)[0].reshape(S, N * c)
-            b2 = (self.proj_b(n) * mk)[0].reshape(S, N * c)
+            a, b = a * mk, b * mk
+        a2, b2 = a[0].reshape(S, N * c), b[0].reshape(S, N * c)
         wo = self.proj_o.weight.to(torch.bfloat16).contiguous()
         bo = self.proj_o.bias.float()
         out = torch.empty((N, N, wo.shape[0]), dtype=torch.bfloat16, device=m.device)
