@@ -210,7 +210,7 @@ LEVERS: Dict[str, Lever] = {l.name: l for l in [
           apply=_fused(_kinds_triatt, "fused_triatt")),
     Lever("fused_apb", "F1.kernel_fusion", "attention_sm100@1", needs_gpu=True, apply=_fused(_kinds_apb, "fused_apb")),
     Lever("fused_opm", "F1.kernel_fusion", "gemm_sm100@1", needs_gpu=True, apply=_fused(_kinds_opm, "fused_opm")),
-    Lever("fused_pwa", "F1.kernel_fusion", "gemm_sm100@1", needs_gpu=True, apply=_fused(_kinds_pwa, "fused_pwa")),
+    Lever("fused_pwa", "F1.kernel_fusion", "pwa+gemm_sm100@1", needs_gpu=True, apply=_fused(_kinds_pwa, "fused_pwa")),
     Lever("fused_dit", "F1.kernel_fusion", "attention_d64+rows_sm100@1", needs_gpu=True,
           apply=_fused(_kinds_dit, "fused_dit")),
     Lever("sampler_graph", "F2.graph_capture", "api.Predictor._step_fn", needs_gpu=True, apply=_flag("use_graphs", True, "The sampler step is captured once per shape in a CUDA graph and replayed for every "

@@ -25,7 +25,7 @@ LEVERS: Dict[str, Tuple[str, str, Tuple[str, ...]]] = {
     # keys from another sequence (cross attention) are outside the kernel's call classes by declaration
     "fused_apb": ("attention_sm100@1", "apb", ("cross_keys",)),
     "fused_opm": ("gemm_sm100@1", "opm", ()),
-    "fused_pwa": ("gemm_sm100@1", "pwa", ()),
+    "fused_pwa": ("pwa+gemm_sm100@1", "pwa", ()),
     "fused_dit": ("attention_d64+rows_sm100@1", "apb", ()),
 }
 
