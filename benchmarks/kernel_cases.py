@@ -6,8 +6,9 @@ Cases: ``attention`` (triangle-attention core, H=4 x D=32, rows = N), ``attentio
 16 heads x 64, 5 samples), ``trimul_proj``, ``trimul_gemm``, ``trimul_out``, ``triatt_proj``, ``transition``,
 ``out_gemm`` (the [N*N,128] x [128,128] output projection with residual), ``trimul`` (three launches),
 ``triatt`` (three launches), ``causal_attention`` (--n tokens, --heads, head dimension 128; --lib 1 = the
-library call), ``gemm_rows`` (--m --k --nn: a row GEMM with bias), ``gemv_rows`` (--m <= 8 rows, --k, --nn, --form), ``decode_attention`` (--n cached keys, --heads), ``fir_inner_gate`` (--n positions, --k channels, --nn taps), ``window_attention`` (--m atoms,
-5 samples, 4 heads x 32).  Inputs are larger than L2 for N >= 768.  Prints one line per case with the
+library call), ``gemm_rows`` (--m --k --nn: a row GEMM with bias), ``gemv_rows`` (--m <= 8 rows, --k, --nn, --form), ``decode_attention`` (--n cached keys, --heads), ``fir_inner_gate`` (--n positions, --k channels, --nn taps), ``pole_conv`` (the same
+with --nn poles), ``qk_norm_rotary`` (--m tokens, --k channels), ``head_bias`` (--heads planes), ``pair_averaging`` (--m sequences),
+``window_attention`` (--m atoms, 5 samples, 4 heads x 32).  Inputs are larger than L2 for N >= 768.  Prints one line per case with the
 mean time, the algorithmic bytes and FLOPs, and the fractions of the measured peaks in MEASURED_PEAKS.json
 (fallback 6.65 TB/s, 1.59 PFLOP/s when the file is absent).
 """
@@ -60,10 +61,10 @@ def main():
     ap.add_argument("--m", type=int, default=7680, help="rows of the gemm_rows case / atoms of window_attention")
     ap.add_argument("--k", type=int, default=768)
     ap.add_argument("--nn", type=int, default=3072)
-    ap.add_argument("--heads", type=int, default=32, help="causal_attention: heads")
+    ap.add_argument("--heads", type=int, default=32, help="causal_attention, decode_attention, head_bias: heads")
     ap.add_argument("--lib", type=int, default=0, help="causal_attention: 1 = time the library attention instead")
     ap.add_argument("--masked", type=int, default=0, help="attention: 1 = key mask with a padded tail of a tenth of the keys")
-    ap.add_argument("--form", default="plain", help="gemv_rows: plain | norm (RMSNorm in front) | res (residual behind) | swiglu (RMSNorm + two matrices); gemm_rows: fp8 = e4m3 operands")
+    ap.add_argument("--form", default="plain", help="gemv_rows: plain | norm (RMSNorm in front) | res (residual behind) | swiglu (RMSNorm + two matrices); gemm_rows: fp8 = e4m3 operands; fir_inner_gate: fp32 = fp32 taps")
     ap.add_argument("--incoming", type=int, default=0, help="trimul / trimul_gemm: 1 = the incoming update (MN-major contraction)")
     a = ap.parse_args()
     N, c = a.n, 128
@@ -72,7 +73,7 @@ def main():
     torch.manual_seed(0)
     r = lambda *s: torch.randn(*s, device=dev) * 0.08  # noqa: E731
     ones, zeros = torch.ones(c, device=dev), torch.zeros(c, device=dev)
-    z = torch.randn(N, N, c, device=dev).bfloat16() if a.case not in ("causal_attention", "gemm_rows", "gemv_rows", "decode_attention", "fir_inner_gate") else None
+    z = torch.randn(N, N, c, device=dev).bfloat16() if a.case not in ("causal_attention", "gemm_rows", "gemv_rows", "decode_attention", "fir_inner_gate", "pole_conv", "qk_norm_rotary") else None
     Np = pair.ceil_to(N, 8)
     st = native.status_tensor(dev)
     stream = native.current_stream(dev)
@@ -178,16 +179,52 @@ def main():
         fn = lambda: seq.gemv_rows(x, wt, **kw)  # noqa: E731
         byts, flops = wt.numel() * 2 * (2 if a.form == "swiglu" else 1), 2.0 * M * K * NN
     elif a.case == "fir_inner_gate":
-        # inner operator of a Hyena layer over --n positions x --k channels with --nn taps (128 = the medium filter:
-        # the tiled direct convolution), gate included
+        # inner operator of a Hyena layer over --n positions x --k channels with --nn taps, gate included.  Taps are a bf16
+        # parameter as in a bf16 model (65 to 128 of them, the medium filter, run as Toeplitz products);
+        # --form fp32 = fp32 taps, which stay on the multiply-add kernels
         from uplifting_biomolecular_modeling_b200.ops import seq
         Lp, ch, taps = N, a.k, a.nn
         u = torch.randn(1, Lp, ch, device=dev).bfloat16()
         x2 = torch.randn(1, Lp, ch, device=dev).bfloat16()
-        ht = seq.taps_major(torch.randn(ch, taps, device=dev) * taps ** -0.5)
+        h = torch.randn(ch, taps, device=dev) * taps ** -0.5
+        ht = seq.taps_major(h if a.form == "fp32" else h.bfloat16())
         Dv = torch.randn(ch, device=dev)
-        fn = lambda: seq.fir_inner_gate(u, ht, Dv, x2, None)  # noqa: E731
+        fn = lambda: seq.fir_inner_gate(u, ht, Dv, x2, None, taps_bf16=a.form != "fp32")  # noqa: E731
         byts, flops = 3 * u.numel() * 2, 2.0 * Lp * ch * taps
+    elif a.case == "pole_conv":
+        # long operator of a Hyena layer over --n positions x --k channels with --nn poles, gate and final state included
+        from uplifting_biomolecular_modeling_b200.ops import seq
+        Lp, ch, S = N, a.k, a.nn
+        u = torch.randn(1, Lp, ch, device=dev).bfloat16()
+        x2 = torch.randn(1, Lp, ch, device=dev).bfloat16()
+        lam, res = torch.rand(ch, S, device=dev) * 0.5 + 0.45, torch.randn(ch, S, device=dev) / S
+        Dv = torch.randn(ch, device=dev)
+        fn = lambda: seq.pole_conv_gate(u, lam, res, Dv, x2)  # noqa: E731
+        byts, flops = 3 * u.numel() * 2, 6.0 * Lp * ch * S
+    elif a.case == "qk_norm_rotary":
+        # LayerNorm and rotary embedding of q and k in place: --m tokens x --k channels in heads of 64
+        from uplifting_biomolecular_modeling_b200.ops import seq
+        qkv = torch.randn(a.m, 3 * a.k, device=dev).bfloat16()
+        pos = torch.arange(a.m, device=dev, dtype=torch.int32) % 2048
+        gq, gk = torch.ones(a.k, device=dev), torch.ones(a.k, device=dev)
+        fn = lambda: seq.qk_norm_rotary_(qkv, pos, gq, gk, a.k // 64, 64)  # noqa: E731
+        byts, flops = 4 * a.m * a.k * 2, 20.0 * a.m * a.k
+    elif a.case == "head_bias":
+        # LayerNorm and projection of the pair tensor to --heads bias planes
+        from uplifting_biomolecular_modeling_b200.ops import rows
+        wb = r(a.heads, c)
+        fn = lambda: rows.pair_head_bias(z, ones, zeros, wb)  # noqa: E731
+        byts, flops = z.numel() * 2 + a.heads * N * Np * 2, 2.0 * N * N * c * a.heads
+    elif a.case == "pair_averaging":
+        # pair-weighted averaging of --m sequences x --n tokens (all launches of the operator)
+        from uplifting_biomolecular_modeling_b200.models import msa
+        mod = msa.PairWeightedAveraging().to(dev).bfloat16().eval().requires_grad_(False)
+        mod.impl = "fused"
+        x = torch.randn(1, a.m, N, 64, device=dev).bfloat16()
+        mask = torch.ones(1, N, N, device=dev, dtype=torch.bfloat16)
+        fn = lambda: mod(x, z[None], mask)  # noqa: E731
+        byts = 2 * x.numel() * 2 + N * N * 130 * 2
+        flops = 2.0 * a.m * N * 64 * 768 + 2.0 * N * N * 128 * 8 + 2.0 * a.m * N * N * 256
     elif a.case == "decode_attention":
         # one new token against a cache of --n keys (--heads heads of 128): rotary + cache write, split-key pass, merge
         from uplifting_biomolecular_modeling_b200.ops import seq

@@ -167,15 +167,6 @@ constexpr int kTpW = (kTpPos + kTpHalo) / 2 + 2;      // 32-bit words per channe
 constexpr int kTpTapW = 84;                           // words per channel of one tap copy (168 taps)
 constexpr int kTpSmem = kTpCh * kTpW * 4 + 2 * kTpCh * kTpTapW * 4;
 
-__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                          uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 __global__ void __launch_bounds__(kTpThreads, 2) fir_toeplitz_kernel(const __nv_bfloat16* __restrict__ u,
                                                                      const float* __restrict__ ht, int K,
                                                                      const float* __restrict__ D,
@@ -264,7 +255,7 @@ __global__ void __launch_bounds__(kTpThreads, 2) fir_toeplitz_kernel(const __nv_
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const uint2 bv = *reinterpret_cast<const uint2*>(row + kTpHalo / 2 + 8 * (8 * q + g - m) + 2 * t);
-        mma_16816(acc[q], ax[2 * m], ax[2 * m + 1], ay[2 * m], ay[2 * m + 1], bv.x, bv.y);
+        mma_bf16_16816(acc[q], ax[2 * m], ax[2 * m + 1], ay[2 * m], ay[2 * m + 1], bv.x, bv.y);
       }
     }
     __syncwarp();

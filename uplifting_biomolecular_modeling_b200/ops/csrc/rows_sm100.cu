@@ -198,15 +198,6 @@ __global__ void __launch_bounds__(256) layernorm_rows_narrow_kernel(const __nv_b
 // A warp takes 32 rows.  The k index is permuted so that a lane's fragments of two products are one 16-byte load, the
 // four lanes of a row reading 64 consecutive bytes; the row statistics come from the same registers.  Results go
 // through shared memory so that a plane is written 64 or 128 consecutive bytes at a time.
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint2 b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
-}
-
 constexpr int kHbRows = 128;            // rows per CTA and iteration: four warps of 32
 constexpr int kHbLd = kHbRows + 2;      // staging row of a head, in elements
 
@@ -282,8 +273,8 @@ __global__ void __launch_bounds__(128) pair_head_bias_kernel(const __nv_bfloat16
           const uint2 b0 = sw[nt][k][2 * c][lane], b1 = sw[nt][k][2 * c + 1][lane];
 #pragma unroll
           for (int m = 0; m < 2; ++m) {
-            mma_bf16_16816(acc[m][nt], x[m][0][c].x, x[m][1][c].x, x[m][0][c].y, x[m][1][c].y, b0);
-            mma_bf16_16816(acc[m][nt], x[m][0][c].z, x[m][1][c].z, x[m][0][c].w, x[m][1][c].w, b1);
+            mma_bf16_16816(acc[m][nt], x[m][0][c].x, x[m][1][c].x, x[m][0][c].y, x[m][1][c].y, b0.x, b0.y);
+            mma_bf16_16816(acc[m][nt], x[m][0][c].z, x[m][1][c].z, x[m][0][c].w, x[m][1][c].w, b1.x, b1.y);
           }
         }
 #pragma unroll
