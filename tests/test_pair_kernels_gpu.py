@@ -294,7 +294,7 @@ def test_segment_mean_and_gather_rows():
 @pytest.mark.parametrize("H", [4, 16, 32])
 @pytest.mark.parametrize("transpose", [False, True])
 def test_pair_head_bias_planes(N, H, transpose):
-    """LN(z) -> H head-bias planes, several pair rows per thread (vector stores when 4 rows share a plane row)."""
+    """LN(z) -> H head-bias planes: row counts around the 128 rows of a CTA, even and odd plane rows, both layouts."""
     from uplifting_biomolecular_modeling_b200.ops import rows
     g = torch.Generator(device="cuda").manual_seed(N + H)
     z = (torch.randn(N, N, 128, device="cuda", generator=g) * 1.5 + 0.3).bfloat16()

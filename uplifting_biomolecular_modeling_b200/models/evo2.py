@@ -9,7 +9,7 @@ short (7-tap FIR), medium (128-tap FIR) and long (implicit, pole/residue) Hyena 
 kernels for the same pieces: evo2/opt/evo2_opt/kit/base.py:55 ``_fir3_kernel``, :160 ``_hcs7_kernel_s``,
 :219/:242 FFT-convolution epilogues, gen/hyenafuse for the decode-step state update).
 
-Prefill runs the medium operator as a direct convolution and the long one as its recurrence over chunks; decoding keeps per-layer state (FIR
+Prefill runs the medium operator as one Toeplitz product per channel and the long one as its recurrence over chunks; decoding keeps per-layer state (FIR
 tails, pole states, attention KV cache) and advances one token per step.  Tensor parallelism shards
 the channel dimension of every operator (``parallel.tp``): column-parallel input projections, row-parallel
 output projections whose reduce-scatter is done by the GEMM epilogue over peer memory.  The causal attention
@@ -210,8 +210,8 @@ class HyenaOperator(nn.Module):
                 state["poles"] = poles
             return gated
         if self.kind in ("hcs", "hcm") and self.h.shape[1] <= 512:
-            # short filters from a register window, the medium filter (128 taps) as a tiled direct convolution:
-            # 17 G multiply-adds per operator at the 7B shape against three FFT-sized fp32 passes
+            # short filters from a register window; the medium filter (128 taps) as Toeplitz products on the tensor cores
+            # where its taps are a bf16 parameter, as a tiled direct convolution where they are fp32
             return seq.fir_inner_gate(u, self._kernel_taps()[1], self.D, x2, taps_bf16=self.h.dtype == torch.bfloat16)
         Hf, n = self.filter_spectrum(u.shape[1])
         X = torch.fft.rfft(seq.fft_pad_transpose(u, n))          # channel-major fp32, zero-padded to the transform size

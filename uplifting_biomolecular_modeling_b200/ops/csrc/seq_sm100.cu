@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(256) fir_step_kernel(const __nv_bfloat16* __re
 
 // Inner operator of hcs / hcm: out = x2 * (fir(u, h) + D * u).  Short filters keep the window in registers, two channels
 // per thread and kFgBatch positions requested together as in fir_gate3_kernel;
-// longer ones (the 128-tap medium filter) re-read the inputs through L1/L2 (generic kernel below).
+// longer ones take the kernels below, or, with bf16 taps and no tail, the Toeplitz products of hyena_sm100.cu.
 template <int K>
 __global__ void __launch_bounds__(128) fir_inner_gate_kernel(const __nv_bfloat16* __restrict__ u,
                                                              const float* __restrict__ ht,   // [K][d]
@@ -488,9 +488,9 @@ __global__ void __launch_bounds__(128) fir_inner_gate_long_kernel(const __nv_bfl
   }
 }
 
-// The same operator for filters of tens to hundreds of taps over a long sequence (the 128-tap medium filter of a
-// prefill), as a direct convolution on the FMA pipes: 17 G multiply-adds per operator at the 7B shape, against
-// three FFT-sized passes over fp32 copies of the sequence.  A CTA owns 32 channels x 512 positions: the input
+// The same operator for filters of tens to hundreds of fp32 taps over a long sequence (and bf16 ones outside the 65 to
+// 128 taps of the Toeplitz form), as a direct convolution on the FMA pipes: 17 G multiply-adds per operator at 8192
+// positions x 4096 channels x 128 taps, against three FFT-sized passes over fp32 copies of the sequence.  A CTA owns 32 channels x 512 positions: the input
 // tile with its halo (bf16) and the taps (fp32, zero-padded to a multiple of 16) sit in shared memory; a thread
 // owns one channel and runs of 16 positions with 16 accumulators, and walks the taps 16 at a time over a
 // 31-value register window (out[p] += h[kb + q] * W[p - q + 15], all indices static), so one shared-memory load
@@ -776,7 +776,8 @@ __global__ void __launch_bounds__(256) rotary_split_qkv_kernel(const __nv_bfloat
 // LayerNorm over the whole q row and over the whole k row of a fused projection [T][3][H][Dh], each followed by the
 // rotary embedding of its heads, in place; one warp per token, the row read once and kept packed in registers.  A lane
 // holds 8-channel chunks 256 channels apart, so with Dh dividing 256 all its chunks sit at one place of their heads and
-// share four (cos, sin) pairs.  Bound by memory: two row reads and two row writes where the separate steps (slices made
+// share four (cos, sin) pairs.  Two row reads and two row writes (DRAM a third busy, issue slots 60 %, at 32768 tokens x 960
+// channels) where the separate steps (slices made
 // contiguous, normalised, written back, then rotated and split into three tensors) made eighteen: 40 us against 247 us
 // at 16376 tokens x 960 channels.
 template <int CHUNKS>

@@ -14,7 +14,7 @@
 // Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = four epilogue groups of 32 output channels each.
 // TMEM: {O, G} x two tiles = 512 columns.  Sixteen epilogue warps instead of eight, the statistics of the x columns
 // taken two columns per lane from whole 128-byte rows (one thread per column read 128 two-byte values), and the output
-// staged over the residual in the z tile: 202 us at 1021 tokens against 265 us.
+// staged over the residual in the z tile: 202 us at 1021 tokens against 265 us (issue slots 55 %, DRAM 45 % busy at 768).
 #include "host_util.h"
 #include "sm100.cuh"
 
