@@ -147,7 +147,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           tma_load_2d(dst + 16384, &tmWab, &w_full[s], 64, h * 128);
           if (g > 0) load_wo(g - 1, h == 0 ? nch - 1 : h - 1);
           if (*abort_flag) break;
-          if (h == 1) {
+          if (h == 1 || nch == 1) {   // nch >= 2; without the second term: 1.452 against 1.440 ms at 1536 tokens
             const int tn = t + gridDim.x;
             if (tn < p.num_tiles) load_x(tn, xt++);
           }
