@@ -135,20 +135,25 @@ def test_pair_weighted_averaging_weights_count_however_written():
         assert _rel(m(x, z, mask), _averaging_exact(m, x, z, mask)) <= 12 * 2.0 ** -9
 
 
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-def test_folded_weights_of_pair_weighted_averaging(dtype):
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("norm", ["weight and bias", "weight", "neither"])
+def test_parameters_of_pair_weighted_averaging(dtype, norm):
+    """Parameter types other than the module's, weights in other strides, a LayerNorm without a bias or without either."""
     from uplifting_biomolecular_modeling_b200.ops import pair
     g = torch.Generator(device="cuda").manual_seed(7)
-    r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)  # noqa: E731
-    wm, wg, wo, nw, nb = r(256, 64), r(256, 64), r(64, 256), r(64), r(64)
-    for gamma, beta in ((nw, nb), (nw, None), (None, None)):
-        p = pair.PwaPacked.pack(gamma, beta, wm, wg, wo, 1e-5)
-        for w, (got, colsum, colbias) in ((wm, (p.wv, p.v_colsum, p.v_colbias)), (wg, (p.wg, p.g_colsum, p.g_colbias))):
-            want = pair.fold_ln_linear(w, gamma, beta)
-            assert torch.equal(got, want[0])
-            # sums of 64 fp32 values in another order
-            assert (colsum - want[1]).abs().max() <= 64 * 2.0 ** -24 * want[0].float().abs().sum(1).max()
-            assert (colbias - want[2]).abs().max() <= 64 * 2.0 ** -24 * 64 * w.float().abs().max() * nb.float().abs().max()
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    S, N = 5, 72
+    wm, wg, wo = (r(64, 256) / 8).to(dtype).t(), (r(256, 64) / 8).to(dtype), (r(64, 256) / 16).to(dtype)
+    nw, nb = (1 + 0.2 * r(64)).to(dtype), (0.2 * r(64)).to(dtype)
+    nw, nb = nw if norm != "neither" else None, nb if norm == "weight and bias" else None
+    m, planes = r(S, N, 64).bfloat16(), r(8, N, N).bfloat16()
+    w = torch.softmax(planes.double(), -1)
+    d = lambda t: None if t is None else t.double()  # noqa: E731
+    n = torch.nn.functional.layer_norm(m.double(), (64,), d(nw), d(nb), 1e-5)
+    o = torch.einsum("hij,sjhc->sihc", w, (n @ d(wm).t()).view(S, N, 8, 32)).reshape(S, N, 256)
+    want = (torch.sigmoid(n @ d(wg).t()) * o) @ d(wo).t()
+    got = pair.pair_weighted_averaging_fused(m, planes.clone(), None, pair.PwaPacked.pack(nw, nb, wm, wg, wo, 1e-5))
+    assert _rel(got, want) <= 12 * 2.0 ** -9
 
 
 @pytest.mark.parametrize("name", ["proj_m", "proj_g", "proj_o"])

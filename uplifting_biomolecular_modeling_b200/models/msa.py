@@ -104,8 +104,9 @@ class PairWeightedAveraging(_Switchable):
         B, S, N, _ = m.shape
         H, c = self.heads, self.c_h
         if m.shape[-1] == 64 and (H, c) == (8, 32) and plain_linears(self.proj_m, self.proj_g, self.proj_o):
-            w = pair.PwaPacked.pack(self.norm_m.weight, self.norm_m.bias, self.proj_m.weight, self.proj_g.weight,
-                                    self.proj_o.weight, self.norm_m.eps)
+            norm = self.norm_m
+            w = pair.PwaPacked.pack(norm.weight, norm.bias, self.proj_m.weight, self.proj_g.weight, self.proj_o.weight,
+                                    norm.eps)
             b = rows.pair_head_bias(z[0].contiguous(), self.norm_z.weight, self.norm_z.bias, self.proj_z.weight)
             return pair.pair_weighted_averaging_fused(m[0].contiguous(), b, mask[0], w).unsqueeze(0)
         mn = rows.layernorm_rows(m.contiguous(), self.norm_m.weight, self.norm_m.bias, self.norm_m.eps)

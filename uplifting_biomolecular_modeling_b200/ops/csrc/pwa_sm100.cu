@@ -530,7 +530,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
 
 // wv, wg: [256][64], gamma, beta: [64] or null, each bf16 (its flag 0) or fp32 (1); w: bf16 [2][256][64];
 // consts: fp32 [4][256] = row sums and biases of the values, row sums and biases of the gates
-extern "C" int ubm_pwa_pack(const void* wv, int wv_fp32, const void* wg, int wg_fp32, const void* gamma, int gamma_fp32,
+static int pwa_pack(const void* wv, int wv_fp32, const void* wg, int wg_fp32, const void* gamma, int gamma_fp32,
                             const void* beta, int beta_fp32, void* w, void* consts, void* stream) {
   using namespace ubm;
   if (wv == nullptr || wg == nullptr || w == nullptr || consts == nullptr) return UBM_ERR_ARGUMENT;
@@ -542,7 +542,7 @@ extern "C" int ubm_pwa_pack(const void* wv, int wv_fp32, const void* wg, int wg_
 }
 
 // b: bf16 [H][N][ld] in place; mask: [N][N] fp32 (mask_bf16 = 0) or bf16 (1), or null
-extern "C" int ubm_pwa_softmax(void* b, const void* mask, int mask_bf16, int H, int N, int ld, void* stream) {
+static int pwa_softmax(void* b, const void* mask, int mask_bf16, int H, int N, int ld, void* stream) {
   using namespace ubm;
   if (H <= 0 || N <= 0 || ld < N) return UBM_ERR_ARGUMENT;
   const long long rows = static_cast<long long>(H) * N;
@@ -559,7 +559,7 @@ extern "C" int ubm_pwa_softmax(void* b, const void* mask, int mask_bf16, int H, 
 }
 
 // m: bf16 [S][N][64]; w: bf16 [256][64] (gamma folded); colsum / colbias: fp32 [256]; v: bf16 [8][S * 32][Np]
-extern "C" int ubm_pwa_value(const void* m, const void* w, const void* colsum, const void* colbias, void* v, int S,
+static int pwa_value(const void* m, const void* w, const void* colsum, const void* colbias, void* v, int S,
                              int N, int Np, float eps, void* status, void* stream) {
   using namespace ubm;
   if (S <= 0 || N <= 0 || Np < N || (Np & 7)) return UBM_ERR_ARGUMENT;
@@ -597,7 +597,7 @@ extern "C" int ubm_pwa_value(const void* m, const void* w, const void* colsum, c
 }
 
 // m, out: bf16 [S][N][64]; o: bf16 [N][S][256]; wg: bf16 [256][64] (gamma folded); wo: bf16 [64][256]
-extern "C" int ubm_pwa_out(const void* m, const void* o, const void* wg, const void* g_colsum, const void* g_colbias,
+static int pwa_out(const void* m, const void* o, const void* wg, const void* g_colsum, const void* g_colbias,
                            const void* wo, void* out, int S, int N, float eps, void* status, void* stream) {
   using namespace ubm;
   if (S <= 0 || N <= 0) return UBM_ERR_ARGUMENT;
@@ -638,4 +638,37 @@ extern "C" int ubm_pwa_out(const void* m, const void* o, const void* wg, const v
   pwa_out_kernel<<<grid, kPoThreads, kPoSmem, static_cast<cudaStream_t>(stream)>>>(tmM, tmO, tmWg, tmWo, tmOut, p);
   UBM_CHECK_LAUNCH("pwa_out_kernel");
   return UBM_OK;
+}
+
+extern "C" int ubm_gemm_bf16_ex(const void* A, const void* B, void* C, const void* bias, const void* residual, int M,
+                                int N, int K, int batch, long long lda, long long ldb, long long ldc, long long ldr,
+                                long long strideA, long long strideB, long long strideC, long long strideR,
+                                int mn_major, int out_fp32, int act, float alpha, long long cblk_hi,
+                                long long cblk_lo, long long cblk_col, const void* gate, long long ld_gate,
+                                int gate_rows, int act_col0, void* status, void* stream);
+
+// The whole operator behind the bias planes, from one call (five separate ones cost a foreign-function caller 17 us more).
+// m, out: bf16 [S][N][64]; b: bf16 [8][N][Np] planes, overwritten; mask: [N][N] bf16 or fp32 (mask_bf16), or null; wv, wg,
+// gamma, beta with their flags as for the folding above; wo: bf16 [64][256]; scratch: fold, 69632 bytes; v, bf16
+// [8][S * 32][Np]; o, bf16 [N][S][256].
+extern "C" int ubm_pair_weighted_averaging(const void* m, void* b, const void* mask, int mask_bf16, const void* wv,
+                                           int wv_fp32, const void* wg, int wg_fp32, const void* gamma, int gamma_fp32,
+                                           const void* beta, int beta_fp32, const void* wo, void* fold, void* v, void* o,
+                                           void* out, int S, int N, int Np, float eps, void* status, void* stream) {
+  using namespace ubm;
+  if (S <= 0 || N <= 0 || S > 0x7fffffff / 32) return UBM_ERR_ARGUMENT;
+  constexpr int kW = kPwHC * kPwC * 2;
+  uint8_t* w = static_cast<uint8_t*>(fold);
+  float* c = reinterpret_cast<float*>(w + 2 * kW);
+  int rc = pwa_pack(wv, wv_fp32, wg, wg_fp32, gamma, gamma_fp32, beta, beta_fp32, w, c, stream);
+  if (rc == UBM_OK) rc = pwa_softmax(b, mask, mask_bf16, 8, N, Np, stream);
+  if (rc == UBM_OK) rc = pwa_value(m, w, c, c + kPwHC, v, S, N, Np, eps, status, stream);
+  if (rc == UBM_OK) {
+    const long long row = static_cast<long long>(S) * kPwHC;       // a token of o; entry (head) h starts 32 h further on
+    rc = ubm_gemm_bf16_ex(b, v, o, nullptr, nullptr, N, S * 32, N, 8, Np, Np, 0, 0, static_cast<long long>(N) * Np,
+                          static_cast<long long>(S) * 32 * Np, 32, 0, 0, 0, 0, 1.0f, 32 * row, row, kPwHC, nullptr, 0, 0, 0,
+                          status, stream);
+  }
+  if (rc == UBM_OK) rc = pwa_out(m, o, w + kW, c + 2 * kPwHC, c + 3 * kPwHC, wo, out, S, N, eps, status, stream);
+  return rc;
 }

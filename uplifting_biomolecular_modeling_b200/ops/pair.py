@@ -468,45 +468,39 @@ def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, r
 
 
 # ------------------------------------------------------------------------------------------
-native.declare("ubm_pwa_pack", [c_void_p, c_int] * 4 + [c_void_p] * 3)
-native.declare("ubm_pwa_softmax", [c_void_p] * 2 + [c_int] * 4 + [c_void_p])
-native.declare("ubm_pwa_value", [c_void_p] * 5 + [c_int] * 3 + [c_float] + [c_void_p] * 2)
-native.declare("ubm_pwa_out", [c_void_p] * 7 + [c_int] * 2 + [c_float] + [c_void_p] * 2)
+native.declare("ubm_pair_weighted_averaging", [c_void_p] * 3 + [c_int] + [c_void_p, c_int] * 4 + [c_void_p] * 5 +
+               [c_int] * 3 + [c_float] + [c_void_p] * 2)
 
 
 @dataclass
 class PwaPacked:
-    wv: torch.Tensor         # bf16 [256, 64], gamma folded
-    v_colsum: torch.Tensor   # fp32 [256]
-    v_colbias: torch.Tensor
-    wg: torch.Tensor         # bf16 [256, 64], gamma folded
-    g_colsum: torch.Tensor
-    g_colbias: torch.Tensor
+    """Parameters of a pair-weighted averaging as the kernels take them.  Nothing is folded ahead: each call folds the
+    LayerNorm into the two projections (one launch over 64 KB), so a weight written by any route counts."""
+    args: tuple              # address and fp32 flag of the value and gate projections and the LayerNorm's weight and bias
+    held: tuple              # the tensors behind the addresses
     wo: torch.Tensor         # bf16 [64, 256]
     eps: float
 
     @classmethod
     def pack(cls, norm_w, norm_b, w_m, w_g, w_o, eps: float) -> "PwaPacked":
-        """Folded weights as they are now, in one launch.  Parameters bf16 or fp32; norm_w / norm_b may be None."""
-        if w_m.shape != (256, 64) or w_g.shape != (256, 64) or w_o.shape != (64, 256) or \
-                any(t is not None and t.shape != (64,) for t in (norm_w, norm_b)):
+        """Parameters bf16 or fp32 (others are converted); norm_w / norm_b may be None."""
+        if w_m.shape != (256, 64) or w_g.shape != (256, 64) or w_o.shape != (64, 256):
             raise ValueError("fused pair-weighted averaging supports c_m = 64 and 8 heads of 32")
-        dev = w_m.device
-        args, held = [], []                   # held: converted copies live until the launch is queued
+        dev, args, held = w_m.device, [], []
         for t in (w_m, w_g, norm_w, norm_b):
-            if t is not None:
-                if t.device != dev:
-                    raise ValueError("fused pair-weighted averaging: parameters on several devices")
-                t = t.detach().contiguous()
-                if t.dtype not in (torch.bfloat16, torch.float32):
-                    t = t.float()
-                held.append(t)
-            args += [native.ptr(t), 1 if t is not None and t.dtype == torch.float32 else 0]
-        w = torch.empty((2, 256, 64), dtype=torch.bfloat16, device=dev)
-        c = torch.empty((4, 256), dtype=torch.float32, device=dev)
-        native.check(native.lib().ubm_pwa_pack(*args, native.ptr(w), native.ptr(c), native.current_stream(dev)),
-                     "ubm_pwa_pack")
-        return cls(w[0], c[0], c[1], w[1], c[2], c[3], w_o.detach().to(torch.bfloat16).contiguous(), float(eps))
+            if t is None:
+                args += (0, 0)
+                continue
+            if t.device != dev or t.shape[-1] != 64:
+                raise ValueError("fused pair-weighted averaging: parameters of one device and 64 channels")
+            fp32 = t.dtype != torch.bfloat16
+            if fp32 or not t.is_contiguous():
+                t = t.detach().to(torch.float32 if fp32 else t.dtype).contiguous()
+            held.append(t)
+            args += (t.data_ptr(), 1 if fp32 else 0)
+        if w_o.dtype != torch.bfloat16 or not w_o.is_contiguous():
+            w_o = w_o.detach().to(torch.bfloat16).contiguous()
+        return cls(tuple(args), tuple(held), w_o, float(eps))
 
 
 def pair_weighted_averaging_fused(m: torch.Tensor, b: torch.Tensor, mask: Optional[torch.Tensor],
@@ -518,23 +512,20 @@ def pair_weighted_averaging_fused(m: torch.Tensor, b: torch.Tensor, mask: Option
     if m.dtype != torch.bfloat16 or c != 64 or not m.is_contiguous() or b.shape != (8, N, N) or b.stride(0) != N * Np:
         raise ValueError("pair_weighted_averaging_fused expects contiguous bf16 [S, N, 64] and planes of 8 heads")
     dev = m.device
-    if b.device != dev or (mask is not None and mask.device != dev):
-        raise ValueError("pair_weighted_averaging_fused: rows, bias planes and mask live on one GPU")
+    if b.device != dev or w.wo.device != dev or (mask is not None and mask.device != dev):
+        raise ValueError("pair_weighted_averaging_fused: rows, bias planes, weights and mask live on one GPU")
     if mask is not None and mask.dtype != torch.bfloat16:
         mask = mask.float()
     mk = None if mask is None else mask.expand(N, N).contiguous()
+    fold = torch.empty(2 * 256 * 64 * 2 + 4 * 256 * 4, dtype=torch.uint8, device=dev)
     v = torch.empty((8, S * 32, Np), dtype=torch.bfloat16, device=dev)
     o = torch.empty((N, S, 256), dtype=torch.bfloat16, device=dev)
     out = torch.empty_like(m)
-    lib, stream, st = native.lib(), native.current_stream(dev), native.status_tensor(dev)
-    native.check(lib.ubm_pwa_softmax(native.ptr(b), native.ptr(mk), 1 if mk is not None and mk.dtype == torch.bfloat16
-                                     else 0, 8, N, Np, stream), "ubm_pwa_softmax")
-    native.check(lib.ubm_pwa_value(native.ptr(m), native.ptr(w.wv), native.ptr(w.v_colsum), native.ptr(w.v_colbias),
-                                   native.ptr(v), S, N, Np, w.eps, native.ptr(st), stream), "ubm_pwa_value")
-    _gemm.gemm(b, v[:, :, :N], out=o, c_blocked=(32 * S * 256, S * 256, 256), c_batch=32)
-    native.check(lib.ubm_pwa_out(native.ptr(m), native.ptr(o), native.ptr(w.wg), native.ptr(w.g_colsum),
-                                 native.ptr(w.g_colbias), native.ptr(w.wo), native.ptr(out), S, N, w.eps,
-                                 native.ptr(st), stream), "ubm_pwa_out")
+    rc = native.lib().ubm_pair_weighted_averaging(
+        m.data_ptr(), b.data_ptr(), 0 if mk is None else mk.data_ptr(), 1 if mk is not None and mk.dtype == torch.bfloat16
+        else 0, *w.args, w.wo.data_ptr(), fold.data_ptr(), v.data_ptr(), o.data_ptr(), out.data_ptr(), S, N, Np, w.eps,
+        native.status_tensor(dev).data_ptr(), native.current_stream(dev))
+    native.check(rc, "ubm_pair_weighted_averaging")
     return out
 
 
