@@ -46,9 +46,7 @@ def pack_swiglu(gate_w: torch.Tensor, value_w: torch.Tensor) -> torch.Tensor:
 
 def _matrix(sh, st, batch: int, M: int, N: int, what: str) -> tuple:
     """(row stride, batch stride) of an output or residual of shape ``sh`` and strides ``st`` that has to cover
-    [batch, M, N]: the kernel addresses it by these two numbers alone."""
-    if len(sh) == 2 and batch == 1 and sh[0] >= M and sh[1] >= N:
-        return st[0], 0
+    [batch, M, N]: the kernel addresses it by these two numbers alone.  (A matrix that does is told apart in front.)"""
     if len(sh) == 3 and sh[0] >= batch and sh[2] >= N:
         # one product over rows that a 3-D tensor holds back to back may run on from one entry into the next
         rows = sh[0] * sh[1] if batch == 1 and st[0] == sh[1] * st[1] else sh[1]
@@ -124,13 +122,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, mn_major: bool = False, bias: Opti
                 raise ValueError(f"{act} output must be bf16 [.., {M}, {n_out}]")
             if sto[-1] != 1:
                 raise ValueError("output innermost dimension must be contiguous")
-            ldc, stride_c = _matrix(sho, sto, batch, M, n_out, "output")
+            if batch == 1 and len(sho) == 2 and sho[0] >= M and sho[1] >= n_out:
+                ldc, stride_c = sto[0], 0
+            else:
+                ldc, stride_c = _matrix(sho, sto, batch, M, n_out, "output")
     ldr = stride_r = 0
     if residual is not None:
         str_ = residual.stride()
         if residual.dtype != torch.bfloat16 or str_[-1] != 1:
             raise ValueError("residual must be bf16 with contiguous rows")
-        ldr, stride_r = _matrix(residual.shape, str_, batch, M, N, "residual")
+        shr = residual.shape
+        if batch == 1 and len(shr) == 2 and shr[0] >= M and shr[1] >= N:
+            ldr = str_[0]
+        else:
+            ldr, stride_r = _matrix(shr, str_, batch, M, N, "residual")
     if bias is not None and bias.dtype != torch.float32:
         bias = bias.float()
     gate_ptr = ld_gate = gate_rows = 0
