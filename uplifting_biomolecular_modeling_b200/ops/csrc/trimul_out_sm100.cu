@@ -179,6 +179,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int et = threadIdx.x - 64;       // 0 .. 511
+    const int fg = lane >> 2, ft = lane & 3;   // rows q * 32 + fg + 8 rr (rr < 4), two columns of every eight
     int stage = 0;
     uint32_t phase = 0;
     int acc = 0;
@@ -245,8 +246,14 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       const float mux = xsum * (1.f / 128.f), muz = zs.x * (1.f / 128.f);
       const float rsx = rsqrtf(fmaxf(xsq * (1.f / 128.f) - mux * mux, 0.f) + 1e-5f);
       const float rsz = rsqrtf(fmaxf(zs.y * (1.f / 128.f) - muz * muz, 0.f) + 1e-5f);
-      const float2 ax = make_float2(rsx, rsx), bx = make_float2(-mux * rsx, -mux * rsx);
-      const float2 az = make_float2(rsz, rsz), bz = make_float2(-muz * rsz, -muz * rsz);
+      float rx[4], nx[4], rz[4], nz[4];      // of this thread's four rows
+#pragma unroll
+      for (int rr = 0; rr < 4; ++rr) {
+        rx[rr] = __shfl_sync(0xffffffffu, rsx, rr * 8 + fg);
+        nx[rr] = __shfl_sync(0xffffffffu, -mux * rsx, rr * 8 + fg);
+        rz[rr] = __shfl_sync(0xffffffffu, rsz, rr * 8 + fg);
+        nz[rr] = __shfl_sync(0xffffffffu, -muz * rsz, rr * 8 + fg);
+      }
 
       mbar_wait(&acc_full[acc], acc_phase, ws, 26, acc);
       tc_fence_after_sync();
@@ -254,42 +261,38 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       const uint32_t tG = tO + 128;
 #pragma unroll 1
       for (int c0 = 0; c0 < 32; c0 += 16) {
-        uint32_t ov[16], gv[16];
-        tmem_ld16(tO + c0, ov);
-        tmem_ld16(tG + c0, gv);
+        uint32_t ov[2][8], gv[2][8];         // [lane half]
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          tmem_ld_frag16(tO + hf * kTmemLane16 + c0, ov[hf]);
+          tmem_ld_frag16(tG + hf * kTmemLane16 + c0, gv[hf]);
+        }
         tmem_ld_wait();
         if (c0 == 16) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[acc]);
         }
-        const int cb0 = grp * 32 + c0;
-        const float4* oc4 = reinterpret_cast<const float4*>(sConst + cb0);
 #pragma unroll
-        for (int j8 = 0; j8 < 2; ++j8) {
-          // in place over the residual: 16 bytes of this row in the z tile, which both products have read
-          uint4* at = reinterpret_cast<uint4*>(sz + (grp >> 1) * 16384 +
-                                               swz128_offset(row, (grp & 1) * 4 + (c0 >> 3) + j8));
-          const uint4 u = p.add_residual ? *at : make_uint4(0u, 0u, 0u, 0u);
-          const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-          uint32_t o[4];
+        for (int u = 0; u < 2; ++u) {
+          const int col = grp * 32 + c0 + u * 8;
+          const float2* oc2 = reinterpret_cast<const float2*>(sConst + col) + ft;
+          const float2 ocs = oc2[0], ocb = oc2[64], gcs = oc2[128], gcb = oc2[192];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float4 ocs = oc4[j8 * 2 + h], ocb = oc4[32 + j8 * 2 + h];
-            const float4 gcs = oc4[64 + j8 * 2 + h], gcb = oc4[96 + j8 * 2 + h];
-            const int k = j8 * 8 + h * 4;
-            const float2 f0 = ln_fold2(ov[k], ov[k + 1], ax, bx, ocs.x, ocs.y, ocb.x, ocb.y);
-            const float2 f1 = ln_fold2(ov[k + 2], ov[k + 3], ax, bx, ocs.z, ocs.w, ocb.z, ocb.w);
-            const float2 g0 = ln_fold2(gv[k], gv[k + 1], az, bz, gcs.x, gcs.y, gcb.x, gcb.y);
-            const float2 g1 = ln_fold2(gv[k + 2], gv[k + 3], az, bz, gcs.z, gcs.w, gcb.z, gcb.w);
-            const float2 v0 = __ffma2_rn(f0, make_float2(sigmoidf_fast(g0.x), sigmoidf_fast(g0.y)),
-                                         make_float2(bf16_lo(w[h * 2]), bf16_hi(w[h * 2])));
-            const float2 v1 = __ffma2_rn(f1, make_float2(sigmoidf_fast(g1.x), sigmoidf_fast(g1.y)),
-                                         make_float2(bf16_lo(w[h * 2 + 1]), bf16_hi(w[h * 2 + 1])));
-            o[h * 2] = pack_bf16x2(v0.x, v0.y);
-            o[h * 2 + 1] = pack_bf16x2(v1.x, v1.y);
+          for (int rr = 0; rr < 4; ++rr) {
+            const int k = u * 4 + (rr & 1) * 2;
+            // in place over the residual: two channels of this row in the z tile, which both products have read
+            uint32_t* at = reinterpret_cast<uint32_t*>(sz + (grp >> 1) * 16384 +
+                                                       swz128_offset(q * 32 + rr * 8 + fg, (col & 63) >> 3)) + ft;
+            const uint32_t w = p.add_residual ? *at : 0u;
+            const float2 f = ln_fold2(ov[rr >> 1][k], ov[rr >> 1][k + 1], make_float2(rx[rr], rx[rr]),
+                                      make_float2(nx[rr], nx[rr]), ocs.x, ocs.y, ocb.x, ocb.y);
+            const float2 gt = ln_fold2(gv[rr >> 1][k], gv[rr >> 1][k + 1], make_float2(rz[rr], rz[rr]),
+                                       make_float2(nz[rr], nz[rr]), gcs.x, gcs.y, gcb.x, gcb.y);
+            const float2 v = __ffma2_rn(f, make_float2(sigmoidf_fast(gt.x), sigmoidf_fast(gt.y)),
+                                        make_float2(bf16_lo(w), bf16_hi(w)));
+            *at = pack_bf16x2(v.x, v.y);
           }
-          *at = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
       fence_proxy_async_smem();

@@ -180,13 +180,18 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const int op = ((warp - 2) >> 2) & 1;   // operand a or b
     const int half = (warp - 2) >> 3;       // columns 64 half .. 64 half + 63
     const int q = warp & 3;                 // TMEM lane quadrant
-    const int ch = q * 32 + lane;           // output channel of this thread
+    const int g = lane >> 2, t4 = lane & 3; // channels q * 32 + g + 8 rr (rr < 4), two columns of every eight
     const int et = threadIdx.x - 64;        // 0 .. 511: four threads take the statistics of one tile row
     const int srow = et >> 2;
-    const float cs_v = p.colsum[op * 256 + ch], cb_v = p.colbias[op * 256 + ch];
-    const float cs_g = p.colsum[op * 256 + 128 + ch], cb_g = p.colbias[op * 256 + 128 + ch];
-    const float2 csv2 = make_float2(cs_v, cs_v), cbv2 = make_float2(cb_v, cb_v);
-    const float2 csg2 = make_float2(cs_g, cs_g), cbg2 = make_float2(cb_g, cb_g);
+    float cs_v[4], cb_v[4], cs_g[4], cb_g[4];
+#pragma unroll
+    for (int rr = 0; rr < 4; ++rr) {
+      const int ch = op * 256 + q * 32 + rr * 8 + g;
+      cs_v[rr] = p.colsum[ch];
+      cb_v[rr] = p.colbias[ch];
+      cs_g[rr] = p.colsum[ch + 128];
+      cb_g[rr] = p.colbias[ch + 128];
+    }
     int stage = 0;
     uint32_t phase = 0;
     uint32_t acc_phase = 0;
@@ -239,12 +244,14 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       mbar_wait(&acc_full[op], acc_phase, ws, 16, op);
       tc_fence_after_sync();
       const uint32_t tbase = tmem_addr(tmem_base, q, op * 256 + half * 64);
-      const float4* st4 = reinterpret_cast<const float4*>(sStat + half * 64);
 #pragma unroll 1
       for (int c16 = 0; c16 < 4; ++c16) {
-        uint32_t v[16], g[16];
-        tmem_ld16(tbase + c16 * 16, v);
-        tmem_ld16(tbase + 128 + c16 * 16, g);
+        uint32_t v[2][8], gt[2][8];                          // [lane half]: value and gate of 16 columns
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          tmem_ld_frag16(tbase + hf * kTmemLane16 + c16 * 16, v[hf]);
+          tmem_ld_frag16(tbase + hf * kTmemLane16 + 128 + c16 * 16, gt[hf]);
+        }
         tmem_ld_wait();
         if (c16 == 3) {
           tc_fence_before_sync();
@@ -256,27 +263,24 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           __syncwarp();
         }
 #pragma unroll
-        for (int j8 = 0; j8 < 2; ++j8) {
-          uint32_t o[4];
+        for (int u = 0; u < 2; ++u) {
+          // two adjacent s at a time in packed fp32 instructions, their constants for four channels
+          const float2* st2 = reinterpret_cast<const float2*>(sStat + half * 64 + c16 * 16 + u * 8) + t4;
+          const float2 rs = st2[0], nm = st2[64], mk = st2[128];
+          const uint32_t at = g * 64 + ((((c16 & 1) * 2 + u) ^ (g >> 1)) << 4) + t4 * 4;   // 64-byte swizzle
 #pragma unroll
-          for (int h4 = 0; h4 < 2; ++h4) {
-            // two adjacent s at a time in packed fp32 instructions
-            const int f4 = c16 * 4 + j8 * 2 + h4, si = j8 * 8 + h4 * 4;
-            const float4 rs = st4[f4], nm = st4[32 + f4], mk = st4[64 + f4];
-            auto gated = [&](int k, float2 rs2, float2 nm2, float2 mk2) {
-              const float2 val = __ffma2_rn(make_float2(__uint_as_float(v[k]), __uint_as_float(v[k + 1])), rs2,
-                                            __ffma2_rn(nm2, csv2, cbv2));
-              const float2 gt = __ffma2_rn(make_float2(__uint_as_float(g[k]), __uint_as_float(g[k + 1])), rs2,
-                                           __ffma2_rn(nm2, csg2, cbg2));
-              const float2 ov = __fmul2_rn(
-                  val, __fmul2_rn(mk2, make_float2(sigmoidf_fast(gt.x), sigmoidf_fast(gt.y))));
-              return pack_bf16x2(ov.x, ov.y);
-            };
-            o[h4 * 2] = gated(si, make_float2(rs.x, rs.y), make_float2(nm.x, nm.y), make_float2(mk.x, mk.y));
-            o[h4 * 2 + 1] = gated(si + 2, make_float2(rs.z, rs.w), make_float2(nm.z, nm.w), make_float2(mk.z, mk.w));
+          for (int rr = 0; rr < 4; ++rr) {
+            const int k = u * 4 + (rr & 1) * 2;
+            const uint32_t(&vr)[8] = v[rr >> 1];
+            const uint32_t(&gr)[8] = gt[rr >> 1];
+            const float2 val = __ffma2_rn(make_float2(__uint_as_float(vr[k]), __uint_as_float(vr[k + 1])), rs,
+                                          make_float2(fmaf(nm.x, cs_v[rr], cb_v[rr]), fmaf(nm.y, cs_v[rr], cb_v[rr])));
+            const float2 gate = __ffma2_rn(make_float2(__uint_as_float(gr[k]), __uint_as_float(gr[k + 1])), rs,
+                                           make_float2(fmaf(nm.x, cs_g[rr], cb_g[rr]), fmaf(nm.y, cs_g[rr], cb_g[rr])));
+            const float2 ov =
+                __fmul2_rn(val, __fmul2_rn(mk, make_float2(sigmoidf_fast(gate.x), sigmoidf_fast(gate.y))));
+            *reinterpret_cast<uint32_t*>(stage_w + rr * 512 + at) = pack_bf16x2(ov.x, ov.y);
           }
-          *reinterpret_cast<uint4*>(stage_w + swz64_offset(lane, (c16 & 1) * 2 + j8)) =
-              make_uint4(o[0], o[1], o[2], o[3]);
         }
         if (c16 & 1) {
           fence_proxy_async_smem();
