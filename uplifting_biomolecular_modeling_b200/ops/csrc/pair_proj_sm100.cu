@@ -66,19 +66,7 @@ struct PairOutMaps {
 };
 constexpr int kPPOutWarpBytes = 32 * 64;
 constexpr int kPPOutBytes = 8 * kPPOutWarpBytes;
-
-// Optional timeline (build with -DUBM_PP_TIMELINE): CTA 0 stamps clock64 at fixed points of its first tiles
-// into a global buffer [4 roles][kPPTlTiles][8 events] (roles: producer, MMA issuer, epilogue group 0, 1).
-#ifdef UBM_PP_TIMELINE
-constexpr int kPPTlTiles = 32;
-__device__ long long g_pp_timeline[4 * kPPTlTiles * 8];
-#define PP_STAMP(role, tile, ev)                                                                              \
-  do {                                                                                                        \
-    if (blockIdx.x == 0 && (tile) < kPPTlTiles) g_pp_timeline[((role) * kPPTlTiles + (tile)) * 8 + (ev)] = clock64(); \
-  } while (0)
-#else
-#define PP_STAMP(role, tile, ev) do { } while (0)
-#endif
+constexpr int kPPWbFrags = 3 * 8 * 32;
 
 template <int MODE>
 __global__ void __launch_bounds__(320, 1)
@@ -92,8 +80,8 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   uint8_t* sOut = sX + kPPStages * kPPXBytes;       // 8 warps x 2 KB of output staging
   float* sColsum = reinterpret_cast<float*>(sOut + kPPOutBytes);          // 512
   float* sColbias = sColsum + 512;                                         // 512
-  float* sWb = sColbias + 512;                                             // kPPMaxHeads * 128
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sWb + kPPMaxHeads * 128);
+  uint2* sWbF = reinterpret_cast<uint2*>(sColbias + 512);                  // [3 parts][8 k-steps][32 lanes]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sWbF + kPPWbFrags);
   uint64_t* x_full = bars;                 // [stages]
   uint64_t* x_empty = x_full + kPPStages;  // [stages]
   uint64_t* w_full = x_empty + kPPStages;  // [1]
@@ -131,7 +119,25 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     sColbias[i] = p.colbias[i];
   }
   if (MODE == MODE_TRIATT) {
-    for (int i = threadIdx.x; i < p.H * 128; i += blockDim.x) sWb[i] = p.wb[i];
+    // head weights as three bf16 parts (high, middle, low: 24 bits), in the order in which a lane of mma.sync takes them as
+    // the second operand of a 16-wide k-step: head lane / 4, channels 2 (lane % 4), + 1 and the same eight further on
+    for (int i = threadIdx.x; i < 8 * 32; i += blockDim.x) {
+      const int head = (i & 31) >> 2, k0 = (i >> 5) * 16 + (i & 3) * 2;
+      uint32_t part[3][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float r = head < p.H ? p.wb[head * 128 + k0 + (e >> 1) * 8 + (e & 1)] : 0.f;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const __nv_bfloat16 h = __float2bfloat16_rn(r);
+          part[q][e] = __bfloat16_as_ushort(h);
+          r -= __bfloat162float(h);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        sWbF[q * 256 + i] = make_uint2(part[q][0] | (part[q][1] << 16), part[q][2] | (part[q][3] << 16));
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -148,11 +154,8 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           tma_load_2d(sW + kb * 65536 + h * 32768, &tmW, w_full, kb * 64, h * 256);
       int stage = 0;
       uint32_t phase = 0;
-      int lt = 0;
-      for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++lt) {
-        PP_STAMP(0, lt, 0);
+      for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
         mbar_wait(&x_empty[stage], phase ^ 1u, ws, 11, stage);
-        PP_STAMP(0, lt, 1);
         if (*abort_flag) break;
         uint8_t* dst = sX + stage * kPPXBytes;
         mbar_expect_tx(&x_full[stage], kPPXBytes);
@@ -186,17 +189,13 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       int stage = 0;
       uint32_t phase = 0;
       uint32_t acc_phase = 0;
-      int lt = 0;
-      for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++lt) {
-        if (lane == 0) PP_STAMP(1, lt, 0);
+      for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
         mbar_wait(&x_full[stage], phase, ws, 13, stage);
-        if (lane == 0) PP_STAMP(1, lt, 1);
         tc_fence_after_sync();
         const uint32_t xa = smem_u32(sX + stage * kPPXBytes);
         const uint32_t wa = smem_u32(sW);
         for (int h = 0; h < 2; ++h) {
           mbar_wait(&acc_empty[h], acc_phase ^ 1u, ws, 14, h);
-          if (lane == 0) PP_STAMP(1, lt, 2 + 2 * h);
           tc_fence_after_sync();
           const uint64_t ad0 = umma_smem_desc(xa, 16, 1024, kSwizzle128);
           const uint64_t bd0 = umma_smem_desc(wa + h * 32768, 16, 1024, kSwizzle128);
@@ -211,7 +210,6 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             umma_commit(&acc_full[h]);
           }
           __syncwarp();
-          if (lane == 0) PP_STAMP(1, lt, 3 + 2 * h);
         }
         if (leader) umma_commit(&x_empty[stage]);
         __syncwarp();
@@ -227,51 +225,43 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     const int grp = (warp - 2) >> 2;  // 0 or 1: which 256-column half
     const int q = warp & 3;           // TMEM lane quadrant
     const int row_in_tile = q * 32 + lane;
-    const bool out_tma = p.out_tma != 0;                 // warp-uniform
+    const int fg = lane >> 2, ft = lane & 3;   // rows q * 32 + fg + 8 rr (rr < 4), two columns of every eight
     uint8_t* stage_w = sOut + (warp - 2) * kPPOutWarpBytes;
     int stage = 0;
     uint32_t phase = 0;
     uint32_t acc_phase = 0;
-    int lt = 0;
-    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++lt) {
+    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
       const long long r = static_cast<long long>(t) * kPPRows + row_in_tile;
       const bool row_ok = r < p.R;
       // ---- row statistics (and head bias) from the shared-memory tile
-      if (q == 0 && lane == 0) PP_STAMP(2 + grp, lt, 0);
       mbar_wait(&x_full[stage], phase, ws, 15, stage);
-      if (q == 0 && lane == 0) PP_STAMP(2 + grp, lt, 1);
       const uint8_t* xs = sX + stage * kPPXBytes;
       float sum = 0.f, sumsq = 0.f;
-      float hb[kPPMaxHeads / 2];
-#pragma unroll
-      for (int h = 0; h < kPPMaxHeads / 2; ++h) hb[h] = 0.f;
-      const int hpg = (MODE == MODE_TRIATT) ? (p.H + 1) / 2 : 0;  // heads per group
 #pragma unroll 4
       for (int c16 = 0; c16 < 16; ++c16) {
-        const int kb = c16 >> 3;
-        const uint4 u = *reinterpret_cast<const uint4*>(xs + kb * 16384 + swz128_offset(row_in_tile, c16 & 7));
+        const uint4 u = *reinterpret_cast<const uint4*>(xs + (c16 >> 3) * 16384 + swz128_offset(row_in_tile, c16 & 7));
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-        float e[8];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          e[2 * j] = bf16_lo(w[j]);
-          e[2 * j + 1] = bf16_hi(w[j]);
+          const float e0 = bf16_lo(w[j]), e1 = bf16_hi(w[j]);
+          sum += e0;
+          sumsq += e0 * e0;
+          sum += e1;
+          sumsq += e1 * e1;
         }
+      }
+      // head products of 16 rows per warp (q * 32 + grp * 16 ..) and up to eight heads on the warp-level matrix instruction
+      float hb[4] = {0.f, 0.f, 0.f, 0.f};
+      if (MODE == MODE_TRIATT) {
+        const int lrow = q * 32 + grp * 16 + (lane & 15);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          sum += e[j];
-          sumsq += e[j] * e[j];
-        }
-        if (MODE == MODE_TRIATT) {
+        for (int ks = 0; ks < 8; ++ks) {
+          uint32_t a0, a1, a2, a3;
+          ldmatrix_x4(xs + (ks >> 2) * 16384 + swz128_offset(lrow, (ks & 3) * 2 + (lane >> 4)), a0, a1, a2, a3);
 #pragma unroll
-          for (int h = 0; h < kPPMaxHeads / 2; ++h) {
-            if (h < hpg) {
-              const float* wrow = sWb + (grp * hpg + h) * 128 + c16 * 8;
-              const float4 w0 = *reinterpret_cast<const float4*>(wrow);
-              const float4 w1 = *reinterpret_cast<const float4*>(wrow + 4);
-              hb[h] += e[0] * w0.x + e[1] * w0.y + e[2] * w0.z + e[3] * w0.w + e[4] * w1.x + e[5] * w1.y +
-                       e[6] * w1.z + e[7] * w1.w;
-            }
+          for (int part = 0; part < 3; ++part) {
+            const uint2 bw = sWbF[(part * 8 + ks) * 32 + lane];
+            mma_bf16_16816(hb, a0, a1, a2, a3, bw.x, bw.y);
           }
         }
       }
@@ -291,23 +281,30 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         pk = static_cast<int>(r - static_cast<long long>(pi) * p.N);
       }
 
-      if (MODE == MODE_TRIATT && row_ok) {
-        const int oi = p.transpose_out ? pk : pi;
-        const int ok = p.transpose_out ? pi : pk;
+      if (MODE == MODE_TRIATT) {
+        // this lane holds heads 2 ft, + 1 of rows grp * 16 + fg and + 8 of the quadrant
 #pragma unroll
-        for (int h = 0; h < kPPMaxHeads / 2; ++h) {
-          const int head = grp * hpg + h;
-          if (h < hpg && head < p.H) {
-            const float val = rstd * (hb[h] - mu * p.wb_colsum[head]) + p.wb_colbias[head];
-            p.headbias[(static_cast<long long>(head) * p.plane_rows + oi) * p.Np + ok] = __float2bfloat16(val);
+        for (int e = 0; e < 2; ++e) {
+          const int src = grp * 16 + e * 8 + fg;
+          const float rs = __shfl_sync(0xffffffffu, rstd, src), m = __shfl_sync(0xffffffffu, mu, src);
+          const int ri = __shfl_sync(0xffffffffu, pi, src), rk = __shfl_sync(0xffffffffu, pk, src);
+          if (static_cast<long long>(t) * kPPRows + q * 32 + src < p.R) {
+            const int oi = p.transpose_out ? rk : ri;
+            const int ok = p.transpose_out ? ri : rk;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              const int head = 2 * ft + c;
+              if (head < p.H) {
+                const float val = rs * (hb[2 * e + c] - m * p.wb_colsum[head]) + p.wb_colbias[head];
+                p.headbias[(static_cast<long long>(head) * p.plane_rows + oi) * p.Np + ok] = __float2bfloat16(val);
+              }
+            }
           }
         }
       }
 
       // ---- accumulator half of this group
-      if (q == 0 && lane == 0) PP_STAMP(2 + grp, lt, 2);
       mbar_wait(&acc_full[grp], acc_phase, ws, 16, grp);
-      if (q == 0 && lane == 0) PP_STAMP(2 + grp, lt, 3);
       tc_fence_after_sync();
       const uint32_t tbase = tmem_addr(tmem_base, q, grp * 256);
       {
@@ -315,47 +312,41 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         const long long orow = p.transpose_out ? (static_cast<long long>(pk) * p.N + pi) : r;
         __nv_bfloat16* o0 = (grp == 0 ? p.q : p.v) + orow * 128;
         __nv_bfloat16* o1 = (grp == 0 ? p.k : p.g) + orow * 128;
-        const float2 a2 = make_float2(rstd, rstd);
-        const float2 b2 = make_float2(-mu * rstd, -mu * rstd);
+        float ra[4], rb[4];      // of this thread's four rows
+#pragma unroll
+        for (int rr = 0; rr < 4; ++rr) {
+          ra[rr] = __shfl_sync(0xffffffffu, rstd, rr * 8 + fg);
+          rb[rr] = __shfl_sync(0xffffffffu, -mu * rstd, rr * 8 + fg);
+        }
         // 32-column chunks, the tensor-memory load of the next chunk in flight while this one is processed;
         // the chunk body exists twice (ping-pong registers), not eight times
         // first row of this warp's 32 (a multiple of 32): its pair index places the warp's output box
         const long long r0 = static_cast<long long>(t) * kPPRows + q * 32;
         const int bi = static_cast<int>(r0 / p.N);
         const int bk = static_cast<int>(r0 - static_cast<long long>(bi) * p.N);
-        auto chunk = [&](const uint32_t (&av)[32], const int c0) {
-          if (out_tma) {
-            if (lane == 0) tma_store_wait_read<0>();    // the previous box of this warp has left the staging rows
-            __syncwarp();
-          }
-          if (row_ok) {
-            if (q == 0 && lane == 0 && c0 == 32) PP_STAMP(2 + grp, lt, 5);
-            float f[32];
-            ln_fold32(av, a2, b2, sColsum + grp * 256 + c0, sColbias + grp * 256 + c0, f);
-            if (grp == 1 && c0 >= 128) {      // gate columns (warp-uniform)
+        // a transposed box holds second indices of one first index: rows that reach into the next one leave by lane
+        const bool boxed = p.out_tma != 0 && (!p.transpose_out || bk + 32 <= p.N || r0 + p.N - bk >= p.R);   // warp-uniform
+        auto chunk = [&](const uint32_t (&lo)[16], const uint32_t (&hi)[16], const int c0) {
+          if (lane == 0) tma_store_wait_read<0>();    // the previous box of this warp has left the staging rows
+          __syncwarp();
+          const bool gate = grp == 1 && c0 >= 128;    // warp-uniform
 #pragma unroll
-              for (int j = 0; j < 32; ++j) f[j] = sigmoidf_fast(f[j]);
-            }
-            if (q == 0 && lane == 0 && c0 == 32) PP_STAMP(2 + grp, lt, 6);
-            if (out_tma) {
+          for (int u = 0; u < 4; ++u) {
+            const int col = grp * 256 + c0 + u * 8;
+            const float2 cs = reinterpret_cast<const float2*>(sColsum + col)[ft];
+            const float2 cb = reinterpret_cast<const float2*>(sColbias + col)[ft];
 #pragma unroll
-              for (int j8 = 0; j8 < 4; ++j8) {
-                uint4 u;
-                u.x = pack_bf16x2(f[j8 * 8], f[j8 * 8 + 1]);
-                u.y = pack_bf16x2(f[j8 * 8 + 2], f[j8 * 8 + 3]);
-                u.z = pack_bf16x2(f[j8 * 8 + 4], f[j8 * 8 + 5]);
-                u.w = pack_bf16x2(f[j8 * 8 + 6], f[j8 * 8 + 7]);
-                *reinterpret_cast<uint4*>(stage_w + swz64_offset(lane, j8)) = u;
-              }
-            } else {
-              __nv_bfloat16* dst = (c0 < 128 ? o0 + c0 : o1 + (c0 - 128));
-              st_bf16x16(dst, f);
-              st_bf16x16(dst + 16, f + 16);
+            for (int rr = 0; rr < 4; ++rr) {
+              const uint32_t(&v)[16] = rr < 2 ? lo : hi;
+              const int k = u * 4 + (rr & 1) * 2;
+              float2 f = ln_fold2(v[k], v[k + 1], make_float2(ra[rr], ra[rr]), make_float2(rb[rr], rb[rr]), cs.x, cs.y,
+                                  cb.x, cb.y);
+              if (gate) f = make_float2(sigmoidf_fast(f.x), sigmoidf_fast(f.y));
+              *reinterpret_cast<uint32_t*>(stage_w + swz64_offset(rr * 8 + fg, u) + ft * 4) = pack_bf16x2(f.x, f.y);
             }
-            if (q == 0 && lane == 0 && c0 == 32) PP_STAMP(2 + grp, lt, 7);
           }
-          if (out_tma) {
-            // rows past R hold stale bytes: the copy clips them
+          if (boxed) {
+            // rows past R hold values of zero rows: the copy clips them
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
@@ -364,21 +355,33 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
               else tma_store_3d(om, stage_w, c0 & 127, static_cast<int>(r0), 0);
               tma_store_commit();
             }
+          } else {
+            __syncwarp();
+            if (row_ok) {
+              uint4* dst = reinterpret_cast<uint4*>(c0 < 128 ? o0 + c0 : o1 + (c0 - 128));
+#pragma unroll
+              for (int j = 0; j < 4; ++j) dst[j] = *reinterpret_cast<const uint4*>(stage_w + swz64_offset(lane, j));
+            }
+            __syncwarp();
           }
         };
-        uint32_t va[32], vb[32];
-        tmem_ld32(tbase, va);
+        uint32_t la[16], ha[16], lb[16], hb2[16];
+        tmem_ld_frag32(tbase, la);
+        tmem_ld_frag32(tbase + kTmemLane16, ha);
 #pragma unroll 1
         for (int c0 = 0; c0 < 256; c0 += 64) {
           tmem_ld_wait();
-          tmem_ld32(tbase + c0 + 32, vb);
-          chunk(va, c0);
+          tmem_ld_frag32(tbase + c0 + 32, lb);
+          tmem_ld_frag32(tbase + kTmemLane16 + c0 + 32, hb2);
+          chunk(la, ha, c0);
           tmem_ld_wait();
-          if (c0 + 64 < 256) tmem_ld32(tbase + c0 + 64, va);
-          chunk(vb, c0 + 32);
+          if (c0 + 64 < 256) {
+            tmem_ld_frag32(tbase + c0 + 64, la);
+            tmem_ld_frag32(tbase + kTmemLane16 + c0 + 64, ha);
+          }
+          chunk(lb, hb2, c0 + 32);
         }
       }
-      if (q == 0 && lane == 0) PP_STAMP(2 + grp, lt, 4);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[grp]);
@@ -388,7 +391,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       }
       acc_phase ^= 1u;
     }
-    if (out_tma && lane == 0) tma_store_wait_all<0>();   // the staging rows are read and the boxes written
+    if (lane == 0) tma_store_wait_all<0>();   // the staging rows are read and the boxes written
   }
 
   tc_fence_before_sync();
@@ -400,7 +403,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 }
 
 constexpr int kPPSmemBytes =
-    kPPWBytes + kPPStages * kPPXBytes + kPPOutBytes + (512 + 512 + kPPMaxHeads * 128) * 4 + 256 + 1024;
+    kPPWBytes + kPPStages * kPPXBytes + kPPOutBytes + (512 + 512) * 4 + kPPWbFrags * 8 + 256 + 1024;
 static_assert(kPPSmemBytes <= 232448, "shared memory of one CTA");
 
 template <int MODE>
@@ -434,7 +437,7 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
       return e == nullptr || e[0] != '0';
     }();
     void* bufs[4] = {p.q, p.k, p.v, p.g};
-    bool ok = on && MODE == MODE_TRIATT && p.R < (1ll << 31) && (!p.transpose_out || (p.N % 32) == 0);
+    bool ok = on && MODE == MODE_TRIATT && p.R < (1ll << 31);
     for (int i = 0; i < 4; ++i) ok = ok && bufs[i] != nullptr && (reinterpret_cast<uintptr_t>(bufs[i]) & 15) == 0;
     if (ok) {
       for (int i = 0; i < 4; ++i) {
@@ -525,12 +528,6 @@ extern "C" int ubm_triatt_proj_rows_peer(const void* const* z_ptrs, const int* p
   return triatt_proj_impl(z_ptrs[me], w, colsum, colbias, wb, wb_colsum, wb_colbias, q, k, v, g, headbias, nullptr,
                           rows, plane_rows, N, Np, H, 0, status, stream, z_ptrs, peer_rows, npeers, me);
 }
-
-#ifdef UBM_PP_TIMELINE
-extern "C" int ubm_pair_proj_read_timeline(long long* host_out) {
-  return cudaMemcpyFromSymbol(host_out, ubm::g_pp_timeline, sizeof(ubm::g_pp_timeline)) == cudaSuccess ? 0 : -1;
-}
-#endif
 
 extern "C" int ubm_triatt_proj(const void* z, const void* w, const void* colsum, const void* colbias, const void* wb,
                                const void* wb_colsum, const void* wb_colbias, void* q, void* k, void* v, void* g,
