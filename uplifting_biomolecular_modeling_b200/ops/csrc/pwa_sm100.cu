@@ -197,11 +197,15 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     }
   } else {
     const int grp = (warp - 2) >> 2;      // channel block: heads 4 grp .. 4 grp + 3
-    const int q = warp & 3;               // lane quadrant = head within the block; lane = channel of the head
+    const int q = warp & 3;               // lane quadrant = head within the block
     const int et = threadIdx.x - 64;      // 0..255: two threads take the statistics of one tile row
-    const int ch = grp * 128 + q * 32 + lane;
-    const float cs = p.colsum[ch], cb = p.colbias[ch];
-    const float2 cs2 = make_float2(cs, cs), cb2 = make_float2(cb, cb);
+    const int fg = lane >> 2, ft = lane & 3;   // channels fg + 8 rr (rr < 4) of the head, two tokens of every eight
+    float cs[4], cb[4];
+#pragma unroll
+    for (int rr = 0; rr < 4; ++rr) {
+      cs[rr] = p.colsum[grp * 128 + q * 32 + rr * 8 + fg];
+      cb[rr] = p.colbias[grp * 128 + q * 32 + rr * 8 + fg];
+    }
     uint8_t* stage_w = sOut + (warp - 2) * 32 * 64;
     int stage = 0;
     uint32_t phase = 0, acc_phase = 0, par = 0;
@@ -239,28 +243,23 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
       const int chunks = min(4, (p.N - j0 + 31) / 32);
 #pragma unroll 1
       for (int c = 0; c < chunks; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tb + c * 32, v);
+        uint32_t v[2][16];                              // [lane half]
+        tmem_ld_frag32(tb + c * 32, v[0]);
+        tmem_ld_frag32(tb + kTmemLane16 + c * 32, v[1]);
         tmem_ld_wait();
         if (lane == 0) tma_store_wait_read<0>();        // the previous box of this warp has left the staging rows
         __syncwarp();
-        const float4* rs4 = reinterpret_cast<const float4*>(st + c * 32);
-        const float4* nm4 = reinterpret_cast<const float4*>(st + 128 + c * 32);
 #pragma unroll
-        for (int j8 = 0; j8 < 4; ++j8) {
-          uint32_t o[4];
+        for (int u = 0; u < 4; ++u) {
+          const float2* st2 = reinterpret_cast<const float2*>(st + c * 32 + u * 8) + ft;
+          const float2 rs = st2[0], nm = st2[64];
 #pragma unroll
-          for (int h4 = 0; h4 < 2; ++h4) {
-            const float4 rs = rs4[j8 * 2 + h4], nm = nm4[j8 * 2 + h4];
-            const int k = j8 * 8 + h4 * 4;
-            const float2 a = __ffma2_rn(make_float2(__uint_as_float(v[k]), __uint_as_float(v[k + 1])),
-                                        make_float2(rs.x, rs.y), __ffma2_rn(make_float2(nm.x, nm.y), cs2, cb2));
-            const float2 b = __ffma2_rn(make_float2(__uint_as_float(v[k + 2]), __uint_as_float(v[k + 3])),
-                                        make_float2(rs.z, rs.w), __ffma2_rn(make_float2(nm.z, nm.w), cs2, cb2));
-            o[h4 * 2] = pack_bf16x2(a.x, a.y);
-            o[h4 * 2 + 1] = pack_bf16x2(b.x, b.y);
+          for (int rr = 0; rr < 4; ++rr) {
+            const int k = u * 4 + (rr & 1) * 2;
+            const float2 a = __ffma2_rn(make_float2(__uint_as_float(v[rr >> 1][k]), __uint_as_float(v[rr >> 1][k + 1])), rs,
+                                        __ffma2_rn(nm, make_float2(cs[rr], cs[rr]), make_float2(cb[rr], cb[rr])));
+            *reinterpret_cast<uint32_t*>(stage_w + swz64_offset(rr * 8 + fg, u) + ft * 4) = pack_bf16x2(a.x, a.y);
           }
-          *reinterpret_cast<uint4*>(stage_w + swz64_offset(lane, j8)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
         fence_proxy_async_smem();
         __syncwarp();
@@ -427,6 +426,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
     const int half = ((warp - 3) >> 2) & 1;      // columns 128 half .. of D_g, 32 half .. of D_o
     const int q = warp & 3;
     const int row = q * 32 + lane;
+    const int fg = lane >> 2, ft = lane & 3;     // rows q * 32 + fg + 8 rr (rr < 4), two columns of every eight
     uint8_t* st = sSt + team * kPoStage;
     const uint32_t tb = tmem_base + team * 256;
     uint32_t n = 0;
@@ -450,32 +450,46 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
       }
       const float mu = sum * (1.f / kPwC);
       const float rstd = row_rstd(mu, sumsq, p.eps);
-      const float2 a2 = make_float2(rstd, rstd), b2 = make_float2(-mu * rstd, -mu * rstd);
+      float ra[4], rb[4];
+#pragma unroll
+      for (int rr = 0; rr < 4; ++rr) {
+        ra[rr] = __shfl_sync(0xffffffffu, rstd, rr * 8 + fg);
+        rb[rr] = __shfl_sync(0xffffffffu, -mu * rstd, rr * 8 + fg);
+      }
       mbar_wait(&g_full[team], ph, ws, 87, team);
       tc_fence_after_sync();
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         const int col = half * 128 + c * 32;
-        uint32_t v[32];
-        tmem_ld32(tmem_addr(tb, q, col), v);
+        uint32_t v[2][16];                       // [lane half]
+        tmem_ld_frag32(tmem_addr(tb, q, col), v[0]);
+        tmem_ld_frag32(tmem_addr(tb, q, col) + kTmemLane16, v[1]);
         tmem_ld_wait();
-        float f[32];
-        ln_fold32(v, a2, b2, sConst + col, sConst + kPwHC + col, f);
-        float low = fminf(f[0], f[1]);
+        float2 f[4][4];                          // [eight columns][row]
+        float low = 0.f;
 #pragma unroll
-        for (int k = 2; k < 32; k += 2) low = min3f(low, f[k], f[k + 1]);
+        for (int u = 0; u < 4; ++u) {
+          const float2* gc = reinterpret_cast<const float2*>(sConst + col + u * 8) + ft;
+          const float2 cs = gc[0], cb = gc[kPwHC / 2];
+#pragma unroll
+          for (int rr = 0; rr < 4; ++rr) {
+            const int k = u * 4 + (rr & 1) * 2;
+            f[u][rr] = ln_fold2(v[rr >> 1][k], v[rr >> 1][k + 1], make_float2(ra[rr], ra[rr]), make_float2(rb[rr], rb[rr]),
+                                cs.x, cs.y, cb.x, cb.y);
+            low = min3f(low, f[u][rr].x, f[u][rr].y);
+          }
+        }
         uint8_t* ob = st + (1 + (col >> 6)) * kPwTile;
         auto apply = [&](auto gate) {
 #pragma unroll
-          for (int j8 = 0; j8 < 4; ++j8) {
-            uint4* at = reinterpret_cast<uint4*>(ob + swz128_offset(row, ((col >> 5) & 1) * 4 + j8));
-            const uint4 u = *at;
-            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-            uint32_t r[4];
+          for (int u = 0; u < 4; ++u) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              r[e] = pack_bf16x2(bf16_lo(w[e]) * gate(f[j8 * 8 + 2 * e]), bf16_hi(w[e]) * gate(f[j8 * 8 + 2 * e + 1]));
-            *at = make_uint4(r[0], r[1], r[2], r[3]);
+            for (int rr = 0; rr < 4; ++rr) {
+              uint32_t* at =
+                  reinterpret_cast<uint32_t*>(ob + swz128_offset(q * 32 + rr * 8 + fg, ((col >> 5) & 1) * 4 + u)) + ft;
+              const uint32_t w = *at;
+              *at = pack_bf16x2(bf16_lo(w) * gate(f[u][rr].x), bf16_hi(w) * gate(f[u][rr].y));
+            }
           }
         };
         // nearly closed gates take the form that keeps their relative precision (for every gate it costs 27 us more)
