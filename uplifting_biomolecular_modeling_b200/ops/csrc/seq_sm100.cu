@@ -1471,6 +1471,195 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_rows_kernel(
   }
 }
 
+// The same products on the warp-level matrix instruction (m16n8k16): 16 weight rows are the rows of the tile, the decode
+// rows its eight columns.  In the kernel above every decode row costs eight FMAs, a shared-memory read and an unpacking per
+// 16 bytes of weights, so eight rows were bound by issue slots; here a 128-byte line of 16 weight rows costs four matrix
+// instructions whatever the number of decode rows, and the weights go to the tensor core as they are.
+// The order of a contraction is free as long as both operands share it: lane (g, t) takes elements 16 t .. 16 t + 15 of a
+// 64-wide block from rows g and g + 8 of the weights and from decode row g, one 32-byte load each, and feeds them to four
+// instructions four at a time.  The blocks of a tile are dealt to the CTA's warps, which add their sums up in shared memory.
+// STAGED: x^ is normalised into shared memory once per CTA; otherwise decode rows come straight from L1 (staging all of
+// x cost every SM up to 176 KB of L2 reads in front of its weights).  Needs K % 64 == 0 and weights on 32 bytes.
+constexpr int kGemvMmaThreads = 256;
+constexpr int kGemvMmaWarps = kGemvMmaThreads / 32;
+
+__device__ __forceinline__ void ld_stream_256(const void* ptr, uint32_t (&v)[8]) {
+  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "l"(ptr));
+}
+
+template <bool DUAL, bool STAGED>
+__global__ void __launch_bounds__(kGemvMmaThreads, 2) gemv_mma_kernel(
+    const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, float eps,
+    const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ w2, const float* __restrict__ bias,
+    const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ out, int M, int N, int K) {
+  constexpr int D = DUAL ? 2 : 1;
+  constexpr int U = DUAL ? 2 : 4;             // 64-wide blocks in flight per warp: 8 loads of 32 bytes per lane
+  extern __shared__ __align__(16) unsigned char gemv_smem[];                    // STAGED: [M][K] bf16, rows 16 bytes apart
+  __shared__ float red[2][kGemvMmaWarps][D][128];
+  __shared__ float part[kGemvMmaWarps];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int nblk = K >> 6;
+  const int tiles = (N + 15) >> 4;
+  const size_t row_bytes = static_cast<size_t>(K) * 2;
+  const size_t xs_stride = row_bytes + 16;    // the reads of two decode rows fall into different halves of the banks
+  {
+    // the first tile starts towards L2 before the kernel waits for the one in front of it
+    const int n0 = blockIdx.x * 16;
+    for (int r = warp; r < 16; r += kGemvMmaWarps) {
+      if (n0 + r < N) {
+        const char* p0 = reinterpret_cast<const char*>(w) + (n0 + r) * row_bytes;
+        const char* p1 = reinterpret_cast<const char*>(w2) + (n0 + r) * row_bytes;
+        for (size_t o = lane * 128; o < row_bytes; o += 32 * 128) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p0 + o));
+          if (DUAL) asm volatile("prefetch.global.L2 [%0];" ::"l"(p1 + o));
+        }
+      }
+    }
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");      // see the kernel above
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if constexpr (STAGED) {
+    // warps per decode row: all eight for one row, one for five rows and more
+    const int wpr = M == 1 ? 8 : M == 2 ? 4 : M <= 4 ? 2 : 1;
+    const int b = warp / wpr, in_row = (warp - b * wpr) * 32 + lane, step = wpr * 32, nv = K >> 3;
+    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(b) * K);
+    float ss = 0.f;
+    if (b < M) {
+#pragma unroll 4
+      for (int i = in_row; i < nv; i += step) {
+        float v[8];
+        unpack8(xr[i], v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
+      }
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) part[warp] = ss;
+    __syncthreads();
+    if (b < M) {
+      float sum = 0.f;
+      for (int i = 0; i < wpr; ++i) sum += part[b * wpr + i];
+      const float rs = rsqrtf(sum / K + eps);
+#pragma unroll 4
+      for (int i = in_row; i < nv; i += step) {
+        const float4 s0 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * i);
+        const float4 s1 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * i + 1);
+        const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        float v[8], o[8];
+        unpack8(xr[i], v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = v[e] * rs * sc[e];
+        *reinterpret_cast<uint4*>(gemv_smem + b * xs_stride + i * 16) = pack8(o);
+      }
+    }
+    __syncthreads();
+  }
+  const bool has_x = g < M;
+  const unsigned char* xrow = STAGED ? gemv_smem + (has_x ? g : 0) * xs_stride
+                                     : reinterpret_cast<const unsigned char*>(x) + (has_x ? g : 0) * row_bytes;
+  int buf = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1) {
+    // rows past N read the last row again; their sums are not stored
+    const size_t r0 = static_cast<size_t>(min(tile * 16 + g, N - 1)) * row_bytes + t * 32;
+    const size_t r1 = static_cast<size_t>(min(tile * 16 + g + 8, N - 1)) * row_bytes + t * 32;
+    float acc[D][4];
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[d][e] = 0.f;
+    for (int kb0 = warp; kb0 < nblk; kb0 += kGemvMmaWarps * U) {
+      uint32_t a0[U][D][8], a1[U][D][8];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t kb = static_cast<size_t>(min(kb0 + u * kGemvMmaWarps, nblk - 1)) * 128;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const char* base = reinterpret_cast<const char*>(d == 0 ? w : w2) + kb;
+          ld_stream_256(base + r0, a0[u][d]);
+          ld_stream_256(base + r1, a1[u][d]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int kb = kb0 + u * kGemvMmaWarps;
+        if (kb < nblk) {                                              // warp-uniform
+          uint4 b0 = make_uint4(0u, 0u, 0u, 0u), b1 = b0;
+          if (has_x) {
+            const uint4* xp = reinterpret_cast<const uint4*>(xrow + static_cast<size_t>(kb) * 128 + t * 32);
+            b0 = xp[0];
+            b1 = xp[1];
+          }
+          const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+          for (int d = 0; d < D; ++d)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              mma_bf16_16816(acc[d], a0[u][d][2 * i], a1[u][d][2 * i], a0[u][d][2 * i + 1], a1[u][d][2 * i + 1], bw[2 * i],
+                             bw[2 * i + 1]);
+        }
+      }
+    }
+    // sums as [decode row][weight row of the tile]
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      float* r = red[buf][warp][d];
+      r[(2 * t) * 16 + g] = acc[d][0];
+      r[(2 * t + 1) * 16 + g] = acc[d][1];
+      r[(2 * t) * 16 + g + 8] = acc[d][2];
+      r[(2 * t + 1) * 16 + g + 8] = acc[d][3];
+    }
+    __syncthreads();        // the other buffer is written before the next one, and read in front of it
+    if (threadIdx.x < 128) {
+      const int b = threadIdx.x >> 4, n = tile * 16 + (threadIdx.x & 15);
+      if (b < M && n < N) {
+        float s = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < kGemvMmaWarps; ++i) {
+          s += red[buf][i][0][threadIdx.x];
+          if (DUAL) s2 += red[buf][i][D - 1][threadIdx.x];
+        }
+        const long long o = static_cast<long long>(b) * N + n;
+        if (bias != nullptr) s += bias[n];
+        if (DUAL) {
+          const float gt = bf16_round(s), up = bf16_round(s2);
+          s = (gt / (1.0f + __expf(-gt))) * up;
+        }
+        if (res != nullptr) s = bf16_round(s) + __bfloat162float(res[o]);
+        out[o] = __float2bfloat16(s);
+      }
+    }
+  }
+}
+
+template <bool DUAL, bool STAGED>
+int launch_gemv_mma(const __nv_bfloat16* x, const float* gamma, float eps, const __nv_bfloat16* w,
+                    const __nv_bfloat16* w2, const float* bias, const __nv_bfloat16* res, __nv_bfloat16* out, int M,
+                    int N, int K, bool pdl, cudaStream_t st) {
+  auto kern = gemv_mma_kernel<DUAL, STAGED>;
+  const size_t smem = STAGED ? static_cast<size_t>(M) * (K * 2 + 16) : 0;
+  if (smem > 0 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvMaxSmem) != cudaSuccess)
+    return UBM_ERR_LAUNCH;
+  const int tiles = (N + 15) / 16;
+  const int slots = sm_count() * (smem > 90 * 1024 ? 1 : 2);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles < slots ? tiles : slots);
+  cfg.blockDim = dim3(kGemvMmaThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, kern, x, gamma, eps, w, w2, bias, res, out, M, N, K) != cudaSuccess) return UBM_ERR_LAUNCH;
+  UBM_CHECK_LAUNCH("gemv_mma_kernel");
+  return UBM_OK;
+}
+
 template <bool DUAL, bool W8>
 int launch_gemv(const __nv_bfloat16* x, const float* gamma, float eps, const __nv_bfloat16* w, const __nv_bfloat16* w2,
                 const float* bias, const __nv_bfloat16* res, __nv_bfloat16* out, int M, int N, int K, float wscale,
@@ -1487,6 +1676,13 @@ int launch_gemv(const __nv_bfloat16* x, const float* gamma, float eps, const __n
     const char* e = getenv("UBM_PDL");
     return e == nullptr || e[0] != '0';
   }();
+  if constexpr (!W8) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(w) | (DUAL ? reinterpret_cast<uintptr_t>(w2) : 0);
+    if ((K & 63) == 0 && (bits & 31) == 0 && static_cast<size_t>(M) * (K * 2 + 16) <= kGemvMaxSmem) {
+      return gamma != nullptr ? launch_gemv_mma<DUAL, true>(x, gamma, eps, w, w2, bias, res, out, M, N, K, pdl, st)
+                              : launch_gemv_mma<DUAL, false>(x, gamma, eps, w, w2, bias, res, out, M, N, K, pdl, st);
+    }
+  }
 #define UBM_GEMV(MBV)                                                                                          \
   do {                                                                                                         \
     auto kern = gemv_rows_kernel<MBV, DUAL, W8>;                                                               \
