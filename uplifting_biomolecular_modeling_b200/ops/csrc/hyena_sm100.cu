@@ -22,48 +22,91 @@
 namespace ubm {
 
 // ------------------------------------------------------------------------------------------ long operator
-constexpr int kPcThreads = 128;
-constexpr int kPcBatch = 8;      // positions whose loads are in flight together
+constexpr int kPcThreads = 128;  // a channel per thread
+constexpr int kPcRows = 16;      // positions per stage of the ring
+constexpr int kPcStages = 4;
 
-template <int S>
-__device__ __forceinline__ void load_poles(const float* __restrict__ src, long long c, int n, float (&v)[S]) {
+// Positions of 128 channels on their way into shared memory while earlier ones are worked on: a ring of [16 positions][128
+// channels] stages filled by 16-byte asynchronous copies, kPcStages - 1 of them in flight (12 to 24 KB per CTA), where a
+// thread that reads its own channel has 2-byte loads and as many in flight as it has registers for.  VEC = false (rows that
+// are not on 16 bytes): each thread fetches its own channel.
+template <bool VEC>
+__device__ __forceinline__ void pc_fetch(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ src, int c0, int d, int rows) {
+  if (VEC) {
 #pragma unroll
-  for (int k = 0; k < S; ++k) v[k] = k < n ? src[c * n + k] : 0.f;
+    for (int i = 0; i < kPcRows * 16 / kPcThreads; ++i) {
+      const int e = i * kPcThreads + threadIdx.x, r = e >> 4, c = (e & 15) * 8;
+      const bool ok = r < rows && c0 + c < d;     // else zeros are written
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * kPcThreads + c)),
+                   "l"(src + (ok ? static_cast<long long>(r) * d + c : 0)), "r"(ok ? 16 : 0)
+                   : "memory");
+    }
+  } else if (c0 + static_cast<int>(threadIdx.x) < d) {
+#pragma unroll
+    for (int r = 0; r < kPcRows; ++r)
+      if (r < rows) dst[r * kPcThreads + threadIdx.x] = src[static_cast<long long>(r) * d + threadIdx.x];
+  }
+}
+__device__ __forceinline__ void pc_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void pc_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// two poles per packed fp32 instruction
 template <int S>
+__device__ __forceinline__ void load_poles(const float* __restrict__ src, long long c, int n, bool ok, float2 (&v)[S / 2]) {
+#pragma unroll
+  for (int k = 0; k < S; k += 2)
+    v[k / 2] = make_float2(ok && k < n ? src[c * n + k] : 0.f, ok && k + 1 < n ? src[c * n + k + 1] : 0.f);
+}
+
+template <int S, bool VEC>
 __global__ void __launch_bounds__(kPcThreads) pole_chunk_kernel(const __nv_bfloat16* __restrict__ u,
                                                                 const float* __restrict__ lam, float* __restrict__ part,
                                                                 int L, int d, int n, int chunk) {
-  const int c = blockIdx.x * kPcThreads + threadIdx.x;
-  if (c >= d) return;
+  __shared__ __align__(16) __nv_bfloat16 ring[kPcStages][kPcRows * kPcThreads];
+  const int c0 = blockIdx.x * kPcThreads, c = c0 + threadIdx.x;
+  const bool ok = c < d;
   const int t0 = blockIdx.y * chunk, t1 = min(L, t0 + chunk);
+  const int stages = (t1 - t0 + kPcRows - 1) / kPcRows;
   const long long b = blockIdx.z;
-  float lm[S], st[S];
-  load_poles<S>(lam, c, n, lm);
+  const __nv_bfloat16* up = u + (b * L + t0) * d + c0;
 #pragma unroll
-  for (int k = 0; k < S; ++k) st[k] = 0.f;
-  const __nv_bfloat16* up = u + (b * L + t0) * d + c;
-  int t = t0;
-  for (; t + kPcBatch <= t1; t += kPcBatch) {
-    float uv[kPcBatch];
-#pragma unroll
-    for (int i = 0; i < kPcBatch; ++i) uv[i] = __bfloat162float(up[static_cast<long long>(i) * d]);
-    up += static_cast<long long>(kPcBatch) * d;
-#pragma unroll
-    for (int i = 0; i < kPcBatch; ++i)
-#pragma unroll
-      for (int k = 0; k < S; ++k) st[k] = fmaf(st[k], lm[k], uv[i]);
+  for (int s = 0; s < kPcStages - 1; ++s) {
+    if (s < stages) pc_fetch<VEC>(ring[s], up + static_cast<long long>(s) * kPcRows * d, c0, d, t1 - t0 - s * kPcRows);
+    pc_commit();
   }
-  for (; t < t1; ++t, up += d) {
-    const float uv = __bfloat162float(*up);
+  float2 lm[S / 2], st[S / 2];
+  load_poles<S>(lam, c, n, ok, lm);
 #pragma unroll
-    for (int k = 0; k < S; ++k) st[k] = fmaf(st[k], lm[k], uv);
+  for (int k = 0; k < S / 2; ++k) st[k] = make_float2(0.f, 0.f);
+  for (int s = 0; s < stages; ++s) {
+    pc_wait<kPcStages - 2>();
+    __syncthreads();            // everybody's part of stage s has landed, everybody is done with stage s - 1
+    const int nx = s + kPcStages - 1;
+    if (nx < stages)
+      pc_fetch<VEC>(ring[nx % kPcStages], up + static_cast<long long>(nx) * kPcRows * d, c0, d, t1 - t0 - nx * kPcRows);
+    pc_commit();
+    const __nv_bfloat16* r = ring[s % kPcStages] + threadIdx.x;
+    const int rows = min(kPcRows, t1 - t0 - s * kPcRows);
+    auto step = [&](int i) {
+      const float uv = __bfloat162float(r[i * kPcThreads]);
+#pragma unroll
+      for (int k = 0; k < S / 2; ++k) st[k] = __ffma2_rn(st[k], lm[k], make_float2(uv, uv));
+    };
+    if (rows == kPcRows) {
+#pragma unroll
+      for (int i = 0; i < kPcRows; ++i) step(i);
+    } else {
+      for (int i = 0; i < rows; ++i) step(i);
+    }
   }
+  if (!ok) return;
   float* o = part + ((b * gridDim.y + blockIdx.y) * d + c) * n;
 #pragma unroll
   for (int k = 0; k < S; ++k)
-    if (k < n) o[k] = st[k];
+    if (k < n) o[k] = (k & 1) ? st[k / 2].y : st[k / 2].x;
 }
 
 // part [B][nch][d * n]: chunk end states in, chunk start states out; state [B][d * n]: the state after position L - 1.
@@ -92,56 +135,61 @@ __global__ void __launch_bounds__(256) pole_carry_kernel(float* __restrict__ par
   state[i] = run;
 }
 
-template <int S>
+template <int S, bool VEC>
 __global__ void __launch_bounds__(kPcThreads) pole_apply_kernel(
     const __nv_bfloat16* __restrict__ u, const float* __restrict__ lam, const float* __restrict__ res,
     const float* __restrict__ part, const float* __restrict__ D, const __nv_bfloat16* __restrict__ x2,
     __nv_bfloat16* __restrict__ out, int L, int d, int n, int chunk) {
-  const int c = blockIdx.x * kPcThreads + threadIdx.x;
-  if (c >= d) return;
+  __shared__ __align__(16) __nv_bfloat16 ring[kPcStages][2][kPcRows * kPcThreads];
+  const int c0 = blockIdx.x * kPcThreads, c = c0 + threadIdx.x;
+  const bool ok = c < d, gated = x2 != nullptr;
   const int t0 = blockIdx.y * chunk, t1 = min(L, t0 + chunk);
+  const int stages = (t1 - t0 + kPcRows - 1) / kPcRows;
   const long long b = blockIdx.z;
-  float lm[S], rs[S], st[S];
-  load_poles<S>(lam, c, n, lm);
-  load_poles<S>(res, c, n, rs);
-  load_poles<S>(part + (b * gridDim.y + blockIdx.y) * d * n, c, n, st);
-  const float dv = D[c];
-  const long long o0 = (b * L + t0) * d + c;
-  const __nv_bfloat16* up = u + o0;
-  const __nv_bfloat16* gp = x2 == nullptr ? nullptr : x2 + o0;
-  __nv_bfloat16* op = out + o0;
-  auto one = [&](float uv, float g) {
-    float y0 = 0.f, y1 = 0.f;
-#pragma unroll
-    for (int k = 0; k < S; k += 2) {
-      st[k] = fmaf(st[k], lm[k], uv);
-      st[k + 1] = fmaf(st[k + 1], lm[k + 1], uv);
-      y0 = fmaf(st[k], rs[k], y0);
-      y1 = fmaf(st[k + 1], rs[k + 1], y1);
-    }
-    // rounded where the transform form rounds: the convolution, the sum with the skip term, the gated product
-    const float conv = __bfloat162float(__float2bfloat16(y0 + y1));
-    return __float2bfloat16(g * __bfloat162float(__float2bfloat16(conv + uv * dv)));
+  const long long o0 = (b * L + t0) * d + c0;
+  auto fetch = [&](int s) {
+    const long long at = o0 + static_cast<long long>(s) * kPcRows * d;
+    pc_fetch<VEC>(ring[s % kPcStages][0], u + at, c0, d, t1 - t0 - s * kPcRows);
+    if (gated) pc_fetch<VEC>(ring[s % kPcStages][1], x2 + at, c0, d, t1 - t0 - s * kPcRows);
   };
-  int t = t0;
-  for (; t + kPcBatch <= t1; t += kPcBatch) {
-    float uv[kPcBatch], g[kPcBatch];
 #pragma unroll
-    for (int i = 0; i < kPcBatch; ++i) {
-      uv[i] = __bfloat162float(up[static_cast<long long>(i) * d]);
-      g[i] = gp == nullptr ? 1.f : __bfloat162float(gp[static_cast<long long>(i) * d]);
-    }
-#pragma unroll
-    for (int i = 0; i < kPcBatch; ++i) op[static_cast<long long>(i) * d] = one(uv[i], g[i]);
-    up += static_cast<long long>(kPcBatch) * d;
-    op += static_cast<long long>(kPcBatch) * d;
-    if (gp != nullptr) gp += static_cast<long long>(kPcBatch) * d;
+  for (int s = 0; s < kPcStages - 1; ++s) {
+    if (s < stages) fetch(s);
+    pc_commit();
   }
-  for (; t < t1; ++t) {
-    *op = one(__bfloat162float(*up), gp == nullptr ? 1.f : __bfloat162float(*gp));
-    up += d;
-    op += d;
-    if (gp != nullptr) gp += d;
+  float2 lm[S / 2], rs[S / 2], st[S / 2];
+  load_poles<S>(lam, c, n, ok, lm);
+  load_poles<S>(res, c, n, ok, rs);
+  load_poles<S>(part + (b * gridDim.y + blockIdx.y) * d * n, c, n, ok, st);
+  const float dv = ok ? D[c] : 0.f;
+  __nv_bfloat16* op = out + o0 + threadIdx.x;
+  for (int s = 0; s < stages; ++s) {
+    pc_wait<kPcStages - 2>();
+    __syncthreads();            // as above
+    if (s + kPcStages - 1 < stages) fetch(s + kPcStages - 1);
+    pc_commit();
+    const __nv_bfloat16* r = ring[s % kPcStages][0] + threadIdx.x;
+    const int rows = min(kPcRows, t1 - t0 - s * kPcRows);
+    auto step = [&](int i) {
+      const float uv = __bfloat162float(r[i * kPcThreads]);
+      const float g = gated ? __bfloat162float(r[(kPcRows + i) * kPcThreads]) : 1.f;
+      float2 y = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < S / 2; ++k) {
+        st[k] = __ffma2_rn(st[k], lm[k], make_float2(uv, uv));
+        y = __ffma2_rn(st[k], rs[k], y);
+      }
+      // rounded where the transform form rounds: the convolution, the sum with the skip term, the gated product
+      const float conv = __bfloat162float(__float2bfloat16(y.x + y.y));
+      if (ok) op[static_cast<long long>(i) * d] = __float2bfloat16(g * __bfloat162float(__float2bfloat16(conv + uv * dv)));
+    };
+    if (rows == kPcRows) {
+#pragma unroll
+      for (int i = 0; i < kPcRows; ++i) step(i);
+    } else {
+      for (int i = 0; i < rows; ++i) step(i);
+    }
+    op += static_cast<long long>(kPcRows) * d;
   }
 }
 
@@ -314,20 +362,29 @@ extern "C" int ubm_pole_conv_gate(const void* u, const void* lam, const void* re
   auto* uu = static_cast<const __nv_bfloat16*>(u);
   auto* ll = static_cast<const float*>(lam);
   auto* pp = static_cast<float*>(part);
-#define UBM_POLE_CONV(SS)                                                                                       \
+  // 16-byte copies need every row on 16 bytes
+  const bool vec = (d & 7) == 0 && ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(x2)) & 15) == 0;
+#define UBM_POLE_CONV(SS, VEC)                                                                                  \
   do {                                                                                                          \
-    pole_chunk_kernel<SS><<<grid, kPcThreads, 0, st>>>(uu, ll, pp, L, d, S, chunk);                             \
+    pole_chunk_kernel<SS, VEC><<<grid, kPcThreads, 0, st>>>(uu, ll, pp, L, d, S, chunk);                        \
     pole_carry_kernel<<<static_cast<unsigned>((B * dn + 255) / 256), 256, 0, st>>>(                             \
         pp, ll, static_cast<float*>(state), B, dn, L, chunk, nch);                                              \
     if (out != nullptr)                                                                                         \
-      pole_apply_kernel<SS><<<grid, kPcThreads, 0, st>>>(uu, ll, static_cast<const float*>(res), pp,              \
-                                                       static_cast<const float*>(D),                            \
-                                                       static_cast<const __nv_bfloat16*>(x2),                   \
-                                                       static_cast<__nv_bfloat16*>(out), L, d, S, chunk);       \
+      pole_apply_kernel<SS, VEC><<<grid, kPcThreads, 0, st>>>(                                                  \
+          uu, ll, static_cast<const float*>(res), pp, static_cast<const float*>(D),                             \
+          static_cast<const __nv_bfloat16*>(x2), static_cast<__nv_bfloat16*>(out), L, d, S, chunk);             \
   } while (0)
-  if (S <= 4) UBM_POLE_CONV(4);
-  else if (S <= 8) UBM_POLE_CONV(8);
-  else UBM_POLE_CONV(16);
+#define UBM_POLE_CONV_S(SS)     \
+  do {                          \
+    if (vec)                    \
+      UBM_POLE_CONV(SS, true);  \
+    else                        \
+      UBM_POLE_CONV(SS, false); \
+  } while (0)
+  if (S <= 4) UBM_POLE_CONV_S(4);
+  else if (S <= 8) UBM_POLE_CONV_S(8);
+  else UBM_POLE_CONV_S(16);
+#undef UBM_POLE_CONV_S
 #undef UBM_POLE_CONV
   UBM_CHECK_LAUNCH("pole_conv kernels");
   return UBM_OK;
