@@ -228,23 +228,54 @@ __global__ void __launch_bounds__(kTpThreads, 2) fir_toeplitz_kernel(const __nv_
   __nv_bfloat16* st1 = st0 + 2 * kTpCh * kTpTapW;
   const int c0 = blockIdx.x * kTpCh, t0 = blockIdx.y * kTpPos;
   const long long base = static_cast<long long>(blockIdx.z) * L * d;
-  for (int i = threadIdx.x; i < kTpCh * 2 * kTpTapW; i += kTpThreads) {
-    const int ch = i % kTpCh, x = i / kTpCh;                // lanes over channels: the tap rows are read coalesced
-    auto tap = [&](int k) { return k >= 0 && k < K && c0 + ch < d ? ht[static_cast<long long>(k) * d + c0 + ch] : 0.f; };
-    st0[ch * 2 * kTpTapW + x] = __float2bfloat16(tap(kTap0 - x));
-    st1[ch * 2 * kTpTapW + x] = __float2bfloat16(tap(kTap0 - x - 1));
-  }
-  uint32_t odd = 0;                                         // a word with an infinite or NaN half was seen
-  for (int i = threadIdx.x; i < (kTpPos + kTpHalo) / 2 * (kTpCh / 8); i += kTpThreads) {
+  // Every phase requests all it reads before it uses any of it: with one access in flight per thread and loop step, the
+  // taps (each read twice, once per copy), the inputs and the gates took 42, 5 and 4 trips to memory one after another.
+  constexpr int kUBatch = (kTpPos + kTpHalo) / 2 * (kTpCh / 8) / kTpThreads;
+  static_assert(kUBatch * kTpThreads == (kTpPos + kTpHalo) / 2 * (kTpCh / 8), "whole batches");
+  uint4 uv[kUBatch][2];
+#pragma unroll
+  for (int j = 0; j < kUBatch; ++j) {
+    const int i = j * kTpThreads + threadIdx.x;
     const int g8 = (i & 3) * 8, p = i >> 2;                 // eight channels, two positions
     const int l = t0 - kTpHalo + 2 * p;
-    uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0;
-    if (c0 + g8 < d) {
-      const __nv_bfloat16* src = u + base + static_cast<long long>(l) * d + c0 + g8;
-      if (l >= 0 && l < L) v0 = *reinterpret_cast<const uint4*>(src);
-      if (l + 1 >= 0 && l + 1 < L) v1 = *reinterpret_cast<const uint4*>(src + d);
+    const __nv_bfloat16* src = u + base + static_cast<long long>(l) * d + c0 + g8;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      uv[j][r] = c0 + g8 < d && l + r >= 0 && l + r < L
+                     ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<long long>(r) * d))
+                     : make_uint4(0u, 0u, 0u, 0u);
+  }
+  {
+    constexpr int kTapBatch = kTpHalo * kTpCh / kTpThreads;
+    float tap[kTapBatch];
+    const int ch = threadIdx.x % kTpCh, k0 = threadIdx.x / kTpCh;   // lanes over channels: the tap rows are read coalesced
+#pragma unroll
+    for (int j = 0; j < kTapBatch; ++j) {
+      const int k = j * (kTpThreads / kTpCh) + k0;
+      tap[j] = k < K && c0 + ch < d ? __ldg(ht + static_cast<long long>(k) * d + c0 + ch) : 0.f;
     }
-    const uint32_t a[4] = {v0.x, v0.y, v0.z, v0.w}, b[4] = {v1.x, v1.y, v1.z, v1.w};
+    __nv_bfloat16* r0 = st0 + ch * 2 * kTpTapW;
+    __nv_bfloat16* r1 = st1 + ch * 2 * kTpTapW;
+#pragma unroll
+    for (int j = 0; j < kTapBatch; ++j) {
+      const int k = j * (kTpThreads / kTpCh) + k0;
+      const __nv_bfloat16 h = __float2bfloat16(tap[j]);
+      r0[kTap0 - k] = h;
+      r1[kTap0 - 1 - k] = h;
+    }
+    // zeros before the last and behind the first tap (copy 0: 16 + 24 of its 168, copy 1: 15 + 25)
+    for (int z = k0; z < 2 * kTpTapW - kTpHalo; z += kTpThreads / kTpCh) {
+      r0[z < kTap0 + 1 - kTpHalo ? z : z + kTpHalo] = __float2bfloat16(0.f);
+      r1[z < kTap0 - kTpHalo ? z : z + kTpHalo] = __float2bfloat16(0.f);
+    }
+  }
+  uint32_t odd = 0;                                         // a word with an infinite or NaN half was seen
+#pragma unroll
+  for (int j = 0; j < kUBatch; ++j) {
+    const int i = j * kTpThreads + threadIdx.x;
+    const int g8 = (i & 3) * 8, p = i >> 2;
+    const uint32_t a[4] = {uv[j][0].x, uv[j][0].y, uv[j][0].z, uv[j][0].w};
+    const uint32_t b[4] = {uv[j][1].x, uv[j][1].y, uv[j][1].z, uv[j][1].w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       odd |= (__vcmpeq2(a[e] & 0x7F807F80u, 0x7F807F80u) | __vcmpeq2(b[e] & 0x7F807F80u, 0x7F807F80u));
@@ -317,30 +348,44 @@ __global__ void __launch_bounds__(kTpThreads, 2) fir_toeplitz_kernel(const __nv_
         *at = __float2bfloat16(conv + __bfloat162float(*at) * dv);
       }
   }
+  constexpr int kOBatch = kTpPos / 2 * (kTpCh / 8) / kTpThreads;
+  static_assert(kOBatch * kTpThreads == kTpPos / 2 * (kTpCh / 8), "whole batches");
+  uint4 gv[kOBatch][2];
+#pragma unroll
+  for (int j = 0; j < kOBatch; ++j) {
+    const int i = j * kTpThreads + threadIdx.x;
+    const int g8 = (i & 3) * 8, l = t0 + 2 * (i >> 2);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      gv[j][r] = x2 != nullptr && l + r < L && c0 + g8 < d
+                     ? __ldg(reinterpret_cast<const uint4*>(x2 + base + static_cast<long long>(l + r) * d + c0 + g8))
+                     : make_uint4(0u, 0u, 0u, 0u);
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < kTpPos / 2 * (kTpCh / 8); i += kTpThreads) {
+#pragma unroll
+  for (int j = 0; j < kOBatch; ++j) {
+    const int i = j * kTpThreads + threadIdx.x;
     const int g8 = (i & 3) * 8, p = i >> 2;
     const int l = t0 + 2 * p;
     if (l >= L || c0 + g8 >= d) continue;
-    uint32_t a[4], b[4];
+    uint32_t v[2][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const uint32_t w0 = su[(g8 + 2 * e) * kTpW + kTpHalo / 2 + p], w1 = su[(g8 + 2 * e + 1) * kTpW + kTpHalo / 2 + p];
-      a[e] = __byte_perm(w0, w1, 0x5410);
-      b[e] = __byte_perm(w0, w1, 0x7632);
+      v[0][e] = __byte_perm(w0, w1, 0x5410);
+      v[1][e] = __byte_perm(w0, w1, 0x7632);
     }
-    const long long o = base + static_cast<long long>(l) * d + c0 + g8;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       if (l + r >= L) break;
-      uint32_t* v = r ? b : a;
       if (x2 != nullptr) {
-        const uint4 gv = *reinterpret_cast<const uint4*>(x2 + o + static_cast<long long>(r) * d);
-        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+        const uint32_t gw[4] = {gv[j][r].x, gv[j][r].y, gv[j][r].z, gv[j][r].w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = pack_bf16x2(bf16_lo(gw[e]) * bf16_lo(v[e]), bf16_hi(gw[e]) * bf16_hi(v[e]));
+        for (int e = 0; e < 4; ++e)
+          v[r][e] = pack_bf16x2(bf16_lo(gw[e]) * bf16_lo(v[r][e]), bf16_hi(gw[e]) * bf16_hi(v[r][e]));
       }
-      *reinterpret_cast<uint4*>(out + o + static_cast<long long>(r) * d) = make_uint4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<uint4*>(out + base + static_cast<long long>(l + r) * d + c0 + g8) =
+          make_uint4(v[r][0], v[r][1], v[r][2], v[r][3]);
     }
   }
 }
