@@ -65,10 +65,14 @@ class OuterProductMean(_Switchable):
         # The mean over sequences: the first GEMM carries 1/S; where sequences are masked the per-pair count
         # differs from S and the (linear) output projection is rescaled by S / count afterwards, on 128
         # channels instead of c*c.
-        scale = None
+        count = None
         if not self.full_mask:
-            cnt = torch.einsum("si,sj->ij", mask[0].float(), mask[0].float()).clamp(min=1.0)
-            scale = (float(S) / cnt).unsqueeze(-1)
+            mk = mask[0].expand(S, N)
+            if mk.dtype == torch.bfloat16 and N % 8 == 0:       # bf16 values: exact products, fp32 sums
+                mk = mk.contiguous()
+                count = gemm.gemm(mk, mk, mn_major=True, out_dtype=torch.float32)
+            else:
+                count = torch.einsum("si,sj->ij", mk.float(), mk.float())
         rb = self.row_block
         blocked = c == 32 and (N * c) % 32 == 0
         t2 = torch.empty((rb * N, c * c), dtype=torch.bfloat16, device=m.device)
@@ -83,11 +87,11 @@ class OuterProductMean(_Switchable):
             else:
                 t = gemm.gemm(a2[:, i0 * c:i1 * c], b2, mn_major=True, alpha=1.0 / S)
                 t = t.view(i1 - i0, c, N, c).permute(0, 2, 1, 3).reshape(nr, c * c)
-            if scale is None:
-                gemm.gemm(t, wo, bias=bo, out=out[i0:i1].view(nr, -1))
-            else:
-                o = gemm.gemm(t, wo).view(i1 - i0, N, -1)
-                out[i0:i1] = (o.float() * scale[i0:i1] + bo).to(torch.bfloat16)
+            gemm.gemm(t, wo, bias=bo if count is None else None, out=out[i0:i1].view(nr, -1))
+        if count is not None and out.shape[-1] % 8 == 0:
+            rows.mean_rescale_(out.view(N * N, -1), count.contiguous().view(-1), bo.contiguous(), S)
+        elif count is not None:
+            out = (out.float() * (S / count.clamp(min=1.0)).unsqueeze(-1) + bo).to(torch.bfloat16)
         return out.unsqueeze(0)
 
 

@@ -128,6 +128,26 @@ __global__ void __launch_bounds__(256) layernorm_rows_wide_kernel(const __nv_bfl
   }
 }
 
+// o[r] = bf16(o[r] * total / max(count[r], 1) + bias), in place: the mean over the sequences that two tokens share, behind a
+// product that carried 1 / total.  One pass over the rows where tensor statements took five and two fp32 copies.
+__global__ void __launch_bounds__(256) mean_rescale_kernel(__nv_bfloat16* __restrict__ o, const float* __restrict__ count,
+                                                           const float* __restrict__ bias, long long vecs, int vpr,
+                                                           float total) {
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < vecs;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long r = i / vpr;
+    const int c = static_cast<int>(i - r * vpr) * 8;
+    const float sc = total / fmaxf(__ldg(count + r), 1.f);
+    const float4 b0 = __ldg(reinterpret_cast<const float4*>(bias + c)), b1 = __ldg(reinterpret_cast<const float4*>(bias + c) + 1);
+    uint4 u = reinterpret_cast<uint4*>(o)[i];
+    u.x = pack_bf16x2(bf16_lo(u.x) * sc + b0.x, bf16_hi(u.x) * sc + b0.y);
+    u.y = pack_bf16x2(bf16_lo(u.y) * sc + b0.z, bf16_hi(u.y) * sc + b0.w);
+    u.z = pack_bf16x2(bf16_lo(u.z) * sc + b1.x, bf16_hi(u.z) * sc + b1.y);
+    u.w = pack_bf16x2(bf16_lo(u.w) * sc + b1.z, bf16_hi(u.w) * sc + b1.w);
+    reinterpret_cast<uint4*>(o)[i] = u;
+  }
+}
+
 // LayerNorm of narrow bf16 rows with 16-byte accesses: C = 8 * LPR channels, LPR lanes per row (8, 16 or 32),
 // 32 / LPR rows per warp instruction; statistics by xor-shuffles inside the LPR lanes of a row.  The MSA track
 // (C = 64, 1.5 M rows per call) spends its LayerNorms here.
@@ -668,6 +688,19 @@ extern "C" int ubm_layernorm_rows(const void* x, const void* gamma, const void* 
 #undef UBM_LN_BY_WIDTH
 #undef UBM_LN_LAUNCH
   UBM_CHECK_LAUNCH("layernorm_rows_kernel");
+  return UBM_OK;
+}
+
+// o: bf16 [R][C] in place (C a multiple of 8, rows on 16 bytes); count: fp32 [R]; bias: fp32 [C]
+extern "C" int ubm_mean_rescale(void* o, const void* count, const void* bias, long long R, int C, float total,
+                                void* stream) {
+  using namespace ubm;
+  if (R <= 0 || C <= 0 || (C & 7) || ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(bias)) & 15))
+    return UBM_ERR_ARGUMENT;
+  const long long vecs = R * (C / 8);
+  mean_rescale_kernel<<<grid_for(vecs, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<__nv_bfloat16*>(o), static_cast<const float*>(count), static_cast<const float*>(bias), vecs, C / 8, total);
+  UBM_CHECK_LAUNCH("mean_rescale_kernel");
   return UBM_OK;
 }
 

@@ -19,6 +19,7 @@ native.declare("ubm_swiglu_rows", [c_void_p] * 2 + [c_ll, c_int, c_void_p])
 native.declare("ubm_swiglu3_rows", [c_void_p] * 2 + [c_ll, c_int, c_void_p])
 native.declare("ubm_segment_mean", [c_void_p] * 3 + [c_int] * 5 + [c_void_p])
 native.declare("ubm_gather_rows_add", [c_void_p] * 4 + [c_int] * 4 + [c_void_p])
+native.declare("ubm_mean_rescale", [c_void_p] * 3 + [c_ll, c_int, c_float, c_void_p])
 
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 
@@ -55,6 +56,19 @@ def layernorm_rows(x: torch.Tensor, weight: Optional[torch.Tensor], bias: Option
                                          float(eps), _DT[x.dtype], _DT[out_dtype], native.current_stream(x.device))
     native.check(rc, "ubm_layernorm_rows")
     return out
+
+
+def mean_rescale_(o: torch.Tensor, count: torch.Tensor, bias: torch.Tensor, total: float) -> torch.Tensor:
+    """o[r] = o[r] * total / max(count[r], 1) + bias in place.  o: bf16 [R, C], contiguous; count: R fp32 elements;
+    bias: fp32 [C]."""
+    R, C = o.shape
+    if o.dtype != torch.bfloat16 or not o.is_contiguous() or count.dtype != torch.float32 or count.numel() != R or \
+            not count.is_contiguous() or bias.dtype != torch.float32 or bias.shape != (C,) or not bias.is_contiguous():
+        raise ValueError(f"mean_rescale_ expects bf16 rows with {R} fp32 counts and {C} fp32 biases")
+    rc = native.lib().ubm_mean_rescale(native.ptr(o), native.ptr(count), native.ptr(bias), R, C, float(total),
+                                       native.current_stream(o.device))
+    native.check(rc, "ubm_mean_rescale")
+    return o
 
 
 _HB_CACHE = {}
