@@ -1,0 +1,69 @@
+"""GEMM tiles shared by two SMs: edges of the 256 x 256 tile and of the k-blocks, both operand layouts, batches and every
+epilogue that has one."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _r(seed, *shape):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(*shape, device="cuda", generator=g).bfloat16()
+
+
+def _close(got, want):
+    # fp32 sums of exact products, one rounding to bf16
+    assert (got.double() - want).norm() <= 1.1 * 2.0 ** -9 * want.norm()
+    assert not ((got.double() - want).abs() > 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).any()
+
+
+@pytest.mark.parametrize("M,N", [(1024, 4096), (4864, 1000), (1153, 4104), (2304, 2176), (4000, 4640)])
+@pytest.mark.parametrize("K", [64, 72, 840])
+@pytest.mark.parametrize("mn_major", [False, True])
+def test_plain(M, N, K, mn_major):
+    from uplifting_biomolecular_modeling_b200.ops import gemm, native
+    Mp, Np, Kp = (-(-v // 8) * 8 for v in (M, N, K))
+    a = _r(M, K, Mp)[:, :M] if mn_major else _r(M, M, Kp)[:, :K]
+    b = _r(N, K, Np)[:, :N] if mn_major else _r(N, N, Kp)[:, :K]
+    bias, res = torch.randn(N, device="cuda"), _r(5, M, Np)[:, :N]
+    prod = (a.double().T @ b.double()) if mn_major else a.double() @ b.double().T
+    _close(gemm.gemm(a, b, mn_major=mn_major), prod)
+    _close(gemm.gemm(a, b, mn_major=mn_major, bias=bias, residual=res, alpha=0.5), 0.5 * prod + bias.double() + res.double())
+    native.raise_on_status("cuda", "gemm")
+
+
+@pytest.mark.parametrize("n", [200, 257, 300, 513])
+@pytest.mark.parametrize("mn_major", [False, True])
+def test_batch(n, mn_major):
+    from uplifting_biomolecular_modeling_b200.ops import gemm, native
+    ld = -(-n // 8) * 8
+    a, b = _r(1, 128, n, ld)[:, :, :n], _r(2, 128, n, ld)[:, :, :n]
+    out = torch.zeros(128, n, ld, device="cuda", dtype=torch.bfloat16)
+    gemm.gemm(a, b, mn_major=mn_major, out=out[:, :, :n])
+    native.raise_on_status("cuda", "gemm")
+    want = torch.bmm(a.double().transpose(1, 2), b.double()) if mn_major else torch.bmm(a.double(), b.double().transpose(1, 2))
+    _close(out[:, :, :n], want)
+    assert not out[:, :, n:].any()
+
+
+@pytest.mark.parametrize("tokens,sequences", [(40, 24), (96, 136)])
+def test_blocked_outer_product(tokens, sequences):
+    from uplifting_biomolecular_modeling_b200.ops import gemm, native
+    a, b = _r(3, sequences, tokens * 32), _r(4, sequences, tokens * 32)
+    out = torch.empty(tokens * tokens, 1024, device="cuda", dtype=torch.bfloat16)
+    gemm.gemm(a, b, mn_major=True, out=out, c_blocked=(tokens * 1024, 32, 1024))
+    native.raise_on_status("cuda", "gemm")
+    want = torch.einsum("sic,sjd->ijcd", a.double().view(sequences, tokens, 32), b.double().view(sequences, tokens, 32))
+    _close(out, want.reshape(tokens * tokens, 1024))
+
+
+@pytest.mark.parametrize("M,hidden,K", [(2050, 2048, 136), (4100, 1056, 64)])
+def test_swiglu(M, hidden, K):
+    from uplifting_biomolecular_modeling_b200.ops import gemm, native
+    x, wg, wv = _r(6, M, K), _r(7, hidden, K) * K ** -0.5, _r(8, hidden, K) * K ** -0.5
+    got = gemm.gemm(x, gemm.pack_swiglu(wg, wv), act="swiglu")
+    native.raise_on_status("cuda", "gemm")
+    want = F.silu(x.double() @ wg.double().T) * (x.double() @ wv.double().T)
+    # the gate's sigmoid has a relative error of 2e-4
+    assert (got.double() - want).norm() <= 1.5 * 2.0 ** -9 * want.norm()
