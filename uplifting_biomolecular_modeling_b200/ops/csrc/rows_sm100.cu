@@ -74,7 +74,9 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restric
 
 // LayerNorm of wide bf16 rows (256 < C <= 2048, C a multiple of 8): one warp per row, 16-byte accesses, the row kept
 // in registers (CHUNKS x 8 values per lane).  The single / token tracks and the LM and genomics trunks land here.
-template <int CHUNKS>
+// VEC: gamma and beta start on 32 bytes (or are absent) and a lane takes its eight values of each in one load.  One value at a
+// time, 32 bytes between lanes, the 64 loads of a row of 960 channels took 512 wavefronts of L1.
+template <int CHUNKS, bool VEC>
 __global__ void __launch_bounds__(256) layernorm_rows_wide_kernel(const __nv_bfloat16* __restrict__ x,
                                                                   const float* __restrict__ gamma,
                                                                   const float* __restrict__ beta,
@@ -114,12 +116,16 @@ __global__ void __launch_bounds__(256) layernorm_rows_wide_kernel(const __nv_bfl
     for (int k = 0; k < CHUNKS; ++k) {
       const int c = k * 256 + lane * 8;
       if (c < C) {
-        float y[8];
+        float y[8], gm[8], bt[8];
+        if (VEC) {
+          if (gamma != nullptr) ld_f32x8(gamma + c, gm);
+          if (beta != nullptr) ld_f32x8(beta + c, bt);
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           y[j] = (v[k][j] - mu) * rstd;
-          if (gamma != nullptr) y[j] *= gamma[c + j];
-          if (beta != nullptr) y[j] += beta[c + j];
+          if (gamma != nullptr) y[j] *= VEC ? gm[j] : gamma[c + j];
+          if (beta != nullptr) y[j] += VEC ? bt[j] : beta[c + j];
         }
         *reinterpret_cast<uint4*>(out + r * C + c) = make_uint4(pack_bf16x2(y[0], y[1]), pack_bf16x2(y[2], y[3]),
                                                                 pack_bf16x2(y[4], y[5]), pack_bf16x2(y[6], y[7]));
@@ -642,9 +648,15 @@ extern "C" int ubm_layernorm_rows(const void* x, const void* gamma, const void* 
     const float* gg = static_cast<const float*>(gamma);
     const float* bb = static_cast<const float*>(beta);
     const int gridw = grid_for(R, 8);
-    if (C <= 512) layernorm_rows_wide_kernel<2><<<gridw, 256, 0, st>>>(xx, gg, bb, oo, R, C, eps);
-    else if (C <= 1024) layernorm_rows_wide_kernel<4><<<gridw, 256, 0, st>>>(xx, gg, bb, oo, R, C, eps);
-    else layernorm_rows_wide_kernel<8><<<gridw, 256, 0, st>>>(xx, gg, bb, oo, R, C, eps);
+    const bool vec = ((reinterpret_cast<uintptr_t>(gg) | reinterpret_cast<uintptr_t>(bb)) & 31) == 0;
+#define UBM_LN_WIDE(CH)                                                                                          \
+  (vec ? layernorm_rows_wide_kernel<CH, true><<<gridw, 256, 0, st>>>(xx, gg, bb, oo, R, C, eps)                  \
+       : layernorm_rows_wide_kernel<CH, false><<<gridw, 256, 0, st>>>(xx, gg, bb, oo, R, C, eps))
+    if (C <= 512) UBM_LN_WIDE(2);
+    else if (C <= 1024) UBM_LN_WIDE(4);
+    else if (C <= 1280) UBM_LN_WIDE(5);
+    else UBM_LN_WIDE(8);
+#undef UBM_LN_WIDE
     UBM_CHECK_LAUNCH("layernorm_rows_wide_kernel");
     return UBM_OK;
   }

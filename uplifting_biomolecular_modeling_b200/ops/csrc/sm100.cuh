@@ -585,6 +585,14 @@ __device__ __forceinline__ void ld_global_256(const void* ptr, uint4& a, uint4& 
                : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                : "l"(ptr));
 }
+// eight fp32 values (32-byte aligned) in one load
+__device__ __forceinline__ void ld_f32x8(const float* src, float (&e)[8]) {
+  uint4 a, b;
+  ld_global_256(src, a, b);
+  const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) e[j] = __uint_as_float(w[j]);
+}
 // 16 fp32 values -> 16 bf16 = 32 bytes, one store.  A lane that writes half a sector (16 bytes) per
 // instruction, as a row-per-lane epilogue does with 16-byte stores, costs the L2 two partial-sector writes;
 // measured on the plane writer of the triangle projection, 32-byte stores cut the kernel from 1.6 to 1.0 ms.
