@@ -392,17 +392,8 @@ __global__ void __launch_bounds__(256) adaln_rows_kernel(const __nv_bfloat16* __
   }
 }
 
-// conditioning row of row r: a 32-bit remainder where the row count fits one (a 64-bit one costs a row about as many
-// instructions as its arithmetic)
-__device__ __forceinline__ long long cond_row(long long r, long long R, long long cond_rows) {
-  return R <= 0x7fffffffLL && cond_rows <= 0x7fffffffLL
-             ? static_cast<long long>(static_cast<uint32_t>(r) % static_cast<uint32_t>(cond_rows))
-             : r % cond_rows;
-}
-
 // The same with 16-byte accesses: a warp per row, the row (up to 1024 channels: four 8-channel chunks per
-// lane) stays in registers between the statistics and the output pass, so it is read once; scale and shift are requested
-// with it, not behind its statistics.
+// lane) stays in registers between the statistics and the output pass, so it is read once.
 template <int CHUNKS>
 __global__ void __launch_bounds__(256) adaln_rows_vec_kernel(const __nv_bfloat16* __restrict__ a,
                                                              const __nv_bfloat16* __restrict__ scale,
@@ -414,18 +405,9 @@ __global__ void __launch_bounds__(256) adaln_rows_vec_kernel(const __nv_bfloat16
   for (long long r = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); r < R;
        r += static_cast<long long>(gridDim.x) * warps_per_block) {
     const __nv_bfloat16* ar = a + r * C;
-    const long long rc = cond_row(r, R, cond_rows);
+    const long long rc = r % cond_rows;
     float x[CHUNKS][8];
-    uint4 us[CHUNKS], uh[CHUNKS];
     float sum = 0.f, sumsq = 0.f;
-#pragma unroll
-    for (int k = 0; k < CHUNKS; ++k) {
-      const int c = k * 256 + lane * 8;
-      if (c < C) {
-        us[k] = __ldg(reinterpret_cast<const uint4*>(scale + rc * ld_cond + c));
-        uh[k] = __ldg(reinterpret_cast<const uint4*>(shift + rc * ld_cond + c));
-      }
-    }
 #pragma unroll
     for (int k = 0; k < CHUNKS; ++k) {
       const int c = k * 256 + lane * 8;
@@ -449,8 +431,10 @@ __global__ void __launch_bounds__(256) adaln_rows_vec_kernel(const __nv_bfloat16
     for (int k = 0; k < CHUNKS; ++k) {
       const int c = k * 256 + lane * 8;
       if (c < C) {
-        const uint32_t ws[4] = {us[k].x, us[k].y, us[k].z, us[k].w};
-        const uint32_t wh[4] = {uh[k].x, uh[k].y, uh[k].z, uh[k].w};
+        const uint4 us = __ldg(reinterpret_cast<const uint4*>(scale + rc * ld_cond + c));
+        const uint4 uh = __ldg(reinterpret_cast<const uint4*>(shift + rc * ld_cond + c));
+        const uint32_t ws[4] = {us.x, us.y, us.z, us.w};
+        const uint32_t wh[4] = {uh.x, uh.y, uh.z, uh.w};
         uint32_t o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -481,12 +465,8 @@ __global__ void __launch_bounds__(256) adaln_rows_c128_kernel(const __nv_bfloat1
     const bool ok = r < R;
     float x[8];
     float sum = 0.f, sumsq = 0.f;
-    uint4 us = make_uint4(0u, 0u, 0u, 0u), uh = us;
     if (ok) {
       const uint4 u = *reinterpret_cast<const uint4*>(a + r * C + c);
-      const long long rc = cond_row(r, R, cond_rows);
-      us = __ldg(reinterpret_cast<const uint4*>(scale + rc * ld_cond + c));
-      uh = __ldg(reinterpret_cast<const uint4*>(shift + rc * ld_cond + c));
       const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -504,6 +484,9 @@ __global__ void __launch_bounds__(256) adaln_rows_c128_kernel(const __nv_bfloat1
     if (!ok) continue;
     const float mu = sum * (1.0f / C);
     const float rstd = rsqrtf(fmaxf(sumsq * (1.0f / C) - mu * mu, 0.f) + eps);
+    const long long rc = r % cond_rows;
+    const uint4 us = __ldg(reinterpret_cast<const uint4*>(scale + rc * ld_cond + c));
+    const uint4 uh = __ldg(reinterpret_cast<const uint4*>(shift + rc * ld_cond + c));
     const uint32_t ws[4] = {us.x, us.y, us.z, us.w};
     const uint32_t wh[4] = {uh.x, uh.y, uh.z, uh.w};
     uint32_t o4[4];
