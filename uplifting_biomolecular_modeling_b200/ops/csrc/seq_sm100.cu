@@ -1480,6 +1480,10 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_rows_kernel(
 // instructions four at a time.  The blocks of a tile are dealt to the CTA's warps, which add their sums up in shared memory.
 // STAGED: x^ is normalised into shared memory once per CTA; otherwise decode rows come straight from L1 (staging all of
 // x cost every SM up to 176 KB of L2 reads in front of its weights).  Needs K % 64 == 0 and weights on 32 bytes.
+// us of the FMA form / of this one, 12288 x 4096 behind a norm, 2 x 11008 x 4096 behind a norm, 4096 x 11008, 4096 x 4096: one
+// decode row 18.2 / 21.3, 33.2 / 36.0, 18.7 / 17.0, 6.1 / 7.3; two 21.1 / 20.6, 36.5 / 34.9, 20.4 / 17.1, 7.9 / 7.3; four 32.5 /
+// 22.4, 47.4 / 36.7, 29.3 / 17.2, 11.5 / 7.5; eight 56.7 / 25.1, 99.9 / 39.3, 59.2 / 17.5, 20.1 / 7.3.  One row stays with the FMAs.
+constexpr int kGemvMmaMinRows = 2;
 constexpr int kGemvMmaThreads = 256;
 constexpr int kGemvMmaWarps = kGemvMmaThreads / 32;
 
@@ -1573,9 +1577,14 @@ __global__ void __launch_bounds__(kGemvMmaThreads, 2) gemv_mma_kernel(
       for (int e = 0; e < 4; ++e) acc[d][e] = 0.f;
     for (int kb0 = warp; kb0 < nblk; kb0 += kGemvMmaWarps * U) {
       uint32_t a0[U][D][8], a1[U][D][8];
+      uint4 xv[U][2];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const size_t kb = static_cast<size_t>(min(kb0 + u * kGemvMmaWarps, nblk - 1)) * 128;
+        // decode rows from L1 or L2 are requested with the weights (shared memory answers soon enough)
+        const uint4* xp = reinterpret_cast<const uint4*>(xrow + kb + t * 32);
+        xv[u][0] = !STAGED && has_x ? __ldg(xp) : make_uint4(0u, 0u, 0u, 0u);
+        xv[u][1] = !STAGED && has_x ? __ldg(xp + 1) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int d = 0; d < D; ++d) {
           const char* base = reinterpret_cast<const char*>(d == 0 ? w : w2) + kb;
@@ -1587,8 +1596,8 @@ __global__ void __launch_bounds__(kGemvMmaThreads, 2) gemv_mma_kernel(
       for (int u = 0; u < U; ++u) {
         const int kb = kb0 + u * kGemvMmaWarps;
         if (kb < nblk) {                                              // warp-uniform
-          uint4 b0 = make_uint4(0u, 0u, 0u, 0u), b1 = b0;
-          if (has_x) {
+          uint4 b0 = xv[u][0], b1 = xv[u][1];
+          if (STAGED && has_x) {
             const uint4* xp = reinterpret_cast<const uint4*>(xrow + static_cast<size_t>(kb) * 128 + t * 32);
             b0 = xp[0];
             b1 = xp[1];
@@ -1678,7 +1687,7 @@ int launch_gemv(const __nv_bfloat16* x, const float* gamma, float eps, const __n
   }();
   if constexpr (!W8) {
     const uintptr_t bits = reinterpret_cast<uintptr_t>(w) | (DUAL ? reinterpret_cast<uintptr_t>(w2) : 0);
-    if ((K & 63) == 0 && (bits & 31) == 0 && static_cast<size_t>(M) * (K * 2 + 16) <= kGemvMaxSmem) {
+    if (M >= kGemvMmaMinRows && (K & 63) == 0 && (bits & 31) == 0 && static_cast<size_t>(M) * (K * 2 + 16) <= kGemvMaxSmem) {
       return gamma != nullptr ? launch_gemv_mma<DUAL, true>(x, gamma, eps, w, w2, bias, res, out, M, N, K, pdl, st)
                               : launch_gemv_mma<DUAL, false>(x, gamma, eps, w, w2, bias, res, out, M, N, K, pdl, st);
     }
