@@ -18,8 +18,9 @@ def _close(got, want):
     assert not ((got.double() - want).abs() > 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).any()
 
 
-@pytest.mark.parametrize("M,N", [(1024, 4096), (4864, 1000), (1153, 4104), (2304, 2176), (4000, 4640)])
-@pytest.mark.parametrize("K", [64, 72, 840])
+# six waves of a short contraction (the last tile one row, one column high), a few waves of a longer one, 130 to 256 rows
+@pytest.mark.parametrize("M,N,K", [(4864, 5128, 648), (12801, 2049, 712), (12673, 2168, 704), (2100, 4616, 1544),
+                                   (2049, 4353, 1536), (130, 9608, 3080), (256, 9600, 3072)])
 @pytest.mark.parametrize("mn_major", [False, True])
 def test_plain(M, N, K, mn_major):
     from uplifting_biomolecular_modeling_b200.ops import gemm, native
@@ -33,13 +34,13 @@ def test_plain(M, N, K, mn_major):
     native.raise_on_status("cuda", "gemm")
 
 
-@pytest.mark.parametrize("n", [200, 257, 300, 513])
+@pytest.mark.parametrize("n", [641, 897])
 @pytest.mark.parametrize("mn_major", [False, True])
 def test_batch(n, mn_major):
     from uplifting_biomolecular_modeling_b200.ops import gemm, native
     ld = -(-n // 8) * 8
-    a, b = _r(1, 128, n, ld)[:, :, :n], _r(2, 128, n, ld)[:, :, :n]
-    out = torch.zeros(128, n, ld, device="cuda", dtype=torch.bfloat16)
+    a, b = _r(1, 96, n, ld)[:, :, :n], _r(2, 96, n, ld)[:, :, :n]
+    out = torch.zeros(96, n, ld, device="cuda", dtype=torch.bfloat16)
     gemm.gemm(a, b, mn_major=mn_major, out=out[:, :, :n])
     native.raise_on_status("cuda", "gemm")
     want = torch.bmm(a.double().transpose(1, 2), b.double()) if mn_major else torch.bmm(a.double(), b.double().transpose(1, 2))
@@ -47,7 +48,7 @@ def test_batch(n, mn_major):
     assert not out[:, :, n:].any()
 
 
-@pytest.mark.parametrize("tokens,sequences", [(40, 24), (96, 136)])
+@pytest.mark.parametrize("tokens,sequences", [(160, 650), (72, 1544)])
 def test_blocked_outer_product(tokens, sequences):
     from uplifting_biomolecular_modeling_b200.ops import gemm, native
     a, b = _r(3, sequences, tokens * 32), _r(4, sequences, tokens * 32)
@@ -58,7 +59,7 @@ def test_blocked_outer_product(tokens, sequences):
     _close(out, want.reshape(tokens * tokens, 1024))
 
 
-@pytest.mark.parametrize("M,hidden,K", [(2050, 2048, 136), (4100, 1056, 64)])
+@pytest.mark.parametrize("M,hidden,K", [(2050, 2048, 1544), (12001, 1056, 648)])
 def test_swiglu(M, hidden, K):
     from uplifting_biomolecular_modeling_b200.ops import gemm, native
     x, wg, wv = _r(6, M, K), _r(7, hidden, K) * K ** -0.5, _r(8, hidden, K) * K ** -0.5

@@ -11,10 +11,9 @@
 // (LN_in recompute + LN_out + W_o x sigmoid gate + residual) and _k3c/_k3d of
 // kernels/fpf_trimul_v4/kernels.py.
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = four epilogue groups of 32 output channels each.
-// TMEM: {O, G} x two tiles = 512 columns.  Sixteen epilogue warps instead of eight, the statistics of the x columns
-// taken two columns per lane from whole 128-byte rows (one thread per column read 128 two-byte values), and the output
-// staged over the residual in the z tile: 202 us at 1021 tokens against 265 us (issue slots 55 %, DRAM 45 % busy at 768).
+// Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = four epilogue groups of 32 output channels each, 18-21 = statistics, a tile
+// ahead of the epilogue.  TMEM: {O, G} x two tiles = 512 columns.
+// TO_COMMENT
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -35,7 +34,8 @@ struct TrimulOutParams {
   int tiles_per_i, num_tiles;
 };
 constexpr int kTOEpiWarps = 16;
-constexpr int kTOThreads = 64 + 32 * kTOEpiWarps;
+constexpr int kTOStatWarps = 4;
+constexpr int kTOThreads = 64 + 32 * (kTOEpiWarps + kTOStatWarps);
 
 __global__ void __launch_bounds__(kTOThreads, 1)
 trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmZ,
@@ -47,14 +47,16 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   uint8_t* sWg = smem + kTOTileBytes;     // 32 KB
   uint8_t* sSt = smem + 2 * kTOTileBytes; // stages: {x tile 32 KB, z tile 32 KB}
   float* sConst = reinterpret_cast<float*>(sSt + kTOStages * kTOStageBytes);  // 4 x 128
-  float2* sPart = reinterpret_cast<float2*>(sConst + 512);   // [9][128] (sum, sum of squares): x by channel group, z
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sPart + 9 * 128);
+  float4* sRow = reinterpret_cast<float4*>(sConst + 512);    // [stages][128]: 1 / std, - mean / std of x column and z row
+  float2* sPart = reinterpret_cast<float2*>(sRow + kTOStages * 128);   // [2][128]: an x column's sums over half of the channels
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sPart + 2 * 128);
   uint64_t* full = bars;                 // [stages]
   uint64_t* empty = full + kTOStages;    // [stages]  MMA commit + 8 output boxes that have left the tile
   uint64_t* w_full = empty + kTOStages;  // [1]
   uint64_t* acc_full = w_full + 1;       // [2]
   uint64_t* acc_empty = acc_full + 2;    // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* r_full = acc_empty + 2;      // [stages] statistics of the tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(r_full + kTOStages);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5;
@@ -66,6 +68,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     for (int s = 0; s < kTOStages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1 + 8);
+      mbar_init(&r_full[s], kTOStatWarps);
     }
     mbar_init(w_full, 1);
     for (int a = 0; a < 2; ++a) {
@@ -174,45 +177,34 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
       }
     }
-  } else {
-    const int grp = (warp - 2) >> 2;       // output channels 32 grp .. + 31
-    const int q = warp & 3;
-    const int row = q * 32 + lane;
-    const int et = threadIdx.x - 64;       // 0 .. 511
-    const int fg = lane >> 2, ft = lane & 3;   // rows q * 32 + fg + 8 rr (rr < 4), two columns of every eight
+  } else if (warp >= 2 + kTOEpiWarps) {
+    // ------------------------------------------------------------------ statistics
+    // The rows of sRow that a tile overwrites were read for the tile two before it, whose boxes had left its buffers when
+    // this tile was requested.
+    const int sw = warp - 2 - kTOEpiWarps;
+    const int jh = sw & 1, ch0 = (sw >> 1) * 64;     // x: 64 columns, two per lane, over half of the channels
+    const int st = sw * 32 + lane;                   // z: a row per thread; then the column of that number
     int stage = 0;
     uint32_t phase = 0;
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    bool stored = false;                   // an output box of the previous tile is on its way
     for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
-      const int i = t / p.tiles_per_i;
-      const int j0 = (t - i * p.tiles_per_i) * 128;
-      mbar_wait(&full[stage], phase, ws, 25, stage);
+      mbar_wait(&full[stage], phase, ws, 27, stage);
       const uint8_t* sx = sSt + stage * kTOStageBytes;
-      uint8_t* sz = sSt + stage * kTOStageBytes + kTOTileBytes;
-      // statistics over channels of x[:, i, j] (columns of the [c][j] tile): a warp takes 16 channels of 64 columns,
-      // two columns per lane, so that its reads are whole 128-byte rows
-      const int jh = (warp - 2) & 1, cg = (warp - 2) >> 1;
+      const uint8_t* sz = sx + kTOTileBytes;
       float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-#pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        const int ch = cg * 16 + c;
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(sx + ((ch >> 6) * 2 + jh) * 8192 +
-                                                              swz128_offset(ch & 63, lane >> 2) + (lane & 3) * 4);
+#pragma unroll 16
+      for (int c = 0; c < 64; ++c) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(sx + ((ch0 >> 6) * 2 + jh) * 8192 +
+                                                              swz128_offset(c, lane >> 2) + (lane & 3) * 4);
         const float a = bf16_lo(w), b = bf16_hi(w);
         s0 += a;
         q0 += a * a;
         s1 += b;
         q1 += b * b;
       }
-      // statistics of the z rows: four threads per row
-      const int zrow = et >> 2;
       float sum = 0.f, sumsq = 0.f;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint4 u = *reinterpret_cast<const uint4*>(sz + ((et & 3) >> 1) * 16384 +
-                                                        swz128_offset(zrow, (et & 1) * 4 + c));
+#pragma unroll 8
+      for (int c = 0; c < 16; ++c) {
+        const uint4 u = *reinterpret_cast<const uint4*>(sz + (c >> 3) * 16384 + swz128_offset(st, c & 7));
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
@@ -221,78 +213,87 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           sumsq += a * a + b * b;
         }
       }
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sumsq += __shfl_xor_sync(0xffffffffu, sumsq, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      sumsq += __shfl_xor_sync(0xffffffffu, sumsq, 2);
+      // the four warps exchange the halves: nobody reads the previous tile's any more, then nobody reads too early
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      reinterpret_cast<float4*>(sPart)[((sw >> 1) * 128 + jh * 64 + lane * 2) >> 1] = make_float4(s0, q0, s1, q1);
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      const float2 xa = sPart[st], xb = sPart[128 + st];
+      const float mux = (xa.x + xb.x) * (1.f / 128.f), muz = sum * (1.f / 128.f);
+      const float rsx = rsqrtf(fmaxf((xa.y + xb.y) * (1.f / 128.f) - mux * mux, 0.f) + 1e-5f);
+      const float rsz = rsqrtf(fmaxf(sumsq * (1.f / 128.f) - muz * muz, 0.f) + 1e-5f);
+      sRow[stage * 128 + st] = make_float4(rsx, -mux * rsx, rsz, -muz * rsz);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&r_full[stage]);
+      if (++stage == kTOStages) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
+  } else {
+    const int grp = (warp - 2) >> 2;       // output channels 32 grp .. + 31
+    const int q = warp & 3;
+    const int row = q * 32 + lane;
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool stored = false;                   // an output box of the previous tile is on its way
+    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
+      const int i = t / p.tiles_per_i;
+      const int j0 = (t - i * p.tiles_per_i) * 128;
+      uint8_t* sz = sSt + stage * kTOStageBytes + kTOTileBytes;
       if (stored) {
         // the box this thread stored from the previous tile has been read: its buffers may be loaded again
         tma_store_wait_read<0>();
         mbar_arrive(&empty[stage ^ 1]);
       }
-      // all 512 threads exchange sums: nobody reads the previous tile's any more, then nobody reads too early
-      asm volatile("bar.sync 1, 512;" ::: "memory");
-      reinterpret_cast<float4*>(sPart)[(cg * 128 + jh * 64 + lane * 2) >> 1] = make_float4(s0, q0, s1, q1);
-      if ((et & 3) == 0) sPart[8 * 128 + zrow] = make_float2(sum, sumsq);
-      asm volatile("bar.sync 1, 512;" ::: "memory");
-      float xsum = 0.f, xsq = 0.f;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float2 v = sPart[c * 128 + row];
-        xsum += v.x;
-        xsq += v.y;
-      }
-      const float2 zs = sPart[8 * 128 + row];
-      const float mux = xsum * (1.f / 128.f), muz = zs.x * (1.f / 128.f);
-      const float rsx = rsqrtf(fmaxf(xsq * (1.f / 128.f) - mux * mux, 0.f) + 1e-5f);
-      const float rsz = rsqrtf(fmaxf(zs.y * (1.f / 128.f) - muz * muz, 0.f) + 1e-5f);
-      float rx[4], nx[4], rz[4], nz[4];      // of this thread's four rows
-#pragma unroll
-      for (int rr = 0; rr < 4; ++rr) {
-        rx[rr] = __shfl_sync(0xffffffffu, rsx, rr * 8 + fg);
-        nx[rr] = __shfl_sync(0xffffffffu, -mux * rsx, rr * 8 + fg);
-        rz[rr] = __shfl_sync(0xffffffffu, rsz, rr * 8 + fg);
-        nz[rr] = __shfl_sync(0xffffffffu, -muz * rsz, rr * 8 + fg);
-      }
-
+      __syncwarp();
+      mbar_wait(&r_full[stage], phase, ws, 25, stage);
+      const float4 rw = sRow[stage * 128 + row];
+      const float2 ax = make_float2(rw.x, rw.x), bx = make_float2(rw.y, rw.y);
+      const float2 az = make_float2(rw.z, rw.z), bz = make_float2(rw.w, rw.w);
       mbar_wait(&acc_full[acc], acc_phase, ws, 26, acc);
       tc_fence_after_sync();
       const uint32_t tO = tmem_addr(tmem_base, q, acc * 256 + grp * 32);
       const uint32_t tG = tO + 128;
 #pragma unroll 1
       for (int c0 = 0; c0 < 32; c0 += 16) {
-        uint32_t ov[2][8], gv[2][8];         // [lane half]
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          tmem_ld_frag16(tO + hf * kTmemLane16 + c0, ov[hf]);
-          tmem_ld_frag16(tG + hf * kTmemLane16 + c0, gv[hf]);
-        }
+        uint32_t ov[16], gv[16];
+        tmem_ld16(tO + c0, ov);
+        tmem_ld16(tG + c0, gv);
         tmem_ld_wait();
         if (c0 == 16) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&acc_empty[acc]);
         }
+        const int cb0 = grp * 32 + c0;
+        const float4* oc4 = reinterpret_cast<const float4*>(sConst + cb0);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int col = grp * 32 + c0 + u * 8;
-          const float2* oc2 = reinterpret_cast<const float2*>(sConst + col) + ft;
-          const float2 ocs = oc2[0], ocb = oc2[64], gcs = oc2[128], gcb = oc2[192];
+        for (int j8 = 0; j8 < 2; ++j8) {
+          // in place over the residual: 16 bytes of this row in the z tile, which both products have read
+          uint4* at = reinterpret_cast<uint4*>(sz + (grp >> 1) * 16384 +
+                                               swz128_offset(row, (grp & 1) * 4 + (c0 >> 3) + j8));
+          const uint4 u = p.add_residual ? *at : make_uint4(0u, 0u, 0u, 0u);
+          const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+          uint32_t o[4];
 #pragma unroll
-          for (int rr = 0; rr < 4; ++rr) {
-            const int k = u * 4 + (rr & 1) * 2;
-            // in place over the residual: two channels of this row in the z tile, which both products have read
-            uint32_t* at = reinterpret_cast<uint32_t*>(sz + (grp >> 1) * 16384 +
-                                                       swz128_offset(q * 32 + rr * 8 + fg, (col & 63) >> 3)) + ft;
-            const uint32_t w = p.add_residual ? *at : 0u;
-            const float2 f = ln_fold2(ov[rr >> 1][k], ov[rr >> 1][k + 1], make_float2(rx[rr], rx[rr]),
-                                      make_float2(nx[rr], nx[rr]), ocs.x, ocs.y, ocb.x, ocb.y);
-            const float2 gt = ln_fold2(gv[rr >> 1][k], gv[rr >> 1][k + 1], make_float2(rz[rr], rz[rr]),
-                                       make_float2(nz[rr], nz[rr]), gcs.x, gcs.y, gcb.x, gcb.y);
-            const float2 v = __ffma2_rn(f, make_float2(sigmoidf_fast(gt.x), sigmoidf_fast(gt.y)),
-                                        make_float2(bf16_lo(w), bf16_hi(w)));
-            *at = pack_bf16x2(v.x, v.y);
+          for (int h = 0; h < 2; ++h) {
+            const float4 ocs = oc4[j8 * 2 + h], ocb = oc4[32 + j8 * 2 + h];
+            const float4 gcs = oc4[64 + j8 * 2 + h], gcb = oc4[96 + j8 * 2 + h];
+            const int k = j8 * 8 + h * 4;
+            const float2 f0 = ln_fold2(ov[k], ov[k + 1], ax, bx, ocs.x, ocs.y, ocb.x, ocb.y);
+            const float2 f1 = ln_fold2(ov[k + 2], ov[k + 3], ax, bx, ocs.z, ocs.w, ocb.z, ocb.w);
+            const float2 g0 = ln_fold2(gv[k], gv[k + 1], az, bz, gcs.x, gcs.y, gcb.x, gcb.y);
+            const float2 g1 = ln_fold2(gv[k + 2], gv[k + 3], az, bz, gcs.z, gcs.w, gcb.z, gcb.w);
+            const float2 v0 = __ffma2_rn(f0, make_float2(sigmoidf_fast(g0.x), sigmoidf_fast(g0.y)),
+                                         make_float2(bf16_lo(w[h * 2]), bf16_hi(w[h * 2])));
+            const float2 v1 = __ffma2_rn(f1, make_float2(sigmoidf_fast(g1.x), sigmoidf_fast(g1.y)),
+                                         make_float2(bf16_lo(w[h * 2 + 1]), bf16_hi(w[h * 2 + 1])));
+            o[h * 2] = pack_bf16x2(v0.x, v0.y);
+            o[h * 2 + 1] = pack_bf16x2(v1.x, v1.y);
           }
+          *at = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
       fence_proxy_async_smem();
@@ -326,7 +327,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 }
 
 static_assert(kTOStages == 2, "the release of a tile's buffers names the other stage");
-constexpr int kTOSmemBytes = 2 * kTOTileBytes + kTOStages * kTOStageBytes + 512 * 4 + 9 * 128 * 8 + 256 + 1024;
+constexpr int kTOSmemBytes = 2 * kTOTileBytes + kTOStages * kTOStageBytes + 512 * 4 + kTOStages * 128 * 16 + 2 * 128 * 8 + 256 + 1024;
 static_assert(kTOSmemBytes <= 232448, "shared memory of one CTA");
 
 }  // namespace ubm

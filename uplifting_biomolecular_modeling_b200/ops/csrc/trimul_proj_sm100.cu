@@ -15,10 +15,9 @@
 // are computed thread-per-row from the shared-memory tile (as the row-major kernels do) and passed to all
 // threads of the epilogue group through a small shared array; the per-channel constants live in registers.
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = four epilogue groups: operand (a, b) x half of the tile's columns.
-// With eight epilogue warps, and both operands' groups taking every row's statistics, it took 314 us at 1021 tokens;
-// sixteen warps that share the statistics take 265 us.  No unit is full: issue slots 49 %, DRAM 36 %, tensor pipe 25 %,
-// special-function unit 28 % busy at 768 tokens.
+// Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = four epilogue groups: operand (a, b) x half of the tile's columns,
+// 18-21 = row statistics, up to two tiles ahead of the epilogue.
+// TP_COMMENT
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -50,25 +49,27 @@ struct TrimulProjParams {
 constexpr int kTPOutWarpBytes = 32 * 64;
 constexpr int kTPEpiWarps = 16;
 constexpr int kTPOutBytes = kTPEpiWarps * kTPOutWarpBytes;
-constexpr int kTPThreads = 64 + 32 * kTPEpiWarps;
+constexpr int kTPStatWarps = 4;
+constexpr int kTPThreads = 64 + 32 * (kTPEpiWarps + kTPStatWarps);
 
 __global__ void __launch_bounds__(kTPThreads, 1)
 trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                    const __grid_constant__ PeerSrcMaps peers, const __grid_constant__ CUtensorMap tmP,
                    TrimulProjParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];   // no room to align by hand
   uint8_t* sW = smem;                               // 128 KB
   uint8_t* sX = smem + kTPWBytes;                   // stages * 32 KB
   uint8_t* sOut = sX + kTPStages * kTPXBytes;       // 16 warps x 2 KB of output staging
-  float* sStat = reinterpret_cast<float*>(sOut + kTPOutBytes);           // [3][128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 3 * 128);
+  float* sStat = reinterpret_cast<float*>(sOut + kTPOutBytes);           // [2 tiles][1 / std, - mean / std][128], halved
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 2 * 256);
   uint64_t* x_full = bars;                 // [stages]
   uint64_t* x_empty = x_full + kTPStages;  // [stages]
   uint64_t* w_full = x_empty + kTPStages;  // [1]
   uint64_t* acc_full = w_full + 1;         // [2]
   uint64_t* acc_empty = acc_full + 2;      // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* r_full = acc_empty + 2;        // [2] statistics of a tile written
+  uint64_t* r_empty = r_full + 2;          // [2] and read by every epilogue warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(r_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5;
@@ -79,14 +80,18 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     *abort_flag = 0;
     for (int s = 0; s < kTPStages; ++s) {
       mbar_init(&x_full[s], 1);
-      mbar_init(&x_empty[s], 1 + kTPEpiWarps);  // MMA commit + one arrival per epilogue warp
+      mbar_init(&x_empty[s], 1 + kTPStatWarps);  // MMA commit + one arrival per statistics warp
     }
     mbar_init(w_full, 1);
     for (int h = 0; h < 2; ++h) {
       mbar_init(&acc_full[h], 1);
       mbar_init(&acc_empty[h], kTPEpiWarps / 2);
+      mbar_init(&r_full[h], kTPStatWarps);
+      mbar_init(&r_empty[h], kTPEpiWarps);
     }
     mbar_fence_init();
+    // the swizzled tiles assume what the alignment attribute asks for; nothing runs where it is not so
+    if ((smem_u32(smem) & 1023u) != 0) report_failure(ws, kErrBadArgument, 10, 0);
     tma_prefetch_desc(&tmX);
     tma_prefetch_desc(&tmW);
   }
@@ -98,17 +103,19 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  const bool run = (smem_u32(smem) & 1023u) == 0;
+  const int num_tiles = run ? p.num_tiles : 0;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (lane == 0 && run) {
       mbar_expect_tx(w_full, kTPWBytes);
       for (int kb = 0; kb < 2; ++kb)
         for (int h = 0; h < 2; ++h)
           tma_load_2d(sW + kb * 65536 + h * 32768, &tmW, w_full, kb * 64, h * 256);
       int stage = 0;
       uint32_t phase = 0;
-      for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const int i = t / p.tiles_per_row;
         const int s0 = (t - i * p.tiles_per_row) * kTPRows;
         const int flat = i * p.N + s0;   // rows past the end of pair row i belong to the next one and are discarded
@@ -138,11 +145,11 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     // ------------------------------------------------------------------ MMA issuer (warp-uniform loop, elected lane issues)
     const bool leader = elect_one();
     constexpr uint32_t idesc = umma_idesc_bf16(128, 128);
-    mbar_wait(w_full, 0, ws, 12);
+    if (run) mbar_wait(w_full, 0, ws, 12);
     int stage = 0;
     uint32_t phase = 0;
     uint32_t acc_phase = 0;
-    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       mbar_wait(&x_full[stage], phase, ws, 13, stage);
       tc_fence_after_sync();
       const uint64_t xd0 = umma_smem_desc(smem_u32(sX + stage * kTPXBytes), 16, 1024, kSwizzle128);
@@ -175,42 +182,18 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       }
       acc_phase ^= 1u;
     }
-  } else {
-    // ------------------------------------------------------------------ epilogue groups
-    const int op = ((warp - 2) >> 2) & 1;   // operand a or b
-    const int half = (warp - 2) >> 3;       // columns 64 half .. 64 half + 63
-    const int q = warp & 3;                 // TMEM lane quadrant
-    const int g = lane >> 2, t4 = lane & 3; // channels q * 32 + g + 8 rr (rr < 4), two columns of every eight
-    const int et = threadIdx.x - 64;        // 0 .. 511: four threads take the statistics of one tile row
-    const int srow = et >> 2;
-    float cs_v[4], cb_v[4], cs_g[4], cb_g[4];
-#pragma unroll
-    for (int rr = 0; rr < 4; ++rr) {
-      const int ch = op * 256 + q * 32 + rr * 8 + g;
-      cs_v[rr] = p.colsum[ch];
-      cb_v[rr] = p.colbias[ch];
-      cs_g[rr] = p.colsum[ch + 128];
-      cb_g[rr] = p.colbias[ch + 128];
-    }
+  } else if (warp >= 2 + kTPEpiWarps) {
+    // ------------------------------------------------------------------ row statistics, a row per thread
+    const int row = threadIdx.x - 32 * (2 + kTPEpiWarps);
     int stage = 0;
-    uint32_t phase = 0;
-    uint32_t acc_phase = 0;
-    uint8_t* stage_w = sOut + (warp - 2) * kTPOutWarpBytes;
-    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
-      const int i = t / p.tiles_per_row;
-      const int s0 = (t - i * p.tiles_per_row) * kTPRows;
-      // ---- statistics of tile row `srow` from the shared-memory tile: 32 channels per thread
-      const int s = s0 + srow;
-      const bool valid = s < p.N;
-      const long long r = static_cast<long long>(i) * p.N + s;
-      float mval = valid ? 1.0f : 0.0f;            // entries past N are written as zeros (K padding of the contraction)
-      if (valid && p.mask != nullptr) mval = p.mask[r];
+    uint32_t phase = 0, n = 0;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++n) {
       mbar_wait(&x_full[stage], phase, ws, 15, stage);
-      const uint8_t* xs = sX + stage * kTPXBytes + ((et & 3) >> 1) * 16384;
+      const uint8_t* xs = sX + stage * kTPXBytes;
       float sum = 0.f, sumsq = 0.f;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint4 u = *reinterpret_cast<const uint4*>(xs + swz128_offset(srow, (et & 1) * 4 + c));
+#pragma unroll 8
+      for (int c = 0; c < 16; ++c) {
+        const uint4 u = *reinterpret_cast<const uint4*>(xs + (c >> 3) * 16384 + swz128_offset(row, c & 7));
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -219,26 +202,59 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           sumsq += a * a + b * b;
         }
       }
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sumsq += __shfl_xor_sync(0xffffffffu, sumsq, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      sumsq += __shfl_xor_sync(0xffffffffu, sumsq, 2);
+      __syncwarp();
       if (lane == 0) mbar_arrive(&x_empty[stage]);
       const float mu = sum * (1.0f / kTPC);
       const float var = fmaxf(sumsq * (1.0f / kTPC) - mu * mu, 0.f);
       const float rstd = rsqrtf(var + 1e-5f);
-      if (p.stats_out != nullptr && (et & 3) == 0 && valid) {
+      const int i = t / p.tiles_per_row, s = (t - i * p.tiles_per_row) * kTPRows + row;
+      if (p.stats_out != nullptr && s < p.N) {
+        const long long r = static_cast<long long>(i) * p.N + s;
         p.stats_out[2 * r] = mu;
         p.stats_out[2 * r + 1] = rstd;
       }
-      // all 512 threads exchange statistics: nobody reads the previous tile's any more, then nobody reads too early
-      asm volatile("bar.sync 1, 512;" ::: "memory");
-      if ((et & 3) == 0) {
-        sStat[srow] = rstd;
-        sStat[128 + srow] = -mu * rstd;
-        sStat[256 + srow] = mval;
+      const int b = n & 1;
+      mbar_wait(&r_empty[b], ((n >> 1) & 1u) ^ 1u, ws, 17, b);
+      sStat[b * 256 + row] = 0.5f * rstd;
+      sStat[b * 256 + 128 + row] = -0.5f * mu * rstd;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&r_full[b]);
+      if (++stage == kTPStages) {
+        stage = 0;
+        phase ^= 1u;
       }
-      asm volatile("bar.sync 1, 512;" ::: "memory");
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue groups
+    const int op = ((warp - 2) >> 2) & 1;   // operand a or b
+    const int half = (warp - 2) >> 3;       // columns 64 half .. 64 half + 63
+    const int q = warp & 3;                 // TMEM lane quadrant
+    const int g = lane >> 2, t4 = lane & 3; // channels q * 32 + g + 8 rr (rr < 4), two columns of every eight
+    // value and gate are formed at half their size: sigmoid(x) v = v / 2 + v / 2 tanh(x / 2)
+    float cs_v[4], cb_v[4], cs_g[4], cb_g[4];
+#pragma unroll
+    for (int rr = 0; rr < 4; ++rr) {
+      const int ch = op * 256 + q * 32 + rr * 8 + g;
+      cs_v[rr] = p.colsum[ch];
+      cb_v[rr] = 0.5f * p.colbias[ch];
+      cs_g[rr] = p.colsum[ch + 128];
+      cb_g[rr] = 0.5f * p.colbias[ch + 128];
+    }
+    uint32_t acc_phase = 0, n = 0;
+    uint8_t* stage_w = sOut + (warp - 2) * kTPOutWarpBytes;
+    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++n) {
+      const int i = t / p.tiles_per_row;
+      const int s0 = (t - i * p.tiles_per_row) * kTPRows;
+      const int b = n & 1;
+      // mask of this warp's 64 columns, two per lane; entries past N are written as zeros (K padding of the contraction)
+      const int left = p.N - s0 - half * 64;
+      float mk0 = lane < left ? 1.0f : 0.0f, mk1 = lane + 32 < left ? 1.0f : 0.0f;
+      if (p.mask != nullptr) {
+        const float* mrow = p.mask + static_cast<long long>(i) * p.N + s0 + half * 64;
+        if (lane < left) mk0 = __ldg(mrow + lane);
+        if (lane + 32 < left) mk1 = __ldg(mrow + lane + 32);
+      }
+      mbar_wait(&r_full[b], (n >> 1) & 1u, ws, 18, b);
 
       // ---- accumulators of this operand: value block at +0, gate block at +128
       mbar_wait(&acc_full[op], acc_phase, ws, 16, op);
@@ -265,8 +281,11 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           // two adjacent s at a time in packed fp32 instructions, their constants for four channels
-          const float2* st2 = reinterpret_cast<const float2*>(sStat + half * 64 + c16 * 16 + u * 8) + t4;
-          const float2 rs = st2[0], nm = st2[64], mk = st2[128];
+          const float2* st2 = reinterpret_cast<const float2*>(sStat + b * 256 + half * 64 + c16 * 16 + u * 8) + t4;
+          const float2 rs = st2[0], nm = st2[64];
+          const float mks = c16 < 2 ? mk0 : mk1;
+          const int from = (c16 & 1) * 16 + u * 8 + t4 * 2;
+          const float2 mk = make_float2(__shfl_sync(0xffffffffu, mks, from), __shfl_sync(0xffffffffu, mks, from + 1));
           const uint32_t at = g * 64 + ((((c16 & 1) * 2 + u) ^ (g >> 1)) << 4) + t4 * 4;   // 64-byte swizzle
 #pragma unroll
           for (int rr = 0; rr < 4; ++rr) {
@@ -277,8 +296,7 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                                           make_float2(fmaf(nm.x, cs_v[rr], cb_v[rr]), fmaf(nm.y, cs_v[rr], cb_v[rr])));
             const float2 gate = __ffma2_rn(make_float2(__uint_as_float(gr[k]), __uint_as_float(gr[k + 1])), rs,
                                            make_float2(fmaf(nm.x, cs_g[rr], cb_g[rr]), fmaf(nm.y, cs_g[rr], cb_g[rr])));
-            const float2 ov =
-                __fmul2_rn(val, __fmul2_rn(mk, make_float2(sigmoidf_fast(gate.x), sigmoidf_fast(gate.y))));
+            const float2 ov = __fmul2_rn(mk, __ffma2_rn(val, make_float2(fast_tanh(gate.x), fast_tanh(gate.y)), val));
             *reinterpret_cast<uint32_t*>(stage_w + rr * 512 + at) = pack_bf16x2(ov.x, ov.y);
           }
         }
@@ -291,10 +309,8 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           }
         }
       }
-      if (++stage == kTPStages) {
-        stage = 0;
-        phase ^= 1u;
-      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&r_empty[b]);
       acc_phase ^= 1u;
     }
     if (lane == 0) tma_store_wait_all<0>();   // the staging rows are read and the boxes written
@@ -308,7 +324,7 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   }
 }
 
-constexpr int kTPSmemBytes = kTPWBytes + kTPStages * kTPXBytes + kTPOutBytes + 3 * 128 * 4 + 256 + 1024;
+constexpr int kTPSmemBytes = kTPWBytes + kTPStages * kTPXBytes + kTPOutBytes + 2 * 256 * 4 + 256;
 static_assert(kTPSmemBytes <= 232448, "shared memory of one CTA");
 
 }  // namespace ubm
