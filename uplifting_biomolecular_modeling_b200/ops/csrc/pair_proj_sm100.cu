@@ -13,9 +13,10 @@
 // fp32 accumulator in the epilogue.  The 512 x 128 weight matrix stays resident in shared memory
 // for the life of the persistent CTA; only row tiles stream.
 //
-// Warps: 0 = TMA producer, 1 = MMA issuer, 2-5 = epilogue group 0 (output half 0),
-// 6-9 = epilogue group 1 (output half 1).  Each half is one 128 x 256 accumulator in TMEM, so
-// the epilogue of half 0 overlaps the MMAs of half 1 and of the next tile.
+// Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = epilogue, four warps (one per lane quadrant) for each of q, k, v and the
+// gate, 18-21 = row statistics and head biases, up to two tiles ahead of the epilogue.  [q | k] and [v | gate] are two 128 x
+// 256 accumulators in TMEM, so the epilogue of one overlaps the MMAs of the other and of the next tile.
+// PP_COMMENT
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -52,24 +53,27 @@ struct PairProjParams {
   KernelStatus* status;
   int num_tiles;
   PeerSrc src;       // src.n > 0: the input rows are columns of z fetched from their owners (see host_util.h)
-  // q | k | v | gate leave through shared memory: every epilogue warp stages its 32 rows x 32 columns (64-byte
-  // swizzle) and one lane stores the box with a bulk tensor copy (maps in PairOutMaps).  Off when a warp's 32 rows
-  // could straddle two values of the first pair index under the transposed write (N not a multiple of 32).
+  // q | k | v | gate leave through shared memory: every epilogue warp stages 16 rows x 32 columns (64-byte swizzle) and one
+  // lane stores the box with a bulk tensor copy (maps in PairOutMaps).  Under the transposed write, 16 rows that straddle
+  // two values of the first pair index leave by lane.
   int out_tma;
 };
 
-// Output maps, one per q / k / v / gate buffer.  Plain write: {128, R, 1} with boxes {32, 32, 1} at (column, row, 0).
-// Transposed write (ending node): {128, N, N} = out[pk][pi][channel] with boxes {32, 1, 32} at (column, pi, pk0):
-// 32 consecutive second indices of one first index land on 32 rows that are N * 128 elements apart.
+// Output maps, one per q / k / v / gate buffer.  Plain write: {128, R, 1} with boxes {32, 16, 1} at (column, row, 0).
+// Transposed write (ending node): {128, N, N} = out[pk][pi][channel] with boxes {32, 1, 16} at (column, pi, pk0):
+// 16 consecutive second indices of one first index land on 16 rows that are N * 128 elements apart.
 struct PairOutMaps {
   CUtensorMap m[4];
 };
-constexpr int kPPOutWarpBytes = 32 * 64;
-constexpr int kPPOutBytes = 8 * kPPOutWarpBytes;
-constexpr int kPPWbFrags = 3 * 8 * 32;
+constexpr int kPPEpiWarps = 16;
+constexpr int kPPStatWarps = 4;
+constexpr int kPPThreads = 64 + 32 * (kPPEpiWarps + kPPStatWarps);
+constexpr int kPPBoxRows = 16;
+constexpr int kPPOutWarpBytes = kPPBoxRows * 64;
+constexpr int kPPOutBytes = kPPEpiWarps * kPPOutWarpBytes;
 
 template <int MODE>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kPPThreads, 1)
 pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                  const __grid_constant__ PeerSrcMaps peers, const __grid_constant__ PairOutMaps outs,
                  PairProjParams p) {
@@ -77,17 +81,19 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sW = smem;                               // 128 KB
   uint8_t* sX = smem + kPPWBytes;                   // stages * 32 KB
-  uint8_t* sOut = sX + kPPStages * kPPXBytes;       // 8 warps x 2 KB of output staging
+  uint8_t* sOut = sX + kPPStages * kPPXBytes;       // 16 warps x 1 KB of output staging
   float* sColsum = reinterpret_cast<float*>(sOut + kPPOutBytes);          // 512
   float* sColbias = sColsum + 512;                                         // 512
-  uint2* sWbF = reinterpret_cast<uint2*>(sColbias + 512);                  // [3 parts][8 k-steps][32 lanes]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sWbF + kPPWbFrags);
+  float2* sRow = reinterpret_cast<float2*>(sColbias + 512);                // [2 tiles][128]: 1 / std, - mean / std
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sRow + 2 * 128);
   uint64_t* x_full = bars;                 // [stages]
   uint64_t* x_empty = x_full + kPPStages;  // [stages]
   uint64_t* w_full = x_empty + kPPStages;  // [1]
   uint64_t* acc_full = w_full + 1;         // [2]
   uint64_t* acc_empty = acc_full + 2;      // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* r_full = acc_empty + 2;        // [2] statistics of a tile written
+  uint64_t* r_empty = r_full + 2;          // [2] and read by every epilogue warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(r_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5;
@@ -98,12 +104,14 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     *abort_flag = 0;
     for (int s = 0; s < kPPStages; ++s) {
       mbar_init(&x_full[s], 1);
-      mbar_init(&x_empty[s], 1 + 8);  // MMA commit + one arrival per epilogue warp
+      mbar_init(&x_empty[s], 1 + kPPStatWarps);  // MMA commit + one arrival per statistics warp
     }
     mbar_init(w_full, 1);
     for (int h = 0; h < 2; ++h) {
       mbar_init(&acc_full[h], 1);
-      mbar_init(&acc_empty[h], 4);
+      mbar_init(&acc_empty[h], kPPEpiWarps / 2);
+      mbar_init(&r_full[h], kPPStatWarps);
+      mbar_init(&r_empty[h], kPPEpiWarps);
     }
     mbar_fence_init();
     tma_prefetch_desc(&tmX);
@@ -117,27 +125,6 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   for (int i = threadIdx.x; i < 512; i += blockDim.x) {
     sColsum[i] = p.colsum[i];
     sColbias[i] = p.colbias[i];
-  }
-  if (MODE == MODE_TRIATT) {
-    // head weights as three bf16 parts (high, middle, low: 24 bits), in the order in which a lane of mma.sync takes them as
-    // the second operand of a 16-wide k-step: head lane / 4, channels 2 (lane % 4), + 1 and the same eight further on
-    for (int i = threadIdx.x; i < 8 * 32; i += blockDim.x) {
-      const int head = (i & 31) >> 2, k0 = (i >> 5) * 16 + (i & 3) * 2;
-      uint32_t part[3][4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float r = head < p.H ? p.wb[head * 128 + k0 + (e >> 1) * 8 + (e & 1)] : 0.f;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const __nv_bfloat16 h = __float2bfloat16_rn(r);
-          part[q][e] = __bfloat16_as_ushort(h);
-          r -= __bfloat162float(h);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 3; ++q)
-        sWbF[q * 256 + i] = make_uint2(part[q][0] | (part[q][1] << 16), part[q][2] | (part[q][3] << 16));
-    }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -220,26 +207,40 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         acc_phase ^= 1u;
       }
     }
-  } else {
-    // ------------------------------------------------------------------ epilogue groups
-    const int grp = (warp - 2) >> 2;  // 0 or 1: which 256-column half
-    const int q = warp & 3;           // TMEM lane quadrant
-    const int row_in_tile = q * 32 + lane;
-    const int fg = lane >> 2, ft = lane & 3;   // rows q * 32 + fg + 8 rr (rr < 4), two columns of every eight
-    uint8_t* stage_w = sOut + (warp - 2) * kPPOutWarpBytes;
+  } else if (warp >= 2 + kPPEpiWarps) {
+    // ------------------------------------------------------------------ row statistics (a row per thread) and head biases
+    const int sw = warp - 2 - kPPEpiWarps;       // rows 32 sw .. + 31 of the tile
+    const int fg = lane >> 2, ft = lane & 3;
+    // Head weights as three bf16 parts (high, middle, low: 24 bits), as a lane of mma.sync takes them for the second operand
+    // of a 16-wide k-step: head lane / 4, channels 2 (lane % 4), + 1 and the same eight further on.
+    uint32_t wb[8][3][2];
+#pragma unroll
+    for (int ks = 0; ks < 8; ++ks) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float r0 = 0.f, r1 = 0.f;
+        if (MODE == MODE_TRIATT && fg < p.H) {
+          const float* src = p.wb + fg * 128 + ks * 16 + e * 8 + ft * 2;
+          r0 = src[0];
+          r1 = src[1];
+        }
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+          wb[ks][part][e] = pack_bf16x2(r0, r1);
+          r0 -= bf16_lo(wb[ks][part][e]);
+          r1 -= bf16_hi(wb[ks][part][e]);
+        }
+      }
+    }
     int stage = 0;
-    uint32_t phase = 0;
-    uint32_t acc_phase = 0;
-    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
-      const long long r = static_cast<long long>(t) * kPPRows + row_in_tile;
-      const bool row_ok = r < p.R;
-      // ---- row statistics (and head bias) from the shared-memory tile
+    uint32_t phase = 0, n = 0;
+    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++n) {
       mbar_wait(&x_full[stage], phase, ws, 15, stage);
       const uint8_t* xs = sX + stage * kPPXBytes;
       float sum = 0.f, sumsq = 0.f;
-#pragma unroll 4
+#pragma unroll 8
       for (int c16 = 0; c16 < 16; ++c16) {
-        const uint4 u = *reinterpret_cast<const uint4*>(xs + (c16 >> 3) * 16384 + swz128_offset(row_in_tile, c16 & 7));
+        const uint4 u = *reinterpret_cast<const uint4*>(xs + (c16 >> 3) * 16384 + swz128_offset(sw * 32 + lane, c16 & 7));
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -250,18 +251,17 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           sumsq += e1 * e1;
         }
       }
-      // head products of 16 rows per warp (q * 32 + grp * 16 ..) and up to eight heads on the warp-level matrix instruction
-      float hb[4] = {0.f, 0.f, 0.f, 0.f};
+      float hb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};     // [16 rows]
       if (MODE == MODE_TRIATT) {
-        const int lrow = q * 32 + grp * 16 + (lane & 15);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          uint32_t a0, a1, a2, a3;
-          ldmatrix_x4(xs + (ks >> 2) * 16384 + swz128_offset(lrow, (ks & 3) * 2 + (lane >> 4)), a0, a1, a2, a3);
 #pragma unroll
-          for (int part = 0; part < 3; ++part) {
-            const uint2 bw = sWbF[(part * 8 + ks) * 32 + lane];
-            mma_bf16_16816(hb, a0, a1, a2, a3, bw.x, bw.y);
+          for (int m16 = 0; m16 < 2; ++m16) {
+            uint32_t a0, a1, a2, a3;
+            ldmatrix_x4(xs + (ks >> 2) * 16384 + swz128_offset(sw * 32 + m16 * 16 + (lane & 15), (ks & 3) * 2 + (lane >> 4)), a0,
+                        a1, a2, a3);
+#pragma unroll
+            for (int part = 0; part < 3; ++part) mma_bf16_16816(hb[m16], a0, a1, a2, a3, wb[ks][part][0], wb[ks][part][1]);
           }
         }
       }
@@ -270,124 +270,137 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       const float mu = sum * (1.0f / kPPC);
       const float var = fmaxf(sumsq * (1.0f / kPPC) - mu * mu, 0.f);
       const float rstd = rsqrtf(var + 1e-5f);
-      if (p.stats_out != nullptr && grp == 0 && row_ok) {
+      const int b = n & 1;
+      mbar_wait(&r_empty[b], ((n >> 1) & 1u) ^ 1u, ws, 17, b);
+      sRow[b * 128 + sw * 32 + lane] = make_float2(rstd, -mu * rstd);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&r_full[b]);
+      const long long r0 = static_cast<long long>(t) * kPPRows + sw * 32, r = r0 + lane;
+      if (p.stats_out != nullptr && r < p.R) {
         p.stats_out[2 * r] = mu;
         p.stats_out[2 * r + 1] = rstd;
       }
-      // pair index of this row
-      int pi = 0, pk = 0;
-      if (row_ok) {
-        pi = static_cast<int>(r / p.N);
-        pk = static_cast<int>(r - static_cast<long long>(pi) * p.N);
-      }
-
       if (MODE == MODE_TRIATT) {
-        // this lane holds heads 2 ft, + 1 of rows grp * 16 + fg and + 8 of the quadrant
+        const int pi = static_cast<int>(r / p.N), pk = static_cast<int>(r - static_cast<long long>(pi) * p.N);
+        // this lane holds heads 2 ft, + 1 of rows fg, + 8, + 16, + 24
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int src = grp * 16 + e * 8 + fg;
+        for (int e = 0; e < 4; ++e) {
+          const int src = e * 8 + fg;
           const float rs = __shfl_sync(0xffffffffu, rstd, src), m = __shfl_sync(0xffffffffu, mu, src);
           const int ri = __shfl_sync(0xffffffffu, pi, src), rk = __shfl_sync(0xffffffffu, pk, src);
-          if (static_cast<long long>(t) * kPPRows + q * 32 + src < p.R) {
+          if (r0 + src < p.R) {
             const int oi = p.transpose_out ? rk : ri;
             const int ok = p.transpose_out ? ri : rk;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
               const int head = 2 * ft + c;
               if (head < p.H) {
-                const float val = rs * (hb[2 * e + c] - m * p.wb_colsum[head]) + p.wb_colbias[head];
+                const float val = rs * (hb[e >> 1][2 * (e & 1) + c] - m * p.wb_colsum[head]) + p.wb_colbias[head];
                 p.headbias[(static_cast<long long>(head) * p.plane_rows + oi) * p.Np + ok] = __float2bfloat16(val);
               }
             }
           }
         }
       }
-
-      // ---- accumulator half of this group
+      if (++stage == kPPStages) {
+        stage = 0;
+        phase ^= 1u;
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue warps
+    const int buf = (warp - 2) >> 2;  // q, k, v, gate
+    const int grp = buf >> 1;         // accumulator half
+    const int q = warp & 3;           // TMEM lane quadrant
+    const int fg = lane >> 2, ft = lane & 3;   // rows q * 32 + fg + 8 rr (rr < 4), two columns of every eight
+    uint8_t* stage_w = sOut + (warp - 2) * kPPOutWarpBytes;
+    __nv_bfloat16* out = buf == 0 ? p.q : buf == 1 ? p.k : buf == 2 ? p.v : p.g;
+    const CUtensorMap* om = &outs.m[buf];
+    uint32_t acc_phase = 0, n = 0;
+    for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++n) {
+      const int b = n & 1;
+      mbar_wait(&r_full[b], (n >> 1) & 1u, ws, 18, b);
+      float ra[4], rb[4];      // of this thread's four rows
+#pragma unroll
+      for (int rr = 0; rr < 4; ++rr) {
+        const float2 v = sRow[b * 128 + q * 32 + rr * 8 + fg];
+        ra[rr] = v.x;
+        rb[rr] = v.y;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&r_empty[b]);
+      // first row of this warp's 32 and its pair index, which places the output boxes
+      const long long r0 = static_cast<long long>(t) * kPPRows + q * 32;
+      const int bi = static_cast<int>(r0 / p.N);
+      const int bk = static_cast<int>(r0 - static_cast<long long>(bi) * p.N);
       mbar_wait(&acc_full[grp], acc_phase, ws, 16, grp);
       tc_fence_after_sync();
-      const uint32_t tbase = tmem_addr(tmem_base, q, grp * 256);
-      {
-        // half 0 = [q | k], half 1 = [v | g]; rows written at (possibly transposed) pair index
-        const long long orow = p.transpose_out ? (static_cast<long long>(pk) * p.N + pi) : r;
-        __nv_bfloat16* o0 = (grp == 0 ? p.q : p.v) + orow * 128;
-        __nv_bfloat16* o1 = (grp == 0 ? p.k : p.g) + orow * 128;
-        float ra[4], rb[4];      // of this thread's four rows
-#pragma unroll
-        for (int rr = 0; rr < 4; ++rr) {
-          ra[rr] = __shfl_sync(0xffffffffu, rstd, rr * 8 + fg);
-          rb[rr] = __shfl_sync(0xffffffffu, -mu * rstd, rr * 8 + fg);
-        }
-        // 32-column chunks, the tensor-memory load of the next chunk in flight while this one is processed;
-        // the chunk body exists twice (ping-pong registers), not eight times
-        // first row of this warp's 32 (a multiple of 32): its pair index places the warp's output box
-        const long long r0 = static_cast<long long>(t) * kPPRows + q * 32;
-        const int bi = static_cast<int>(r0 / p.N);
-        const int bk = static_cast<int>(r0 - static_cast<long long>(bi) * p.N);
-        // a transposed box holds second indices of one first index: rows that reach into the next one leave by lane
-        const bool boxed = p.out_tma != 0 && (!p.transpose_out || bk + 32 <= p.N || r0 + p.N - bk >= p.R);   // warp-uniform
-        auto chunk = [&](const uint32_t (&lo)[16], const uint32_t (&hi)[16], const int c0) {
-          if (lane == 0) tma_store_wait_read<0>();    // the previous box of this warp has left the staging rows
+      const uint32_t tbase = tmem_addr(tmem_base, q, buf * 128);
+#pragma unroll 1
+      for (int c0 = 0; c0 < 128; c0 += 32) {
+        uint32_t v[2][16];     // [lane half]
+        tmem_ld_frag32(tbase + c0, v[0]);
+        tmem_ld_frag32(tbase + kTmemLane16 + c0, v[1]);
+        tmem_ld_wait();
+        if (c0 == 96) {
+          tc_fence_before_sync();
           __syncwarp();
-          const bool gate = grp == 1 && c0 >= 128;    // warp-uniform
+          if (lane == 0) mbar_arrive(&acc_empty[grp]);       // the accumulators are in registers
+        }
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t o[4][2];    // [eight columns][row]
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            const int col = grp * 256 + c0 + u * 8;
-            const float2 cs = reinterpret_cast<const float2*>(sColsum + col)[ft];
-            const float2 cb = reinterpret_cast<const float2*>(sColbias + col)[ft];
+            const float2 cs = reinterpret_cast<const float2*>(sColsum + buf * 128 + c0 + u * 8)[ft];
+            const float2 cb = reinterpret_cast<const float2*>(sColbias + buf * 128 + c0 + u * 8)[ft];
 #pragma unroll
-            for (int rr = 0; rr < 4; ++rr) {
-              const uint32_t(&v)[16] = rr < 2 ? lo : hi;
-              const int k = u * 4 + (rr & 1) * 2;
-              float2 f = ln_fold2(v[k], v[k + 1], make_float2(ra[rr], ra[rr]), make_float2(rb[rr], rb[rr]), cs.x, cs.y,
-                                  cb.x, cb.y);
-              if (gate) f = make_float2(sigmoidf_fast(f.x), sigmoidf_fast(f.y));
-              *reinterpret_cast<uint32_t*>(stage_w + swz64_offset(rr * 8 + fg, u) + ft * 4) = pack_bf16x2(f.x, f.y);
+            for (int e = 0; e < 2; ++e) {
+              const int rr = hf * 2 + e, k = u * 4 + e * 2;
+              float2 f = ln_fold2(v[hf][k], v[hf][k + 1], make_float2(ra[rr], ra[rr]), make_float2(rb[rr], rb[rr]), cs.x,
+                                  cs.y, cb.x, cb.y);
+              if (buf == 3)    // warp-uniform
+                f = make_float2(sigmoidf_fast(f.x), sigmoidf_fast(f.y));
+              o[u][e] = pack_bf16x2(f.x, f.y);
             }
           }
-          if (boxed) {
-            // rows past R hold values of zero rows: the copy clips them
+          if (lane == 0) tma_store_wait_read<0>();    // the previous box of this warp has left the staging rows
+          __syncwarp();
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              *reinterpret_cast<uint32_t*>(stage_w + swz64_offset(e * 8 + fg, u) + ft * 4) = o[u][e];
+          // a transposed box holds second indices of one first index: rows that reach into the next one leave by lane
+          int xi = bi, xk = bk + hf * kPPBoxRows;
+          if (xk >= p.N) {     // 16 rows further on (a first index is no shorter than a box, or the box is not taken)
+            xi += 1;
+            xk -= p.N;
+          }
+          const long long h0 = r0 + hf * kPPBoxRows;
+          const bool boxed = p.out_tma != 0 && (!p.transpose_out || (xk < p.N && (xk + kPPBoxRows <= p.N || h0 + p.N - xk >= p.R)));
+          if (boxed) {         // warp-uniform; rows past R hold values of zero rows: the copy clips them
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              const CUtensorMap* om = &outs.m[grp * 2 + (c0 >> 7)];
-              if (p.transpose_out) tma_store_3d(om, stage_w, c0 & 127, bi, bk);
-              else tma_store_3d(om, stage_w, c0 & 127, static_cast<int>(r0), 0);
+              if (p.transpose_out) tma_store_3d(om, stage_w, c0, xi, xk);
+              else tma_store_3d(om, stage_w, c0, static_cast<int>(h0), 0);
               tma_store_commit();
             }
           } else {
             __syncwarp();
-            if (row_ok) {
-              uint4* dst = reinterpret_cast<uint4*>(c0 < 128 ? o0 + c0 : o1 + (c0 - 128));
-#pragma unroll
-              for (int j = 0; j < 4; ++j) dst[j] = *reinterpret_cast<const uint4*>(stage_w + swz64_offset(lane, j));
+            // two lanes per row, 32 bytes each
+            const long long r = h0 + (lane >> 1);
+            if (r < p.R) {
+              const long long pi = r / p.N, pk = r - pi * p.N;
+              const long long orow = p.transpose_out ? pk * p.N + pi : r;
+              uint4* dst = reinterpret_cast<uint4*>(out + orow * 128 + c0) + (lane & 1) * 2;
+              dst[0] = *reinterpret_cast<const uint4*>(stage_w + swz64_offset(lane >> 1, (lane & 1) * 2));
+              dst[1] = *reinterpret_cast<const uint4*>(stage_w + swz64_offset(lane >> 1, (lane & 1) * 2 + 1));
             }
             __syncwarp();
           }
-        };
-        uint32_t la[16], ha[16], lb[16], hb2[16];
-        tmem_ld_frag32(tbase, la);
-        tmem_ld_frag32(tbase + kTmemLane16, ha);
-#pragma unroll 1
-        for (int c0 = 0; c0 < 256; c0 += 64) {
-          tmem_ld_wait();
-          tmem_ld_frag32(tbase + c0 + 32, lb);
-          tmem_ld_frag32(tbase + kTmemLane16 + c0 + 32, hb2);
-          chunk(la, ha, c0);
-          tmem_ld_wait();
-          if (c0 + 64 < 256) {
-            tmem_ld_frag32(tbase + c0 + 64, la);
-            tmem_ld_frag32(tbase + kTmemLane16 + c0 + 64, ha);
-          }
-          chunk(lb, hb2, c0 + 32);
         }
-      }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[grp]);
-      if (++stage == kPPStages) {
-        stage = 0;
-        phase ^= 1u;
       }
       acc_phase ^= 1u;
     }
@@ -403,7 +416,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 }
 
 constexpr int kPPSmemBytes =
-    kPPWBytes + kPPStages * kPPXBytes + kPPOutBytes + (512 + 512) * 4 + kPPWbFrags * 8 + 256 + 1024;
+    kPPWBytes + kPPStages * kPPXBytes + kPPOutBytes + (512 + 512) * 4 + 2 * 128 * 8 + 256 + 1024;
 static_assert(kPPSmemBytes <= 232448, "shared memory of one CTA");
 
 template <int MODE>
@@ -444,13 +457,13 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
         if (p.transpose_out) {
           uint64_t d[3] = {128, (uint64_t)p.N, (uint64_t)p.N};
           uint64_t st[2] = {128 * 2, (uint64_t)p.N * 128 * 2};
-          uint32_t b[3] = {32, 1, 32};
+          uint32_t b[3] = {32, 1, kPPBoxRows};
           rc = make_tmap(&outs.m[i], bufs[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, d, st, b,
                          CU_TENSOR_MAP_SWIZZLE_64B);
         } else {
           uint64_t d[3] = {128, (uint64_t)p.R, 1};
           uint64_t st[2] = {128 * 2, (uint64_t)p.R * 128 * 2};
-          uint32_t b[3] = {32, 32, 1};
+          uint32_t b[3] = {32, kPPBoxRows, 1};
           rc = make_tmap(&outs.m[i], bufs[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, d, st, b,
                          CU_TENSOR_MAP_SWIZZLE_64B);
         }
@@ -463,7 +476,7 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
   rc = set_smem(kern, kPPSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  kern<<<grid, 320, kPPSmemBytes, stream>>>(tmX, tmW, maps, outs, p);
+  kern<<<grid, kPPThreads, kPPSmemBytes, stream>>>(tmX, tmW, maps, outs, p);
   UBM_CHECK_LAUNCH("pair_proj_kernel");
   return UBM_OK;
 }
