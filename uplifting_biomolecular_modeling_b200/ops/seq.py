@@ -7,7 +7,6 @@ three-term sum, width-2 pooling, residual + LayerNorm).  Every wrapper has a pla
 """
 from __future__ import annotations
 
-import functools
 from typing import Optional, Tuple
 
 import torch
@@ -196,22 +195,12 @@ def pole_step(state: torch.Tensor, lam: torch.Tensor, res: torch.Tensor, u: torc
     return out
 
 
-@functools.lru_cache(maxsize=256)
 def _pole_chunk(B: int, L: int, d: int) -> int:
-    """Positions per chunk of :func:`pole_conv_gate`: near 16 CTAs of 128 channels per SM (148 of them), between 32 (below that
-    the chunk states outweigh the sequence) and 1024, in whole stages of 16; long sequences take longer chunks so that the
-    chunk count fits a grid.  Among the lengths within a quarter of that, the one whose waves (9 CTAs of the chunk pass and 6
-    of the apply pass on an SM) end soonest, a stage of theirs taking about 2.6 and 3.6 us (8192 positions x 4096 channels:
-    128 positions 42 + 86 us in 2 and 3 waves)."""
+    """Positions per chunk of :func:`pole_conv_gate`: about 16 CTAs of 128 channels per SM (148 of them), between 32
+    (below that the chunk states outweigh the sequence) and 1024, in whole batches of 32; long sequences take longer
+    chunks so that the chunk count fits a grid."""
     per = B * L * d // (128 * 148 * 16)
-    least = (L + 65534) // 65535
-    if per <= 32 or per >= 1024 or least > 32:
-        return max(32, min(1024, (per + 31) // 32 * 32), least)
-
-    def cost(chunk):
-        ctas = -(-L // chunk) * -(-d // 128) * B
-        return chunk * (2.6 * -(-ctas // (148 * 9)) + 3.6 * -(-ctas // (148 * 6)))
-    return min(range(max(32, per * 3 // 4 // 16 * 16), per * 5 // 4 + 16, 16), key=cost)
+    return max(32, min(1024, (per + 31) // 32 * 32), (L + 65534) // 65535)
 
 
 def pole_conv_gate(u: torch.Tensor, lam: torch.Tensor, res: torch.Tensor, D: torch.Tensor,
