@@ -778,7 +778,8 @@ def _bf16_weight(module: nn.Linear):
     """(contiguous bf16 weight, fp32 bias or None) of a linear layer, kept until the weight is written again."""
     key = id(module)
     ent = _W_CACHE.get(key)
-    if ent is None or ent[0] is not module.weight or ent[1] != module.weight._version:
+    weight = module.weight               # one look-up: a module's attributes are found through its dictionaries
+    if ent is None or ent[0] is not weight or ent[1] != weight._version:
         ent = (module.weight, module.weight._version, module.weight.detach().to(torch.bfloat16).contiguous(),
                None if module.bias is None else module.bias.detach().float().contiguous())
         _W_CACHE[key] = ent
@@ -829,7 +830,7 @@ def folded_linear(module: nn.Linear, rows: torch.Tensor, gamma=None, eps: float 
     kernel with RMSNorm (``gamma``) in front, the residual (``res``) behind and, with ``second``, the SwiGLU of
     two projections."""
     from ..ops import seq
-    if getattr(module, "fp8_weights", False) and second is None and rows.shape[-1] % 16 == 0:
+    if second is None and getattr(module, "fp8_weights", False) and rows.shape[-1] % 16 == 0:
         q, dq, b8 = _e4m3_weight(module)          # the prefill's e4m3 weights: half the bytes of the step
         return seq.gemv_rows(rows, q, b8, gamma=gamma, eps=eps, res=res, wscale=dq)
     w, b = _bf16_weight(module)

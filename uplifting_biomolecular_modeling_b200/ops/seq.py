@@ -7,6 +7,8 @@ three-term sum, width-2 pooling, residual + LayerNorm).  Every wrapper has a pla
 """
 from __future__ import annotations
 
+import ctypes
+import struct
 from typing import Optional, Tuple
 
 import torch
@@ -27,6 +29,8 @@ native.declare("ubm_pool2", [c_void_p] * 3 + [c_int] * 4 + [c_void_p])
 native.declare("ubm_residual_ln", [c_void_p] * 6 + [c_ll, c_int, c_float, c_void_p])
 
 native.declare("ubm_gemv_fused", [c_void_p] * 2 + [c_float] + [c_void_p] * 5 + [c_int] * 3 + [c_void_p])
+native.declare("ubm_gemv_fused_packed", [ctypes.c_char_p])
+_GEMV_ARGS = struct.Struct("=11qd")      # the integer arguments of ubm_gemv_fused_packed in order, then eps
 native.declare("ubm_gemv_fused_w8", [c_void_p] * 2 + [c_float, c_void_p, c_float] + [c_void_p] * 3 + [c_int] * 3 + [c_void_p])
 native.declare("ubm_rmsnorm_fp8", [c_void_p] * 5 + [c_ll, c_int, c_float, c_void_p])
 native.declare("ubm_qk_norm_rotary", [c_void_p] * 4 + [c_ll] + [c_int] * 3 + [c_float] * 2 + [c_void_p])
@@ -377,7 +381,7 @@ def gemv_rows(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
     x = _bf16c(x)
     M, K = x.shape
     N = w.shape[0]
-    out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    out = x.new_empty((M, N))
     if w2 is not None and (w2.shape != w.shape or not w2.is_contiguous()):
         raise ValueError("gemv_rows: w2 must match w")
     if res is not None:
@@ -390,9 +394,10 @@ def gemv_rows(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
                                             native.ptr(bias), native.ptr(res), native.ptr(out), M, N, K, _stream(x))
         native.check(rc, "ubm_gemv_fused_w8")
         return out
-    rc = native.lib().ubm_gemv_fused(native.ptr(x), native.ptr(gamma), float(eps), native.ptr(w), native.ptr(w2),
-                                     native.ptr(bias), native.ptr(res), native.ptr(out), M, N, K, _stream(x))
-    native.check(rc, "ubm_gemv_fused")
+    ptr = native.ptr
+    rc = native.lib().ubm_gemv_fused_packed(_GEMV_ARGS.pack(ptr(x), ptr(gamma), ptr(w), ptr(w2), ptr(bias), ptr(res), ptr(out),
+                                                            M, N, K, _stream(x), eps))
+    native.check(rc, "ubm_gemv_fused_packed")
     return out
 
 
