@@ -8,10 +8,12 @@
 //   3. pole_apply_kernel    the recurrence again from those states, with the skip term and the gate (32 per position)
 // The transform form of the same convolution (zero-padded fp32 FFT, product, inverse FFT, transposing epilogue) moves
 // about 14 passes over fp32 copies padded to twice the length and rebuilds or keeps a spectrum per length; this moves
-// four bf16 passes plus the chunk states.  8192 positions x 4096 channels x 16 poles: 0.20 ms (63 + 11 + 124 us, the
-// state for decoding included) against 0.75 ms of transform kernels, their epilogue and a separate state scan, and
-// 0.16 ms of copies around them.  Bound by the 48 multiply-adds per position and channel (45 us) and the waits of the
-// 2-byte accesses of a thread per channel.
+// four bf16 passes plus the chunk states.  8192 positions x 4096 channels x 16 poles: 0.14 ms (42 + 11 + 86 us, the
+// state for decoding included; 63 + 11 + 124 with 2-byte loads of a thread per channel instead of the ring) against
+// 0.75 ms of transform kernels, their epilogue and a separate state scan, and 0.16 ms of copies around them.  Bound by
+// the 48 multiply-adds per position and channel (45 us, two per instruction) and the chain of a state from position to
+// position.  Chunks of 80 positions, which fill the last wave better, instead of 128:
+// 51 + 17 + 90 us.
 //
 // Medium operator (up to 128 taps): a depthwise convolution as one Toeplitz product per channel on mma.sync
 // m16n8k16 (see fir_toeplitz_kernel).  tcgen05 has no use here: a channel's operand is 16 x 144, its 128 x 64 tiles
@@ -205,8 +207,8 @@ __global__ void __launch_bounds__(kPcThreads) pole_apply_kernel(
 // A CTA owns 32 channels x 512 positions (+ 128 of halo), transposed into shared memory as [channel][position];
 // a warp owns four channels.  Results replace the inputs of their channel in place (the skip term is added there)
 // and leave through the same transpose, 16 bytes (8 channels) per access.
-// 8192 x 4096, 128 taps: 133 us against 248 us on the FMA pipes (17 G multiply-adds); what is left is the two
-// transposes through shared memory around 31 us of traffic.
+// 8192 x 4096, 128 taps: 97 us (136 with the loads of one batch waited for before the next was asked for) against 248 us
+// on the FMA pipes (17 G multiply-adds); what is left is the two transposes through shared memory around 31 us of traffic.
 constexpr int kTpCh = 32;
 constexpr int kTpPos = 512;
 constexpr int kTpHalo = 128;

@@ -372,7 +372,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 // 8 N columns, lane (g, t) = (lane / 4, lane % 4) reads columns 8 u + 2 t, + 1 of rows g and g + 8 into r[4 u .. 4 u + 3].
 // A thread then owns two columns of several rows, so a constant of a column is read from shared memory once for all of
 // them, 8 bytes per lane; with a row per lane, every lane reads every column's constants (512 bytes per 16-byte load and
-// warp, four clocks of the shared-memory port), which bounded the projection and output kernels.
+// warp, four clocks of the shared-memory port).
 __device__ __forceinline__ void tmem_ld_frag16(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])

@@ -17,7 +17,9 @@
 //
 // Warps: 0 = TMA producer, 1 = MMA issuer, 2-17 = four epilogue groups: operand (a, b) x half of the tile's columns,
 // 18-21 = row statistics, up to two tiles ahead of the epilogue.
-// TP_COMMENT
+// Bound by latency, not by a unit (0.8 GB at 1021 x 1021 tokens, 122 us at copy bandwidth): with the row statistics in the
+// epilogue warps their time added to a tile's; in warps of their own they are ready when the products are, and the gate's halves
+// are folded into its weights' scale: 243 -> 199 us at 1021, 145 -> 117 at 768, 37.6 -> 31.7 at 300, 15.5 -> 15.0 at 137.
 #include "host_util.h"
 #include "sm100.cuh"
 
