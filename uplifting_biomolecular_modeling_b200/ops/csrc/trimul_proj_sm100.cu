@@ -20,6 +20,8 @@
 // Bound by latency, not by a unit (0.8 GB at 1021 x 1021 tokens, 122 us at copy bandwidth): with the row statistics in the
 // epilogue warps their time added to a tile's; in warps of their own they are ready when the products are, and the gate's halves
 // are folded into its weights' scale: 243 -> 199 us at 1021, 145 -> 117 at 768, 37.6 -> 31.7 at 300, 15.5 -> 15.0 at 137.
+// From about 1200 tokens on it is the memory side (360 us before and after at 1200, 575 at 1536: 3.1 TB/s into 256 planes at
+// once); hints to keep or drop lines of either side in L2 change nothing.
 #include "host_util.h"
 #include "sm100.cuh"
 
