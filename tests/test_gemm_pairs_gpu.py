@@ -68,3 +68,16 @@ def test_swiglu(M, hidden, K):
     want = F.silu(x.double() @ wg.double().T) * (x.double() @ wv.double().T)
     # the gate's sigmoid has a relative error of 2e-4
     assert (got.double() - want).norm() <= 1.5 * 2.0 ** -9 * want.norm()
+
+
+@pytest.mark.parametrize("blocks", range(48, 54))
+def test_ring_ends_at_any_stage(blocks):
+    """One tile per pair that ends at each of the ring's six stages, launched back to back: no commit of a launch may still be
+    under way to a CTA that has left."""
+    from uplifting_biomolecular_modeling_b200.ops import gemm, native
+    M, N, K = 200, 9608, 64 * blocks
+    a, b = _r(9, M, K), _r(10, N, K)
+    got = [gemm.gemm(a, b) for _ in range(8)]
+    native.raise_on_status("cuda", "gemm")
+    _close(got[0], a.double() @ b.double().T)
+    assert all(torch.equal(g, got[0]) for g in got)
