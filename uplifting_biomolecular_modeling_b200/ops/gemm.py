@@ -19,6 +19,7 @@ native.declare("ubm_gemm_fp8", [native.c_void_p] * 5 + [native.c_int] * 3 + [nat
                [native.c_int, native.c_float, native.c_void_p, native.c_void_p, native.c_void_p])
 
 native.declare("ubm_gemm_bf16_packed", [ctypes.c_char_p])
+native.declare("ubm_gemm_bf16_tiles", [ctypes.c_char_p])      # the tiles such a call would take; launches nothing
 _ARGS = struct.Struct("=29qd")       # the integer arguments of ubm_gemm_bf16_ex in order, then alpha
 
 ACT = {None: 0, "none": 0, "silu": 1, "sigmoid": 2, "gelu": 3, "relu": 4, "swiglu3": 5, "swiglu": 6}
