@@ -426,7 +426,6 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
     const int half = ((warp - 3) >> 2) & 1;      // columns 128 half .. of D_g, 32 half .. of D_o
     const int q = warp & 3;
     const int row = q * 32 + lane;
-    const int fg = lane >> 2, ft = lane & 3;     // rows q * 32 + fg + 8 rr (rr < 4), two columns of every eight
     uint8_t* st = sSt + team * kPoStage;
     const uint32_t tb = tmem_base + team * 256;
     uint32_t n = 0;
@@ -450,46 +449,32 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
       }
       const float mu = sum * (1.f / kPwC);
       const float rstd = row_rstd(mu, sumsq, p.eps);
-      float ra[4], rb[4];
-#pragma unroll
-      for (int rr = 0; rr < 4; ++rr) {
-        ra[rr] = __shfl_sync(0xffffffffu, rstd, rr * 8 + fg);
-        rb[rr] = __shfl_sync(0xffffffffu, -mu * rstd, rr * 8 + fg);
-      }
+      const float2 a2 = make_float2(rstd, rstd), b2 = make_float2(-mu * rstd, -mu * rstd);
       mbar_wait(&g_full[team], ph, ws, 87, team);
       tc_fence_after_sync();
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         const int col = half * 128 + c * 32;
-        uint32_t v[2][16];                       // [lane half]
-        tmem_ld_frag32(tmem_addr(tb, q, col), v[0]);
-        tmem_ld_frag32(tmem_addr(tb, q, col) + kTmemLane16, v[1]);
+        uint32_t v[32];
+        tmem_ld32(tmem_addr(tb, q, col), v);
         tmem_ld_wait();
-        float2 f[4][4];                          // [eight columns][row]
-        float low = 0.f;
+        float f[32];
+        ln_fold32(v, a2, b2, sConst + col, sConst + kPwHC + col, f);
+        float low = fminf(f[0], f[1]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float2* gc = reinterpret_cast<const float2*>(sConst + col + u * 8) + ft;
-          const float2 cs = gc[0], cb = gc[kPwHC / 2];
-#pragma unroll
-          for (int rr = 0; rr < 4; ++rr) {
-            const int k = u * 4 + (rr & 1) * 2;
-            f[u][rr] = ln_fold2(v[rr >> 1][k], v[rr >> 1][k + 1], make_float2(ra[rr], ra[rr]), make_float2(rb[rr], rb[rr]),
-                                cs.x, cs.y, cb.x, cb.y);
-            low = min3f(low, f[u][rr].x, f[u][rr].y);
-          }
-        }
+        for (int k = 2; k < 32; k += 2) low = min3f(low, f[k], f[k + 1]);
         uint8_t* ob = st + (1 + (col >> 6)) * kPwTile;
         auto apply = [&](auto gate) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+          for (int j8 = 0; j8 < 4; ++j8) {
+            uint4* at = reinterpret_cast<uint4*>(ob + swz128_offset(row, ((col >> 5) & 1) * 4 + j8));
+            const uint4 u = *at;
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+            uint32_t r[4];
 #pragma unroll
-            for (int rr = 0; rr < 4; ++rr) {
-              uint32_t* at =
-                  reinterpret_cast<uint32_t*>(ob + swz128_offset(q * 32 + rr * 8 + fg, ((col >> 5) & 1) * 4 + u)) + ft;
-              const uint32_t w = *at;
-              *at = pack_bf16x2(bf16_lo(w) * gate(f[u][rr].x), bf16_hi(w) * gate(f[u][rr].y));
-            }
+            for (int e = 0; e < 4; ++e)
+              r[e] = pack_bf16x2(bf16_lo(w[e]) * gate(f[j8 * 8 + 2 * e]), bf16_hi(w[e]) * gate(f[j8 * 8 + 2 * e + 1]));
+            *at = make_uint4(r[0], r[1], r[2], r[3]);
           }
         };
         // nearly closed gates take the form that keeps their relative precision (for every gate it costs 27 us more)
