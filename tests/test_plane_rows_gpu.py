@@ -50,3 +50,31 @@ def test_head_bias_rows(N):
     assert planes.stride(1) % 16 == 0 and torch.equal(planes, given[:, :, :N])
     whole = planes.as_strided((4, N, planes.stride(1)), planes.stride())
     assert not whole[:, :, N:].any()
+
+
+@pytest.mark.parametrize("N", [9, 129])
+def test_projection_statistics(N):
+    """Row means of the projection as the sum of four parts of 32 channels: results do not depend on which warp takes them."""
+    from uplifting_biomolecular_modeling_b200.ops import native, pair
+    g = torch.Generator(device="cuda").manual_seed(N)
+    c = 128
+    z = (_rand((N, N, c), g, 3.0) + 40.0).bfloat16()
+    one, zero = torch.ones(c, device="cuda"), torch.zeros(c, device="cuda")
+    w = pair.TrimulPacked.pack(one, zero, *(_rand((2 * c, c), g) for _ in range(2)), one, zero, *(_rand((c, c), g) for _ in range(2)))
+    Np = pair.ceil_to(N, pair.PLANE_ROW)
+    planes = torch.empty(2, 128, N, Np, device="cuda", dtype=torch.bfloat16)
+    stats = torch.empty(N * N, 2, device="cuda")
+    rc = native.lib().ubm_trimul_proj(native.ptr(z), native.ptr(w.w_in), native.ptr(w.in_colsum), native.ptr(w.in_colbias), 0,
+                                      native.ptr(planes), native.ptr(stats), N, Np, native.ptr(native.status_tensor(z.device)),
+                                      native.current_stream(z.device))
+    native.check(rc, "ubm_trimul_proj")
+    native.raise_on_status("cuda", "trimul_proj")
+    x = z.float().view(N * N, 4, 16, 2)
+    pairs, part = x[..., 0] + x[..., 1], torch.zeros(N * N, 4, device="cuda")
+    for k in range(16):
+        part = part + pairs[:, :, k]
+    mean = ((part[:, 0] + part[:, 1]) + (part[:, 2] + part[:, 3])) / 128
+    assert torch.equal(stats[:, 0], mean)
+    var = z.double().view(N * N, c).var(-1, unbiased=False)
+    # single-pass variance: fp32 sums of squares near 40^2 + 3^2 (2^-24 of 1609 for each of about 40 roundings) against 9
+    assert ((stats[:, 1].double() * (var + 1e-5).sqrt() - 1).abs() <= 40 * 2 ** -24 * 1609 / 9).all()

@@ -692,6 +692,30 @@ __device__ __forceinline__ void ldmatrix_x4(const void* row, uint32_t& a0, uint3
                : "memory");
 }
 
+// Sum and sum of squares of a row of 128 bf16 values, two k-blocks of [128 rows][64] in the 128-byte swizzle at `tile`: four
+// sums of 32 values in a tree, shorter chains and less rounding than one of 128.
+__device__ __forceinline__ void row_sums128(const uint8_t* tile, uint32_t row, float& sum, float& sumsq) {
+  sum = 0.f;
+  sumsq = 0.f;
+#pragma unroll 1
+  for (int kb = 0; kb < 2; ++kb) {
+    float s[2] = {0.f, 0.f}, q[2] = {0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const uint4 u = *reinterpret_cast<const uint4*>(tile + kb * 16384 + swz128_offset(row, c));
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = bf16_lo(w[j]), b = bf16_hi(w[j]);
+        s[c >> 2] += a + b;
+        q[c >> 2] += a * a + b * b;
+      }
+    }
+    sum += s[0] + s[1];
+    sumsq += q[0] + q[1];
+  }
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

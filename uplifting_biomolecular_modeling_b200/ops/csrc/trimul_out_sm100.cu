@@ -15,8 +15,10 @@
 // ahead of the epilogue.  TMEM: {O, G} x two tiles = 512 columns.
 // Bound by latency, not by a unit (0.8 GB at 1021 x 1021 tokens, 122 us at copy bandwidth): what an epilogue warp does one
 // after the other sets the pace.  With the statistics of both operands in the epilogue warps a tile waited for them before its
-// accumulators could be read; in warps of their own they are ready when the products are: 195 -> 187 us at 1021, 118 -> 113 at
-// 768, 30.6 -> 28.7 at 300, 421 -> 407 at 1536.  Not faster: the x tile given back before the z tile (197 against 197 us).
+// accumulators could be read; in warps of their own they are ready when the products are.  Inside a whole multiplication,
+// before -> now: 12.1 -> 11.4 us at 137 tokens, 30.0 -> 28.9 at 300, 114.7 -> 112.3 at 768, 447 -> 440 at 1536, but 204 -> 207 at
+// 1021 and 289 -> 293 at 1200, where the planes come from a GEMM that now writes them in another order (by itself 195 -> 187 at
+// 1021).  Not faster: the x tile given back before the z tile (197 against 197 us).
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -51,8 +53,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   uint8_t* sSt = smem + 2 * kTOTileBytes; // stages: {x tile 32 KB, z tile 32 KB}
   float* sConst = reinterpret_cast<float*>(sSt + kTOStages * kTOStageBytes);  // 4 x 128
   float4* sRow = reinterpret_cast<float4*>(sConst + 512);    // [stages][128]: 1 / std, - mean / std of x column and z row
-  float2* sPart = reinterpret_cast<float2*>(sRow + kTOStages * 128);   // [2][128]: an x column's sums over half of the channels
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sPart + 2 * 128);
+  float2* sPart = reinterpret_cast<float2*>(sRow + kTOStages * 128);   // [stages][5][128]: an x column's sums
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sPart + kTOStages * 5 * 128);
   uint64_t* full = bars;                 // [stages]
   uint64_t* empty = full + kTOStages;    // [stages]  MMA commit + 8 output boxes that have left the tile
   uint64_t* w_full = empty + kTOStages;  // [1]
@@ -193,36 +195,42 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       mbar_wait(&full[stage], phase, ws, 27, stage);
       const uint8_t* sx = sSt + stage * kTOStageBytes;
       const uint8_t* sz = sx + kTOTileBytes;
-      float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-#pragma unroll 16
-      for (int c = 0; c < 64; ++c) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(sx + ((ch0 >> 6) * 2 + jh) * 8192 +
-                                                              swz128_offset(c, lane >> 2) + (lane & 3) * 4);
-        const float a = bf16_lo(w), b = bf16_hi(w);
-        s0 += a;
-        q0 += a * a;
-        s1 += b;
-        q1 += b * b;
-      }
-      float sum = 0.f, sumsq = 0.f;
-#pragma unroll 8
-      for (int c = 0; c < 16; ++c) {
-        const uint4 u = *reinterpret_cast<const uint4*>(sz + (c >> 3) * 16384 + swz128_offset(st, c & 7));
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+      // a column's sums: channels 0 - 63 in one warp, 64 - 79, .. each by itself in the other, added up in ascending order below.
+      // Two sets of them, by turns: whoever writes one has passed the barrier behind the reading of the other.
+      float4* part = reinterpret_cast<float4*>(sPart + stage * 5 * 128) + ((jh * 64 + lane * 2) >> 1);
+      float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+      for (int k = 0; k < 4; ++k) {
+        float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const float a = bf16_lo(w[m]), b = bf16_hi(w[m]);
-          sum += a + b;
-          sumsq += a * a + b * b;
+        for (int c = 0; c < 16; ++c) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(sx + ((ch0 >> 6) * 2 + jh) * 8192 +
+                                                                swz128_offset(k * 16 + c, lane >> 2) + (lane & 3) * 4);
+          const float a = bf16_lo(w), b = bf16_hi(w);
+          s0 += a;
+          q0 += a * a;
+          s1 += b;
+          q1 += b * b;
+        }
+        if (ch0 == 0) {
+          run = make_float4(run.x + s0, run.y + q0, run.z + s1, run.w + q1);
+        } else {
+          part[(k + 1) * 64] = make_float4(s0, q0, s1, q1);
         }
       }
-      // the four warps exchange the halves: nobody reads the previous tile's any more, then nobody reads too early
+      if (ch0 == 0) part[0] = run;
+      float sum, sumsq;
+      row_sums128(sz, st, sum, sumsq);
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      reinterpret_cast<float4*>(sPart)[((sw >> 1) * 128 + jh * 64 + lane * 2) >> 1] = make_float4(s0, q0, s1, q1);
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      const float2 xa = sPart[st], xb = sPart[128 + st];
-      const float mux = (xa.x + xb.x) * (1.f / 128.f), muz = sum * (1.f / 128.f);
-      const float rsx = rsqrtf(fmaxf((xa.y + xb.y) * (1.f / 128.f) - mux * mux, 0.f) + 1e-5f);
+      float2 x = sPart[stage * 5 * 128 + st];
+#pragma unroll
+      for (int k = 1; k < 5; ++k) {
+        const float2 v = sPart[(stage * 5 + k) * 128 + st];
+        x.x += v.x;
+        x.y += v.y;
+      }
+      const float mux = x.x * (1.f / 128.f), muz = sum * (1.f / 128.f);
+      const float rsx = rsqrtf(fmaxf(x.y * (1.f / 128.f) - mux * mux, 0.f) + 1e-5f);
       const float rsz = rsqrtf(fmaxf(sumsq * (1.f / 128.f) - muz * muz, 0.f) + 1e-5f);
       sRow[stage * 128 + st] = make_float4(rsx, -mux * rsx, rsz, -muz * rsz);
       __syncwarp();
@@ -330,7 +338,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 }
 
 static_assert(kTOStages == 2, "the release of a tile's buffers names the other stage");
-constexpr int kTOSmemBytes = 2 * kTOTileBytes + kTOStages * kTOStageBytes + 512 * 4 + kTOStages * 128 * 16 + 2 * 128 * 8 + 256 + 1024;
+constexpr int kTOSmemBytes = 2 * kTOTileBytes + kTOStages * kTOStageBytes + 512 * 4 + kTOStages * 128 * 16 +
+                             kTOStages * 5 * 128 * 8 + 256 + 1024;
 static_assert(kTOSmemBytes <= 232448, "shared memory of one CTA");
 
 }  // namespace ubm

@@ -19,9 +19,10 @@
 // 18-21 = row statistics, up to two tiles ahead of the epilogue.
 // Bound by latency, not by a unit (0.8 GB at 1021 x 1021 tokens, 122 us at copy bandwidth): with the row statistics in the
 // epilogue warps their time added to a tile's; in warps of their own they are ready when the products are, and the gate's halves
-// are folded into its weights' scale: 243 -> 199 us at 1021, 145 -> 117 at 768, 37.6 -> 31.7 at 300, 15.5 -> 15.0 at 137.
-// From about 1200 tokens on it is the memory side (360 us before and after at 1200, 575 at 1536: 3.1 TB/s into 256 planes at
-// once); hints to keep or drop lines of either side in L2 change nothing.
+// are folded into its weights' scale.  Inside a whole multiplication, before -> now: 13.8 -> 12.4 us at 137 tokens, 35.2 -> 29.3 at
+// 300, 140 -> 113 at 768, 238 -> 202 at 1021.  From about 1200 tokens on it is the memory side: 363 -> 351 at 1200, 480 -> 477 at
+// 1400, 590 -> 570 to 590 at 1536 (3.1 TB/s into 256 planes at once); hints to keep or drop lines of either side in L2 change
+// nothing.  The mask multiplies the gate, not the product: 2 % slower at 768, and the planes are what they were bit for bit.
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -193,19 +194,8 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     uint32_t phase = 0, n = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++n) {
       mbar_wait(&x_full[stage], phase, ws, 15, stage);
-      const uint8_t* xs = sX + stage * kTPXBytes;
-      float sum = 0.f, sumsq = 0.f;
-#pragma unroll 8
-      for (int c = 0; c < 16; ++c) {
-        const uint4 u = *reinterpret_cast<const uint4*>(xs + (c >> 3) * 16384 + swz128_offset(row, c & 7));
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float a = bf16_lo(w[j]), b = bf16_hi(w[j]);
-          sum += a + b;
-          sumsq += a * a + b * b;
-        }
-      }
+      float sum, sumsq;
+      row_sums128(sX + stage * kTPXBytes, row, sum, sumsq);
       __syncwarp();
       if (lane == 0) mbar_arrive(&x_empty[stage]);
       const float mu = sum * (1.0f / kTPC);
@@ -234,7 +224,7 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const int half = (warp - 2) >> 3;       // columns 64 half .. 64 half + 63
     const int q = warp & 3;                 // TMEM lane quadrant
     const int g = lane >> 2, t4 = lane & 3; // channels q * 32 + g + 8 rr (rr < 4), two columns of every eight
-    // value and gate are formed at half their size: sigmoid(x) v = v / 2 + v / 2 tanh(x / 2)
+    // value and gate are formed at half their size: mask sigmoid(x) v = (mask + mask tanh(x / 2)) v / 2
     float cs_v[4], cb_v[4], cs_g[4], cb_g[4];
 #pragma unroll
     for (int rr = 0; rr < 4; ++rr) {
@@ -300,7 +290,7 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                                           make_float2(fmaf(nm.x, cs_v[rr], cb_v[rr]), fmaf(nm.y, cs_v[rr], cb_v[rr])));
             const float2 gate = __ffma2_rn(make_float2(__uint_as_float(gr[k]), __uint_as_float(gr[k + 1])), rs,
                                            make_float2(fmaf(nm.x, cs_g[rr], cb_g[rr]), fmaf(nm.y, cs_g[rr], cb_g[rr])));
-            const float2 ov = __fmul2_rn(mk, __ffma2_rn(val, make_float2(fast_tanh(gate.x), fast_tanh(gate.y)), val));
+            const float2 ov = __fmul2_rn(val, __ffma2_rn(make_float2(fast_tanh(gate.x), fast_tanh(gate.y)), mk, mk));
             *reinterpret_cast<uint32_t*>(stage_w + rr * 512 + at) = pack_bf16x2(ov.x, ov.y);
           }
         }
