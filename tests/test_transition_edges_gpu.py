@@ -46,3 +46,30 @@ def test_fewest_chunks_with_several_tiles_per_cta(hidden):
     assert (got.double() - want).norm() <= 5 * 2.0 ** -8 * want.norm()
     far = (got.double() - want).norm(dim=1) > 0.1 * want.norm(dim=1)        # no tile left out
     assert not far.any()
+
+
+def _weights(seed, hidden):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    return r, (1 + 0.1 * r(128), 0.1 * r(128), r(hidden, 128) / 128 ** 0.5, r(hidden, 128) / 128 ** 0.5, r(128, hidden) / hidden ** 0.5)
+
+
+def test_rows_whose_squares_overflow():
+    """Such a row has no variance in fp32; as in the tensor statements what is left of its norm is the bias."""
+    from uplifting_biomolecular_modeling_b200.ops import native, pair
+    r, (nw, nb, a, b, o) = _weights(7, 256)
+    x = torch.sign(r(300, 128)).bfloat16()
+    x[:, 64:] = -x[:, :64]                                       # mean 0
+    x[5], x[17], x[200:232] = x[5] * 1e19, x[17] * 3e25, x[200:232] * 1e30
+    x[60], x[299] = float("nan"), float("inf")
+    got = pair.transition_fused(x, pair.TransitionPacked.pack(nw, nb, a, b, o), residual=False)
+    native.raise_on_status("cuda", "transition")
+    bias = (torch.nn.functional.silu(a.double() @ nb.double()) * (b.double() @ nb.double())) @ o.double().T
+    both = pair.transition_fused(x, pair.TransitionPacked.pack(nw, nb, a, b, o), residual=True)
+    rows = [5, 17, *range(200, 232)]
+    assert torch.equal(both[rows], x[rows])                      # the residual dwarfs the bias
+    assert ((got[rows].double() - bias).norm(dim=1) <= 5 * 2.0 ** -8 * bias.norm()).all()
+    assert got[[60, 299]].isnan().all()
+    rest = [i for i in range(300) if i not in rows + [60, 299]]
+    want = R.transition(x[rest].double(), *(t.double() for t in (nw, nb, a, b, o)), residual=False)
+    assert (got[rest].double() - want).norm() <= 5 * 2.0 ** -8 * want.norm()

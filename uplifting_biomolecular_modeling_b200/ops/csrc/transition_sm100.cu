@@ -43,6 +43,7 @@ constexpr int kTRWStages = 2;
 constexpr int kTRMaxHidden = 1024;
 
 struct TransitionParams {
+  const __nv_bfloat16* x;   // [R][128]
   long long R;
   int hidden;               // multiple of 64
   const float* ab_colsum;   // [hidden/64][128] in packed order
@@ -352,7 +353,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     auto statistics = [&](uint32_t tl) {
       const int xs = tl & 1;
       mbar_wait(&x_full[xs], (tl >> 1) & 1u, ws, 45, xs);
-      const uint8_t* xsm = sX + xs * kTRXBytes;
+      uint8_t* xsm = sX + xs * kTRXBytes;
       float sum = 0.f, sumsq = 0.f;
 #pragma unroll
       for (int c = 0; c < 16; ++c) {
@@ -368,21 +369,32 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       const float mu = sum * (1.f / kTRC);
       const float var = fmaxf(sumsq * (1.f / kTRC) - mu * mu, 0.f);
       const float rstd = rsqrtf(var + 1e-5f);
+      // A row whose squares overflow has no deviation (rstd 0), and nothing but the bias is left of its norm, as in fp32 tensor
+      // statements.  No deviation carries the bias through the products (infinity, times 0 behind them), so the row enters them as
+      // zeros of deviation 1; the residual is read again.
+      const bool flat = rstd == 0.f;
+      if (flat) {
+#pragma unroll 1
+        for (int c = 0; c < 16; ++c)
+          *reinterpret_cast<uint4*>(xsm + (c >> 3) * 16384 + swz128_offset(row, c & 7)) = make_uint4(0u, 0u, 0u, 0u);
+      }
       // the buffers of tile t + 1 were last read for tile t - 1, all of whose products this warp has waited for (y_full)
-      sRstd[xs * 128 + row] = rstd;
-      store_row_factors(sXext + xs * kTRExtBytes, row, -mu, (var + 1e-5f) * rstd);
+      sRstd[xs * 128 + row] = flat ? 1.f : rstd;
+      store_row_factors(sXext + xs * kTRExtBytes, row, flat ? 0.f : -mu, flat ? 1.f : (var + 1e-5f) * rstd);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&r_full[xs]);
+      return flat;
     };
-    if (my_tiles > 0) statistics(0);
+    bool next_flat = my_tiles > 0 && statistics(0);
     for (uint32_t tl = 0; tl < my_tiles; ++tl) {
       if (tl > 0 && lane == 0) {
         // the boxes this thread stored from the previous tile have been read: its buffer may be loaded again
         tma_store_wait_read<0>();
         mbar_arrive(&x_empty[(tl & 1) ^ 1]);
       }
-      if (tl + 1 < my_tiles) statistics(tl + 1);
+      const bool flat = next_flat;
+      if (tl + 1 < my_tiles) next_flat = statistics(tl + 1);
       const int t = static_cast<int>(blockIdx.x + tl * gridDim.x);
       const long long r = static_cast<long long>(t) * 128 + row;
       const float mval = (p.mask != nullptr && r < p.R) ? p.mask[r] : 1.0f;
@@ -421,6 +433,17 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           }
           *at = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
                            pack_bf16x2(f[6], f[7]));
+        }
+      }
+      if (flat && p.add_residual) {   // behind the release of the accumulator, which the next tile waits for
+#pragma unroll 1
+        for (int c = 0; c < 16; ++c) {
+          uint4* at = reinterpret_cast<uint4*>(xsm + (c >> 3) * 16384 + swz128_offset(row, c & 7));
+          const uint4 y = *at, u = *reinterpret_cast<const uint4*>(p.x + r * 128 + c * 8);
+          *at = make_uint4(pack_bf16x2(bf16_lo(y.x) + bf16_lo(u.x), bf16_hi(y.x) + bf16_hi(u.x)),
+                           pack_bf16x2(bf16_lo(y.y) + bf16_lo(u.y), bf16_hi(y.y) + bf16_hi(u.y)),
+                           pack_bf16x2(bf16_lo(y.z) + bf16_lo(u.z), bf16_hi(y.z) + bf16_hi(u.z)),
+                           pack_bf16x2(bf16_lo(y.w) + bf16_lo(u.w), bf16_hi(y.w) + bf16_hi(u.w)));
         }
       }
       fence_proxy_async_smem();
@@ -488,6 +511,7 @@ extern "C" int ubm_transition(const void* x, const void* wab, const void* wo, co
     if (rc) return rc;
   }
   TransitionParams p = {};
+  p.x = static_cast<const __nv_bfloat16*>(x);
   p.R = R;
   p.hidden = hidden;
   p.ab_colsum = static_cast<const float*>(ab_colsum);
