@@ -54,6 +54,31 @@ def _weights(seed, hidden):
     return r, (1 + 0.1 * r(128), 0.1 * r(128), r(hidden, 128) / 128 ** 0.5, r(hidden, 128) / 128 ** 0.5, r(128, hidden) / hidden ** 0.5)
 
 
+@pytest.mark.parametrize("hidden", [64, 512])
+@pytest.mark.parametrize("ratio", [1, 10, 100])
+def test_rows_far_from_zero(ratio, hidden):
+    """Mean and bias enter the first product as three bf16 parts each: a mean of many deviations shows every one of them."""
+    from uplifting_biomolecular_modeling_b200.ops import native, pair
+    r, w = _weights(ratio + hidden, hidden)
+    # powers of two and 7-bit fractions, so that the deviations survive the rounding of a row to bf16
+    x = (ratio * 2.0 ** r(3000, 1).round() + torch.sign(r(3000, 128)) * 2.0 ** r(3000, 1).round()).bfloat16()
+    packed = pair.TransitionPacked.pack(*w)
+    got = pair.transition_fused(x, packed, residual=False)
+    native.raise_on_status("cuda", "transition")
+    # float64 on the kernel's own folded weights: their rounding is not what is tested
+    xd = x.double()
+    mu, rstd = xd.mean(-1, keepdim=True), (xd.var(-1, unbiased=False, keepdim=True) + 1e-5).rsqrt()
+    ab = (rstd * (xd @ packed.wab.double().T - mu * packed.colsum.double()) + packed.colbias.double()).view(len(x), -1, 2, 64)
+    h = torch.nn.functional.silu(ab[:, :, 0]) * ab[:, :, 1]
+    want = h.reshape(len(x), -1) @ packed.wo.double().T
+    # fp32 sums of 128 products of the size of the mean against the deviation, the variance from sums of squares likewise; then
+    # tanh.approx (2^-11) and two roundings to bf16
+    size = (xd.abs().amax(-1, keepdim=True) * rstd).clamp(min=1)
+    bound = 2.5 * 2.0 ** -9 + 32 * 2.0 ** -24 * size ** 2
+    err = (got.double() - want).norm(dim=1, keepdim=True) / want.norm(dim=1, keepdim=True)
+    assert (err <= bound).all(), (err / bound).max()
+
+
 def test_rows_whose_squares_overflow():
     """Such a row has no variance in fp32; as in the tensor statements what is left of its norm is the bias."""
     from uplifting_biomolecular_modeling_b200.ops import native, pair
