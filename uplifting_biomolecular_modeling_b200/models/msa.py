@@ -70,6 +70,8 @@ class OuterProductMean(_Switchable):
             mk = mask[0].expand(S, N)
             if mk.dtype == torch.bfloat16 and N % 8 == 0:       # bf16 values: exact products, fp32 sums
                 mk = mk.contiguous()
+                if mk.data_ptr() % 16:                          # the GEMM's tensor maps start on 16 bytes
+                    mk = mk.clone()
                 count = gemm.gemm(mk, mk, mn_major=True, out_dtype=torch.float32)
             else:
                 count = torch.einsum("si,sj->ij", mk.float(), mk.float())

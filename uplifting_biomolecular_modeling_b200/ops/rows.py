@@ -65,6 +65,10 @@ def mean_rescale_(o: torch.Tensor, count: torch.Tensor, bias: torch.Tensor, tota
     if o.dtype != torch.bfloat16 or not o.is_contiguous() or count.dtype != torch.float32 or count.numel() != R or \
             not count.is_contiguous() or bias.dtype != torch.float32 or bias.shape != (C,) or not bias.is_contiguous():
         raise ValueError(f"mean_rescale_ expects bf16 rows with {R} fp32 counts and {C} fp32 biases")
+    if not o.is_cuda or count.device != o.device or bias.device != o.device:
+        raise ValueError("mean_rescale_: rows, counts and biases live on one GPU")
+    if bias.data_ptr() % 16:                                    # read four at a time
+        bias = bias.clone()
     rc = native.lib().ubm_mean_rescale(native.ptr(o), native.ptr(count), native.ptr(bias), R, C, float(total),
                                        native.current_stream(o.device))
     native.check(rc, "ubm_mean_rescale")
