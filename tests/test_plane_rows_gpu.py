@@ -78,3 +78,39 @@ def test_projection_statistics(N):
     var = z.double().view(N * N, c).var(-1, unbiased=False)
     # single-pass variance: fp32 sums of squares near 40^2 + 3^2 (2^-24 of 1609 for each of about 40 roundings) against 9
     assert ((stats[:, 1].double() * (var + 1e-5).sqrt() - 1).abs() <= 40 * 2 ** -24 * 1609 / 9).all()
+
+
+@pytest.mark.parametrize("row", [8, 16])
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("H", [4, 16])
+@pytest.mark.parametrize("N", [7, 8, 24, 33, 48, 129])
+def test_head_bias_padding(monkeypatch, N, H, transpose, row):
+    """Planes of its own have zeros behind every row, whatever the memory held; planes given to it keep their rows' length and what
+    lies behind column N."""
+    from uplifting_biomolecular_modeling_b200.ops import rows
+    g = torch.Generator(device="cuda").manual_seed(N + H)
+    z, w = _rand((N, N, 128), g).bfloat16(), _rand((H, 128), g, 128 ** -0.5)
+    one, zero = torch.ones(128, device="cuda"), torch.zeros(128, device="cuda")
+    Np = (N + row - 1) // row * row
+    real = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: real(*a, **k).fill_(float("nan")))
+    own = rows.pair_head_bias(z, one, zero, w, transpose=transpose, row=row)
+    monkeypatch.undo()
+    whole = own.as_strided((H, N, Np), (N * Np, Np, 1))
+    assert own.stride() == (N * Np, Np, 1) and not whole[:, :, N:].any() and own.isfinite().all()
+    for ld in {(N + 7) // 8 * 8, Np, Np + 8}:
+        planes = torch.full((H, N, ld), 5.0, device="cuda", dtype=torch.bfloat16)
+        for given in (planes, planes[:, :, :N]):
+            planes[:, :, :N] = 5.0
+            got = rows.pair_head_bias(z, one, zero, w, transpose=transpose, out=given)
+            assert torch.equal(got, own) and torch.equal(planes[:, :, :N], own) and (planes[:, :, N:] == 5).all()
+
+
+def test_head_bias_planes_that_do_not_fit():
+    from uplifting_biomolecular_modeling_b200.ops import rows
+    z, w = torch.zeros(24, 24, 128, device="cuda", dtype=torch.bfloat16), torch.zeros(4, 128, device="cuda")
+    planes = torch.zeros(4, 24, 32, device="cuda", dtype=torch.bfloat16)
+    for out in (planes.float(), planes[:3], planes[:, :23], planes[:, :, :23], planes.cpu(), planes[:, ::2], planes.view(4, -1),
+                torch.zeros(4, 24, 28, device="cuda", dtype=torch.bfloat16), torch.zeros(4, 25, 24, device="cuda", dtype=torch.bfloat16)):
+        with pytest.raises(ValueError):
+            rows.pair_head_bias(z, None, None, w, out=out)

@@ -79,14 +79,26 @@ _HB_CACHE = {}
 
 
 def pair_head_bias(z: torch.Tensor, ln_w, ln_b, w, scale: float = 1.0, transpose: bool = False,
-                   out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """z: bf16 [N, N, 128]; w: [H, 128].  Returns bf16 [H, N, N] (a view of planes padded to whole 32-byte
-    sectors, 16 columns; planes given as ``out`` to a multiple of 8) with ``scale * Linear(LN(z))`` laid out head-major."""
+                   out: Optional[torch.Tensor] = None, row: int = 16) -> torch.Tensor:
+    """z: bf16 [N, N, 128]; w: [H, 128].  Returns bf16 [H, N, N] (a view of planes whose rows are padded with zeros to a
+    multiple of ``row`` elements, 8 or more) with ``scale * Linear(LN(z))`` laid out head-major.  ``out``: bf16 planes [H, N, N or more] to
+    write instead, one behind the other with rows of a multiple of 8 elements; columns behind N are left as they are."""
     N = z.shape[0]
     H = w.shape[0]
-    # whole sectors: the contraction of the pair-weighted averaging reads the planes and values of their row length (760 tokens
-    # x 1024 sequences 845 -> 701 us, 405 x 500 221 -> 204; the attention's bias tiles alone gain nothing, 602 us both ways)
-    Np = (N + 15) // 16 * 16 if out is None else (N + 7) // 8 * 8
+    # Whole 32-byte sectors (16): the contraction of the pair-weighted averaging reads the planes and values of their row length
+    # (760 tokens x 1024 sequences 845 -> 701 us, 405 x 500 221 -> 204).  The attention's bias tiles gain nothing (602 us both ways),
+    # and where only they are padded (136 tokens) the fill costs 1 us of 4.8: it asks for 8.
+    if out is not None:
+        Np = out.stride(1) if out.dim() == 3 else 0
+        if out.dtype != torch.bfloat16 or out.device != z.device or out.dim() != 3 or out.shape[0] < H or out.shape[1] != N or \
+                out.shape[2] < N or out.stride(2) != 1 or Np < N or Np % 8 or out.stride(0) != N * Np:
+            raise ValueError(f"pair_head_bias: planes of {H} heads are bf16 [{H}, {N}, {N} or more], rows of a multiple of 8 elements")
+    else:
+        if row < 8 or row % 8:
+            raise ValueError("pair_head_bias: rows of a multiple of 8 elements")
+        Np = (N + row - 1) // row * row
+        make = torch.zeros if Np != N else torch.empty       # the kernel writes no padding
+        out = make((H, N, Np), dtype=torch.bfloat16, device=z.device)
     # the cache entry is tied to the live weight tensor object (a freed tensor's address may be reused)
     key = (id(w), w._version, None if ln_w is None else ln_w._version, float(scale), str(z.device))
     entry = _HB_CACHE.get(key)
@@ -102,9 +114,6 @@ def pair_head_bias(z: torch.Tensor, ln_w, ln_b, w, scale: float = 1.0, transpose
             _HB_CACHE.clear()
         _HB_CACHE[key] = (weakref.ref(w), packed)
     wf, colsum, colbias = packed
-    if out is None:
-        out = torch.zeros((H, N, Np), dtype=torch.bfloat16, device=z.device) if Np != N else \
-            torch.empty((H, N, Np), dtype=torch.bfloat16, device=z.device)
     rc = native.lib().ubm_pair_head_bias(native.ptr(z), native.ptr(wf), native.ptr(colsum), native.ptr(colbias),
                                          native.ptr(out), N, Np, H, 1 if transpose else 0,
                                          native.current_stream(z.device))
