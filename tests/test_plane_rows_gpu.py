@@ -114,3 +114,14 @@ def test_head_bias_planes_that_do_not_fit():
                 torch.zeros(4, 24, 28, device="cuda", dtype=torch.bfloat16), torch.zeros(4, 25, 24, device="cuda", dtype=torch.bfloat16)):
         with pytest.raises(ValueError):
             rows.pair_head_bias(z, None, None, w, out=out)
+
+
+@pytest.mark.parametrize("N", [24, 33])
+def test_attention_asks_for_rows_of_eight(N):
+    """Padding to sectors would cost the planes of 24 tokens a fill and gain the attention nothing."""
+    from uplifting_biomolecular_modeling_b200.models import pairformer
+    with torch.device("cuda"):
+        m = pairformer.AttentionPairBias().bfloat16().eval().requires_grad_(False)
+    pairformer.set_impl(m, "fused")
+    planes = m.pair_bias(torch.zeros(1, N, N, 128, device="cuda", dtype=torch.bfloat16))
+    assert planes.ld == (N + 7) // 8 * 8

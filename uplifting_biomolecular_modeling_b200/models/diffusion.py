@@ -476,7 +476,7 @@ class DiffusionModule(nn.Module):
             from ..ops import rows
             from .pairformer import BiasPlanes
             zc = z_cond[0].contiguous()
-            tb = [BiasPlanes(rows.pair_head_bias(zc, m[0].weight, m[0].bias, m[1].weight, scale=BiasPlanes.LOG2E))
+            tb = [BiasPlanes(rows.pair_head_bias(zc, m[0].weight, m[0].bias, m[1].weight, scale=BiasPlanes.LOG2E, row=8))
                   for m in self.token_pair_bias]
         else:
             tb = [m(z_cond).permute(0, 3, 1, 2) for m in self.token_pair_bias]

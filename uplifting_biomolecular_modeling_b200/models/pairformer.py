@@ -356,7 +356,7 @@ class AttentionPairBias(_Switchable):
         if self._fusable(z) and z.shape[0] == 1:
             from ..ops import rows
             return BiasPlanes(rows.pair_head_bias(z[0].contiguous(), self.proj_z[0].weight, self.proj_z[0].bias,
-                                                  self.proj_z[1].weight, scale=BiasPlanes.LOG2E))
+                                                  self.proj_z[1].weight, scale=BiasPlanes.LOG2E, row=8))
         return self.proj_z[1](self.proj_z[0](z)).permute(0, 3, 1, 2)
 
     def _fused_forward(self, s: torch.Tensor, planes: "BiasPlanes", out_gate=None, out_residual=None,
