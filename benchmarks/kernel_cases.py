@@ -98,6 +98,7 @@ def main():
         flops = 4.0 * rows * H * N * N * D
     elif a.case in ("trimul_proj", "trimul_gemm", "trimul_out", "trimul"):
         w = pair.TrimulPacked.pack(ones, zeros, r(256, c), r(256, c), ones, zeros, r(c, c), r(c, c))
+        Np = pair.ceil_to(N, pair.PLANE_ROW)
         planes = torch.empty((2, 128, N, Np), dtype=torch.bfloat16, device=dev)
         x = torch.empty((128, N, Np), dtype=torch.bfloat16, device=dev)
         out = torch.empty_like(z)

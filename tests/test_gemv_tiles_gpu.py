@@ -30,7 +30,7 @@ def _want(x, w, w2, gamma, b, res):
 
 @pytest.mark.parametrize("M", range(1, 9))
 @pytest.mark.parametrize("N,K", [(1, 64), (15, 128), (17, 576), (4752, 1024)])
-@pytest.mark.parametrize("dual,gamma", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("dual,gamma", [(False, False), (False, True), (True, False), (True, True)])
 def test_gemv_tiles(M, N, K, dual, gamma):
     from uplifting_biomolecular_modeling_b200.ops import seq
     x, w, w2, gm, b, res = _inputs(M, N, K, dual, gamma, M + N + K)

@@ -1,6 +1,6 @@
 // Fused LayerNorm -> 512-wide projection of pair rows, with the op-specific epilogue.
 //
-// Epilogue (MODE_TRIATT): q | k | v | sigmoid(g) rows (bf16, [row][128]) plus the per-head pair bias
+// Epilogue: q | k | v | sigmoid(g) rows (bf16, [row][128]) plus the per-head pair bias
 // planes bias[h][j][k]; optionally at the transposed pair index (ending node).  Reference: the
 // triangle-attention prologue (common/opt_core/opt_core/attn/pair_fused.py:1136, N15
 // triatt_procuda_sm90.cu).  (The triangle-multiplication projection, whose planes want the transposed
@@ -31,8 +31,6 @@ constexpr int kPPStages = 2;   // row-tile ring
 constexpr int kPPXBytes = kPPRows * kPPC * 2;        // 32 KB, two k-blocks of [128][64]
 constexpr int kPPWBytes = 512 * kPPC * 2;            // 128 KB, two k-blocks of [512][64]
 constexpr int kPPMaxHeads = 8;
-
-enum { MODE_TRIMUL = 0, MODE_TRIATT = 1 };
 
 struct PairProjParams {
   long long R;       // number of pair rows (rows * N)
@@ -75,7 +73,6 @@ constexpr int kPPBoxRows = 16;
 constexpr int kPPOutWarpBytes = kPPBoxRows * 64;
 constexpr int kPPOutBytes = kPPEpiWarps * kPPOutWarpBytes;
 
-template <int MODE>
 __global__ void __launch_bounds__(kPPThreads, 1)
 pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                  const __grid_constant__ PeerSrcMaps peers, const __grid_constant__ PairOutMaps outs,
@@ -222,7 +219,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         float r0 = 0.f, r1 = 0.f;
-        if (MODE == MODE_TRIATT && fg < p.H) {
+        if (fg < p.H) {
           const float* src = p.wb + fg * 128 + ks * 16 + e * 8 + ft * 2;
           r0 = src[0];
           r1 = src[1];
@@ -255,17 +252,15 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         }
       }
       float hb[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};     // [16 rows]
-      if (MODE == MODE_TRIATT) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
+      for (int ks = 0; ks < 8; ++ks) {
 #pragma unroll
-          for (int m16 = 0; m16 < 2; ++m16) {
-            uint32_t a0, a1, a2, a3;
-            ldmatrix_x4(xs + (ks >> 2) * 16384 + swz128_offset(sw * 32 + m16 * 16 + (lane & 15), (ks & 3) * 2 + (lane >> 4)), a0,
-                        a1, a2, a3);
+        for (int m16 = 0; m16 < 2; ++m16) {
+          uint32_t a0, a1, a2, a3;
+          ldmatrix_x4(xs + (ks >> 2) * 16384 + swz128_offset(sw * 32 + m16 * 16 + (lane & 15), (ks & 3) * 2 + (lane >> 4)), a0,
+                      a1, a2, a3);
 #pragma unroll
-            for (int part = 0; part < 3; ++part) mma_bf16_16816(hb[m16], a0, a1, a2, a3, wb[ks][part][0], wb[ks][part][1]);
-          }
+          for (int part = 0; part < 3; ++part) mma_bf16_16816(hb[m16], a0, a1, a2, a3, wb[ks][part][0], wb[ks][part][1]);
         }
       }
       __syncwarp();
@@ -283,24 +278,22 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         p.stats_out[2 * r] = mu;
         p.stats_out[2 * r + 1] = rstd;
       }
-      if (MODE == MODE_TRIATT) {
-        const int pi = static_cast<int>(r / p.N), pk = static_cast<int>(r - static_cast<long long>(pi) * p.N);
-        // this lane holds heads 2 ft, + 1 of rows fg, + 8, + 16, + 24
+      const int pi = static_cast<int>(r / p.N), pk = static_cast<int>(r - static_cast<long long>(pi) * p.N);
+      // this lane holds heads 2 ft, + 1 of rows fg, + 8, + 16, + 24
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int src = e * 8 + fg;
-          const float rs = __shfl_sync(0xffffffffu, rstd, src), m = __shfl_sync(0xffffffffu, mu, src);
-          const int ri = __shfl_sync(0xffffffffu, pi, src), rk = __shfl_sync(0xffffffffu, pk, src);
-          if (r0 + src < p.R) {
-            const int oi = p.transpose_out ? rk : ri;
-            const int ok = p.transpose_out ? ri : rk;
+      for (int e = 0; e < 4; ++e) {
+        const int src = e * 8 + fg;
+        const float rs = __shfl_sync(0xffffffffu, rstd, src), m = __shfl_sync(0xffffffffu, mu, src);
+        const int ri = __shfl_sync(0xffffffffu, pi, src), rk = __shfl_sync(0xffffffffu, pk, src);
+        if (r0 + src < p.R) {
+          const int oi = p.transpose_out ? rk : ri;
+          const int ok = p.transpose_out ? ri : rk;
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const int head = 2 * ft + c;
-              if (head < p.H) {
-                const float val = rs * (hb[e >> 1][2 * (e & 1) + c] - m * p.wb_colsum[head]) + p.wb_colbias[head];
-                p.headbias[(static_cast<long long>(head) * p.plane_rows + oi) * p.Np + ok] = __float2bfloat16(val);
-              }
+          for (int c = 0; c < 2; ++c) {
+            const int head = 2 * ft + c;
+            if (head < p.H) {
+              const float val = rs * (hb[e >> 1][2 * (e & 1) + c] - m * p.wb_colsum[head]) + p.wb_colbias[head];
+              p.headbias[(static_cast<long long>(head) * p.plane_rows + oi) * p.Np + ok] = __float2bfloat16(val);
             }
           }
         }
@@ -422,7 +415,6 @@ constexpr int kPPSmemBytes =
     kPPWBytes + kPPStages * kPPXBytes + kPPOutBytes + (512 + 512) * 4 + 2 * 128 * 8 + 256 + 1024;
 static_assert(kPPSmemBytes <= 232448, "shared memory of one CTA");
 
-template <int MODE>
 static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cudaStream_t stream,
                             const void* const* z_ptrs = nullptr, const int* peer_rows = nullptr, int npeers = 0,
                             int me = 0) {
@@ -453,7 +445,7 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
       return e == nullptr || e[0] != '0';
     }();
     void* bufs[4] = {p.q, p.k, p.v, p.g};
-    bool ok = on && MODE == MODE_TRIATT && p.R < (1ll << 31);
+    bool ok = on && p.R < (1ll << 31);
     for (int i = 0; i < 4; ++i) ok = ok && bufs[i] != nullptr && (reinterpret_cast<uintptr_t>(bufs[i]) & 15) == 0;
     if (ok) {
       for (int i = 0; i < 4; ++i) {
@@ -475,7 +467,7 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
       p.out_tma = 1;
     }
   }
-  auto kern = pair_proj_kernel<MODE>;
+  auto kern = pair_proj_kernel;
   rc = set_smem(kern, kPPSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
@@ -518,7 +510,7 @@ static int triatt_proj_impl(const void* z, const void* w, const void* colsum, co
   p.transpose_out = transpose_out;
   p.stats_out = static_cast<float*>(stats_out);
   p.status = static_cast<KernelStatus*>(status);
-  return launch_pair_proj<MODE_TRIATT>(z, w, p, static_cast<cudaStream_t>(stream), z_ptrs, peer_rows, npeers, me);
+  return launch_pair_proj(z, w, p, static_cast<cudaStream_t>(stream), z_ptrs, peer_rows, npeers, me);
 }
 
 extern "C" int ubm_triatt_proj_rows(const void* z, const void* w, const void* colsum, const void* colbias,

@@ -1482,9 +1482,11 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_rows_kernel(
 // instructions four at a time.  The blocks of a tile are dealt to the CTA's warps, which add their sums up in shared memory.
 // STAGED: x^ is normalised into shared memory once per CTA; otherwise decode rows come straight from L1 (staging all of
 // x cost every SM up to 176 KB of L2 reads in front of its weights).  Needs K % 64 == 0 and weights on 32 bytes.
-// us of the FMA form / of this one, 12288 x 4096 behind a norm, 2 x 11008 x 4096 behind a norm, 4096 x 11008, 4096 x 4096: one
-// decode row 18.2 / 21.3, 33.2 / 36.0, 18.7 / 17.0, 6.1 / 7.3; two 21.1 / 20.6, 36.5 / 34.9, 20.4 / 17.1, 7.9 / 7.3; four 32.5 /
-// 22.4, 47.4 / 36.7, 29.3 / 17.2, 11.5 / 7.5; eight 56.7 / 25.1, 99.9 / 39.3, 59.2 / 17.5, 20.1 / 7.3.  One row stays with the FMAs.
+// us of the FMA form / of this one for 12288 x 4096 behind a norm, 2 x 11008 x 4096 behind a norm, 4096 x 11008 and 4096 x 4096, launch
+// behind launch with weights from memory (600 MB of them in rotation; each launch's prefetch runs under the one before): one decode
+// row 18.6 / 21.4, 33.4 / 35.5, 17.2 / 17.3, 7.1 / 7.3; two 21.4 / 21.0, 36.4 / 35.1, 20.8 / 17.3, 8.0 / 7.4; four 32.7 / 22.7, 48.0 /
+// 36.9, 29.5 / 17.4, 11.5 / 7.4; eight 57.2 / 25.4, 100 / 40.0, 60.3 / 17.7, 20.2 / 7.2.  One row stays with the FMAs, which lose
+// nowhere.  (A launch by itself with a cold L2, start and end included, takes 8 us more: 26.7 for the first shape.)
 constexpr int kGemvMmaMinRows = 2;
 constexpr int kGemvMmaThreads = 256;
 constexpr int kGemvMmaWarps = kGemvMmaThreads / 32;
@@ -1529,8 +1531,7 @@ __global__ void __launch_bounds__(kGemvMmaThreads, 2) gemv_mma_kernel(
   asm volatile("griddepcontrol.wait;" ::: "memory");      // see the kernel above
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (STAGED) {
-    // warps per decode row: all eight for one row, one for five rows and more
-    const int wpr = M == 1 ? 8 : M == 2 ? 4 : M <= 4 ? 2 : 1;
+    const int wpr = M == 2 ? 4 : M <= 4 ? 2 : 1;           // warps per decode row
     const int b = warp / wpr, in_row = (warp - b * wpr) * 32 + lane, step = wpr * 32, nv = K >> 3;
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(b) * K);
     float ss = 0.f;
