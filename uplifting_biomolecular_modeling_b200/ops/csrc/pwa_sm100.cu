@@ -9,9 +9,9 @@
 //   pwa_out_kernel       gate projection, gating and output projection of 128 tokens of one sequence
 // Between them the [S N, 256] intermediates cross memory once as v and once as o; as tensor statements around the same
 // GEMM they crossed it eleven times (projections, the transpose into planes, gate, product, transpose back).
-// 1024 sequences x 768 tokens: 0.68 ms (weights 3, softmax 15, values 92, GEMM 282, output stage 165 us, bias planes 44)
+// 1024 sequences x 768 tokens: 0.67 ms (weights 3, softmax 15, values 94, GEMM 276, output stage 166 us, bias planes 45)
 // against 2.54 ms.  Values and output stage move the 0.4 GB of v and o (60 us each at copy bandwidth); neither fills a unit
-// (512 x 512: DRAM 39 and 36 %, issue slots 35 and 45 %, special-function unit 2 and 30 % busy), their warps wait for
+// (512 x 512: DRAM 43 and 35 %, issue slots 51 and 45 %, special-function unit 2 and 30 % busy), their warps wait for
 // tensor and shared memory.
 #include "host_util.h"
 #include "sm100.cuh"

@@ -24,7 +24,7 @@
 // take alternate hidden chunks (in a group two warps share each lane quadrant, 32 of the chunk's 64 columns each),
 // 20-23 = row warps: statistics of the next tile, output of the present one.
 //
-// 1021 x 1021 rows, hidden 512: 647 us with one issuer for both GEMMs, column factors from shared memory, and the
+// 1021 x 1021 rows, hidden 512 (single launches): 647 us with one issuer for both GEMMs, column factors from shared memory, and the
 // statistics and the output in the SwiGLU warps; 557 with the issuers apart and the row tiles requested where nothing waits
 // behind them (5200 of a tile's 23700 clocks went by in front of weights that stood behind the next row tile); 413 as it
 // is.  A third weight stage (411) and the row tile as an operand in tensor memory (410) change nothing; without any weight
