@@ -63,3 +63,28 @@ def test_operands_that_start_between_16_bytes(what):
     got = m(x, mask)
     native.raise_on_status("cuda", "outer product")
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("S,N", [(3, 9), (17, 64), (40, 131)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_one_row_of_the_mask_for_all_sequences(S, N, dtype):
+    """The plain statements count such a row once; so does the kernel path."""
+    from uplifting_biomolecular_modeling_b200.models import msa, pairformer
+    from uplifting_biomolecular_modeling_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(S + N)
+    with torch.device("cuda"):
+        m = msa.OuterProductMean()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(torch.randn(p.shape, device="cuda", generator=g) / max(1, p.shape[-1]) ** 0.5)
+    m = m.bfloat16().eval().requires_grad_(False)
+    pairformer.set_impl(m, "fused")
+    x = torch.randn(1, S, N, 64, device="cuda", generator=g).bfloat16()
+    mask = (torch.rand(1, 1, N, device="cuda", generator=g) < 0.6).to(dtype)
+    got = m(x, mask)
+    native.raise_on_status("cuda", "outer product")
+    d = lambda t: t.double()  # noqa: E731
+    want = R.outer_product_mean(d(x), d(mask), d(m.norm.weight), d(m.norm.bias), d(m.proj_a.weight), d(m.proj_b.weight),
+                                d(m.proj_o.weight), d(m.proj_o.bias))
+    # as above
+    assert (d(got) - want).norm() <= 6 * 2.0 ** -9 * (want.norm() + d(m.proj_o.bias).norm() * N)

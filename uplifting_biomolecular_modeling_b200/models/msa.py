@@ -67,7 +67,7 @@ class OuterProductMean(_Switchable):
         # channels instead of c*c.
         count = None
         if not self.full_mask:
-            mk = mask[0].expand(S, N)
+            mk = mask[0].expand(-1, N)      # a mask with one row for all sequences counts once, as in the plain statements
             if mk.dtype == torch.bfloat16 and N % 8 == 0:       # bf16 values: exact products, fp32 sums
                 mk = mk.contiguous()
                 if mk.data_ptr() % 16:                          # the GEMM's tensor maps start on 16 bytes
