@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
 causal_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, CausalParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + smem_pad1024(smem_raw);
   uint8_t* sQ = smem;                      // 2 x Q tile
   uint8_t* sSt = sQ + 2 * kCQBytes;        // stages of {K, V}
   float* sX = reinterpret_cast<float*>(sSt + kCStages * kCStageBytes);

@@ -78,7 +78,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                  const __grid_constant__ PeerSrcMaps peers, const __grid_constant__ PairOutMaps outs,
                  PairProjParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + smem_pad1024(smem_raw);
   uint8_t* sW = smem;                               // 128 KB
   uint8_t* sX = smem + kPPWBytes;                   // stages * 32 KB
   uint8_t* sOut = sX + kPPStages * kPPXBytes;       // 16 warps x 1 KB of output staging

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(320, 2)
 pwa_value_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmW,
                  const __grid_constant__ CUtensorMap tmV, PwaValueParams p) {
   extern __shared__ uint8_t smem_raw[];
+  // rounded as an integer (generic accesses): by smem_pad1024 the pass of 1024 x 768 takes 677 us, this way 672
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sW = smem;
   uint8_t* sX = sW + kPvWBytes;

@@ -42,6 +42,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Bytes to the next multiple of 1024 (swizzled tiles) in dynamic shared memory.  The aligned pointer is formed by adding them, not
+// by rounding the address: a pointer that went through an integer no longer belongs to shared memory for the compiler, and
+// every access by it becomes a generic one.
+__device__ __forceinline__ uint32_t smem_pad1024(const void* p) {
+  return (0u - static_cast<uint32_t>(__cvta_generic_to_shared(p))) & 1023u;
+}
+
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -101,7 +101,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                   const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmOut,
                   TransitionParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + smem_pad1024(smem_raw);
   uint8_t* sX = smem;                                   // 2 x 32 KB
   uint8_t* sW = sX + 2 * kTRXBytes;                     // first-GEMM weights
   uint8_t* sWo = sW + kTRWStages * kTRWabBytes;         // 2 x 16 KB

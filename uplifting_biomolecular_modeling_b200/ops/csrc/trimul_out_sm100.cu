@@ -47,7 +47,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                   const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmWg,
                   const __grid_constant__ CUtensorMap tmO, TrimulOutParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + smem_pad1024(smem_raw);
   uint8_t* sWo = smem;                    // 32 KB: two k-blocks [128][64]
   uint8_t* sWg = smem + kTOTileBytes;     // 32 KB
   uint8_t* sSt = smem + 2 * kTOTileBytes; // stages: {x tile 32 KB, z tile 32 KB}

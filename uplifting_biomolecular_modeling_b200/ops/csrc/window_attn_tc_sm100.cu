@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(128, 2)
 window_attention_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                            const __grid_constant__ CUtensorMap tmV, WindowTcParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw + smem_pad1024(smem_raw);
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + kWTQBytes;
   uint8_t* sV = sK + kWTKBytes;
