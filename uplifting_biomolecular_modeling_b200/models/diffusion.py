@@ -126,24 +126,22 @@ class DiffusionTransformerLayer(_Switchable):
         GEMM) -> attention with the hoisted pair-bias planes shared by all samples -> output projection whose
         epilogue applies the conditioning gate and the residual; then the conditioned SwiGLU transition the same
         way (one GEMM for swish_gated and a_to_b, a three-way row kernel, an output GEMM with gate and residual)."""
-        from ..ops import gemm, pair, rows
+        from ..ops import atom, gemm, pair, rows
         B, N, C = a.shape
         attn = self.pair_bias_attn
         a = a.contiguous()
-        a2 = a.view(B * N, C)
         gate, t_gate = h["gate_sig"], h["t_gate_sig"]
         gate = gate.reshape(-1, C) if gate.dim() == 3 else gate
         t_gate = t_gate.reshape(-1, C) if t_gate.dim() == 3 else t_gate
-        b = rows.adaln_rows(a, h["adaln"][0], h["adaln"][1])
         if isinstance(bias, WindowBias):
             if attn._packed is None:
                 attn._packed = pair.ApbPacked.pack(attn.proj_q.weight, attn.proj_q.bias, attn.proj_k.weight,
                                                    attn.proj_v.weight, attn.proj_g.weight, attn.proj_o.weight,
                                                    attn.heads)
-            a = pair.window_attention_fused(b, attn._packed, bias.data, out_gate=gate, out_residual=a2)
+            a = atom.attention(a, h["adaln"][0], h["adaln"][1], attn._packed, bias.data, gate)
         else:
-            a = attn._fused_forward(b, bias, out_gate=gate, out_residual=a2, mask=mask)
-        a2 = a.view(B * N, C)
+            b = rows.adaln_rows(a, h["adaln"][0], h["adaln"][1])
+            a = attn._fused_forward(b, bias, out_gate=gate, out_residual=a.view(B * N, C), mask=mask)
         tr = self.transition
         if self._packed is None:
             # silu(gates half) * values half * a_to_b: upstream's swish_gate stores the values first
@@ -156,9 +154,7 @@ class DiffusionTransformerLayer(_Switchable):
                 w_in = torch.cat([wsg[hid:], wsg[:hid], tr.a_to_b.weight.detach()], 0).to(torch.bfloat16).contiguous()
             self._packed = (w_in, tr.b_to_a.weight.detach().to(torch.bfloat16).contiguous(), hid % 32 == 0)
         w_in, w_ba, in_epilogue = self._packed
-        x = rows.adaln_rows(a, h["t_adaln"][0], h["t_adaln"][1]).view(B * N, C)
-        u = gemm.gemm(x, w_in, act="swiglu3") if in_epilogue else rows.swiglu3_rows(gemm.gemm(x, w_in))
-        return gemm.gemm(u, w_ba, gate=t_gate, residual=a2).view(B, N, C)
+        return atom.transition(a.view(B, N, C), h["t_adaln"][0], h["t_adaln"][1], t_gate, w_in, w_ba, in_epilogue)
 
     def forward(self, a, s, bias, mask=None, multiplicity: int = 1, hoisted: Optional[dict] = None,
                 window: Optional[tuple] = None):

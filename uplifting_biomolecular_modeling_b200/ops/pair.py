@@ -540,7 +540,7 @@ def pair_weighted_averaging_fused(m: torch.Tensor, b: torch.Tensor, mask: Option
 native.declare("ubm_window_attention", [c_void_p] * 6 + [c_int, c_int, c_int, c_ll, c_int, c_void_p])
 native.declare("ubm_window_attention_tc", [c_void_p] * 6 + [c_int, c_int, c_int, c_ll, c_int, c_void_p, c_void_p])
 
-WINDOW_KERNEL = "tc"     # "tc": tcgen05 kernel (four windows per CTA); "simt": CUDA-core kernel (one window per CTA)
+WINDOW_KERNEL = "tc"     # "tc": matrix instructions (4 heads at 128 channels: ops.atom; else the tcgen05 kernel); "simt": CUDA cores
 
 
 def window_attention_fused(x: torch.Tensor, w: ApbPacked, bias: Optional[torch.Tensor],
@@ -553,6 +553,11 @@ def window_attention_fused(x: torch.Tensor, w: ApbPacked, bias: Optional[torch.T
         raise ValueError("window attention supports head dimension 32")
     HD = w.H * 32
     x2 = x.reshape(B * A, c)
+    from . import atom
+    if atom._window_serves(w, bias, B, A, c) and (out_gate is None or atom._gate_of(out_gate, B * A) is not None) and \
+            (out_residual is None or (atom._plain(out_residual) and out_residual.numel() == B * A * c)):
+        qkvg = _gemm.gemm(x2, w.wqkvg, bias=w.bqkvg, act="sigmoid", act_from=3 * HD)
+        return atom.window_layer(qkvg, w, bias, out_gate, out_residual, B, A)
     qkv = _gemm.gemm(x2, w.wqkv, bias=w.bqkv)
     g = _gemm.gemm(x2, w.wg, act="sigmoid")
     o = torch.empty((B * A, HD), dtype=torch.bfloat16, device=x.device)

@@ -9,7 +9,7 @@ statements under a kernel mode's label.
 | family | tuned | safe |
 |---|---|---|
 | triattn | four rows per CTA, one exponential in four on the FMA pipe | every exponential on the special-function unit |
-| window (atom attention) | tcgen05 kernel, four windows per CTA | CUDA-core kernel, one window per CTA |
+| window (atom attention) | two windows per CTA with their output projection (other head counts: tcgen05 kernel) | CUDA-core kernel, one window per CTA |
 
 Reference: common/opt_core/opt_core/kernels/safe_settings.py (one-stage launch cells when a tuned Triton cell fails
 to build).
