@@ -17,7 +17,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.nn.modules.module import _has_any_global_hook as _any_global_hook
 
-from ..ops import reference as R
+from ..ops import dispatch, gemm, pair, reference as R, rows
 
 IMPLS = ("reference", "fused")
 
@@ -41,7 +41,6 @@ class _Switchable(nn.Module):
         undeclared reason ends the run PARTIAL).  With the plain implementation there is nothing to count."""
         if self.impl != "fused":
             return False
-        from ..ops import dispatch
         return dispatch.decide(self.lever, reason, klass, tokens, call, row)
 
     @staticmethod
@@ -106,7 +105,6 @@ class Transition(_Switchable):
                               {"c": self.dim, "expansion": self.hidden // max(1, self.dim), "dtype": "bf16"},
                               "tcgen05_fused" if one_kernel else "rows_gemm")
         if served and one_kernel:
-            from ..ops import pair
             if self._packed is None:
                 self._packed = pair.TransitionPacked.pack(self.norm.weight, self.norm.bias, self.fc1.weight,
                                                           self.fc2.weight, self.fc3.weight)
@@ -114,7 +112,6 @@ class Transition(_Switchable):
         if served:
             # other widths (the MSA track at 64, the template stack): LayerNorm rows -> one GEMM for both hidden
             # projections -> SwiGLU rows -> output GEMM with the residual in its epilogue
-            from ..ops import gemm, rows
             in_epilogue = self.hidden % 32 == 0     # silu(fc1) * fc2 formed on the accumulator of one product
             if self._packed is None:
                 w12 = gemm.pack_swiglu(self.fc1.weight.detach(), self.fc2.weight.detach()) if in_epilogue else \
@@ -122,8 +119,12 @@ class Transition(_Switchable):
                 self._packed = (w12, self.fc3.weight.detach().to(torch.bfloat16).contiguous())
             w12, w3 = self._packed
             x2 = x.reshape(-1, self.dim).contiguous()
+            if in_epilogue:
+                y = pair.transition_rows(x2, self.norm.weight, self.norm.bias, self.norm.eps, w12, w3,
+                                         residual and self.out_dim == self.dim)
+                return y.view(*x.shape[:-1], self.out_dim)
             n = rows.layernorm_rows(x2, self.norm.weight, self.norm.bias, self.norm.eps)
-            h = gemm.gemm(n, w12, act="swiglu") if in_epilogue else rows.swiglu_rows(gemm.gemm(n, w12))
+            h = rows.swiglu_rows(gemm.gemm(n, w12))
             y = gemm.gemm(h, w3, residual=x2 if residual and self.out_dim == self.dim else None)
             return y.view(*x.shape[:-1], self.out_dim)
         return R.transition(x, self.norm.weight, self.norm.bias, self.fc1.weight, self.fc2.weight, self.fc3.weight,
@@ -149,7 +150,6 @@ class TriangleMultiplication(_Switchable):
         the batched contraction GEMM (K-major for outgoing, MN-major for incoming) -> LayerNorm rows -> output GEMM
         whose epilogue applies the output gate and the residual.  Gating products and the two layout changes are
         plain tensor statements."""
-        from ..ops import gemm, rows
         N, c = z.shape[1], z.shape[-1]
         h = self.p_in.weight.shape[0] // 2
         if self._packed is None:
@@ -188,7 +188,6 @@ class TriangleMultiplication(_Switchable):
         if served and not one_kernel_set:
             return self._rows_gemm_forward(z, mask, residual)
         if served:
-            from ..ops import pair
             if self._packed is None:
                 self._packed = pair.TrimulPacked.pack(self.norm_in.weight, self.norm_in.bias, self.p_in.weight,
                                                       self.g_in.weight, self.norm_out.weight, self.norm_out.bias,
@@ -242,7 +241,6 @@ class TriangleAttention(_Switchable):
         q | k | v | gate (heads padded to the kernel's head dimension 32 or 64, sigmoid on the gate columns) -> the
         attention kernel on column slices of that output with the head-bias planes and the key mask -> output GEMM
         with bias and residual.  The ending node runs on the transposed pair tensor (a tensor statement)."""
-        from ..ops import gemm, pair, rows
         m = self.mha
         N, c = z.shape[1], z.shape[-1]
         H, D = self.heads, self.c_hidden
@@ -289,17 +287,14 @@ class TriangleAttention(_Switchable):
         if served and not one_kernel_set:
             return self._rows_gemm_forward(z, mask, residual)
         if served:
-            from ..ops import pair
-            km = None
-            if mask is not None:
-                km = pair.KeyMask.lay_out(mask[0] if self.starting else mask[0].t(), z.shape[1:3], z.device)
+            keep = None if mask is None else mask[0] if self.starting else mask[0].t()
             if self._packed is None:
                 self._packed = pair.TriattPacked.pack(self.layer_norm.weight, self.layer_norm.bias,
                                                       self.linear.weight, m.linear_q.weight, m.linear_k.weight,
                                                       m.linear_v.weight, m.linear_g.weight, m.linear_g.bias,
                                                       m.linear_o.weight, m.linear_o.bias, self.heads)
             out = pair.triangle_attention_fused(z[0].contiguous(), self._packed, self.starting, residual=residual,
-                                                workspace=self._workspace, mask=km)
+                                                workspace=self._workspace, keep=keep)
             return out.unsqueeze(0)
         outs = [R.triangle_attention(z[b], None if mask is None else mask[b], self.layer_norm.weight,
                                      self.layer_norm.bias, self.linear.weight, m.linear_q.weight, m.linear_k.weight,
@@ -354,25 +349,20 @@ class AttentionPairBias(_Switchable):
     def pair_bias(self, z: torch.Tensor):
         """[B, H, N, N] bias from the pair tensor (a :class:`BiasPlanes` on the fused path)."""
         if self._fusable(z) and z.shape[0] == 1:
-            from ..ops import rows
             return BiasPlanes(rows.pair_head_bias(z[0].contiguous(), self.proj_z[0].weight, self.proj_z[0].bias,
                                                   self.proj_z[1].weight, scale=BiasPlanes.LOG2E, row=8))
         return self.proj_z[1](self.proj_z[0](z)).permute(0, 3, 1, 2)
 
     def _fused_forward(self, s: torch.Tensor, planes: "BiasPlanes", out_gate=None, out_residual=None,
                        mask: Optional[torch.Tensor] = None) -> torch.Tensor:
-        from ..ops import pair
-        km = None
-        if mask is not None:
-            km = pair.KeyMask.lay_out(mask if mask.shape[0] == s.shape[0] else
-                                      mask.expand(s.shape[0], -1) if mask.shape[0] == 1 else
-                                      mask.repeat_interleave(s.shape[0] // mask.shape[0], 0), s.shape[:2], s.device)
+        if mask is not None and mask.shape[0] != s.shape[0]:
+            mask = mask.expand(s.shape[0], -1) if mask.shape[0] == 1 else mask.repeat_interleave(s.shape[0] // mask.shape[0], 0)
         if self._packed is None:
             self._packed = pair.ApbPacked.pack(self.proj_q.weight, self.proj_q.bias, self.proj_k.weight,
                                                self.proj_v.weight, self.proj_g.weight, self.proj_o.weight,
                                                self.heads)
         return pair.apb_fused(s.to(torch.bfloat16).contiguous(), self._packed, planes.view, planes.ld,
-                              out_gate=out_gate, out_residual=out_residual, mask=km)
+                              out_gate=out_gate, out_residual=out_residual, keep=mask)
 
     def forward(self, s: torch.Tensor, z: Optional[torch.Tensor], mask: Optional[torch.Tensor],
                 bias: Optional[torch.Tensor] = None, k_in: Optional[torch.Tensor] = None,
@@ -407,6 +397,14 @@ class AttentionPairBias(_Switchable):
         return self.proj_o(g * o)
 
 
+# what :meth:`PairformerLayer._pair_track` stands for: the forward and the packed weights of each operator
+_PAIR_TRACK = {"tri_mul_out": (TriangleMultiplication.forward, pair.TrimulPacked),
+               "tri_mul_in": (TriangleMultiplication.forward, pair.TrimulPacked),
+               "tri_att_start": (TriangleAttention.forward, pair.TriattPacked),
+               "tri_att_end": (TriangleAttention.forward, pair.TriattPacked),
+               "transition_z": (Transition.forward, pair.TransitionPacked)}
+
+
 class PairformerLayer(nn.Module):
     def __init__(self, c_s: int = 384, c_z: int = 128, heads: int = 16, pair_heads: int = 4, no_seq: bool = False,
                  transition_n: int = 4):
@@ -422,7 +420,45 @@ class PairformerLayer(nn.Module):
         self.tri_att_end = TriangleAttentionEndingNode(c_z, c_z // pair_heads, pair_heads)
         self.transition_z = Transition(c_z, c_z * transition_n)
 
+    def _pair_track(self, z: torch.Tensor, mask: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+        """The five operators below from one call of the library (it spends 70 us on what takes them 175 one by one), or None where
+        a call of any of them would do anything else: another implementation, a hook, a replaced forward, weights that are not
+        packed yet, row blocks, a size window, an input or mask that has to be converted."""
+        N = z.shape[1] if z.dim() == 4 else 0
+        if N == 0 or z.shape != (1, N, N, 128) or not z.is_cuda or z.dtype != torch.bfloat16 or not z.is_contiguous() or \
+                (mask is not None and (mask.shape != (1, N, N) or mask.dtype != torch.bfloat16 or mask.device != z.device or
+                                       not mask.is_contiguous())) or _any_global_hook():
+            return None
+        at = self._modules
+        mods = tuple(at.get(name) for name in _PAIR_TRACK)
+        ws = getattr(mods[0], "_workspace", None)
+        if ws is None or ws.get("row_block"):
+            return None
+        for m, (forward, packed) in zip(mods, _PAIR_TRACK.values()):
+            if getattr(type(m), "forward", None) is not forward:
+                return None
+            d, gate = m.__dict__, dispatch.size_gate(m.lever)
+            if type(d["_packed"]) is not packed or d["impl"] != "fused" or d["_workspace"] is not ws or "forward" in d or \
+                    d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or \
+                    N < gate.min_tokens or (gate.max_tokens is not None and N > gate.max_tokens):
+                return None
+        if not mods[0].outgoing or mods[1].outgoing or not mods[2].starting or mods[3].starting:
+            return None
+        for m, (klass, call, row) in zip(mods, self._pair_calls()):
+            m._decide(None, klass, N, call, row)
+        return pair.pair_track(z, mask, *(m._packed for m in mods), ws)
+
+    def _pair_calls(self) -> tuple:
+        """What the five operators record of a call (:meth:`_Switchable._decide`)."""
+        tm = ("C128H128", {"c_z": 128, "c_hidden": 128, "dtype": "bf16"}, "tcgen05_3stage")
+        ta = ("D32H4", {"head_dim": 32, "dtype": "bf16"}, "tcgen05_4row")
+        x = max(1, self.transition_z.hidden // 128)
+        return tm, tm, ta, ta, (f"C128X{x}", {"c": 128, "expansion": self.transition_z.hidden // 128, "dtype": "bf16"}, "tcgen05_fused")
+
     def pair_update(self, z: torch.Tensor, pair_mask: Optional[torch.Tensor]) -> torch.Tensor:
+        out = self._pair_track(z, pair_mask)
+        if out is not None:
+            return out
         z = self.tri_mul_out(z, pair_mask, residual=True)
         z = self.tri_mul_in(z, pair_mask, residual=True)
         z = self.tri_att_start(z, pair_mask, residual=True)
@@ -442,24 +478,22 @@ class PairformerLayer(nn.Module):
                 and s.shape[-1] % 8 == 0 and s.shape[-1] <= 1024 and not torch.is_autocast_enabled("cuda") \
                 and not (torch.is_grad_enabled() and (s.requires_grad or norm.weight.requires_grad)):
             # normalised in fp32 and rounded once to the projection's type, in one launch
-            from ..ops import rows
-            upd = self.attention(rows.layernorm_rows(s32.contiguous(), norm.weight, norm.bias, 1e-5, torch.bfloat16), z,
-                                 mask).float()
+            upd = self.attention(rows.layernorm_rows(s32.contiguous(), norm.weight, norm.bias, 1e-5, torch.bfloat16), z, mask)
         else:
             sn = F.layer_norm(s32, (s32.shape[-1],), norm.weight.float(), norm.bias.float())
             with torch.autocast(device_type=s.device.type, enabled=False):
-                upd = _run_fp32(self.attention, sn, z, mask)
-        s32 = s32 + upd
-        s32 = s32 + _run_fp32(self.transition_s, s32)
+                upd = _run_own_type(self.attention, sn, z, mask)
+        s32 = s32 + upd                                  # sums in fp32, whatever the update's type
+        s32 = s32 + _run_own_type(self.transition_s, s32)
         return s32.to(s.dtype), z
 
 
-def _run_fp32(module: nn.Module, x: torch.Tensor, *args):
-    """Run a module whose parameters may be bf16 on an fp32 activation (weights up-cast on the fly)."""
-    p = next(module.parameters())
-    if p.dtype == torch.float32:
-        return module(x, *args)
-    return module(x.to(p.dtype), *args).float()
+def _run_own_type(module: nn.Module, x: torch.Tensor, *args):
+    """Run a module on an fp32 activation in the type of its parameters.  A 16-bit result is left as it is: an fp32 sum takes it
+    in exactly, without a conversion of its own."""
+    p = module.norm.weight if type(module) is Transition else next(module.parameters())    # its first; the search costs 8 us
+    y = module(x if p.dtype == torch.float32 else x.to(p.dtype), *args)
+    return y if y.dtype in (torch.bfloat16, torch.float16) else y.float()
 
 
 class PairformerModule(nn.Module):

@@ -44,7 +44,8 @@ struct TrimulProjParams {
   int num_tiles;        // rows * tiles_per_row
   const float* colsum;  // [512] rowsum(W') per output channel
   const float* colbias; // [512]
-  const float* mask;    // [R] or null
+  const void* mask;     // [R] fp32, or bf16 (mask_bf16), or null
+  int mask_bf16;
   float* stats_out;       // optional [R][2]
   KernelStatus* status;
   PeerSrc src;            // src.n > 0: the input rows are columns of z fetched from their owners (see host_util.h)
@@ -242,17 +243,27 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       const int b = n & 1;
       // mask of this warp's 64 columns, two per lane; entries past N are written as zeros (K padding of the contraction)
       const int left = p.N - s0 - half * 64;
-      float mk0 = lane < left ? 1.0f : 0.0f, mk1 = lane + 32 < left ? 1.0f : 0.0f;
+      // (as bits: converted behind the waits, so that nothing stands in front of them for the loads)
+      uint32_t mb0 = lane < left ? 0x3F80u : 0u, mb1 = lane + 32 < left ? 0x3F80u : 0u, shift = 16u;
       if (p.mask != nullptr) {
-        const float* mrow = p.mask + static_cast<long long>(i) * p.N + s0 + half * 64;
-        if (lane < left) mk0 = __ldg(mrow + lane);
-        if (lane + 32 < left) mk1 = __ldg(mrow + lane + 32);
+        const long long m0 = static_cast<long long>(i) * p.N + s0 + half * 64 + lane;
+        if (p.mask_bf16) {
+          const uint16_t* mrow = static_cast<const uint16_t*>(p.mask) + m0;
+          if (lane < left) mb0 = __ldg(mrow);
+          if (lane + 32 < left) mb1 = __ldg(mrow + 32);
+        } else {
+          const uint32_t* mrow = static_cast<const uint32_t*>(p.mask) + m0;
+          if (lane < left) mb0 = __ldg(mrow);
+          if (lane + 32 < left) mb1 = __ldg(mrow + 32);
+          shift = 0u;
+        }
       }
       mbar_wait(&r_full[b], (n >> 1) & 1u, ws, 18, b);
 
       // ---- accumulators of this operand: value block at +0, gate block at +128
       mbar_wait(&acc_full[op], acc_phase, ws, 16, op);
       tc_fence_after_sync();
+      const float mk0 = __uint_as_float(mb0 << shift), mk1 = __uint_as_float(mb1 << shift);
       const uint32_t tbase = tmem_addr(tmem_base, q, op * 256 + half * 64);
 #pragma unroll 1
       for (int c16 = 0; c16 < 4; ++c16) {
@@ -330,7 +341,7 @@ static_assert(kTPSmemBytes <= 232448, "shared memory of one CTA");
 static int trimul_proj_impl(const void* z, const void* w, const void* colsum, const void* colbias,
                                     const void* mask, void* planes, void* stats_out, int rows, int plane_rows, int N,
                                     int Np, void* status, void* stream, const void* const* z_ptrs,
-                                    const int* peer_rows, int npeers, int me) {
+                                    const int* peer_rows, int npeers, int me, int mask_bf16 = 0) {
   using namespace ubm;
   if (N <= 0 || rows <= 0 || plane_rows < rows || Np < N || (Np & 7)) return UBM_ERR_ARGUMENT;
   TrimulProjParams p = {};
@@ -344,7 +355,8 @@ static int trimul_proj_impl(const void* z, const void* w, const void* colsum, co
   p.num_tiles = rows * p.tiles_per_row;
   p.colsum = static_cast<const float*>(colsum);
   p.colbias = static_cast<const float*>(colbias);
-  p.mask = static_cast<const float*>(mask);
+  p.mask = mask;
+  p.mask_bf16 = mask_bf16;
   p.stats_out = static_cast<float*>(stats_out);
   p.status = static_cast<KernelStatus*>(status);
   CUtensorMap tmX, tmW;
@@ -403,4 +415,11 @@ extern "C" int ubm_trimul_proj_rows_peer(const void* const* z_ptrs, const int* p
 extern "C" int ubm_trimul_proj(const void* z, const void* w, const void* colsum, const void* colbias, const void* mask,
                                void* planes, void* stats_out, int N, int Np, void* status, void* stream) {
   return ubm_trimul_proj_rows(z, w, colsum, colbias, mask, planes, stats_out, N, N, N, Np, status, stream);
+}
+
+// The same with an [N][N] mask that may be bf16 (mask_bf16) as the model holds it.
+extern "C" int ubm_trimul_proj_masked(const void* z, const void* w, const void* colsum, const void* colbias, const void* mask,
+                                      int mask_bf16, void* planes, int N, int Np, void* status, void* stream) {
+  return trimul_proj_impl(z, w, colsum, colbias, mask, planes, nullptr, N, N, N, Np, status, stream, nullptr, nullptr, 0, 0,
+                          mask_bf16);
 }

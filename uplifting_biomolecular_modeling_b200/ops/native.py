@@ -101,7 +101,7 @@ class _LibProxy:
             if name in _SIGNATURES:
                 fn.argtypes = _SIGNATURES[name]
                 fn.restype = c_int
-            c = _Counted(fn, name)
+            c = _CountedSequence(fn, SEQUENCES[name]) if name in SEQUENCES else _Counted(fn, name)
             self._cache[name] = c
         return c
 
@@ -116,6 +116,31 @@ class _Counted:
 
     def __call__(self, *a):
         _COUNTS[self.name] = _COUNTS.get(self.name, 0) + 1
+        return self.fn(*a)
+
+
+# entry points that run a whole operator, and the launches that one call of them stands for
+SEQUENCES = {
+    "ubm_trimul": ("ubm_trimul_proj", "ubm_gemm_bf16_packed", "ubm_trimul_out"),
+    "ubm_triatt": ("ubm_triatt_proj", "ubm_attention_d32", "ubm_gemm_bf16_packed"),
+    "ubm_pair_track": ("ubm_trimul_proj", "ubm_gemm_bf16_packed", "ubm_trimul_out") * 2 +
+                      ("ubm_triatt_proj", "ubm_attention_d32", "ubm_gemm_bf16_packed") * 2 + ("ubm_transition",),
+    "ubm_apb": ("ubm_gemm_bf16_packed", "ubm_attention", "ubm_gemm_bf16_packed"),
+    "ubm_transition_rows": ("ubm_layernorm_rows", "ubm_gemm_bf16_packed", "ubm_gemm_bf16_packed"),
+}
+
+
+class _CountedSequence:
+    """The same for one of :data:`SEQUENCES`: every launch is counted under its own name."""
+
+    __slots__ = ("fn", "parts")
+
+    def __init__(self, fn, parts):
+        self.fn, self.parts = fn, parts
+
+    def __call__(self, *a):
+        for name in self.parts:
+            _COUNTS[name] = _COUNTS.get(name, 0) + 1
         return self.fn(*a)
 
 

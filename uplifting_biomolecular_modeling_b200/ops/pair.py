@@ -12,6 +12,8 @@ levers (common/opt_core/opt_core/of3_trunk/castcache.py, evo2/CHANGES.md lever L
 """
 from __future__ import annotations
 
+import ctypes
+import struct
 from dataclasses import dataclass
 from typing import Optional
 
@@ -30,6 +32,13 @@ native.declare("ubm_transition", [c_void_p] * 8 + [c_ll, c_int, c_int, c_void_p,
 native.declare("ubm_trimul_proj_rows", [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_void_p, c_void_p])
 native.declare("ubm_triatt_proj_rows", [c_void_p] * 13 + [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
 native.declare("ubm_trimul_out_rows", [c_void_p] * 9 + [c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+
+
+# whole operators from one call (csrc/sequences_sm100.cu): their arguments as 8-byte integers, in the order the library reads them
+for _name in ("ubm_trimul", "ubm_triatt", "ubm_pair_track", "ubm_apb", "ubm_transition_rows"):
+    native.declare(_name, [ctypes.c_char_p])
+_TRIMUL_ARGS, _TRIATT_ARGS, _APB_ARGS = struct.Struct("=21q"), struct.Struct("=26q"), struct.Struct("=28q")
+_TRANSITION_ROWS_ARGS, _PAIR_TRACK_ARGS = struct.Struct("=3qd12q"), struct.Struct("=56q")
 
 
 def ceil_to(n: int, m: int) -> int:
@@ -98,6 +107,24 @@ def transition_fused(x: torch.Tensor, w: TransitionPacked, residual: bool = True
     return out
 
 
+def transition_rows(x: torch.Tensor, norm_w, norm_b, eps: float, w12: torch.Tensor, w3: torch.Tensor, residual: bool) -> torch.Tensor:
+    """Transition of other widths in one call: x bf16 [R, dim] contiguous, w12 as ``gemm.pack_swiglu`` packs it, w3 bf16 [out, hidden]."""
+    from . import rows as _rows
+    R, dim = x.shape
+    out_dim, hidden = w3.shape
+    dev = x.device
+    g, b = _rows._f32_param(norm_w), _rows._f32_param(norm_b)
+    scratch = torch.empty(R * (dim + hidden), dtype=torch.bfloat16, device=dev)      # norm rows, then hidden rows
+    n = scratch.data_ptr()
+    out = torch.empty((R, out_dim), dtype=torch.bfloat16, device=dev)
+    rc = native.lib().ubm_transition_rows(_TRANSITION_ROWS_ARGS.pack(
+        x.data_ptr(), native.ptr(g), native.ptr(b), eps, w12.data_ptr(), w3.data_ptr(), x.data_ptr() if residual else 0,
+        n, n + 2 * R * dim, out.data_ptr(), R, dim, hidden, out_dim, native.status_tensor(dev).data_ptr(),
+        native.current_stream(dev)))
+    native.check(rc, "ubm_transition_rows")
+    return out
+
+
 # ------------------------------------------------------------------------------------------
 @dataclass
 class TrimulPacked:
@@ -122,6 +149,11 @@ class TrimulPacked:
         wo, so, bo = fold_ln_linear(p_out, norm_out_w, norm_out_b)
         wg, sg, bg = fold_ln_linear(g_out, norm_in_w, norm_in_b)
         return cls(w_in, s_in, b_in, wo, so, bo, wg, sg, bg)
+
+    def pointers(self) -> tuple:
+        return (self.w_in.data_ptr(), self.in_colsum.data_ptr(), self.in_colbias.data_ptr(), self.wo.data_ptr(),
+                self.o_colsum.data_ptr(), self.o_colbias.data_ptr(), self.wg.data_ptr(), self.g_colsum.data_ptr(),
+                self.g_colbias.data_ptr())
 
 
 # Elements by which a row of the channel-major planes is padded: whole 32-byte sectors.  On 16 bytes (8 elements), which is all
@@ -165,6 +197,14 @@ def _trimul_blocked(z, m, w: TrimulPacked, outgoing: bool, residual: bool, out, 
     return out
 
 
+def _trimul_scratch(ws: dict, N: int, Np: int, dev) -> tuple:
+    key = ("trimul", N, dev)
+    if key not in ws:
+        ws[key] = (torch.empty((2, 128, N, Np), dtype=torch.bfloat16, device=dev),
+                   torch.empty((128, N, Np), dtype=torch.bfloat16, device=dev))
+    return ws[key]
+
+
 def trimul_fused(z: torch.Tensor, mask: Optional[torch.Tensor], w: TrimulPacked, outgoing: bool,
                  residual: bool = True, out: Optional[torch.Tensor] = None,
                  workspace: Optional[dict] = None) -> torch.Tensor:
@@ -181,27 +221,18 @@ def trimul_fused(z: torch.Tensor, mask: Optional[torch.Tensor], w: TrimulPacked,
     if 0 < rb < N:
         m = None if mask is None else mask.to(torch.float32).contiguous()
         return _trimul_blocked(z, m, w, outgoing, residual, out, ws, rb // 8 * 8 or 8)
-    key = ("trimul", N, dev)
-    if key not in ws:
-        ws[key] = (torch.empty((2, 128, N, Np), dtype=torch.bfloat16, device=dev),
-                   torch.empty((128, N, Np), dtype=torch.bfloat16, device=dev))
-    planes, x = ws[key]
-    st = native.status_tensor(dev)
-    stream = native.current_stream(dev)
-    m = None
+    planes, x = _trimul_scratch(ws, N, Np, dev)
+    kind = 0
     if mask is not None:
-        m = mask.to(torch.float32).contiguous()
-    rc = native.lib().ubm_trimul_proj(native.ptr(z), native.ptr(w.w_in), native.ptr(w.in_colsum),
-                                      native.ptr(w.in_colbias), native.ptr(m), native.ptr(planes), 0, N, Np,
-                                      native.ptr(st), stream)
-    native.check(rc, "ubm_trimul_proj")
-    _gemm.gemm(planes[0][:, :, :N], planes[1][:, :, :N], mn_major=not outgoing, out=x[:, :, :N])
+        # a bf16 mask of the pair tensor is read as it is; others are converted
+        kind = 2 if mask.dtype == torch.bfloat16 and mask.shape == (N, N) and mask.device == dev and mask.is_contiguous() else 1
+        if kind == 1:
+            mask = mask.to(torch.float32).contiguous()
     out = torch.empty_like(z) if out is None else out
-    rc = native.lib().ubm_trimul_out(native.ptr(x), native.ptr(z), native.ptr(w.wo), native.ptr(w.wg),
-                                     native.ptr(w.o_colsum), native.ptr(w.o_colbias), native.ptr(w.g_colsum),
-                                     native.ptr(w.g_colbias), native.ptr(out), N, Np, 1 if residual else 0,
-                                     native.ptr(st), stream)
-    native.check(rc, "ubm_trimul_out")
+    rc = native.lib().ubm_trimul(_TRIMUL_ARGS.pack(
+        z.data_ptr(), 0 if mask is None else mask.data_ptr(), kind, *w.pointers(), planes.data_ptr(), x.data_ptr(), out.data_ptr(), N, Np,
+        1 if outgoing else 0, 1 if residual else 0, native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
+    native.check(rc, "ubm_trimul")
     return out
 
 
@@ -255,22 +286,29 @@ class KeyMask:
         """:meth:`pack` of a mask as one launch and without the host read: a mask that keeps everything gets clear
         flags, with which the kernel runs its mask-free loop.  ``shape`` = (rows, Nk) that sizes of one broadcast to, ``device`` = the
         GPU it is wanted on (a mask made on the host is copied there)."""
-        if device is not None and keep.device != device:
-            keep = keep.to(device)
-        if not keep.is_cuda:
-            raise ValueError("a key mask is laid out on a GPU")
-        if shape is not None and 1 in keep.shape:
-            keep = keep.expand(*(to if n == 1 else -1 for n, to in zip(keep.shape, shape)))
+        keep = cls.readable(keep, shape, device)
         rows, nk = keep.shape
         steps = ceil_to(nk, MASK_STEP) // MASK_STEP
-        if keep.dtype not in (torch.float32, torch.bfloat16, torch.bool, torch.uint8):
-            keep = keep != 0
         add = torch.empty((rows, steps * MASK_STEP), dtype=torch.bfloat16, device=keep.device)
         flags = torch.empty((rows, steps), dtype=torch.uint8, device=keep.device)
         rc = native.lib().ubm_key_mask(native.ptr(keep), keep.element_size(), keep.stride(0), keep.stride(1),
                                        native.ptr(add), native.ptr(flags), rows, nk, native.current_stream(keep.device))
         native.check(rc, "ubm_key_mask")
         return cls(add, flags)
+
+
+    @staticmethod
+    def readable(keep: torch.Tensor, shape: Optional[tuple], device: Optional[torch.device]) -> torch.Tensor:
+        """The mask as the laying-out kernel reads it: on the GPU, of its full size (strides free), a type of 1, 2 or 4 bytes."""
+        if device is not None and keep.device != device:
+            keep = keep.to(device)
+        if not keep.is_cuda:
+            raise ValueError("a key mask is laid out on a GPU")
+        if shape is not None and 1 in keep.shape:
+            keep = keep.expand(*(to if n == 1 else -1 for n, to in zip(keep.shape, shape)))
+        if keep.dtype not in (torch.float32, torch.bfloat16, torch.bool, torch.uint8):
+            keep = keep != 0
+        return keep
 
 
 @dataclass
@@ -308,6 +346,10 @@ class TriattPacked:
         return cls(w, colsum, colbias, wb, wb_colsum, wb_colbias.contiguous(),
                    w_o.detach().to(torch.bfloat16).contiguous(),
                    None if b_o is None else b_o.detach().float().contiguous(), heads, (ln_w, ln_b, w_bias))
+
+    def pointers(self) -> tuple:
+        return (self.w.data_ptr(), self.colsum.data_ptr(), self.colbias.data_ptr(), self.wb.data_ptr(), self.wb_colsum.data_ptr(),
+                self.wb_colbias.data_ptr(), self.wo.data_ptr(), 0 if self.bo is None else self.bo.data_ptr())
 
 
 def attention(q, k, v, bias, gate, out, rows: int, Nq: int, Nk: int, H: int, D: int = 32, ldb: int = 0,
@@ -375,16 +417,57 @@ class ApbPacked:
                    wo.view(w_o.shape[0], heads * Dp).to(torch.bfloat16).contiguous(), heads, Dp)
 
 
+def _one_call(gate: Optional[torch.Tensor], residual: Optional[torch.Tensor], rows: int, cols: int) -> bool:
+    """Gate and residual of an output product as the operators that run in one call take them; others go product by product."""
+    return (gate is None or (gate.dtype == torch.bfloat16 and gate.dim() == 2 and gate.shape[1] == cols and gate.stride(1) == 1)) \
+        and (residual is None or (residual.dtype == torch.bfloat16 and residual.shape == (rows, cols) and residual.is_contiguous()))
+
+
 def apb_fused(x: torch.Tensor, w: ApbPacked, bias_planes: torch.Tensor, ldb: int,
               out_gate: Optional[torch.Tensor] = None, out_residual: Optional[torch.Tensor] = None,
-              mask: Optional[KeyMask] = None) -> torch.Tensor:
+              mask: Optional[KeyMask] = None, keep: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Gated attention with pair bias on rows x: bf16 [B, N, c]; bias_planes: bf16 [H, N, ldb] holding
-    log2(e) * bias (shared by the B rows); mask: key mask over [B, N] or None.
+    log2(e) * bias (shared by the B rows); mask: key mask over [B, N] or None, or ``keep`` in its place: the mask as the model
+    holds it, laid out on the way.
     Returns proj_o(sigmoid(proj_g x) * attention) as [B, N, c];
     with ``out_gate`` ([N, c], shared by the B rows) and ``out_residual`` ([B*N, c]) the output projection's
     epilogue returns residual + gate * projection."""
     B, N, c = x.shape
     HD = w.H * w.Dp
+    c_out = w.wo.shape[0]
+    if keep is not None:
+        keep = KeyMask.readable(keep, (B, N), x.device)
+        if keep.shape != (B, N):
+            keep, mask = None, KeyMask.lay_out(keep, None, x.device)
+    if x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and _one_call(out_gate, out_residual, B * N, c_out):
+        dev = x.device
+        rows_bytes = 2 * B * N * HD                     # scratch: q | k | v | gate rows, o, additive mask rows and their flags
+        ld_mask = add = flags = mask_bytes = keep_ptr = keep_bytes = keep_row = keep_key = 0
+        if keep is not None:
+            ld_mask = ceil_to(N, MASK_STEP)
+            mask_bytes = B * (2 * ld_mask + ld_mask // MASK_STEP)
+        scratch = torch.empty(5 * rows_bytes + mask_bytes, dtype=torch.uint8, device=dev)
+        qkvg = scratch.data_ptr()
+        if keep is not None:
+            add = qkvg + 5 * rows_bytes
+            flags = add + 2 * B * ld_mask
+            keep_ptr, keep_bytes = keep.data_ptr(), keep.element_size()
+            keep_row, keep_key = keep.stride()
+            native.add_launches(1, "ubm_key_mask")
+        elif mask is not None:
+            if mask.add.shape[0] != B or mask.add.shape[1] < N:
+                raise ValueError(f"key mask of shape {tuple(mask.add.shape)} does not cover [{B}, {N}]")
+            add, flags, ld_mask = mask.add.data_ptr(), mask.flags.data_ptr(), mask.add.stride(0)
+        out = torch.empty((B, N, c_out), dtype=torch.bfloat16, device=dev)
+        rc = native.lib().ubm_apb(_APB_ARGS.pack(
+            x.data_ptr(), w.wqkvg.data_ptr(), w.bqkvg.data_ptr(), w.wo.data_ptr(), native.ptr(bias_planes), ldb, keep_ptr, keep_bytes,
+            keep_row, keep_key, add, flags, ld_mask, native.ptr(out_gate), 0 if out_gate is None else out_gate.stride(0),
+            0 if out_gate is None else out_gate.shape[0], native.ptr(out_residual), qkvg, qkvg + 4 * rows_bytes, out.data_ptr(),
+            B, N, c, c_out, w.H, w.Dp, native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
+        native.check(rc, "ubm_apb")
+        return out
+    if keep is not None:
+        mask = KeyMask.lay_out(keep, None, x.device)
     x2 = x.reshape(B * N, c)
     # q | k | v | gate from one GEMM (sigmoid on the gate columns); the attention kernel reads all four as column
     # slices of its output
@@ -438,11 +521,20 @@ def _triatt_blocked(z, w: TriattPacked, starting: bool, residual: bool, out, ws:
     return out
 
 
+def _triatt_scratch(ws: dict, N: int, Np: int, heads: int, dev) -> tuple:
+    key = ("triatt", N, dev)
+    if key not in ws:
+        ws[key] = (torch.empty((5, N * N, 128), dtype=torch.bfloat16, device=dev),
+                   torch.zeros((heads, N, Np), dtype=torch.bfloat16, device=dev))
+    return ws[key]
+
+
 def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, residual: bool = True,
                              out: Optional[torch.Tensor] = None, workspace: Optional[dict] = None,
-                             mask: Optional[KeyMask] = None) -> torch.Tensor:
+                             mask: Optional[KeyMask] = None, keep: Optional[torch.Tensor] = None) -> torch.Tensor:
     """z: bf16 [N, N, 128] contiguous; mask: key mask over [attention row, key] (for the ending node the
-    attention rows are the columns of z, so the caller packs the transposed pair mask).  Three launches:
+    attention rows are the columns of z, so the caller packs the transposed pair mask), or ``keep`` in its place: the mask as
+    the model holds it, laid out on the way.  Three launches:
     projection (LN folded, q|k|v|gate rows + head bias planes, written at the transposed pair index for the
     ending node) -> attention -> output projection with residual."""
     if z.dtype != torch.bfloat16 or z.dim() != 3 or z.shape[-1] != 128 or not z.is_contiguous():
@@ -453,24 +545,56 @@ def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, r
     ws = workspace if workspace is not None else {}
     rb = int(ws.get("row_block", 0) or 0)
     if 0 < rb < N:
+        if keep is not None:
+            mask = KeyMask.lay_out(keep, (N, N), dev)
         return _triatt_blocked(z, w, starting, residual, out, ws, mask, rb)
-    key = ("triatt", N, dev)
-    if key not in ws:
-        ws[key] = (torch.empty((5, N * N, 128), dtype=torch.bfloat16, device=dev),
-                   torch.zeros((w.heads, N, Np), dtype=torch.bfloat16, device=dev))
-    qkvgo, hb = ws[key]
-    q, k, v, g, og = qkvgo[0], qkvgo[1], qkvgo[2], qkvgo[3], qkvgo[4]
-    st = native.status_tensor(dev)
-    stream = native.current_stream(dev)
-    rc = native.lib().ubm_triatt_proj(native.ptr(z), native.ptr(w.w), native.ptr(w.colsum), native.ptr(w.colbias),
-                                      native.ptr(w.wb), native.ptr(w.wb_colsum), native.ptr(w.wb_colbias),
-                                      native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(g), native.ptr(hb), 0,
-                                      N, Np, w.heads, 0 if starting else 1, native.ptr(st), stream)
-    native.check(rc, "ubm_triatt_proj")
-    attention_d32(q, k, v, hb, g, og, rows=N, Nq=N, Nk=N, H=w.heads, ldb=Np, transpose_out=not starting, mask=mask)
-    z2 = z.view(N * N, 128)
+    add = flags = keep_ptr = keep_bytes = keep_row = keep_key = ld_mask = 0
+    if keep is not None:
+        keep = KeyMask.readable(keep, (N, N), dev)
+        if keep.shape != (N, N):
+            keep, mask = None, KeyMask.lay_out(keep, None, dev)
+    if keep is not None:
+        ld_mask = ceil_to(N, MASK_STEP)
+        laid = torch.empty(N * (2 * ld_mask + ld_mask // MASK_STEP), dtype=torch.uint8, device=dev)     # additive rows, then flags
+        add, keep_ptr, keep_bytes = laid.data_ptr(), keep.data_ptr(), keep.element_size()
+        flags = add + 2 * N * ld_mask
+        keep_row, keep_key = keep.stride()
+        native.add_launches(1, "ubm_key_mask")
+    elif mask is not None:
+        if mask.add.shape[0] != N or mask.add.shape[1] < N:
+            raise ValueError(f"key mask of shape {tuple(mask.add.shape)} does not cover [{N}, {N}]")
+        add, flags, ld_mask = mask.add.data_ptr(), mask.flags.data_ptr(), mask.add.stride(0)
+    qkvgo, hb = _triatt_scratch(ws, N, Np, w.heads, dev)
     out = torch.empty_like(z) if out is None else out
-    _gemm.gemm(og, w.wo, bias=w.bo, residual=z2 if residual else None, out=out.view(N * N, 128))
+    rc = native.lib().ubm_triatt(_TRIATT_ARGS.pack(
+        z.data_ptr(), keep_ptr, keep_bytes, keep_row, keep_key, add, flags, ld_mask, *w.pointers(), qkvgo.data_ptr(), hb.data_ptr(), out.data_ptr(), N, Np, w.heads,
+        1 if starting else 0, 1 if residual else 0, native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
+    native.check(rc, "ubm_triatt")
+    return out
+
+
+def pair_track(z: torch.Tensor, mask: Optional[torch.Tensor], tm_out: TrimulPacked, tm_in: TrimulPacked, ta_start: TriattPacked,
+               ta_end: TriattPacked, tr: TransitionPacked, workspace: dict) -> torch.Tensor:
+    """The five pair operators of a Pairformer layer, each with its residual, from one call.  z: bf16 [1, N, N, 128] contiguous; mask:
+    bf16 [1, N, N] contiguous or None."""
+    N, dev = z.shape[1], z.device
+    Np, bias_row = ceil_to(N, PLANE_ROW), ceil_to(N, 8)
+    planes, x = _trimul_scratch(workspace, N, Np, dev)
+    qkvgo, hb = _triatt_scratch(workspace, N, bias_row, ta_start.heads, dev)
+    out, other = torch.empty_like(z), torch.empty_like(z)
+    add = flags = ld_mask = mask_ptr = 0
+    if mask is not None:
+        ld_mask, mask_ptr = ceil_to(N, MASK_STEP), mask.data_ptr()
+        laid = torch.empty(N * (2 * ld_mask + ld_mask // MASK_STEP), dtype=torch.uint8, device=dev)     # additive rows, then flags
+        add = laid.data_ptr()
+        flags = add + 2 * N * ld_mask
+        native.add_launches(2, "ubm_key_mask")
+    rc = native.lib().ubm_pair_track(_PAIR_TRACK_ARGS.pack(
+        z.data_ptr(), out.data_ptr(), other.data_ptr(), mask_ptr, add, flags, ld_mask, *tm_out.pointers(), *tm_in.pointers(),
+        *ta_start.pointers(), *ta_end.pointers(), tr.wab.data_ptr(), tr.wo.data_ptr(), tr.colsum.data_ptr(), tr.colbias.data_ptr(),
+        tr.hidden, planes.data_ptr(), x.data_ptr(), qkvgo.data_ptr(), hb.data_ptr(), N, Np, bias_row, ta_start.heads,
+        native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
+    native.check(rc, "ubm_pair_track")
     return out
 
 
