@@ -129,6 +129,7 @@ atom_qkvg_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  grid_dependency_sync(short_grid(p.num_tiles, 8));
   for (int i = threadIdx.x; i < 384; i += blockDim.x) sBias[i] = p.bias[i];
   tc_fence_before_sync();
   __syncthreads();
@@ -364,6 +365,7 @@ cond_transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  grid_dependency_sync(short_grid(p.num_tiles, 8));
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -659,7 +661,7 @@ extern "C" int ubm_atom_qkvg(const void* a, const void* scale, const void* shift
   int rc = set_smem(atom_qkvg_kernel, kAQSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  atom_qkvg_kernel<<<grid, kAQThreads, kAQSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmW, tmOut, p);
+  launch_after(true, atom_qkvg_kernel, grid, kAQThreads, kAQSmemBytes, static_cast<cudaStream_t>(stream), tmW, tmOut, p);
   UBM_CHECK_LAUNCH("atom_qkvg_kernel");
   return UBM_OK;
 }
@@ -717,7 +719,7 @@ extern "C" int ubm_cond_transition(const void* a, const void* scale, const void*
   int rc = set_smem(cond_transition_kernel, kCTSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  cond_transition_kernel<<<grid, kCTThreads, kCTSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmX, tmGate, tmWin, tmWo, tmOut, p);
+  launch_after(true, cond_transition_kernel, grid, kCTThreads, kCTSmemBytes, static_cast<cudaStream_t>(stream), tmX, tmGate, tmWin, tmWo, tmOut, p);
   UBM_CHECK_LAUNCH("cond_transition_kernel");
   return UBM_OK;
 }

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <stdlib.h>
 
 namespace ubm {
 
@@ -99,6 +100,37 @@ inline int sm_count() {
       return ubm::UBM_ERR_LAUNCH;                                                           \
     }                                                                                       \
   } while (0)
+
+// UBM_PDL=0: launches wait for the whole of the kernel in front of them
+inline bool overlap_launches() {
+  static const bool on = [] {
+    const char* e = getenv("UBM_PDL");
+    return e == nullptr || e[0] != '0';
+  }();
+  return on;
+}
+
+// Launch of a kernel that calls grid_dependency_sync() in every thread: with `overlap` its CTAs may be placed, and do their set-up,
+// while the kernel in front of it drains.  Between two kernels of one wave that hides about 3 us of launch, barrier and
+// tensor-memory set-up (a Pairformer block of 137 tokens 298 -> 268 us, three atom layers 345 -> 327).  The CTAs then start in the
+// order in which SMs become free, no longer in the order of the tiles that share operands in L2.  So kernels that re-read theirs
+// from L2 for long ask for it, and let the next one begin, only while they are short (attention of 1536 tokens 6064 -> 6122 us, pair
+// averaging 672 -> 678, token layers 635 -> 639 where they did not).
+template <typename... P, typename... A>
+inline cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream,
+                                const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap && overlap_launches() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 
 template <typename K>
 inline int set_smem(K kernel, int bytes) {

@@ -121,6 +121,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  grid_dependency_sync(short_grid(p.num_tiles, 4));
   // column constants
   for (int i = threadIdx.x; i < 512; i += blockDim.x) {
     sColsum[i] = p.colsum[i];
@@ -471,7 +472,7 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
   rc = set_smem(kern, kPPSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  kern<<<grid, kPPThreads, kPPSmemBytes, stream>>>(tmX, tmW, maps, outs, p);
+  launch_after(p.num_tiles <= 4 * grid, kern, grid, kPPThreads, kPPSmemBytes, stream, tmX, tmW, maps, outs, p);
   UBM_CHECK_LAUNCH("pair_proj_kernel");
   return UBM_OK;
 }

@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(256) pwa_pack_kernel(const void* __restrict__ 
                                                        const void* __restrict__ gamma, int gamma_fp32,
                                                        const void* __restrict__ beta, int beta_fp32,
                                                        __nv_bfloat16* __restrict__ w, float* __restrict__ consts) {
+  grid_dependency_sync(true);
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;     // 0 .. 511: values, then gates
   const int ch = row & (kPwHC - 1), gate = row / kPwHC;
   float sum = 0.f, bias = 0.f;
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(256) pwa_pack_kernel(const void* __restrict__ 
 template <typename MT>
 __global__ void __launch_bounds__(256) pwa_softmax_kernel(__nv_bfloat16* __restrict__ b, const MT* __restrict__ mask,
                                                           int H, int N, int ld) {
+  grid_dependency_sync(gridDim.x <= 2048);
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= static_cast<long long>(H) * N) return;
@@ -141,6 +143,7 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
+  grid_dependency_sync(short_grid(p.num_tiles, 4));
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -348,6 +351,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  grid_dependency_sync(short_grid(p.num_tiles, 4));
   for (int i = threadIdx.x; i < kPwHC; i += blockDim.x) {
     sConst[i] = p.g_colsum[i];
     sConst[kPwHC + i] = p.g_colbias[i];
@@ -534,7 +538,7 @@ static int pwa_pack(const void* wv, int wv_fp32, const void* wg, int wg_fp32, co
                             const void* beta, int beta_fp32, void* w, void* consts, void* stream) {
   using namespace ubm;
   if (wv == nullptr || wg == nullptr || w == nullptr || consts == nullptr) return UBM_ERR_ARGUMENT;
-  pwa_pack_kernel<<<2 * kPwHC / 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_after(true, pwa_pack_kernel, 2 * kPwHC / 8, 256, 0, static_cast<cudaStream_t>(stream),
       wv, wv_fp32, wg, wg_fp32, gamma, gamma_fp32, beta, beta_fp32, static_cast<__nv_bfloat16*>(w),
       static_cast<float*>(consts));
   UBM_CHECK_LAUNCH("pwa_pack_kernel");
@@ -549,10 +553,10 @@ static int pwa_softmax(void* b, const void* mask, int mask_bf16, int H, int N, i
   const unsigned grid = static_cast<unsigned>((rows + 7) / 8);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (mask_bf16)
-    pwa_softmax_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<__nv_bfloat16*>(b),
+    launch_after(grid <= 2048, pwa_softmax_kernel<__nv_bfloat16>, grid, 256, 0, st, static_cast<__nv_bfloat16*>(b),
                                                             static_cast<const __nv_bfloat16*>(mask), H, N, ld);
   else
-    pwa_softmax_kernel<float><<<grid, 256, 0, st>>>(static_cast<__nv_bfloat16*>(b), static_cast<const float*>(mask), H,
+    launch_after(grid <= 2048, pwa_softmax_kernel<float>, grid, 256, 0, st, static_cast<__nv_bfloat16*>(b), static_cast<const float*>(mask), H,
                                                     N, ld);
   UBM_CHECK_LAUNCH("pwa_softmax_kernel");
   return UBM_OK;
@@ -590,8 +594,8 @@ static int pwa_value(const void* m, const void* w, const void* colsum, const voi
   rc = set_smem(pwa_value_kernel, kPvSmem);
   if (rc) return rc;
   const int slots = 2 * sm_count();
-  pwa_value_kernel<<<p.num_tiles < slots ? p.num_tiles : slots, 320, kPvSmem, static_cast<cudaStream_t>(stream)>>>(
-      tmM, tmW, tmV, p);
+  launch_after(p.num_tiles <= 4 * slots, pwa_value_kernel, p.num_tiles < slots ? p.num_tiles : slots, 320, kPvSmem, static_cast<cudaStream_t>(stream), tmM,
+               tmW, tmV, p);
   UBM_CHECK_LAUNCH("pwa_value_kernel");
   return UBM_OK;
 }
@@ -635,7 +639,7 @@ static int pwa_out(const void* m, const void* o, const void* wg, const void* g_c
   rc = set_smem(pwa_out_kernel, kPoSmem);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  pwa_out_kernel<<<grid, kPoThreads, kPoSmem, static_cast<cudaStream_t>(stream)>>>(tmM, tmO, tmWg, tmWo, tmOut, p);
+  launch_after(p.num_tiles <= 4 * grid, pwa_out_kernel, grid, kPoThreads, kPoSmem, static_cast<cudaStream_t>(stream), tmM, tmO, tmWg, tmWo, tmOut, p);
   UBM_CHECK_LAUNCH("pwa_out_kernel");
   return UBM_OK;
 }

@@ -15,6 +15,10 @@
 
 namespace ubm {
 
+// Row kernels of up to 16 MB take a few us each: their launch may overlap the kernel in front.  (Conditioned norms of 4 MB: two
+// token layers of 5 x 1536, 12 MB a norm, 635 without and 639 us with.)
+__host__ __device__ inline bool short_rows(long long R, long long C) { return R * C <= (8ll << 20); }
+
 template <typename T>
 __device__ __forceinline__ float to_f(T v);
 template <>
@@ -34,6 +38,7 @@ template <typename TI, typename TO, int MAXPL>
 __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restrict__ x, const float* __restrict__ gamma,
                                                              const float* __restrict__ beta, TO* __restrict__ out,
                                                              long long R, int C, float eps) {
+  grid_dependency_sync(short_rows(R, C));
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (long long r = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); r < R;
@@ -82,6 +87,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_wide_kernel(const __nv_bfl
                                                                   const float* __restrict__ beta,
                                                                   __nv_bfloat16* __restrict__ out, long long R, int C,
                                                                   float eps) {
+  grid_dependency_sync(short_rows(R, C));
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (long long r = static_cast<long long>(blockIdx.x) * wpb + (threadIdx.x >> 5); r < R;
@@ -139,6 +145,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_wide_kernel(const __nv_bfl
 __global__ void __launch_bounds__(256) mean_rescale_kernel(__nv_bfloat16* __restrict__ o, const float* __restrict__ count,
                                                            const float* __restrict__ bias, long long vecs, int vpr,
                                                            float total) {
+  grid_dependency_sync(short_rows(vecs, 8));
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < vecs;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long r = i / vpr;
@@ -163,6 +170,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_narrow_kernel(const __nv_b
                                                                     const float* __restrict__ beta,
                                                                     __nv_bfloat16* __restrict__ out, long long R,
                                                                     float eps) {
+  grid_dependency_sync(short_rows(R, 256));
   constexpr int C = 8 * LPR;
   constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31;
@@ -234,6 +242,7 @@ __global__ void __launch_bounds__(128) pair_head_bias_kernel(const __nv_bfloat16
                                                              const float* __restrict__ colbias,
                                                              __nv_bfloat16* __restrict__ out, int N, int Np,
                                                              int transpose_out) {
+  grid_dependency_sync(short_rows(static_cast<long long>(N) * N, 128));
   constexpr int NT = (H + 7) / 8;
   __shared__ uint2 sw[NT][3][8][32];                       // B fragments: [head tile][part][product][lane]
   __shared__ __align__(4) __nv_bfloat16 so[NT * 8][kHbLd];
@@ -364,6 +373,7 @@ __global__ void __launch_bounds__(256) adaln_rows_kernel(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ shift,
                                                          __nv_bfloat16* __restrict__ out, long long R, int C,
                                                          long long cond_rows, long long ld_cond, float eps) {
+  grid_dependency_sync(short_rows(4 * R, C));
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (long long r = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); r < R;
@@ -400,6 +410,7 @@ __global__ void __launch_bounds__(256) adaln_rows_vec_kernel(const __nv_bfloat16
                                                              const __nv_bfloat16* __restrict__ shift,
                                                              __nv_bfloat16* __restrict__ out, long long R, int C,
                                                              long long cond_rows, long long ld_cond, float eps) {
+  grid_dependency_sync(short_rows(4 * R, C));
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (long long r = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); r < R;
@@ -455,6 +466,7 @@ __global__ void __launch_bounds__(256) adaln_rows_c128_kernel(const __nv_bfloat1
                                                               const __nv_bfloat16* __restrict__ shift,
                                                               __nv_bfloat16* __restrict__ out, long long R,
                                                               long long cond_rows, long long ld_cond, float eps) {
+  grid_dependency_sync(short_rows(4 * R, 128));
   constexpr int C = 128;
   const int halves_per_block = blockDim.x >> 4;
   const int l16 = threadIdx.x & 15;
@@ -590,6 +602,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) key_mask_kernel(const T* __restrict__ keep, long long s_row, long long s_key,
                                                        __nv_bfloat16* __restrict__ add, unsigned char* __restrict__ flags,
                                                        int rows, int nk, int steps) {
+  grid_dependency_sync(true);
   const int lane = threadIdx.x & 31;
   const long long w = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   const int step = static_cast<int>(w % steps);
@@ -609,6 +622,7 @@ __global__ void __launch_bounds__(256) key_mask_rows_kernel(const T* __restrict_
                                                             __nv_bfloat16* __restrict__ add,
                                                             unsigned char* __restrict__ flags, int rows, int nk,
                                                             int steps) {
+  grid_dependency_sync(true);
   __shared__ uint32_t masked[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int step = static_cast<int>(blockIdx.x % steps);
@@ -650,8 +664,8 @@ extern "C" int ubm_layernorm_rows(const void* x, const void* gamma, const void* 
     const int gridw = grid_for(R, 8);
     const bool vec = ((reinterpret_cast<uintptr_t>(gg) | reinterpret_cast<uintptr_t>(bb)) & 31) == 0;
 #define UBM_LN_WIDE(CH)                                                                                          \
-  (vec ? layernorm_rows_wide_kernel<CH, true><<<gridw, 256, 0, st>>>(xx, gg, bb, oo, R, C, eps)                  \
-       : layernorm_rows_wide_kernel<CH, false><<<gridw, 256, 0, st>>>(xx, gg, bb, oo, R, C, eps))
+  (vec ? launch_after(short_rows(R, C), layernorm_rows_wide_kernel<CH, true>, gridw, 256, 0, st, xx, gg, bb, oo, R, C, eps)                  \
+       : launch_after(short_rows(R, C), layernorm_rows_wide_kernel<CH, false>, gridw, 256, 0, st, xx, gg, bb, oo, R, C, eps))
     if (C <= 512) UBM_LN_WIDE(2);
     else if (C <= 1024) UBM_LN_WIDE(4);
     else if (C <= 1280) UBM_LN_WIDE(5);
@@ -669,9 +683,9 @@ extern "C" int ubm_layernorm_rows(const void* x, const void* gamma, const void* 
     const float* bb = static_cast<const float*>(beta);
     const int rows_per_block = 8 * (256 / C);
     const int grid2 = grid_for(R, rows_per_block);
-    if (C == 64) layernorm_rows_narrow_kernel<8><<<grid2, 256, 0, st>>>(xx, gg, bb, oo, R, eps);
-    else if (C == 128) layernorm_rows_narrow_kernel<16><<<grid2, 256, 0, st>>>(xx, gg, bb, oo, R, eps);
-    else layernorm_rows_narrow_kernel<32><<<grid2, 256, 0, st>>>(xx, gg, bb, oo, R, eps);
+    if (C == 64) launch_after(short_rows(R, C), layernorm_rows_narrow_kernel<8>, grid2, 256, 0, st, xx, gg, bb, oo, R, eps);
+    else if (C == 128) launch_after(short_rows(R, C), layernorm_rows_narrow_kernel<16>, grid2, 256, 0, st, xx, gg, bb, oo, R, eps);
+    else launch_after(short_rows(R, C), layernorm_rows_narrow_kernel<32>, grid2, 256, 0, st, xx, gg, bb, oo, R, eps);
     UBM_CHECK_LAUNCH("layernorm_rows_narrow_kernel");
     return UBM_OK;
   }
@@ -679,7 +693,7 @@ extern "C" int ubm_layernorm_rows(const void* x, const void* gamma, const void* 
   const float* g = static_cast<const float*>(gamma);
   const float* b = static_cast<const float*>(beta);
 #define UBM_LN_LAUNCH(TI, TO, MP)                                                                          \
-  layernorm_rows_kernel<TI, TO, MP><<<grid, 256, 0, st>>>(static_cast<const TI*>(x), g, b, static_cast<TO*>(out), R, \
+  launch_after(short_rows(R, C), layernorm_rows_kernel<TI, TO, MP>, grid, 256, 0, st, static_cast<const TI*>(x), g, b, static_cast<TO*>(out), R, \
                                                           C, eps)
 #define UBM_LN_BY_WIDTH(TI, TO)      \
   do {                               \
@@ -710,7 +724,7 @@ extern "C" int ubm_mean_rescale(void* o, const void* count, const void* bias, lo
   if (R <= 0 || C <= 0 || (C & 7) || ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(bias)) & 15))
     return UBM_ERR_ARGUMENT;
   const long long vecs = R * (C / 8);
-  mean_rescale_kernel<<<grid_for(vecs, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_after(short_rows(R, C), mean_rescale_kernel, grid_for(vecs, 256), 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<__nv_bfloat16*>(o), static_cast<const float*>(count), static_cast<const float*>(bias), vecs, C / 8, total);
   UBM_CHECK_LAUNCH("mean_rescale_kernel");
   return UBM_OK;
@@ -728,10 +742,10 @@ extern "C" int ubm_pair_head_bias(const void* z, const void* w, const void* cols
   const float* cb = static_cast<const float*>(colbias);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   switch (H) {
-    case 4: pair_head_bias_kernel<4><<<grid, 128, 0, st>>>(zz, ww, cs, cb, o, N, Np, transpose_out); break;
-    case 8: pair_head_bias_kernel<8><<<grid, 128, 0, st>>>(zz, ww, cs, cb, o, N, Np, transpose_out); break;
-    case 16: pair_head_bias_kernel<16><<<grid, 128, 0, st>>>(zz, ww, cs, cb, o, N, Np, transpose_out); break;
-    case 32: pair_head_bias_kernel<32><<<grid, 128, 0, st>>>(zz, ww, cs, cb, o, N, Np, transpose_out); break;
+    case 4: launch_after(short_rows(static_cast<long long>(N) * N, 128), pair_head_bias_kernel<4>, grid, 128, 0, st, zz, ww, cs, cb, o, N, Np, transpose_out); break;
+    case 8: launch_after(short_rows(static_cast<long long>(N) * N, 128), pair_head_bias_kernel<8>, grid, 128, 0, st, zz, ww, cs, cb, o, N, Np, transpose_out); break;
+    case 16: launch_after(short_rows(static_cast<long long>(N) * N, 128), pair_head_bias_kernel<16>, grid, 128, 0, st, zz, ww, cs, cb, o, N, Np, transpose_out); break;
+    case 32: launch_after(short_rows(static_cast<long long>(N) * N, 128), pair_head_bias_kernel<32>, grid, 128, 0, st, zz, ww, cs, cb, o, N, Np, transpose_out); break;
     default: return UBM_ERR_ARGUMENT;
   }
   UBM_CHECK_LAUNCH("pair_head_bias_kernel");
@@ -753,17 +767,17 @@ extern "C" int ubm_adaln_rows(const void* a, const void* scale, const void* shif
                      reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   const int grid = grid_for(R, 8);
   if (vec && C == 128) {
-    adaln_rows_c128_kernel<<<grid_for((R + 1) / 2 * 2, 16), 256, 0, st>>>(aa, sc, sh, oo, R, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_c128_kernel, grid_for((R + 1) / 2 * 2, 16), 256, 0, st, aa, sc, sh, oo, R, cond_rows, ld_cond, eps);
   } else if (vec && C <= 256) {
-    adaln_rows_vec_kernel<1><<<grid, 256, 0, st>>>(aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<1>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else if (vec && C <= 512) {
-    adaln_rows_vec_kernel<2><<<grid, 256, 0, st>>>(aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<2>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else if (vec && C <= 768) {
-    adaln_rows_vec_kernel<3><<<grid, 256, 0, st>>>(aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<3>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else if (vec) {
-    adaln_rows_vec_kernel<4><<<grid, 256, 0, st>>>(aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<4>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else {
-    adaln_rows_kernel<<<grid, 256, 0, st>>>(aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_kernel, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   }
   UBM_CHECK_LAUNCH("adaln_rows_kernel");
   return UBM_OK;
@@ -816,11 +830,11 @@ extern "C" int ubm_key_mask(const void* keep, int elem_bytes, long long s_row, l
 #define UBM_KEY_MASK(T)                                                                                            \
   do {                                                                                                             \
     if (on_keys)                                                                                                   \
-      key_mask_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T*>(keep), s_row, s_key,                          \
+      launch_after(true, key_mask_kernel<T>, grid, 256, 0, st, static_cast<const T*>(keep), s_row, s_key,                          \
                                                static_cast<__nv_bfloat16*>(add),                                   \
                                                static_cast<unsigned char*>(flags), rows, nk, steps);               \
     else                                                                                                           \
-      key_mask_rows_kernel<T><<<grid, 256, 0, st>>>(static_cast<const T*>(keep), s_row, s_key,                     \
+      launch_after(true, key_mask_rows_kernel<T>, grid, 256, 0, st, static_cast<const T*>(keep), s_row, s_key,                     \
                                                     static_cast<__nv_bfloat16*>(add),                              \
                                                     static_cast<unsigned char*>(flags), rows, nk, steps);          \
   } while (0)

@@ -69,6 +69,18 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Programmatic dependent launch (host_util.h, launch_after): what stands in front of this touches nothing that an earlier kernel of
+// the stream writes and may run while that kernel drains; from here on everything it wrote is there.  With `next` the kernel
+// behind this one, if it was launched that way, may begin its own set-up as soon as every CTA has passed; without, when this one
+// ends.  The wait does nothing in a launch without the attribute.
+__device__ __forceinline__ void grid_dependency_sync(bool next) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (next) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// at most `waves` tiles for every CTA of the launch
+__device__ __forceinline__ bool short_grid(int tiles, int waves) { return tiles <= waves * static_cast<int>(gridDim.x); }
+
 // ----------------------------------------------------------------------------------------
 // mbarrier
 

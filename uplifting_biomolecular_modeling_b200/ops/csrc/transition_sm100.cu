@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(kTRThreads, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWab,
                   const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmOut,
                   TransitionParams p) {
+  grid_dependency_sync(short_grid(p.num_tiles, 8));
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + smem_pad1024(smem_raw);
   uint8_t* sX = smem;                                   // 2 x 32 KB
@@ -525,7 +526,7 @@ extern "C" int ubm_transition(const void* x, const void* wab, const void* wo, co
   int rc = set_smem(transition_kernel, smem);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  transition_kernel<<<grid, kTRThreads, smem, static_cast<cudaStream_t>(stream)>>>(tmX, tmWab, tmWo, tmOut, p);
+  launch_after(true, transition_kernel, grid, kTRThreads, smem, static_cast<cudaStream_t>(stream), tmX, tmWab, tmWo, tmOut, p);
   UBM_CHECK_LAUNCH("transition_kernel");
   return UBM_OK;
 }

@@ -88,6 +88,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  grid_dependency_sync(short_grid(p.num_tiles, 8));
   for (int i = threadIdx.x; i < 128; i += blockDim.x) {
     sConst[i] = p.o_colsum[i];
     sConst[128 + i] = p.o_colbias[i];
@@ -399,7 +400,7 @@ extern "C" int ubm_trimul_out_rows(const void* x, const void* z, const void* wo,
   int rc = set_smem(trimul_out_kernel, kTOSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  trimul_out_kernel<<<grid, kTOThreads, kTOSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmX, tmZ, tmWo, tmWg, tmO, p);
+  launch_after(true, trimul_out_kernel, grid, kTOThreads, kTOSmemBytes, static_cast<cudaStream_t>(stream), tmX, tmZ, tmWo, tmWg, tmO, p);
   UBM_CHECK_LAUNCH("trimul_out_kernel");
   return UBM_OK;
 }

@@ -105,6 +105,7 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  grid_dependency_sync(short_grid(p.num_tiles, 8));
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -385,7 +386,7 @@ static int trimul_proj_impl(const void* z, const void* w, const void* colsum, co
   rc = set_smem(trimul_proj_kernel, kTPSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  trimul_proj_kernel<<<grid, kTPThreads, kTPSmemBytes, static_cast<cudaStream_t>(stream)>>>(tmX, tmW, maps, tmP, p);
+  launch_after(true, trimul_proj_kernel, grid, kTPThreads, kTPSmemBytes, static_cast<cudaStream_t>(stream), tmX, tmW, maps, tmP, p);
   UBM_CHECK_LAUNCH("trimul_proj_kernel");
   return UBM_OK;
 }

@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(kWLThreads, 1) window_layer_kernel(WindowLayer
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
+  grid_dependency_sync(short_grid(p.units, 8));
   const uint32_t base0 = smem_u32(smem);         // the offsets below count from smem
   constexpr uint32_t sO = 4 * kWLKV, sWo = sO + kWLO;   // in front: K and V of an even unit, of an odd one
   auto lds128 = [&](uint32_t at) { return *reinterpret_cast<const uint4*>(smem + at); };
@@ -415,7 +416,7 @@ extern "C" int ubm_window_layer(const void* qkvg, const void* bias, const void* 
   int rc = set_smem(kernel, kWLSmemBytes);
   if (rc) return rc;
   const int grid = p.units < sm_count() ? p.units : sm_count();
-  kernel<<<grid, kWLThreads, kWLSmemBytes, static_cast<cudaStream_t>(stream)>>>(p);
+  launch_after(true, kernel, grid, kWLThreads, kWLSmemBytes, static_cast<cudaStream_t>(stream), p);
   UBM_CHECK_LAUNCH("window_layer_kernel");
   return UBM_OK;
 }
