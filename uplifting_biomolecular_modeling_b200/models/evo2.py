@@ -27,6 +27,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops import seq
+
 
 @dataclass(frozen=True)
 class Evo2Config:
@@ -74,7 +76,6 @@ class RMSNorm(nn.Module):
 
     def forward(self, x):
         if _fusable(self, x):
-            from ..ops import seq
             return seq.rmsnorm_rows(x, self.scale, self.eps)
         x32 = x.float()
         y = x32 * torch.rsqrt(x32.pow(2).mean(-1, keepdim=True) + self.eps)
@@ -191,7 +192,6 @@ class HyenaOperator(nn.Module):
 
     def _kernel_taps(self):
         if self._taps is None:
-            from ..ops import seq
             self._taps = (seq.taps_major(self.fir), None if self.kind == "hcl" else seq.taps_major(self.h))
         return self._taps
 
@@ -203,7 +203,6 @@ class HyenaOperator(nn.Module):
     def _fused_inner(self, u, x2, state: Optional[dict] = None):
         """x2 * (conv(u) + D u) with the gate folded into the convolution's epilogue.  The recurrence form of the long
         operator ends with the pole state, which goes into ``state``."""
-        from ..ops import seq
         if self._scans(u):
             gated, poles = seq.pole_conv_gate(u, self._lam(), self.residues, self.D, x2)
             if state is not None:
@@ -228,7 +227,6 @@ class HyenaOperator(nn.Module):
         z = fp8_projection(self.in_proj, x, pre_norm) if pre_norm is not None else lin(self.in_proj, x)
         fused = _fusable(self, z) and self.cfg.fir_len <= 4
         if fused:
-            from ..ops import seq
             u, x2 = seq.fir_gate3(z, self._kernel_taps()[0])
             gated = self._fused_inner(u, x2, state)
         else:
@@ -253,7 +251,6 @@ class HyenaOperator(nn.Module):
         lin = linear or (lambda m, t: m(t))
         z = lin(self.in_proj, x)
         if _fusable(self, z) and self.cfg.fir_len <= 4:
-            from ..ops import seq
             # a static state (fixed-address buffers that only this decode loop holds) is moved on inside the
             # kernels; any other state may be shared with a snapshot and is replaced, not written
             inplace = bool(state.get("static")) and z.shape[1] == 1 and _kernel_tail(state["fir_tail"])
@@ -408,7 +405,6 @@ class AttentionOperator(nn.Module):
         H = qkv.shape[-1] // (3 * hd)
         if _fusable(self, qkv) and L > 8 and hd % 2 == 0:
             # one pass over the projection: rotary embedding of q and k, the three tensors written apart
-            from ..ops import seq
             q, k, v = seq.rotary_split_qkv(qkv.view(B * L, -1), pos.to(torch.int32).repeat(B), H, hd,
                                            self.cfg.rope_base)
             return q.view(B, L, H, hd), k.view(B, L, H, hd), v.view(B, L, H, hd)
@@ -437,7 +433,6 @@ class AttentionOperator(nn.Module):
             if _fusable(self, x) and x.shape[1] == 1 and hd == 128 and state["k"].dtype == torch.bfloat16 and \
                     state["k"].is_contiguous() and state["v"].is_contiguous():
                 # rotary embedding, cache write and the masked attention as three launches of the kernel path
-                from ..ops import seq
                 o = seq.decode_attention(lin(self.qkv, x).view(B, -1), pos, state["k"], state["v"],
                                          self.cfg.rope_base)
                 return lin(self.out_proj, o.view(B, 1, -1))
@@ -500,7 +495,6 @@ class SwiGLU(nn.Module):
             return lin(self.l3, h.view(*x.shape[:-1], h.shape[-1]))
         g, up = lin(self.l1, x), lin(self.l2, x)
         if _fusable(self, g):
-            from ..ops import seq
             return lin(self.l3, seq.silu_mul(g, up))
         return lin(self.l3, F.silu(g) * up)
 
@@ -534,8 +528,57 @@ class Block(nn.Module):
         x = x + self.mixer(self.pre_norm(x), state, linear)
         return x + self.mlp(self.post_norm(x), linear)
 
+    def _step_call(self, x, state, folded) -> Optional[torch.Tensor]:
+        """A step of the folded block from one call of the library (some 45 us of the host; its seven launches one by one take 115),
+        or None where any of its parts would do anything else: another projection hook or step, e4m3 weights, a state that is
+        replaced and not written, an input that has to be copied."""
+        mix, mlp, B, d = self.mixer, self.mlp, x.shape[0], x.shape[-1]
+        first = mix.qkv if self.kind == "attn" else mix.in_proj
+        if folded is not folded_linear or x.shape[1] != 1 or not x.is_contiguous() or not state.get("static") or \
+                getattr(mix, "impl", "") != "fused" or type(mix).step is not _STEPS[self.kind == "attn"] or "step" in mix.__dict__ or \
+                any(getattr(m, "fp8_weights", False) for m in (first, mix.out_proj, mlp.l3)):
+            return None
+        if self.kind == "attn":
+            kc, vc, pos = state["k"], state["v"], state["pos"]
+            if kc.dim() != 4 or kc.shape[0] != B or kc.shape[2] * 128 != d or kc.shape[3] != 128 or vc.shape != kc.shape or \
+                    kc.dtype != torch.bfloat16 or vc.dtype != torch.bfloat16 or not kc.is_contiguous() or not vc.is_contiguous() or \
+                    pos.dtype != torch.int64 or pos.numel() != 1 or pos.device != x.device or mix.cfg.d_model // mix.cfg.n_heads != 128:
+                return None
+            kind, operands = 2, (pos, kc, vc)
+            sizes = (kc.shape[2], kc.shape[1], max(1, min(64, (kc.shape[1] + 1023) // 1024)))       # splits as decode_attention's
+            factors = (float(mix.cfg.rope_base), 128.0 ** -0.5)
+        else:
+            tail = state["fir_tail"]
+            taps, inner = mix._kernel_taps()
+            if mix.cfg.fir_len > 4 or not _kernel_tail(tail) or tail.shape != (B, taps.shape[0] - 1, 3 * d):
+                return None
+            if self.kind == "hcl":
+                st = state["poles"]
+                if st.dtype != torch.float32 or not st.is_contiguous() or st.shape[:2] != (B, d):
+                    return None
+                kind, operands = 1, (taps, tail, mix._lam(), seq._f32(mix.D), seq._f32(mix.residues), st)
+                sizes = (taps.shape[0], st.shape[2], 0)
+            else:
+                st = state["inner_tail"]
+                if not 2 <= inner.shape[0] <= 256 or not _kernel_tail(st) or st.shape != (B, inner.shape[0] - 1, d):
+                    return None
+                kind, operands = 0, (taps, tail, inner, seq._f32(mix.D), None, st)
+                sizes = (taps.shape[0], inner.shape[0], 0)
+            factors = (0.0, 0.0)
+        pre, post = self.pre_norm, self.post_norm
+        w_in, w_out, w1, w2, w3 = (_bf16_weight(m) for m in (first, mix.out_proj, mlp.l1, mlp.l2, mlp.l3))
+        ffn = w1[0].shape[0]
+        if w_in[0].shape != (3 * d, d) or w_out[0].shape != (d, d) or w1[0].shape != (ffn, d) or w2[0].shape != (ffn, d) or \
+                w3[0].shape != (d, ffn):
+            return None
+        return seq.decode_block(kind, x.view(B, d), (seq._f32(pre.scale), pre.eps), w_in, w_out, (seq._f32(post.scale), post.eps), w1,
+                                w2, w3, operands, sizes, factors)
+
     def step(self, x, state, linear=None, folded=None):
         if folded is not None and _decode_rows(self, x):
+            out = self._step_call(x, state, folded)
+            if out is not None:
+                return out
             return self._folded(x, state, self.mixer.step, folded)
         x = x + self.mixer.step(self.pre_norm(x), state, linear)
         return x + self.mlp(self.post_norm(x), linear)
@@ -571,6 +614,9 @@ class Block(nn.Module):
         r1 = x1.reshape(B * L, d)
         h = folded(self.mlp.l1, r1, gamma=self.post_norm.scale, eps=self.post_norm.eps, second=self.mlp.l2)
         return folded(self.mlp.l3, h, res=r1).view(B, L, d)
+
+
+_STEPS = (HyenaOperator.step, AttentionOperator.step)        # what Block._step_call stands for
 
 
 class StripedHyena2(nn.Module):
@@ -829,7 +875,6 @@ def folded_linear(module: nn.Linear, rows: torch.Tensor, gamma=None, eps: float 
     """A projection of the folded decode block on one GPU: rows [M <= 8, K] -> [M, N] on the weight-streaming
     kernel with RMSNorm (``gamma``) in front, the residual (``res``) behind and, with ``second``, the SwiGLU of
     two projections."""
-    from ..ops import seq
     if second is None and getattr(module, "fp8_weights", False) and rows.shape[-1] % 16 == 0:
         q, dq, b8 = _e4m3_weight(module)          # the prefill's e4m3 weights: half the bytes of the step
         return seq.gemv_rows(rows, q, b8, gamma=gamma, eps=eps, res=res, wscale=dq)
@@ -855,7 +900,6 @@ def fused_linear(module: nn.Linear, x: torch.Tensor, residual: Optional[torch.Te
         if r2.dtype != torch.bfloat16 or not r2.is_contiguous():
             r2 = r2.to(torch.bfloat16).contiguous()
     if x2.shape[0] <= 8:                      # decode rows: stream the weights once (memory bound)
-        from ..ops import seq
         return seq.gemv_rows(x2, w, b, res=r2).view(*x.shape[:-1], w.shape[0])
     return gemm.gemm(x2, w, bias=b, residual=r2).view(*x.shape[:-1], w.shape[0])
 

@@ -31,6 +31,16 @@ int ubm_attention_d32(const void* q, const void* k, const void* v, const void* b
 int ubm_attention_d64(const void* q, const void* k, const void* v, const void* bias, const void* gate, void* out,
                       const void* kmask, const void* kflags, int rows, int Nq, int Nk, int H, long long ldb, long long ld_in,
                       long long ld_gate, long long ld_mask, int transpose_out, void* status, void* stream);
+int ubm_gemv_fused(const void* x, const void* gamma, float eps, const void* w, const void* w2, const void* bias, const void* res,
+                   void* out, int M, int N, int K, void* stream);
+int ubm_fir_gate3(const void* z, const void* h, const void* tail, void* u, void* x2, int B, int L, int d, int K, int push,
+                  void* stream);
+int ubm_fir_step(const void* u, const void* h, const void* D, const void* x2, void* tail, void* out, int B, int d, int K,
+                 void* stream);
+int ubm_pole_step(void* state, const void* lam, const void* res, const void* u, const void* D, const void* x2, void* out, int B,
+                  int d, int S, void* stream);
+int ubm_decode_attention(const void* qkv, const void* pos, void* kc, void* vc, void* q_rot, void* part, void* out, int B, int H,
+                         int Lmax, int splits, float base, float scale, void* status, void* stream);
 int ubm_transition(const void* x, const void* wab, const void* wo, const void* ab_colsum, const void* ab_colbias, const void* o_bias,
                    const void* mask, void* out, long long R, int hidden, int add_residual, void* status, void* stream);
 int ubm_layernorm_rows(const void* x, const void* gamma, const void* beta, void* out, long long R, int C, float eps, int in_dtype,
@@ -244,4 +254,41 @@ extern "C" int ubm_transition_rows(const void* args) {
   rc = product(n, w12, h, nullptr, nullptr, R, 2 * hidden, dim, kActSwiglu, hidden, 0, nullptr, 0, 0, status, stream);
   if (rc) return rc;
   return product(h, w3, out, nullptr, residual, R, out_dim, hidden, 0, out_dim, 0, nullptr, 0, 0, status, stream);
+}
+
+// One decoding step of a block of the genomic decoder on B rows (at most 8): norm -> input projection -> operator -> output projection
+// + x -> norm -> SwiGLU of two projections -> third projection + residual.  kind: 0 = short and medium operator (two filters, tails
+// moved on in place), 1 = long operator (poles moved on in place), 2 = attention over a cache with its position in device memory.
+// work: z or q | k | v [B][n_in], a, b, c [B][d] (u, x2, gated; or rotated q, unused, o), r1 [B][d], h [B][ffn], part (attention), each
+// at its own pointer.
+extern "C" int ubm_decode_block(const void* args) {
+  Args a{static_cast<const char*>(args)};
+  const int kind = a.i32(), B = a.i32(), d = a.i32(), n_in = a.i32(), ffn = a.i32();
+  const void* x = a.ptr();
+  const void* gamma1 = a.ptr();
+  const float eps1 = a.f32();
+  const void *w_in = a.ptr(), *b_in = a.ptr(), *w_out = a.ptr(), *b_out = a.ptr(), *gamma2 = a.ptr();
+  const float eps2 = a.f32();
+  const void *w1 = a.ptr(), *b1 = a.ptr(), *w2 = a.ptr(), *w3 = a.ptr(), *b3 = a.ptr();
+  void *z = a.ptr(), *t0 = a.ptr(), *t1 = a.ptr(), *t2 = a.ptr(), *r1 = a.ptr(), *h = a.ptr(), *out = a.ptr();
+  const void* m[6];                    // kinds 0, 1: first filter, its tail, second filter / poles' factors, D, residues, state; 2: pos, k, v, part
+  for (const void*& q : m) q = a.ptr();
+  const int n0 = a.i32(), n1 = a.i32(), n2 = a.i32();     // kinds 0, 1: taps, taps or poles; 2: heads, cache rows, splits
+  const float f0 = a.f32(), f1 = a.f32();                 // 2: rotary base, score scale
+  void *status = a.ptr(), *stream = a.ptr();
+  if (!a.ok || kind > 2) return ubm::UBM_ERR_ARGUMENT;
+  int rc = ubm_gemv_fused(x, gamma1, eps1, w_in, nullptr, b_in, nullptr, z, B, n_in, d, stream);
+  if (rc == 0 && kind != 2) {
+    rc = ubm_fir_gate3(z, m[0], m[1], t0, t1, B, 1, d, n0, 1, stream);
+    if (rc == 0)
+      rc = kind == 0 ? ubm_fir_step(t0, m[2], m[3], t1, const_cast<void*>(m[5]), t2, B, d, n1, stream)
+                     : ubm_pole_step(const_cast<void*>(m[5]), m[2], m[4], t0, m[3], t1, t2, B, d, n1, stream);
+  } else if (rc == 0) {
+    rc = ubm_decode_attention(z, m[0], const_cast<void*>(m[1]), const_cast<void*>(m[2]), t0, const_cast<void*>(m[3]), t2, B, n0, n1,
+                              n2, f0, f1, status, stream);
+  }
+  if (rc == 0) rc = ubm_gemv_fused(t2, nullptr, 0.f, w_out, nullptr, b_out, x, r1, B, d, d, stream);
+  if (rc == 0) rc = ubm_gemv_fused(r1, gamma2, eps2, w1, w2, b1, nullptr, h, B, ffn, d, stream);
+  if (rc == 0) rc = ubm_gemv_fused(h, nullptr, 0.f, w3, nullptr, b3, r1, out, B, d, ffn, stream);
+  return rc;
 }

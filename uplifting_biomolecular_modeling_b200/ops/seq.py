@@ -30,6 +30,8 @@ native.declare("ubm_residual_ln", [c_void_p] * 6 + [c_ll, c_int, c_float, c_void
 
 native.declare("ubm_gemv_fused_packed", [ctypes.c_char_p])
 _GEMV_ARGS = struct.Struct("=11qd")      # the integer arguments of ubm_gemv_fused_packed in order, then eps
+native.declare("ubm_decode_block", [ctypes.c_char_p])
+_BLOCK_ARGS = struct.Struct("=7qd5qd21q2d2q")    # as ubm_decode_block reads them
 native.declare("ubm_gemv_fused_w8", [c_void_p] * 2 + [c_float, c_void_p, c_float] + [c_void_p] * 3 + [c_int] * 3 + [c_void_p])
 native.declare("ubm_rmsnorm_fp8", [c_void_p] * 5 + [c_ll, c_int, c_float, c_void_p])
 native.declare("ubm_qk_norm_rotary", [c_void_p] * 4 + [c_ll] + [c_int] * 3 + [c_float] * 2 + [c_void_p])
@@ -425,6 +427,40 @@ def decode_attention(qkv: torch.Tensor, pos: torch.Tensor, kc: torch.Tensor, vc:
                                            float(rope_base), sc, native.ptr(native.status_tensor(qkv.device)),
                                            _stream(qkv))
     native.check(rc, "ubm_decode_attention")
+    return out
+
+
+def decode_block(kind: int, x: torch.Tensor, norm1: tuple, w_in: tuple, w_out: tuple, norm2: tuple, w1: tuple, w2: tuple, w3: tuple,
+                 operands: tuple, sizes: tuple, factors: tuple = (0.0, 0.0)) -> torch.Tensor:
+    """One decoding step of a block from one call (``csrc/sequences_sm100.cu``: four weight-streaming projections and the operator
+    between them, the same launches as one by one).  x: bf16 [B <= 8, d] contiguous; norms as (fp32 gamma, eps); weights as (bf16 [N, K]
+    contiguous, fp32 bias or None); kind 0 / 1 / 2 with ``operands`` (tensors or None) and ``sizes`` as the library's comment lists
+    them.  States among the operands are moved on in place."""
+    B, d = x.shape
+    n_in, ffn = w_in[0].shape[0], w1[0].shape[0]
+    dev = x.device
+    part = 0
+    if kind == 2:
+        heads, _, splits = sizes
+        part = B * heads * splits * (128 + 2) * 4
+    wide, step, hid = (-(-2 * B * n // 64) * 64 for n in (n_in, d, ffn))        # rows of n bf16 values, on 64 bytes
+    scratch = torch.empty(wide + 4 * step + hid + part, dtype=torch.uint8, device=dev)
+    z = scratch.data_ptr()
+    t0 = z + wide
+    h = t0 + 4 * step
+    out = torch.empty((B, 1, d), dtype=torch.bfloat16, device=dev)
+    ptr = native.ptr
+    names = [ptr(t) for t in operands]
+    if kind == 2:
+        names.append(h + hid)
+    names += [0] * (6 - len(names))
+    for name in ("ubm_decode_attention",) if kind == 2 else ("ubm_fir_gate3", "ubm_fir_step" if kind == 0 else "ubm_pole_step"):
+        native.add_launches(1, name)
+    rc = native.lib().ubm_decode_block(_BLOCK_ARGS.pack(
+        kind, B, d, n_in, ffn, x.data_ptr(), ptr(norm1[0]), norm1[1], ptr(w_in[0]), ptr(w_in[1]), ptr(w_out[0]), ptr(w_out[1]),
+        ptr(norm2[0]), norm2[1], ptr(w1[0]), ptr(w1[1]), ptr(w2[0]), ptr(w3[0]), ptr(w3[1]), z, t0, t0 + step, t0 + 2 * step,
+        t0 + 3 * step, h, out.data_ptr(), *names, *sizes, *factors, native.status_tensor(dev).data_ptr(), _stream(x)))
+    native.check(rc, "ubm_decode_block")
     return out
 
 
