@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(256) decode_qkv_kernel(const __nv_bfloat16* __
                                                          __nv_bfloat16* __restrict__ q_out,
                                                          __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
                                                          int B, int H, int Lmax, float base, KernelStatus* status) {
+  grid_dependency_sync(true);
   const long long pos = *pos_ptr;
   if (pos < 0 || pos >= Lmax) {                 // a full cache: nothing is written, the host reads the word
     if (blockIdx.x == 0 && threadIdx.x == 0 && atomicCAS(&status->code, 0u, 3u) == 0u) {
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_kernel(const __nv_bfl
                                                                   const long long* __restrict__ pos_ptr,
                                                                   float* __restrict__ part, int H, int Lmax, int chunk,
                                                                   float scale_log2e) {
+  grid_dependency_sync(true);
   __shared__ float s_acc[kDecThreads / 16][kDecHd];
   __shared__ float s_m[kDecThreads / 16], s_l[kDecThreads / 16];
   const int s = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
@@ -182,7 +184,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_attn_kernel(const __nv_bfl
 __global__ void __launch_bounds__(kDecHd) decode_merge_kernel(const float* __restrict__ part,
                                                               __nv_bfloat16* __restrict__ out, int H, int S) {
   const int h = blockIdx.x, b = blockIdx.y;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the projection behind may prefetch its weights
+  grid_dependency_sync(true);   // the projection behind may prefetch its weights
   const float* rec = part + (static_cast<long long>(b) * H + h) * S * kDecRec;
   float M = -INFINITY;
   for (int s = 0; s < S; ++s) M = fmaxf(M, rec[s * kDecRec + kDecHd]);
@@ -214,17 +216,17 @@ extern "C" int ubm_decode_attention(const void* qkv, const void* pos, void* kc, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int chunk = (Lmax + splits - 1) / splits;
   const int total = B * H * (kDecHd / 2);
-  decode_qkv_kernel<<<(total + 255) / 256, 256, 0, st>>>(
+  launch_after(true, decode_qkv_kernel, (total + 255) / 256, 256, 0, st,
       static_cast<const __nv_bfloat16*>(qkv), static_cast<const long long*>(pos), static_cast<__nv_bfloat16*>(q_rot),
       static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), B, H, Lmax, rope_base,
       static_cast<KernelStatus*>(status));
   UBM_CHECK_LAUNCH("decode_qkv_kernel");
-  decode_attn_kernel<<<dim3(splits, H, B), kDecThreads, 0, st>>>(
+  launch_after(true, decode_attn_kernel, dim3(splits, H, B), kDecThreads, 0, st,
       static_cast<const __nv_bfloat16*>(q_rot), static_cast<const __nv_bfloat16*>(kc),
       static_cast<const __nv_bfloat16*>(vc), static_cast<const long long*>(pos), static_cast<float*>(part), H, Lmax,
       chunk, scale * 1.4426950408889634f);
   UBM_CHECK_LAUNCH("decode_attn_kernel");
-  decode_merge_kernel<<<dim3(H, B), kDecHd, 0, st>>>(static_cast<const float*>(part), static_cast<__nv_bfloat16*>(out),
+  launch_after(true, decode_merge_kernel, dim3(H, B), kDecHd, 0, st, static_cast<const float*>(part), static_cast<__nv_bfloat16*>(out),
                                                      H, splits);
   UBM_CHECK_LAUNCH("decode_merge_kernel");
   return UBM_OK;

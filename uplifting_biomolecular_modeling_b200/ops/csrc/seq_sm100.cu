@@ -42,11 +42,14 @@ __device__ __forceinline__ uint4 pack8(const float (&e)[8]) {
 
 // ------------------------------------------------------------------------------------------ RMSNorm
 // one warp per row, the row read once (kept in registers for C <= 8192: up to 32 chunks of 8 per lane)
+constexpr long long kRmsDecodeRows = 64;   // few rows: launched to overlap the kernel in front
+
 template <int CHUNKS>
 __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const __nv_bfloat16* __restrict__ x,
                                                            const float* __restrict__ scale,
                                                            __nv_bfloat16* __restrict__ out, long long R, int C,
                                                            float eps) {
+  if (R <= kRmsDecodeRows) grid_dependency_sync(true);
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (long long r = static_cast<long long>(blockIdx.x) * wpb + (threadIdx.x >> 5); r < R;
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(128) fir_gate3_kernel(const __nv_bfloat16* __r
                                                         __nv_bfloat16* tail,  // [B][K-1][3d] or null
                                                         __nv_bfloat16* __restrict__ u, __nv_bfloat16* __restrict__ x2,
                                                         int B, int L, int d, int push) {
+  if (push) grid_dependency_sync(true);   // the decode form is launched to overlap the projection in front
   constexpr int KW = K > 1 ? K - 1 : 1;
   const int c2 = d / 2;
   const int runs = (L + kFirTL - 1) / kFirTL;
@@ -295,7 +299,7 @@ __global__ void __launch_bounds__(256) fir_step_kernel(const __nv_bfloat16* __re
                                                        __nv_bfloat16* tail,                     // [B][K-1][d]
                                                        __nv_bfloat16* __restrict__ out, int d) {
   __shared__ float part[32][8][8];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the projection behind may prefetch its weights
+  grid_dependency_sync(true);   // the projection behind may prefetch its weights
   const int cg = threadIdx.x & 7;
   const int rg = threadIdx.x >> 3;
   const int b = blockIdx.y;
@@ -629,7 +633,7 @@ __global__ void __launch_bounds__(256) pole_step_kernel(float* __restrict__ stat
                                                         const __nv_bfloat16* __restrict__ x2,
                                                         __nv_bfloat16* __restrict__ out, int B, int d, int S) {
   const long long total = static_cast<long long>(B) * d;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the projection behind may prefetch its weights
+  grid_dependency_sync(true);   // the projection behind may prefetch its weights
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int c = static_cast<int>(i % d);
@@ -992,9 +996,9 @@ extern "C" int ubm_rmsnorm_rows(const void* x, const void* scale, void* out, lon
   const __nv_bfloat16* xx = static_cast<const __nv_bfloat16*>(x);
   const float* sc = static_cast<const float*>(scale);
   __nv_bfloat16* oo = static_cast<__nv_bfloat16*>(out);
-  if (C <= 1024) rmsnorm_rows_kernel<4><<<grid, 256, 0, st>>>(xx, sc, oo, R, C, eps);
-  else if (C <= 2048) rmsnorm_rows_kernel<8><<<grid, 256, 0, st>>>(xx, sc, oo, R, C, eps);
-  else if (C <= 4096) rmsnorm_rows_kernel<16><<<grid, 256, 0, st>>>(xx, sc, oo, R, C, eps);
+  if (C <= 1024) launch_after(R <= kRmsDecodeRows, rmsnorm_rows_kernel<4>, grid, 256, 0, st, xx, sc, oo, R, C, eps);
+  else if (C <= 2048) launch_after(R <= kRmsDecodeRows, rmsnorm_rows_kernel<8>, grid, 256, 0, st, xx, sc, oo, R, C, eps);
+  else if (C <= 4096) launch_after(R <= kRmsDecodeRows, rmsnorm_rows_kernel<16>, grid, 256, 0, st, xx, sc, oo, R, C, eps);
   else rmsnorm_rows_wide_kernel<<<grid, 256, 0, st>>>(xx, sc, oo, R, C, eps);
   UBM_CHECK_LAUNCH("rmsnorm_rows_kernel");
   return UBM_OK;
@@ -1039,7 +1043,7 @@ extern "C" int ubm_fir_gate3(const void* z, const void* ht, void* tail, void* u,
   if ((total + 127) / 128 > 0x7fffffffLL) return UBM_ERR_TOO_LARGE;
   const unsigned grid = static_cast<unsigned>((total + 127) / 128);
 #define UBM_FG3(KK)                                                                                            \
-  fir_gate3_kernel<KK><<<grid, 128, 0, st>>>(static_cast<const __nv_bfloat16*>(z), static_cast<const float*>(ht), \
+  launch_after(push != 0, fir_gate3_kernel<KK>, grid, 128, 0, st, static_cast<const __nv_bfloat16*>(z), static_cast<const float*>(ht), \
                                              static_cast<__nv_bfloat16*>(tail),                                 \
                                              static_cast<__nv_bfloat16*>(u), static_cast<__nv_bfloat16*>(x2), B, L, d, \
                                              push)
@@ -1105,7 +1109,7 @@ extern "C" int ubm_fir_step(const void* u, const void* ht, const void* D, const 
   if (B <= 0 || B > 65535 || d <= 0 || (d & 7) || K < 2 || K > 32 * kFirStepMaxTapsPerThread || tail == nullptr)
     return UBM_ERR_ARGUMENT;
   const dim3 grid((d + 63) / 64, B);
-  fir_step_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_after(true, fir_step_kernel, grid, 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(u), static_cast<const float*>(ht), K, static_cast<const float*>(D),
       static_cast<const __nv_bfloat16*>(x2), static_cast<__nv_bfloat16*>(tail), static_cast<__nv_bfloat16*>(out), d);
   UBM_CHECK_LAUNCH("fir_step_kernel");
@@ -1146,7 +1150,7 @@ extern "C" int ubm_spectrum_mul(void* X, const void* H, int B, long long per_bat
 extern "C" int ubm_pole_step(void* state, const void* lam, const void* res, const void* u, const void* D,
                              const void* x2, void* out, int B, int d, int S, void* stream) {
   if (B <= 0 || d <= 0 || S <= 0) return UBM_ERR_ARGUMENT;
-  pole_step_kernel<<<seq_grid(static_cast<long long>(B) * d, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_after(true, pole_step_kernel, seq_grid(static_cast<long long>(B) * d, 256), 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<float*>(state), static_cast<const float*>(lam), static_cast<const float*>(res),
       static_cast<const __nv_bfloat16*>(u), static_cast<const float*>(D), static_cast<const __nv_bfloat16*>(x2),
       static_cast<__nv_bfloat16*>(out), B, d, S);
@@ -1308,21 +1312,21 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_rows_kernel(
   // rows go to the warps CTA by CTA (dealing them round-robin over the CTAs for an even row count per SM measured
   // slower: 27.5 against 26.7 us for 4096 -> 12288 and 4.2 against 3.5 ms for the whole decode step)
   const int n_first = blockIdx.x * wpb + warp;
-  // the first weight row of this warp starts towards L2 while x^ is staged
-  if (n_first < N) {
+  // The first 2 KB of this warp's first weight row (of each matrix 1 KB) start towards L2 while x^ is staged.  More of it only holds
+  // up what the warps ask for next: whole rows 78.3, 4 KB 74.0, 2 KB 71.6, 1 KB 72.6, nothing 75.9 us for the four projections
+  // of a block (405 MB, one decode row, launch behind launch).
+  constexpr int kAhead = DUAL ? 1024 : 2048;
+  if (n_first < N && lane * 128 < kAhead) {
     const char* p0 = reinterpret_cast<const char*>(w) + static_cast<long long>(n_first) * K * wbytes;
-    for (int o = lane * 128; o < K * wbytes; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p0 + o));
-    if (DUAL) {
-      const char* p1 = reinterpret_cast<const char*>(w2 + static_cast<long long>(n_first) * K);
-      for (int o = lane * 128; o < K * 2; o += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p1 + o));
-    }
+    if (lane * 128 < K * wbytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(p0 + lane * 128));
+    if (DUAL && lane * 128 < K * 2)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(w2 + static_cast<long long>(n_first) * K) + lane * 128));
   }
   // Programmatic dependent launch: the prefetch above read only weights, so this CTA may have started while the
-  // previous kernel of the stream drains; x, the residual and the output are touched from here on.  The kernel
-  // behind this one may start its own prefetch as soon as every CTA here has passed this point.  Both
-  // instructions are no-ops for a launch without the attribute.
+  // previous kernel of the stream drains; x, the residual and the output are touched from here on.  The kernel behind this
+  // one is not let in before this one's CTAs leave: its prefetch would take bandwidth from the rows still being read (71.6
+  // us against 69.8).
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // ---- stage x^
   if (gamma != nullptr) {
     float ss[MB];
@@ -1486,7 +1490,8 @@ __global__ void __launch_bounds__(kGemvThreads) gemv_rows_kernel(
 // behind launch with weights from memory (600 MB of them in rotation; each launch's prefetch runs under the one before): one decode
 // row 18.6 / 21.4, 33.4 / 35.5, 17.2 / 17.3, 7.1 / 7.3; two 21.4 / 21.0, 36.4 / 35.1, 20.8 / 17.3, 8.0 / 7.4; four 32.7 / 22.7, 48.0 /
 // 36.9, 29.5 / 17.4, 11.5 / 7.4; eight 57.2 / 25.4, 100 / 40.0, 60.3 / 17.7, 20.2 / 7.2.  One row stays with the FMAs, which lose
-// nowhere.  (A launch by itself with a cold L2, start and end included, takes 8 us more: 26.7 for the first shape.)
+// nowhere.  (With whole rows prefetched; as it is, one row by the FMAs 17.1, 31.0, 15.7, 7.0, here two rows 20.4, 34.2, 16.5, 7.8 and
+// eight 24.2, 38.2, 16.8, 7.8.  A launch by itself with a cold L2, start and end included, takes 8 us more: 26.7 for the first shape.)
 constexpr int kGemvMmaMinRows = 2;
 constexpr int kGemvMmaThreads = 256;
 constexpr int kGemvMmaWarps = kGemvMmaThreads / 32;
@@ -1515,21 +1520,21 @@ __global__ void __launch_bounds__(kGemvMmaThreads, 2) gemv_mma_kernel(
   const size_t row_bytes = static_cast<size_t>(K) * 2;
   const size_t xs_stride = row_bytes + 16;    // the reads of two decode rows fall into different halves of the banks
   {
-    // the first tile starts towards L2 before the kernel waits for the one in front of it
+    // the first KB of each row of the first tile starts towards L2 before the kernel waits for the one in front of it (the four
+    // projections of a block, two / eight rows: whole rows 82.5 / 89.7 us, 4 KB 78.7 / 87.3, 2 KB 78.6 / 87.1, 1 KB 78.0 / 86.0)
     const int n0 = blockIdx.x * 16;
     for (int r = warp; r < 16; r += kGemvMmaWarps) {
       if (n0 + r < N) {
         const char* p0 = reinterpret_cast<const char*>(w) + (n0 + r) * row_bytes;
         const char* p1 = reinterpret_cast<const char*>(w2) + (n0 + r) * row_bytes;
-        for (size_t o = lane * 128; o < row_bytes; o += 32 * 128) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(p0 + o));
-          if (DUAL) asm volatile("prefetch.global.L2 [%0];" ::"l"(p1 + o));
+        if (lane < 8 && lane * 128 < row_bytes) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p0 + lane * 128));
+          if (DUAL) asm volatile("prefetch.global.L2 [%0];" ::"l"(p1 + lane * 128));
         }
       }
     }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");      // see the kernel above
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (STAGED) {
     const int wpr = M == 2 ? 4 : M <= 4 ? 2 : 1;           // warps per decode row
     const int b = warp / wpr, in_row = (warp - b * wpr) * 32 + lane, step = wpr * 32, nv = K >> 3;
