@@ -455,6 +455,46 @@ class PairformerLayer(nn.Module):
         x = max(1, self.transition_z.hidden // 128)
         return tm, tm, ta, ta, (f"C128X{x}", {"c": 128, "expansion": self.transition_z.hidden // 128, "dtype": "bf16"}, "tcgen05_fused")
 
+    def _single_track(self, s: torch.Tensor, z: torch.Tensor, mask: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+        """The single track from one call of the library, or None where a call of its operators would do anything else (as
+        :meth:`_pair_track`; other widths of the norm, an autocast region and recorded gradients among it)."""
+        at = self._modules
+        attn, tr, norm = at.get("attention"), at.get("transition_s"), at.get("pre_norm_s")
+        if getattr(type(attn), "forward", None) is not AttentionPairBias.forward or \
+                getattr(type(tr), "forward", None) is not Transition.forward or _any_global_hook():
+            return None
+        N, c = s.shape[-2], s.shape[-1]
+        da, dt = attn.__dict__, tr.__dict__
+        for m, d in ((attn, da), (tr, dt)):
+            gate = dispatch.size_gate(m.lever)
+            if d["impl"] != "fused" or "forward" in d or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or \
+                    d["_backward_pre_hooks"] or N < gate.min_tokens or (gate.max_tokens is not None and N > gate.max_tokens):
+                return None
+        if type(da["_packed"]) is not pair.ApbPacked or type(dt["_packed"]) is not tuple or tr.hidden % 32 or tr.dim != c or \
+                tr.out_dim != c or not da["compute_pair_bias"] or "pair_bias" in da or "_fused_forward" in da or \
+                type(attn)._fused_forward is not AttentionPairBias._fused_forward or \
+                type(attn).pair_bias is not AttentionPairBias.pair_bias or da["c_s"] != c or type(norm) is not nn.LayerNorm or \
+                norm.weight is None:
+            return None
+        if s.dim() != 3 or s.shape[0] != 1 or s.dtype != torch.bfloat16 or not s.is_contiguous() or s.data_ptr() % 16 or c % 8 or \
+                c > 1024 or z.shape != (1, N, N, 128) or z.dtype != torch.bfloat16 or not z.is_cuda or not z.is_contiguous() or \
+                s.device != z.device or attn.proj_q.weight.dtype != torch.bfloat16 or tr.norm.weight.dtype != torch.bfloat16 or \
+                attn.heads not in (4, 8, 16, 32):
+            return None
+        if mask is not None and (mask.shape != (1, N) or mask.device != s.device or
+                                 mask.dtype not in (torch.float32, torch.bfloat16, torch.bool, torch.uint8)):
+            return None
+        if torch.is_autocast_enabled("cuda") or (torch.is_grad_enabled() and (s.requires_grad or norm.weight.requires_grad)):
+            return None
+        w = da["_packed"]
+        attn._decide(None, f"D{w.Dp}H{attn.heads}S1", N, {"head_dim": w.Dp, "dtype": "bf16"})
+        tr._decide(None, f"C{c}X{max(1, tr.hidden // c)}", N, {"c": c, "expansion": tr.hidden // c, "dtype": "bf16"}, "rows_gemm")
+        ln, lin = attn.proj_z[0], attn.proj_z[1]
+        n2 = tr.norm
+        return pair.single_track(s, z, mask, (rows._f32_param(norm.weight), rows._f32_param(norm.bias), 1e-5),
+                                 rows._head_bias_weights(lin.weight, ln.weight, ln.bias, BiasPlanes.LOG2E, z.device), w,
+                                 (rows._f32_param(n2.weight), rows._f32_param(n2.bias), n2.eps), *dt["_packed"])
+
     def pair_update(self, z: torch.Tensor, pair_mask: Optional[torch.Tensor]) -> torch.Tensor:
         out = self._pair_track(z, pair_mask)
         if out is not None:
@@ -471,6 +511,9 @@ class PairformerLayer(nn.Module):
         z = self.pair_update(z, pair_mask)
         if self.no_seq:
             return s, z
+        out = self._single_track(s, z, mask)
+        if out is not None:
+            return out, z
         # single track in fp32, as upstream (pairformer.py:103-111)
         s32 = s.float()
         norm = self.pre_norm_s

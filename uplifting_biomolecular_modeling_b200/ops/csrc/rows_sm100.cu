@@ -8,6 +8,7 @@
 //   ubm_adaln_rows       sigmoid(scale[r]) * LN_noaffine(a[r]) + shift[r]   (DiT AdaLN)
 //   ubm_gate_residual    out = res + sigmoid(gate) * x
 //   ubm_swiglu_rows      out = silu(a) * b for a | b halves of one row
+//   ubm_single_add/_out  the two fp32 sums of the single track with their roundings
 // Reference for the last three: _ln_mod_kernel / _gate_res_kernel / _swiglu_kernel in
 // common/opt_core/opt_core/kernels/dtk_kernels.py.
 #include "host_util.h"
@@ -576,6 +577,46 @@ __global__ void __launch_bounds__(256) swiglu3_rows_kernel(const __nv_bfloat16* 
   }
 }
 
+// The single track's two sums; see the entry points.  Bound by their launches (105 KB at 137 tokens x 384 channels): each takes the place
+// of two or three of conversions and sums, and is part of the one call whose figures stand at ubm_single_track.  Eight elements a thread.
+__global__ void __launch_bounds__(256) single_add_kernel(const __nv_bfloat16* __restrict__ s, const __nv_bfloat16* __restrict__ upd,
+                                                         float* __restrict__ s32, __nv_bfloat16* __restrict__ rounded,
+                                                         long long vecs) {
+  grid_dependency_sync(true);
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < vecs;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const uint4 a = reinterpret_cast<const uint4*>(s)[i], b = reinterpret_cast<const uint4*>(upd)[i];
+    const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
+    float f[8];
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f[2 * j] = bf16_lo(wa[j]) + bf16_lo(wb[j]);
+      f[2 * j + 1] = bf16_hi(wa[j]) + bf16_hi(wb[j]);
+      o[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
+    }
+    reinterpret_cast<float4*>(s32)[2 * i] = make_float4(f[0], f[1], f[2], f[3]);
+    reinterpret_cast<float4*>(s32)[2 * i + 1] = make_float4(f[4], f[5], f[6], f[7]);
+    reinterpret_cast<uint4*>(rounded)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+__global__ void __launch_bounds__(256) single_out_kernel(const float* __restrict__ s32, const __nv_bfloat16* __restrict__ upd,
+                                                         __nv_bfloat16* __restrict__ out, long long vecs) {
+  grid_dependency_sync(true);
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < vecs;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const float4 a = reinterpret_cast<const float4*>(s32)[2 * i], c = reinterpret_cast<const float4*>(s32)[2 * i + 1];
+    const uint4 b = reinterpret_cast<const uint4*>(upd)[i];
+    reinterpret_cast<uint4*>(out)[i] =
+        make_uint4(pack_bf16x2(a.x + bf16_lo(b.x), a.y + bf16_hi(b.x)), pack_bf16x2(a.z + bf16_lo(b.y), a.w + bf16_hi(b.y)),
+                   pack_bf16x2(c.x + bf16_lo(b.z), c.y + bf16_hi(b.z)), pack_bf16x2(c.z + bf16_lo(b.w), c.w + bf16_hi(b.w)));
+  }
+}
+
+static inline bool aligned_16(const void* a, const void* b) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
 static inline int grid_for(long long work, int per_block) {
   long long b = (work + per_block - 1) / per_block;
   const long long cap = static_cast<long long>(sm_count()) * 16;
@@ -714,6 +755,43 @@ extern "C" int ubm_layernorm_rows(const void* x, const void* gamma, const void* 
 #undef UBM_LN_BY_WIDTH
 #undef UBM_LN_LAUNCH
   UBM_CHECK_LAUNCH("layernorm_rows_kernel");
+  return UBM_OK;
+}
+
+// bf16 rows normalised in the order of sums that fp32 rows are (the single track's fp32 copy of them holds the same values)
+extern "C" int ubm_layernorm_rows_as_f32(const void* x, const void* gamma, const void* beta, void* out, long long R, int C, float eps,
+                                         void* stream) {
+  using namespace ubm;
+  if (R <= 0 || C <= 0 || C > 1024) return UBM_ERR_ARGUMENT;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto kernel = C <= 128   ? layernorm_rows_kernel<__nv_bfloat16, __nv_bfloat16, 4>
+                : C <= 256 ? layernorm_rows_kernel<__nv_bfloat16, __nv_bfloat16, 8>
+                : C <= 512 ? layernorm_rows_kernel<__nv_bfloat16, __nv_bfloat16, 16>
+                           : layernorm_rows_kernel<__nv_bfloat16, __nv_bfloat16, 32>;
+  launch_after(short_rows(R, C), kernel, grid_for(R, 8), 256, 0, st, static_cast<const __nv_bfloat16*>(x),
+               static_cast<const float*>(gamma), static_cast<const float*>(beta), static_cast<__nv_bfloat16*>(out), R, C, eps);
+  UBM_CHECK_LAUNCH("layernorm_rows_kernel");
+  return UBM_OK;
+}
+
+// s32 = s + upd in fp32 and its bf16 rounding: the single track behind its attention.  n: elements, a multiple of 8; all on 16 bytes.
+extern "C" int ubm_single_add(const void* s, const void* upd, void* s32, void* rounded, long long n, void* stream) {
+  using namespace ubm;
+  if (n <= 0 || (n & 7) || !aligned_16(s, upd) || !aligned_16(s32, rounded)) return UBM_ERR_ARGUMENT;
+  launch_after(true, single_add_kernel, grid_for(n / 8, 256), 256, 0, static_cast<cudaStream_t>(stream),
+               static_cast<const __nv_bfloat16*>(s), static_cast<const __nv_bfloat16*>(upd), static_cast<float*>(s32),
+               static_cast<__nv_bfloat16*>(rounded), n / 8);
+  UBM_CHECK_LAUNCH("single_add_kernel");
+  return UBM_OK;
+}
+
+// out = s32 + upd, rounded to bf16
+extern "C" int ubm_single_out(const void* s32, const void* upd, void* out, long long n, void* stream) {
+  using namespace ubm;
+  if (n <= 0 || (n & 7) || !aligned_16(s32, upd) || !aligned_16(out, out)) return UBM_ERR_ARGUMENT;
+  launch_after(true, single_out_kernel, grid_for(n / 8, 256), 256, 0, static_cast<cudaStream_t>(stream),
+               static_cast<const float*>(s32), static_cast<const __nv_bfloat16*>(upd), static_cast<__nv_bfloat16*>(out), n / 8);
+  UBM_CHECK_LAUNCH("single_out_kernel");
   return UBM_OK;
 }
 

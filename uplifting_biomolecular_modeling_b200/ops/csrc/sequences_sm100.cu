@@ -41,6 +41,12 @@ int ubm_pole_step(void* state, const void* lam, const void* res, const void* u, 
                   int d, int S, void* stream);
 int ubm_decode_attention(const void* qkv, const void* pos, void* kc, void* vc, void* q_rot, void* part, void* out, int B, int H,
                          int Lmax, int splits, float base, float scale, void* status, void* stream);
+int ubm_layernorm_rows_as_f32(const void* x, const void* gamma, const void* beta, void* out, long long R, int C, float eps,
+                              void* stream);
+int ubm_pair_head_bias(const void* z, const void* w, const void* colsum, const void* colbias, void* out, int N, int Np, int H,
+                       int transpose_out, void* stream);
+int ubm_single_add(const void* s, const void* upd, void* s32, void* rounded, long long n, void* stream);
+int ubm_single_out(const void* s32, const void* upd, void* out, long long n, void* stream);
 int ubm_transition(const void* x, const void* wab, const void* wo, const void* ab_colsum, const void* ab_colbias, const void* o_bias,
                    const void* mask, void* out, long long R, int hidden, int add_residual, void* status, void* stream);
 int ubm_layernorm_rows(const void* x, const void* gamma, const void* beta, void* out, long long R, int C, float eps, int in_dtype,
@@ -137,6 +143,40 @@ int triatt(const void* z, const Keep& keep, void* add, void* flags, long long ld
                  stream);
 }
 
+bool apb_sizes(int B, int N, int H, int Dp) {
+  return B > 0 && N > 0 && (Dp == 32 || Dp == 64) && H > 0 && H <= 1024 && static_cast<long long>(B) * N <= 0x7fffffffLL;
+}
+
+// key mask -> q | k | v | gate projection -> attention -> output projection
+int apb(const void* x, const void* wqkvg, const void* bqkvg, const void* wo, const void* planes, long long ldb, const Keep& keep,
+        void* add, void* flags, long long ld_mask, const void* gate, long long ld_gate, int gate_rows, const void* residual, void* qkvg,
+        void* o, void* out, int B, int N, int c, int c_out, int H, int Dp, void* status, void* stream) {
+  const int M = B * N, HD = H * Dp;
+  int rc;
+  if (keep.ptr != nullptr) {
+    rc = ubm_key_mask(keep.ptr, keep.bytes, keep.row, keep.key, add, flags, B, N, stream);
+    if (rc) return rc;
+  }
+  rc = product(x, wqkvg, qkvg, bqkvg, nullptr, M, 4 * HD, c, kActSigmoid, 4 * HD, 3 * HD, nullptr, 0, 0, status, stream);
+  if (rc) return rc;
+  const uint16_t* q = static_cast<const uint16_t*>(qkvg);
+  rc = (Dp == 32 ? ubm_attention_d32 : ubm_attention_d64)(q, q + HD, q + 2 * HD, planes, q + 3 * HD, o, add, flags, B, N, N, H, ldb,
+                                                          4ll * HD, 4ll * HD, ld_mask, 0, status, stream);
+  if (rc) return rc;
+  return product(o, wo, out, nullptr, residual, M, c_out, HD, 0, c_out, 0, gate, ld_gate, gate_rows, status, stream);
+}
+
+// norm rows -> hidden product with SwiGLU -> output product
+int transition_rows(const void* x, const void* gamma, const void* beta, float eps, const void* w12, const void* w3,
+                    const void* residual, void* n, void* h, void* out, int R, int dim, int hidden, int out_dim, void* status,
+                    void* stream) {
+  int rc = ubm_layernorm_rows(x, gamma, beta, n, R, dim, eps, 0, 0, stream);
+  if (rc) return rc;
+  rc = product(n, w12, h, nullptr, nullptr, R, 2 * hidden, dim, kActSwiglu, hidden, 0, nullptr, 0, 0, status, stream);
+  if (rc) return rc;
+  return product(h, w3, out, nullptr, residual, R, out_dim, hidden, 0, out_dim, 0, nullptr, 0, 0, status, stream);
+}
+
 bool square(int N) { return N > 0 && static_cast<long long>(N) * N <= 0x7fffffffLL; }
 
 }  // namespace
@@ -202,16 +242,18 @@ extern "C" int ubm_pair_track(const void* args) {
   return rc;
 }
 
-// Attention with pair bias over B batch entries of N rows (key mask as above): q | k | v | gate projection -> attention -> output projection (times the gate's
-// rows and plus the residual, where given).  x: bf16 [B * N][c]; qkvg: bf16 [B * N][4 H Dp]; o: bf16 [B * N][H Dp]; out: bf16
-// [B * N][c_out]; planes: bf16 [H][N][ldb].
+// Attention with pair bias over B batch entries of N rows (key mask as above): q | k | v | gate projection -> attention -> output
+// projection (times the gate's rows and plus the residual, where given).  x: bf16 [B * N][c]; qkvg: bf16 [B * N][4 H Dp]; o: bf16
+// [B * N][H Dp]; out: bf16 [B * N][c_out]; planes: bf16 [H][N][ldb].
 extern "C" int ubm_apb(const void* args) {
   Args a{static_cast<const char*>(args)};
   const void *x = a.ptr(), *wqkvg = a.ptr(), *bqkvg = a.ptr(), *wo = a.ptr(), *planes = a.ptr();
   const long long ldb = a.i64();
-  const void* keep = a.ptr();
-  const int keep_bytes = a.i32();
-  const long long keep_row = a.i64(), keep_key = a.i64();
+  Keep keep{};
+  keep.ptr = a.ptr();
+  keep.bytes = a.i32();
+  keep.row = a.i64();
+  keep.key = a.i64();
   void *add = a.ptr(), *flags = a.ptr();
   const long long ld_mask = a.i64();
   const void* gate = a.ptr();
@@ -221,21 +263,9 @@ extern "C" int ubm_apb(const void* args) {
   void *qkvg = a.ptr(), *o = a.ptr(), *out = a.ptr();
   const int B = a.i32(), N = a.i32(), c = a.i32(), c_out = a.i32(), H = a.i32(), Dp = a.i32();
   void *status = a.ptr(), *stream = a.ptr();
-  if (!a.ok || B <= 0 || N <= 0 || (Dp != 32 && Dp != 64) || H <= 0 || H > 1024 || static_cast<long long>(B) * N > 0x7fffffffLL)
-    return ubm::UBM_ERR_ARGUMENT;
-  const int M = B * N, HD = H * Dp;
-  int rc;
-  if (keep != nullptr) {
-    rc = ubm_key_mask(keep, keep_bytes, keep_row, keep_key, add, flags, B, N, stream);
-    if (rc) return rc;
-  }
-  rc = product(x, wqkvg, qkvg, bqkvg, nullptr, M, 4 * HD, c, kActSigmoid, 4 * HD, 3 * HD, nullptr, 0, 0, status, stream);
-  if (rc) return rc;
-  const uint16_t* q = static_cast<const uint16_t*>(qkvg);
-  rc = (Dp == 32 ? ubm_attention_d32 : ubm_attention_d64)(q, q + HD, q + 2 * HD, planes, q + 3 * HD, o, add, flags, B, N, N, H, ldb,
-                                                          4ll * HD, 4ll * HD, ld_mask, 0, status, stream);
-  if (rc) return rc;
-  return product(o, wo, out, nullptr, residual, M, c_out, HD, 0, c_out, 0, gate, ld_gate, gate_rows, status, stream);
+  if (!a.ok || !apb_sizes(B, N, H, Dp)) return ubm::UBM_ERR_ARGUMENT;
+  return apb(x, wqkvg, bqkvg, wo, planes, ldb, keep, add, flags, ld_mask, gate, ld_gate, gate_rows, residual, qkvg, o, out, B, N, c,
+             c_out, H, Dp, status, stream);
 }
 
 // SwiGLU transition of widths without a kernel of their own: norm rows -> hidden product (SwiGLU in its epilogue) -> output product.  x:
@@ -249,11 +279,44 @@ extern "C" int ubm_transition_rows(const void* args) {
   const int R = a.i32(), dim = a.i32(), hidden = a.i32(), out_dim = a.i32();
   void *status = a.ptr(), *stream = a.ptr();
   if (!a.ok || R <= 0 || hidden <= 0 || hidden > 0x3fffffff) return ubm::UBM_ERR_ARGUMENT;
-  int rc = ubm_layernorm_rows(x, gamma, beta, n, R, dim, eps, 0, 0, stream);
+  return transition_rows(x, gamma, beta, eps, w12, w3, residual, n, h, out, R, dim, hidden, out_dim, status, stream);
+}
+
+// The single track of a Pairformer layer: s + attention with pair bias of its norm, then + transition, sums in fp32.  Its kernels are
+// of 2 to 9 us at 137 tokens and their set-up by separate calls takes longer: a layer took 268 us so, 247 from this one.  s, out: bf16 [N][c];
+// z: bf16 [N][N][128]; planes: bf16 [H][N][ldb] scratch; mask: [N] or null (its layout into add / flags); n: bf16 [N][c]; qkvg, o
+// as above; upd: bf16 [N][c]; s32: fp32 [N][c]; x: bf16 [N][c]; h: bf16 [N][hidden].
+extern "C" int ubm_single_track(const void* args) {
+  Args a{static_cast<const char*>(args)};
+  const void *s = a.ptr(), *z = a.ptr();
+  const void *gamma1 = a.ptr(), *beta1 = a.ptr(), *wb = a.ptr(), *wb_colsum = a.ptr(), *wb_colbias = a.ptr();
+  const void *wqkvg = a.ptr(), *bqkvg = a.ptr(), *wo = a.ptr();
+  const void *gamma2 = a.ptr(), *beta2 = a.ptr(), *w12 = a.ptr(), *w3 = a.ptr();
+  const float eps1 = a.f32(), eps2 = a.f32();
+  Keep keep{};
+  keep.ptr = a.ptr();
+  keep.bytes = a.i32();
+  keep.key = a.i64();
+  void *add = a.ptr(), *flags = a.ptr();
+  const long long ld_mask = a.i64();
+  void *planes = a.ptr(), *n = a.ptr(), *qkvg = a.ptr(), *o = a.ptr(), *upd = a.ptr(), *s32 = a.ptr(), *x = a.ptr(), *h = a.ptr(),
+       *out = a.ptr();
+  const int N = a.i32(), ldb = a.i32(), c = a.i32(), H = a.i32(), Dp = a.i32(), hidden = a.i32();
+  void *status = a.ptr(), *stream = a.ptr();
+  if (!a.ok || !square(N) || !apb_sizes(1, N, H, Dp) || ldb < N || hidden <= 0 || hidden > 0x3fffffff) return ubm::UBM_ERR_ARGUMENT;
+  const long long elements = static_cast<long long>(N) * c;
+  int rc = ubm_layernorm_rows_as_f32(s, gamma1, beta1, n, N, c, eps1, stream);
   if (rc) return rc;
-  rc = product(n, w12, h, nullptr, nullptr, R, 2 * hidden, dim, kActSwiglu, hidden, 0, nullptr, 0, 0, status, stream);
-  if (rc) return rc;
-  return product(h, w3, out, nullptr, residual, R, out_dim, hidden, 0, out_dim, 0, nullptr, 0, 0, status, stream);
+  if (ldb != N && cudaMemsetAsync(planes, 0, static_cast<size_t>(H) * N * ldb * 2, static_cast<cudaStream_t>(stream)) != cudaSuccess)
+    return ubm::UBM_ERR_LAUNCH;
+  rc = ubm_pair_head_bias(z, wb, wb_colsum, wb_colbias, planes, N, ldb, H, 0, stream);
+  if (rc == 0)
+    rc = apb(n, wqkvg, bqkvg, wo, planes, ldb, keep, add, flags, ld_mask, nullptr, 0, 0, nullptr, qkvg, o, upd, 1, N, c, c, H, Dp,
+             status, stream);
+  if (rc == 0) rc = ubm_single_add(s, upd, s32, x, elements, stream);
+  if (rc == 0) rc = transition_rows(x, gamma2, beta2, eps2, w12, w3, nullptr, n, h, upd, N, c, hidden, c, status, stream);
+  if (rc == 0) rc = ubm_single_out(s32, upd, out, elements, stream);
+  return rc;
 }
 
 // One decoding step of a block of the genomic decoder on B rows (at most 8): norm -> input projection -> operator -> output projection

@@ -126,6 +126,8 @@ SEQUENCES = {
     "ubm_pair_track": ("ubm_trimul_proj", "ubm_gemm_bf16_packed", "ubm_trimul_out") * 2 +
                       ("ubm_triatt_proj", "ubm_attention_d32", "ubm_gemm_bf16_packed") * 2 + ("ubm_transition",),
     "ubm_apb": ("ubm_gemm_bf16_packed", "ubm_attention", "ubm_gemm_bf16_packed"),
+    "ubm_single_track": ("ubm_layernorm_rows", "ubm_pair_head_bias", "ubm_gemm_bf16_packed", "ubm_attention", "ubm_gemm_bf16_packed",
+                         "ubm_single_add", "ubm_layernorm_rows", "ubm_gemm_bf16_packed", "ubm_gemm_bf16_packed", "ubm_single_out"),
     "ubm_decode_block": ("ubm_gemv_fused_packed",) * 4,        # the operator between them is counted by its wrapper
     "ubm_transition_rows": ("ubm_layernorm_rows", "ubm_gemm_bf16_packed", "ubm_gemm_bf16_packed"),
 }

@@ -35,10 +35,10 @@ native.declare("ubm_trimul_out_rows", [c_void_p] * 9 + [c_int, c_int, c_int, c_i
 
 
 # whole operators from one call (csrc/sequences_sm100.cu): their arguments as 8-byte integers, in the order the library reads them
-for _name in ("ubm_trimul", "ubm_triatt", "ubm_pair_track", "ubm_apb", "ubm_transition_rows"):
+for _name in ("ubm_trimul", "ubm_triatt", "ubm_pair_track", "ubm_single_track", "ubm_apb", "ubm_transition_rows"):
     native.declare(_name, [ctypes.c_char_p])
 _TRIMUL_ARGS, _TRIATT_ARGS, _APB_ARGS = struct.Struct("=21q"), struct.Struct("=26q"), struct.Struct("=28q")
-_TRANSITION_ROWS_ARGS, _PAIR_TRACK_ARGS = struct.Struct("=3qd12q"), struct.Struct("=56q")
+_TRANSITION_ROWS_ARGS, _PAIR_TRACK_ARGS, _SINGLE_TRACK_ARGS = struct.Struct("=3qd12q"), struct.Struct("=56q"), struct.Struct("=14q2d23q")
 
 
 def ceil_to(n: int, m: int) -> int:
@@ -476,6 +476,40 @@ def apb_fused(x: torch.Tensor, w: ApbPacked, bias_planes: torch.Tensor, ldb: int
     attention(qkvg[:, :HD], qkvg[:, HD:2 * HD], qkvg[:, 2 * HD:3 * HD], bias_planes, qkvg[:, 3 * HD:], o, rows=B,
               Nq=N, Nk=N, H=w.H, D=w.Dp, ldb=ldb, ld_in=4 * HD, ld_gate=4 * HD, mask=mask)
     return _gemm.gemm(o, w.wo, gate=out_gate, residual=out_residual).view(B, N, -1)
+
+
+def single_track(s: torch.Tensor, z: torch.Tensor, keep: Optional[torch.Tensor], norm: tuple, bias: tuple, w: ApbPacked,
+                 norm2: tuple, w12: torch.Tensor, w3: torch.Tensor) -> torch.Tensor:
+    """The single track of a Pairformer layer from one call: s + attention of its norm with the bias from z, then + transition, sums in
+    fp32.  s: bf16 [1, N, c], z: bf16 [1, N, N, 128], contiguous; keep: [1, N] of a type :meth:`KeyMask.readable` leaves alone, or None;
+    norms as (fp32 gamma, beta or None, eps); bias: :func:`ops.rows._head_bias_weights`; w12, w3 as :func:`transition_rows` takes them."""
+    N, c = s.shape[1:]
+    dev = s.device
+    hidden = w3.shape[1]
+    ldb, ld_mask, HD = ceil_to(N, 8), ceil_to(N, MASK_STEP), w.H * w.Dp
+    row = 2 * N * c                                         # one [N, c] in bf16
+    sizes = (2 * w.H * N * ldb, row, 8 * N * HD, 2 * N * HD, row, 2 * row, row, 2 * N * hidden, 2 * ld_mask, ld_mask // MASK_STEP)
+    at = [0]
+    for n in sizes:
+        at.append(at[-1] + ceil_to(n, 256))
+    scratch = torch.empty(at[-1], dtype=torch.uint8, device=dev)
+    p = scratch.data_ptr()
+    planes, n, qkvg, o, upd, s32, x, h, add, flags = (p + a for a in at[:-1])
+    keep_ptr = keep_bytes = keep_key = 0
+    if keep is None:
+        add = flags = ld_mask = 0
+    else:
+        keep_ptr, keep_bytes, keep_key = keep.data_ptr(), keep.element_size(), keep.stride(1)
+        native.add_launches(1, "ubm_key_mask")
+    out = torch.empty_like(s)
+    ptr = native.ptr
+    rc = native.lib().ubm_single_track(_SINGLE_TRACK_ARGS.pack(
+        s.data_ptr(), z.data_ptr(), ptr(norm[0]), ptr(norm[1]), *(t.data_ptr() for t in bias), w.wqkvg.data_ptr(), w.bqkvg.data_ptr(),
+        w.wo.data_ptr(), ptr(norm2[0]), ptr(norm2[1]), w12.data_ptr(), w3.data_ptr(), norm[2], norm2[2], keep_ptr, keep_bytes, keep_key,
+        add, flags, ld_mask, planes, n, qkvg, o, upd, s32, x, h, out.data_ptr(), N, ldb, c, w.H, w.Dp, hidden,
+        native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
+    native.check(rc, "ubm_single_track")
+    return out
 
 
 def _triatt_blocked(z, w: TriattPacked, starting: bool, residual: bool, out, ws: dict, mask, rb: int):

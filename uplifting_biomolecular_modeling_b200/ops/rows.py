@@ -78,6 +78,25 @@ def mean_rescale_(o: torch.Tensor, count: torch.Tensor, bias: torch.Tensor, tota
 _HB_CACHE = {}
 
 
+def _head_bias_weights(w: torch.Tensor, ln_w, ln_b, scale: float, device) -> tuple:
+    """(fp32 weights with the norm's scale folded in, their row sums, their products with the norm's shift), kept per weight."""
+    # the cache entry is tied to the live weight tensor object (a freed tensor's address may be reused)
+    key = (id(w), w._version, None if ln_w is None else ln_w._version, float(scale), str(device))
+    entry = _HB_CACHE.get(key)
+    packed = entry[1] if entry is not None and entry[0]() is w else None
+    if packed is None:
+        gam = torch.ones(128, device=device) if ln_w is None else ln_w.detach().float()
+        wf = (w.detach().float() * gam[None, :] * scale).contiguous()
+        colsum = wf.sum(1).contiguous()
+        colbias = torch.zeros(w.shape[0], device=device) if ln_b is None else \
+            ((w.detach().float() @ ln_b.detach().float()) * scale).contiguous()
+        packed = (wf, colsum, colbias)
+        if len(_HB_CACHE) > 4096:
+            _HB_CACHE.clear()
+        _HB_CACHE[key] = (weakref.ref(w), packed)
+    return packed
+
+
 def pair_head_bias(z: torch.Tensor, ln_w, ln_b, w, scale: float = 1.0, transpose: bool = False,
                    out: Optional[torch.Tensor] = None, row: int = 16) -> torch.Tensor:
     """z: bf16 [N, N, 128]; w: [H, 128].  Returns bf16 [H, N, N] (a view of planes whose rows are padded with zeros to a
@@ -99,20 +118,7 @@ def pair_head_bias(z: torch.Tensor, ln_w, ln_b, w, scale: float = 1.0, transpose
         Np = (N + row - 1) // row * row
         make = torch.zeros if Np != N else torch.empty       # the kernel writes no padding
         out = make((H, N, Np), dtype=torch.bfloat16, device=z.device)
-    # the cache entry is tied to the live weight tensor object (a freed tensor's address may be reused)
-    key = (id(w), w._version, None if ln_w is None else ln_w._version, float(scale), str(z.device))
-    entry = _HB_CACHE.get(key)
-    packed = entry[1] if entry is not None and entry[0]() is w else None
-    if packed is None:
-        gam = torch.ones(128, device=z.device) if ln_w is None else ln_w.detach().float()
-        wf = (w.detach().float() * gam[None, :] * scale).contiguous()
-        colsum = wf.sum(1).contiguous()
-        colbias = torch.zeros(H, device=z.device) if ln_b is None else \
-            ((w.detach().float() @ ln_b.detach().float()) * scale).contiguous()
-        packed = (wf, colsum, colbias)
-        if len(_HB_CACHE) > 4096:
-            _HB_CACHE.clear()
-        _HB_CACHE[key] = (weakref.ref(w), packed)
+    packed = _head_bias_weights(w, ln_w, ln_b, scale, z.device)
     wf, colsum, colbias = packed
     rc = native.lib().ubm_pair_head_bias(native.ptr(z), native.ptr(wf), native.ptr(colsum), native.ptr(colbias),
                                          native.ptr(out), N, Np, H, 1 if transpose else 0,
