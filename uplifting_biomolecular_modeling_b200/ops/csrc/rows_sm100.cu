@@ -14,6 +14,8 @@
 #include "host_util.h"
 #include "sm100.cuh"
 
+#include <algorithm>
+
 namespace ubm {
 
 // Row kernels of up to 16 MB take a few us each: their launch may overlap the kernel in front.  (Conditioned norms of 4 MB: two
@@ -233,6 +235,10 @@ __global__ void __launch_bounds__(256) layernorm_rows_narrow_kernel(const __nv_b
 // A warp takes 32 rows.  The k index is permuted so that a lane's fragments of two products are one 16-byte load, the
 // four lanes of a row reading 64 consecutive bytes; the row statistics come from the same registers.  Results go
 // through shared memory so that a plane is written 64 or 128 consecutive bytes at a time.
+// Bound by memory (151 MB in 23 us at 768 tokens and 8 heads) once a warp's next rows are fetched while the planes are written, a thread's
+// place in the planes is found once per tile instead of by a 64-bit division per word, and the weights are split once per resident CTA
+// instead of once per two tiles (a grid of 16 CTAs per SM): 52 -> 39 us there (60 -> 41 at 767 tokens), 215 -> 154 at 1536 tokens and
+// 16 heads (131 -> 76 at 1021), 128 -> 76 at 768 and 32.  Planes of the transposed order are bound by their 2-byte stores (86 -> 82).
 constexpr int kHbRows = 128;            // rows per CTA and iteration: four warps of 32
 constexpr int kHbLd = kHbRows + 2;      // staging row of a head, in elements
 
@@ -282,17 +288,19 @@ __global__ void __launch_bounds__(128) pair_head_bias_kernel(const __nv_bfloat16
   const long long R = static_cast<long long>(N) * N;
   const long long tiles = (R + kHbRows - 1) / kHbRows;
   const bool pairs = !transpose_out && ((N | Np) & 1) == 0;   // two neighbouring rows share a 4-byte word of a plane
-  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const long long r0 = tile * kHbRows + warp * 32;
-    uint4 x[2][2][4];                                         // [16-row half][row g, g + 8][64-byte chunk]
+  uint4 x[2][2][4];                                           // [16-row half][row g, g + 8][64-byte chunk]
+  auto load = [&](long long tile) {
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        const long long r = min(r0 + m * 16 + p * 8 + g, R - 1);
+        const long long r = min(tile * kHbRows + warp * 32 + m * 16 + p * 8 + g, R - 1);
 #pragma unroll
         for (int c = 0; c < 4; ++c) x[m][p][c] = __ldg(reinterpret_cast<const uint4*>(z + r * 128 + c * 32 + t * 8));
       }
+  };
+  load(blockIdx.x);
+  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     float acc[2][NT][4];
 #pragma unroll
     for (int m = 0; m < 2; ++m)
@@ -343,24 +351,27 @@ __global__ void __launch_bounds__(128) pair_head_bias_kernel(const __nv_bfloat16
             so[nt * 8 + 2 * t + e][warp * 32 + m * 16 + p * 8 + g] =
                 __float2bfloat16(fmaf(rstd, acc[m][nt][p * 2 + e] - mu * cs[nt][e], cb[nt][e]));
       }
+    if (tile + gridDim.x < tiles) load(tile + gridDim.x);      // on their way while the planes are written
     __syncthreads();
+    // a thread's place in the planes is the same for all of its heads: one division by N, and that of the tile's first row
+    const int q = pairs ? 2 * (threadIdx.x % (kHbRows / 2)) : threadIdx.x;
     const long long base = tile * kHbRows;
-    if (pairs) {
-      for (int f = threadIdx.x; f < H * (kHbRows / 2); f += blockDim.x) {
-        const int h = f / (kHbRows / 2), q = (f % (kHbRows / 2)) * 2;
-        const long long r = base + q;
-        if (r >= R) continue;
-        const int i = static_cast<int>(r / N), j = static_cast<int>(r - static_cast<long long>(i) * N);
-        *reinterpret_cast<uint32_t*>(out + (static_cast<long long>(h) * N + i) * Np + j) =
-            *reinterpret_cast<const uint32_t*>(&so[h][q]);
-      }
-    } else {
-      for (int f = threadIdx.x; f < H * kHbRows; f += blockDim.x) {
-        const int h = f / kHbRows, q = f % kHbRows;
-        const long long r = base + q;
-        if (r >= R) continue;
-        const int i = static_cast<int>(r / N), j = static_cast<int>(r - static_cast<long long>(i) * N);
-        out[(static_cast<long long>(h) * N + (transpose_out ? j : i)) * Np + (transpose_out ? i : j)] = so[h][q];
+    int i = static_cast<int>(base / N), j = static_cast<int>(base - static_cast<long long>(i) * N) + q;
+    const int over = static_cast<unsigned>(j) / static_cast<unsigned>(N);
+    i += over;
+    j -= over * N;
+    if (base + q < R) {
+      const long long plane = static_cast<long long>(N) * Np;
+      if (pairs) {
+        const int h0 = threadIdx.x / (kHbRows / 2);
+        __nv_bfloat16* o = out + h0 * plane + static_cast<long long>(i) * Np + j;
+#pragma unroll
+        for (int h = 0; h < H; h += 2)
+          *reinterpret_cast<uint32_t*>(o + h * plane) = *reinterpret_cast<const uint32_t*>(&so[h0 + h][q]);
+      } else {
+        __nv_bfloat16* o = out + static_cast<long long>(transpose_out ? j : i) * Np + (transpose_out ? i : j);
+#pragma unroll
+        for (int h = 0; h < H; ++h) o[h * plane] = so[h][q];
       }
     }
     __syncthreads();
@@ -813,7 +824,9 @@ extern "C" int ubm_pair_head_bias(const void* z, const void* w, const void* cols
   using namespace ubm;
   if (N <= 0 || Np < N) return UBM_ERR_ARGUMENT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = grid_for(static_cast<long long>(N) * N, kHbRows);
+  // every CTA resident (168 registers a thread at 32 heads, up to 128 at the others)
+  const long long tiles = (static_cast<long long>(N) * N + kHbRows - 1) / kHbRows;
+  const int grid = static_cast<int>(std::min<long long>(tiles, sm_count() * (H == 32 ? 3 : 4)));
   const __nv_bfloat16* zz = static_cast<const __nv_bfloat16*>(z);
   const float* ww = static_cast<const float*>(w);
   const float* cs = static_cast<const float*>(colsum);
