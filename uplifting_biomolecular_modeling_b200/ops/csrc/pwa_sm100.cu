@@ -9,10 +9,10 @@
 //   pwa_out_kernel       gate projection, gating and output projection of 128 tokens of one sequence
 // Between them the [S N, 256] intermediates cross memory once as v and once as o; as tensor statements around the same
 // GEMM they crossed it eleven times (projections, the transpose into planes, gate, product, transpose back).
-// 1024 sequences x 768 tokens: 0.67 ms (weights 3, softmax 15, values 94, GEMM 276, output stage 166 us, bias planes 45)
+// 1024 sequences x 768 tokens: 0.65 ms (weights 3, softmax 17, values 93, GEMM 277, output stage 165 us, bias planes 34)
 // against 2.54 ms.  Values and output stage move the 0.4 GB of v and o (60 us each at copy bandwidth); neither fills a unit
-// (512 x 512: DRAM 43 and 35 %, issue slots 51 and 45 %, special-function unit 2 and 30 % busy), their warps wait for
-// tensor and shared memory.
+// (values at 512 x 512: DRAM 43 %, issue slots 51 %, special-function unit 2 % busy; output stage at 1024 x 768: DRAM 53, issue slots 50,
+// special-function unit 33 %), their warps wait for tensor and shared memory.
 #include "host_util.h"
 #include "sm100.cuh"
 
@@ -292,10 +292,12 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------ output stage
-// A tile is 128 tokens of one sequence.  D_g[token][256] = m W_g'^T; two teams of eight warps take alternate tiles:
-// gate = sigmoid(LayerNorm fold of D_g), multiplied into the o tile where it lies in shared memory (the K-major
-// operand of the second product), D_o[token][64] = (gate o) W_o^T over the first columns of D_g, and the rows leave
-// through the m tile's own buffer.  One team alone idled through its second product and its loads.
+// A tile is 128 tokens of one sequence.  D_g[token][256] = m W_g'^T; two teams of eight warps take alternate tiles: gate = sigmoid(LayerNorm
+// fold of D_g) times o is written over D_g as the second product's operand in tensor memory, D_o[token][64] = (gate o) W_o^T over columns of
+// D_g that have been read, and the rows leave from registers.  So the m tile's buffer is free behind the first product and the halves of
+// the o tile's each behind the gating of its channels: the team's next tile arrives under the rest of this one.  (With the gated operand
+// written over the o tile and the rows staged in the m tile, a team waited for its second product, its stores and then its loads:
+// 170 -> 165 us at 1024 x 768, 90 at copy bandwidth.)
 // Warps: 0 = TMA producer, 1 = first product, 2 = second product (its own issuer: behind the first product of the
 // next tile it would wait for that tile's load), 3-10 / 11-18 = the teams.
 constexpr int kPoThreads = 96 + 512;
@@ -309,24 +311,27 @@ struct PwaOutParams {
   float eps;
   const float* g_colsum;    // [256]
   const float* g_colbias;   // [256]
+  __nv_bfloat16* out;       // [S][N][64]
   KernelStatus* status;
 };
 
 __global__ void __launch_bounds__(kPoThreads, 1)
 pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmO,
                const __grid_constant__ CUtensorMap tmWg, const __grid_constant__ CUtensorMap tmWo,
-               const __grid_constant__ CUtensorMap tmOut, PwaOutParams p) {
+               PwaOutParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sWg = smem;                                   // [256][64]
   uint8_t* sWo = sWg + kPoWBytes;                        // four k-blocks [64][64]
   uint8_t* sSt = sWo + kPoWBytes;
   float* sConst = reinterpret_cast<float*>(sSt + 2 * kPoStage);
-  uint64_t* full = reinterpret_cast<uint64_t*>(sConst + 2 * kPwHC);   // [2] everything below: one per team
-  uint64_t* empty = full + 2;      // 8 arrivals: the rows have been read out of shared memory
-  uint64_t* g_full = empty + 2;    // D_g complete
-  uint64_t* a_full = g_full + 2;   // 8 arrivals: D_g read, gated operand written
-  uint64_t* o_full = a_full + 2;   // D_o complete
-  uint64_t* t_empty = o_full + 2;  // 8 arrivals: D_o read
+  uint64_t* m_full = reinterpret_cast<uint64_t*>(sConst + 2 * kPwHC);   // [2] everything below: one per team
+  uint64_t* m_empty = m_full + 2;    // 8 arrivals: statistics taken, first product done
+  uint64_t* h_full = m_empty + 2;    // [2][2] o, channels 0-63 | 128-191 and 64-127 | 192-255
+  uint64_t* h_empty = h_full + 4;    // [2][2] 8 arrivals: gated
+  uint64_t* g_full = h_empty + 4;    // D_g complete
+  uint64_t* a_full = g_full + 2;     // 8 arrivals: D_g read, gated operand written
+  uint64_t* o_full = a_full + 2;     // D_o complete
+  uint64_t* t_empty = o_full + 2;    // 8 arrivals: D_o read
   uint64_t* w_full = t_empty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(w_full + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -335,8 +340,12 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&full[b], 1);
-      mbar_init(&empty[b], 8);
+      mbar_init(&m_full[b], 1);
+      mbar_init(&m_empty[b], 8);
+      for (int hf = 0; hf < 2; ++hf) {
+        mbar_init(&h_full[2 * b + hf], 1);
+        mbar_init(&h_empty[2 * b + hf], 8);
+      }
       mbar_init(&g_full[b], 1);
       mbar_init(&a_full[b], 8);
       mbar_init(&o_full[b], 1);
@@ -374,12 +383,19 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
         const int b = n & 1;
         const int s = t / p.tiles_per_row;
         const int i0 = (t - s * p.tiles_per_row) * 128;
-        mbar_wait(&empty[b], ((n >> 1) & 1u) ^ 1u, ws, 81, b);
-        if (*abort_flag) break;
+        const uint32_t ph = ((n >> 1) & 1u) ^ 1u;
         uint8_t* dst = sSt + b * kPoStage;
-        mbar_expect_tx(&full[b], kPoStage);
-        tma_load_3d(dst, &tmM, &full[b], 0, i0, s);
-        for (int kb = 0; kb < 4; ++kb) tma_load_3d(dst + (1 + kb) * kPwTile, &tmO, &full[b], kb * 64, s, i0);
+        mbar_wait(&m_empty[b], ph, ws, 81, b);
+        if (*abort_flag) break;
+        mbar_expect_tx(&m_full[b], kPwTile);
+        tma_load_3d(dst, &tmM, &m_full[b], 0, i0, s);
+        for (int hf = 0; hf < 2; ++hf) {
+          mbar_wait(&h_empty[2 * b + hf], ph, ws, 90, 2 * b + hf);
+          if (*abort_flag) break;
+          mbar_expect_tx(&h_full[2 * b + hf], 2 * kPwTile);
+          for (int kb = hf; kb < 4; kb += 2) tma_load_3d(dst + (1 + kb) * kPwTile, &tmO, &h_full[2 * b + hf], kb * 64, s, i0);
+        }
+        if (*abort_flag) break;
       }
     }
   } else if (warp == 1) {
@@ -390,7 +406,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++n) {
       const int b = n & 1;
       const uint32_t ph = (n >> 1) & 1u;
-      mbar_wait(&full[b], ph, ws, 83, b);
+      mbar_wait(&m_full[b], ph, ws, 83, b);
       mbar_wait(&t_empty[b], ph ^ 1u, ws, 84, b);
       tc_fence_after_sync();
       const uint64_t ad = umma_smem_desc(smem_u32(sSt + b * kPoStage), 16, 1024, kSwizzle128);
@@ -413,22 +429,20 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
       const int b = n & 1;
       mbar_wait(&a_full[b], (n >> 1) & 1u, ws, 85, b);
       tc_fence_after_sync();
-      const uint64_t ad = umma_smem_desc(smem_u32(sSt + b * kPoStage + kPwTile), 16, 1024, kSwizzle128);
       const uint64_t bd = umma_smem_desc(smem_u32(sWo), 16, 1024, kSwizzle128);
+      const uint32_t tb = tmem_base + b * 256;
       if (leader) {
 #pragma unroll
-        for (int kb = 0; kb < 4; ++kb)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_ss(tmem_base + b * 256, ad + static_cast<uint64_t>(kb * (kPwTile >> 4) + k * 2),
-                    bd + static_cast<uint64_t>(kb * (8192 >> 4) + k * 2), idesc, (kb | k) != 0 ? 1u : 0u);
+        for (int k = 0; k < 16; ++k)      // 16 channels each: columns 0 .. 63 and 128 .. 191 hold the operand
+          umma_ts(tb + 64, tb + (k >> 3) * 128 + (k & 7) * 8, bd + static_cast<uint64_t>((k >> 2) * (8192 >> 4) + (k & 3) * 2), idesc,
+                  k != 0 ? 1u : 0u);
         umma_commit(&o_full[b]);
       }
       __syncwarp();
     }
   } else {
     const int team = (warp - 3) >> 3;
-    const int half = ((warp - 3) >> 2) & 1;      // columns 128 half .. of D_g, 32 half .. of D_o
+    const int half = ((warp - 3) >> 2) & 1;      // columns 128 half .. of D_g, 64 + 32 half .. (D_o)
     const int q = warp & 3;
     const int row = q * 32 + lane;
     uint8_t* st = sSt + team * kPoStage;
@@ -439,7 +453,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
       const uint32_t ph = (n >> 1) & 1u;
       const int s = t / p.tiles_per_row;
       const int i0 = (t - s * p.tiles_per_row) * 128;
-      mbar_wait(&full[team], ph, ws, 86, team);
+      mbar_wait(&m_full[team], ph, ws, 86, team);
       float sum = 0.f, sumsq = 0.f;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -457,9 +471,12 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
       const float2 a2 = make_float2(rstd, rstd), b2 = make_float2(-mu * rstd, -mu * rstd);
       mbar_wait(&g_full[team], ph, ws, 87, team);
       tc_fence_after_sync();
+      __syncwarp();                                    // every lane has read its row
+      if (lane == 0) mbar_arrive(&m_empty[team]);
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         const int col = half * 128 + c * 32;
+        if ((c & 1) == 0) mbar_wait(&h_full[2 * team + (c >> 1)], ph, ws, 91, 2 * team + (c >> 1));
         uint32_t v[32];
         tmem_ld32(tmem_addr(tb, q, col), v);
         tmem_ld_wait();
@@ -468,18 +485,16 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
         float low = fminf(f[0], f[1]);
 #pragma unroll
         for (int k = 2; k < 32; k += 2) low = min3f(low, f[k], f[k + 1]);
-        uint8_t* ob = st + (1 + (col >> 6)) * kPwTile;
+        const uint8_t* ob = st + (1 + (col >> 6)) * kPwTile;
+        uint32_t r[16];
         auto apply = [&](auto gate) {
 #pragma unroll
           for (int j8 = 0; j8 < 4; ++j8) {
-            uint4* at = reinterpret_cast<uint4*>(ob + swz128_offset(row, ((col >> 5) & 1) * 4 + j8));
-            const uint4 u = *at;
+            const uint4 u = *reinterpret_cast<const uint4*>(ob + swz128_offset(row, ((col >> 5) & 1) * 4 + j8));
             const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-            uint32_t r[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              r[e] = pack_bf16x2(bf16_lo(w[e]) * gate(f[j8 * 8 + 2 * e]), bf16_hi(w[e]) * gate(f[j8 * 8 + 2 * e + 1]));
-            *at = make_uint4(r[0], r[1], r[2], r[3]);
+              r[j8 * 4 + e] = pack_bf16x2(bf16_lo(w[e]) * gate(f[j8 * 8 + 2 * e]), bf16_hi(w[e]) * gate(f[j8 * 8 + 2 * e + 1]));
           }
         };
         // nearly closed gates take the form that keeps their relative precision (for every gate it costs 27 us more)
@@ -487,40 +502,32 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
           apply([](float x) { return x < kSigmoidTail ? sigmoidf_rel(x) : sigmoidf_fast(x); });
         else
           apply([](float x) { return sigmoidf_fast(x); });
+        tmem_st16(tmem_addr(tb, q, half * 128 + c * 16), r);      // columns that this warp has read: 32 of D_g hold 64 of the operand
+        __syncwarp();
+        if ((c & 1) != 0 && lane == 0) mbar_arrive(&h_empty[2 * team + (c >> 1)]);
       }
+      tmem_st_wait();
       tc_fence_before_sync();
-      fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&a_full[team]);
       mbar_wait(&o_full[team], ph, ws, 88, team);
       tc_fence_after_sync();
       uint32_t v[32];
-      tmem_ld32(tmem_addr(tb, q, half * 32), v);
+      tmem_ld32(tmem_addr(tb, q, 64 + half * 32), v);
       tmem_ld_wait();
       tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&t_empty[team]);
+      if (i0 + row < p.N) {
+        uint4* o = reinterpret_cast<uint4*>(p.out + (static_cast<long long>(s) * p.N + i0 + row) * kPwC + half * 32);
 #pragma unroll
-      for (int j8 = 0; j8 < 4; ++j8) {
-        uint4 u;
-        u.x = pack_bf16x2(__uint_as_float(v[j8 * 8]), __uint_as_float(v[j8 * 8 + 1]));
-        u.y = pack_bf16x2(__uint_as_float(v[j8 * 8 + 2]), __uint_as_float(v[j8 * 8 + 3]));
-        u.z = pack_bf16x2(__uint_as_float(v[j8 * 8 + 4]), __uint_as_float(v[j8 * 8 + 5]));
-        u.w = pack_bf16x2(__uint_as_float(v[j8 * 8 + 6]), __uint_as_float(v[j8 * 8 + 7]));
-        // D_o complete means D_g was complete: the first product has read the m tile, and both halves took their
-        // statistics before they arrived on a_full; each warp owns 2 KB of it, [32 rows][64 bytes]
-        *reinterpret_cast<uint4*>(st + half * 8192 + q * 2048 + swz64_offset(lane, j8)) = u;
+        for (int j8 = 0; j8 < 4; ++j8)
+          o[j8] = make_uint4(pack_bf16x2(__uint_as_float(v[j8 * 8]), __uint_as_float(v[j8 * 8 + 1])),
+                             pack_bf16x2(__uint_as_float(v[j8 * 8 + 2]), __uint_as_float(v[j8 * 8 + 3])),
+                             pack_bf16x2(__uint_as_float(v[j8 * 8 + 4]), __uint_as_float(v[j8 * 8 + 5])),
+                             pack_bf16x2(__uint_as_float(v[j8 * 8 + 6]), __uint_as_float(v[j8 * 8 + 7])));
       }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&t_empty[team]);
-        if (i0 + q * 32 < p.N) tma_store_3d(&tmOut, st + half * 8192 + q * 2048, half * 32, i0 + q * 32, s);
-        tma_store_commit();
-        tma_store_wait_read<0>();
-        mbar_arrive(&empty[team]);
-      }
-      __syncwarp();
     }
-    if (lane == 0) tma_store_wait_all<0>();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -604,7 +611,7 @@ static int pwa_value(const void* m, const void* w, const void* colsum, const voi
 static int pwa_out(const void* m, const void* o, const void* wg, const void* g_colsum, const void* g_colbias,
                            const void* wo, void* out, int S, int N, float eps, void* status, void* stream) {
   using namespace ubm;
-  if (S <= 0 || N <= 0) return UBM_ERR_ARGUMENT;
+  if (S <= 0 || N <= 0 || (reinterpret_cast<uintptr_t>(out) & 15)) return UBM_ERR_ARGUMENT;
   PwaOutParams p = {};
   p.S = S;
   p.N = N;
@@ -616,7 +623,8 @@ static int pwa_out(const void* m, const void* o, const void* wg, const void* g_c
   p.g_colsum = static_cast<const float*>(g_colsum);
   p.g_colbias = static_cast<const float*>(g_colbias);
   p.status = static_cast<KernelStatus*>(status);
-  CUtensorMap tmM, tmO, tmWg, tmWo, tmOut;
+  p.out = static_cast<__nv_bfloat16*>(out);
+  CUtensorMap tmM, tmO, tmWg, tmWo;
   uint64_t dM[3] = {64, (uint64_t)N, (uint64_t)S}, sM[2] = {128, (uint64_t)N * 128};
   uint32_t bM[3] = {64, 128, 1};
   int rc = make_tmap(&tmM, m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dM, sM, bM, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -633,13 +641,10 @@ static int pwa_out(const void* m, const void* o, const void* wg, const void* g_c
   uint32_t bW[2] = {64, 64};
   rc = make_tmap(&tmWo, wo, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dW, sW, bW, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
-  uint32_t bOut[3] = {32, 32, 1};
-  rc = make_tmap(&tmOut, out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, dM, sM, bOut, CU_TENSOR_MAP_SWIZZLE_64B);
-  if (rc) return rc;
   rc = set_smem(pwa_out_kernel, kPoSmem);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  launch_after(p.num_tiles <= 4 * grid, pwa_out_kernel, grid, kPoThreads, kPoSmem, static_cast<cudaStream_t>(stream), tmM, tmO, tmWg, tmWo, tmOut, p);
+  launch_after(p.num_tiles <= 4 * grid, pwa_out_kernel, grid, kPoThreads, kPoSmem, static_cast<cudaStream_t>(stream), tmM, tmO, tmWg, tmWo, p);
   UBM_CHECK_LAUNCH("pwa_out_kernel");
   return UBM_OK;
 }
