@@ -17,6 +17,6 @@ def test_tiles_and_rows(N, H, transpose):
     out = rows.pair_head_bias(z, gamma, beta, w, transpose=transpose, out=planes)
     n = torch.nn.functional.layer_norm(z.double(), (128,), gamma.double(), beta.double(), 1e-5)
     ref = torch.einsum("ijc,hc->hji" if transpose else "ijc,hc->hij", n, w.double())
-    # one rounding to bf16 (2^-9 of the value) of fp32 sums of 128 terms of about one, the mean taken off behind them
+    # one rounding to bf16 (2^-8 of the value) of fp32 sums of 128 terms of about one, the mean taken off behind them
     assert ((out[:H].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()
     assert (planes[H] == 7).all() and (planes[:, :, N:] == 7).all()            # nothing beside its planes

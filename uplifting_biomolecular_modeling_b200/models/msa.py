@@ -41,10 +41,23 @@ class OuterProductMean(_Switchable):
         from ..ops import gemm, rows
         B, S, N, _ = m.shape
         c = self.c_hidden
-        n = rows.layernorm_rows(m.contiguous(), self.norm.weight, self.norm.bias, self.norm.eps)
         # [S, N, c] seen as [S, N*c]: sequences (the contraction) along rows, (token, channel) contiguous - the
         # operand form of the MN-major GEMM, so no [N*c, S] transposed copies are made
-        if c == 32 and n.shape[-1] % 8 == 0 and plain_linears(self.proj_a, self.proj_b):
+        m = m.contiguous()
+        plain = c == 32 and m.shape[-1] % 8 == 0 and plain_linears(self.proj_a, self.proj_b)
+        in_place = self.full_mask or (mask.dim() == 3 and mask.device == m.device and mask.shape[0] == 1)
+        n = None
+        if plain and m.shape[-1] == 64 and in_place and m.data_ptr() % 16 == 0:
+            # norm, both projections and the mask in one pass over the rows
+            mk = None if self.full_mask else mask[0].to(torch.bfloat16).expand(S, N).reshape(-1).contiguous()
+            ab = rows.outer_projections(m.view(S * N, 64), self.norm.weight, self.norm.bias, self.norm.eps, self.proj_a.weight,
+                                        self.proj_b.weight, mk)
+            a2, b2 = ab[0].view(S, N * c), ab[1].view(S, N * c)
+        else:
+            n = rows.layernorm_rows(m, self.norm.weight, self.norm.bias, self.norm.eps)
+        if n is None:
+            pass
+        elif plain:
             # both projections from one product, its two 32-wide column blocks stored apart: 7 % of the call where the host
             # bounds it (up to 300 tokens), no difference at 1024 sequences x 768 tokens
             wab = torch.cat([self.proj_a.weight, self.proj_b.weight], 0)

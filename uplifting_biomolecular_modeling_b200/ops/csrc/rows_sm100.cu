@@ -5,6 +5,7 @@
 //   ubm_pair_head_bias   bias[h][i][j] = Linear_{c->H}(LN(z[i][j])) as channel-major bf16 planes
 //                        (the proj_z of attention with pair bias; reference: _pf_bias_kernel,
 //                        common/opt_core/opt_core/kernels/apb/fpf_apb)
+//   ubm_outer_proj       the outer product mean's projections of LN(m), masked
 //   ubm_adaln_rows       sigmoid(scale[r]) * LN_noaffine(a[r]) + shift[r]   (DiT AdaLN)
 //   ubm_gate_residual    out = res + sigmoid(gate) * x
 //   ubm_swiglu_rows      out = silu(a) * b for a | b halves of one row
@@ -375,6 +376,125 @@ __global__ void __launch_bounds__(128) pair_head_bias_kernel(const __nv_bfloat16
       }
     }
     __syncthreads();
+  }
+}
+
+// The two projections of the outer product mean (64 -> 2 x 32 channels) of the LayerNorm of their rows, times the row's mask: x: [R][64] bf16
+// -> out[2][R][32].  As norm, product and mask pass the rows crossed memory six times; a product of 64 channels by 64 fills a
+// quarter of a tcgen05 tile's time and half of its columns.  Here they cross it once each way, on mma.sync m16n8k16 as above.
+// A warp takes 32 rows, the next ones on their way: a lane holds 16 channels of a row, the row's four lanes form the
+// statistics (in the order of layernorm_rows_narrow_kernel, rounded to bf16 as there).  The weights' rows are permuted so that
+// a lane's sums are 8 neighbouring channels: one 16-byte store per row, 512 consecutive bytes per instruction.
+// 786432 rows (1024 sequences x 768 tokens): norm 37 and product 77 us before (a mask pass on top), 42 now (45 with the mask), 30 at copy
+// bandwidth.  Three CTAs per SM: four (128 registers, a few spilled) take the same time.
+constexpr int kOpWarps = 4;
+
+__global__ void __launch_bounds__(32 * kOpWarps, 3) outer_proj_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
+                                                                      const float* __restrict__ beta,
+                                                                      const __nv_bfloat16* __restrict__ wa,
+                                                                      const __nv_bfloat16* __restrict__ wb,
+                                                                      const __nv_bfloat16* __restrict__ mask,
+                                                                      __nv_bfloat16* __restrict__ out, long long R, float eps) {
+  __shared__ uint2 sw[8][4][32];                            // B fragments: [column tile][product][lane]
+  __shared__ __align__(16) float sg[64], sb[64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  grid_dependency_sync(short_rows(R, 64));
+  for (int f = threadIdx.x; f < 8 * 4 * 32; f += blockDim.x) {
+    const int fl = f & 31, prod = (f >> 5) & 3, nt = f >> 7;
+    const int n = fl >> 2, ch = (n >> 1) * 8 + (nt & 3) * 2 + (n & 1);
+    const uint16_t* w = reinterpret_cast<const uint16_t*>(nt < 4 ? wa : wb) + ch * 64 + (prod >> 1) * 32 + (fl & 3) * 8 + (prod & 1) * 4;
+    sw[nt][prod][fl] = make_uint2(w[0] | static_cast<uint32_t>(w[1]) << 16, w[2] | static_cast<uint32_t>(w[3]) << 16);
+  }
+  if (threadIdx.x < 64) {
+    sg[threadIdx.x] = gamma != nullptr ? gamma[threadIdx.x] : 1.f;
+    sb[threadIdx.x] = beta != nullptr ? beta[threadIdx.x] : 0.f;
+  }
+  __syncthreads();
+  const long long tiles = (R + 31) / 32, step = static_cast<long long>(gridDim.x) * kOpWarps;
+  long long tile = static_cast<long long>(blockIdx.x) * kOpWarps + warp;
+  uint4 x4[4][2];                                           // rows g, g + 8, .. of the tile; 64-byte chunk
+  uint16_t mk[4];
+  auto load = [&](long long at) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const long long r = min(at * 32 + m * 8 + g, R - 1);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) x4[m][c] = __ldg(reinterpret_cast<const uint4*>(x + r * 64 + c * 32 + t * 8));
+      if (mask != nullptr) mk[m] = __ldg(reinterpret_cast<const uint16_t*>(mask) + r);
+    }
+  };
+  if (tile < tiles) load(tile);
+  for (; tile < tiles; tile += step) {
+    uint32_t a[4][2][4];                                    // normalised rows
+    float keep[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      float v[2][8], sum[2] = {0.f, 0.f}, sq[2] = {0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const uint32_t w[4] = {x4[m][c].x, x4[m][c].y, x4[m][c].z, x4[m][c].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          v[c][2 * j] = bf16_lo(w[j]);
+          v[c][2 * j + 1] = bf16_hi(w[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[c] += v[c][j];
+      }
+      float total = sum[0] + sum[1];
+      total += __shfl_xor_sync(0xffffffffu, total, 2);
+      total += __shfl_xor_sync(0xffffffffu, total, 1);
+      const float mu = total * (1.0f / 64);
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sq[c] += (v[c][j] - mu) * (v[c][j] - mu);
+      float q = sq[0] + sq[1];
+      q += __shfl_xor_sync(0xffffffffu, q, 2);
+      q += __shfl_xor_sync(0xffffffffu, q, 1);
+      const float rstd = rsqrtf(q * (1.0f / 64) + eps);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float4* gp = reinterpret_cast<const float4*>(sg + c * 32 + t * 8);
+        const float4* bp = reinterpret_cast<const float4*>(sb + c * 32 + t * 8);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 gg = gp[h], bb = bp[h];
+          a[m][c][2 * h] = pack_bf16x2((v[c][4 * h] - mu) * rstd * gg.x + bb.x, (v[c][4 * h + 1] - mu) * rstd * gg.y + bb.y);
+          a[m][c][2 * h + 1] = pack_bf16x2((v[c][4 * h + 2] - mu) * rstd * gg.z + bb.z, (v[c][4 * h + 3] - mu) * rstd * gg.w + bb.w);
+        }
+      }
+      keep[m] = mask != nullptr ? __uint_as_float(static_cast<uint32_t>(mk[m]) << 16) : 1.f;
+    }
+    if (tile + step < tiles) load(tile + step);
+#pragma unroll
+    for (int which = 0; which < 2; ++which) {
+      float acc[2][4][4];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) (&acc[0][0][0])[i] = 0.f;
+#pragma unroll
+      for (int prod = 0; prod < 4; ++prod)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          const uint2 b = sw[which * 4 + nt][prod][lane];
+          const int c = prod >> 1, e = 2 * (prod & 1);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            mma_bf16_16816(acc[h][nt], a[2 * h][c][e], a[2 * h + 1][c][e], a[2 * h][c][e + 1], a[2 * h + 1][c][e + 1], b.x, b.y);
+        }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const long long r = tile * 32 + m * 8 + g;
+        uint32_t o[4];
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+          o[nt] = pack_bf16x2(acc[m >> 1][nt][(m & 1) * 2], acc[m >> 1][nt][(m & 1) * 2 + 1]);
+          if (mask != nullptr) o[nt] = pack_bf16x2(bf16_lo(o[nt]) * keep[m], bf16_hi(o[nt]) * keep[m]);
+        }
+        if (r < R) *reinterpret_cast<uint4*>(out + (which * R + r) * 32 + t * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    }
   }
 }
 
@@ -840,6 +960,21 @@ extern "C" int ubm_pair_head_bias(const void* z, const void* w, const void* cols
     default: return UBM_ERR_ARGUMENT;
   }
   UBM_CHECK_LAUNCH("pair_head_bias_kernel");
+  return UBM_OK;
+}
+
+// x: bf16 [R][64], gamma, beta: fp32 [64] or null, wa, wb: bf16 [32][64], mask: bf16 [R] or null, out: bf16 [2][R][32]; x and out on
+// 16 bytes.
+extern "C" int ubm_outer_proj(const void* x, const void* gamma, const void* beta, const void* wa, const void* wb, const void* mask,
+                              void* out, long long R, float eps, void* stream) {
+  using namespace ubm;
+  if (R <= 0 || !aligned_16(x, out)) return UBM_ERR_ARGUMENT;
+  const int grid = static_cast<int>(std::min<long long>((R + 32 * kOpWarps - 1) / (32 * kOpWarps), sm_count() * 3));
+  launch_after(short_rows(R, 64), outer_proj_kernel, grid, 32 * kOpWarps, 0, static_cast<cudaStream_t>(stream),
+               static_cast<const __nv_bfloat16*>(x), static_cast<const float*>(gamma), static_cast<const float*>(beta),
+               static_cast<const __nv_bfloat16*>(wa), static_cast<const __nv_bfloat16*>(wb), static_cast<const __nv_bfloat16*>(mask),
+               static_cast<__nv_bfloat16*>(out), R, eps);
+  UBM_CHECK_LAUNCH("outer_proj_kernel");
   return UBM_OK;
 }
 

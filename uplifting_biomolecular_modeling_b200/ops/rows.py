@@ -12,6 +12,7 @@ from . import native
 from .native import c_float, c_int, c_ll, c_void_p
 
 native.declare("ubm_layernorm_rows", [c_void_p] * 4 + [c_ll, c_int, c_float, c_int, c_int, c_void_p])
+native.declare("ubm_outer_proj", [c_void_p] * 7 + [c_ll, c_float, c_void_p])
 native.declare("ubm_pair_head_bias", [c_void_p] * 5 + [c_int, c_int, c_int, c_int, c_void_p])
 native.declare("ubm_adaln_rows", [c_void_p] * 4 + [c_ll, c_int, c_ll, c_ll, c_float, c_void_p])
 native.declare("ubm_gate_residual", [c_void_p] * 4 + [c_ll, c_int, c_ll, c_ll, c_void_p])
@@ -125,6 +126,24 @@ def pair_head_bias(z: torch.Tensor, ln_w, ln_b, w, scale: float = 1.0, transpose
                                          native.current_stream(z.device))
     native.check(rc, "ubm_pair_head_bias")
     return out[:, :, :N]
+
+
+def outer_projections(m: torch.Tensor, ln_w, ln_b, eps: float, wa: torch.Tensor, wb: torch.Tensor,
+                      mask: Optional[torch.Tensor]) -> torch.Tensor:
+    """bf16 [2, R, 32]: the projections by wa and wb (bf16 [32, 64]) of LN(m), times the row's mask.  m: bf16 [R, 64], contiguous, on 16
+    bytes; mask: bf16 [R], contiguous, or None."""
+    R = m.shape[0]
+    if m.dtype != torch.bfloat16 or m.shape != (R, 64) or not m.is_contiguous() or wa.shape != (32, 64) or wb.shape != (32, 64) or \
+            wa.dtype != torch.bfloat16 or wb.dtype != torch.bfloat16 or wa.device != m.device or wb.device != m.device or \
+            (mask is not None and (mask.dtype != torch.bfloat16 or mask.shape != (R,) or not mask.is_contiguous() or
+                                   mask.device != m.device)):
+        raise ValueError("outer_projections: bf16 rows of 64 channels, two weights of [32, 64], a mask of one value per row")
+    out = torch.empty((2, R, 32), dtype=torch.bfloat16, device=m.device)
+    wa, wb, g, b = wa.contiguous(), wb.contiguous(), _f32_param(ln_w), _f32_param(ln_b)
+    rc = native.lib().ubm_outer_proj(native.ptr(m), native.ptr(g), native.ptr(b), native.ptr(wa), native.ptr(wb), native.ptr(mask),
+                                     native.ptr(out), R, float(eps), native.current_stream(m.device))
+    native.check(rc, "ubm_outer_proj")
+    return out
 
 
 def _cond2d(t: torch.Tensor, C: int) -> torch.Tensor:
