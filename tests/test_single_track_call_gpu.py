@@ -25,7 +25,7 @@ def _apart(m, s, z, mask, monkeypatch):
     from uplifting_biomolecular_modeling_b200.models import pairformer
     with monkeypatch.context() as mp:
         mp.setattr(pairformer.PairformerLayer, "_single_track", lambda self, s, z, mask: None)
-        mp.setattr(m, "pair_update", lambda z, mask: z)
+        mp.setattr(pairformer.PairformerLayer, "pair_update", lambda self, z, mask: z)
         return m(s, z, mask, None)[0]
 
 
