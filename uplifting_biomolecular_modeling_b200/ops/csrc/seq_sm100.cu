@@ -21,6 +21,8 @@
 #include "host_util.h"
 #include "sm100.cuh"
 
+#include <algorithm>
+
 namespace ubm {
 
 static inline int seq_grid(long long work, int per_block) {
@@ -780,14 +782,18 @@ __global__ void __launch_bounds__(256) rotary_split_qkv_kernel(const __nv_bfloat
 }
 
 // LayerNorm over the whole q row and over the whole k row of a fused projection [T][3][H][Dh], each followed by the
-// rotary embedding of its heads, in place; one warp per token, the row read once and kept packed in registers.  A lane
+// rotary embedding of its heads, in place; one warp per row, read once and kept packed in registers.  A lane
 // holds 8-channel chunks 256 channels apart, so with Dh dividing 256 all its chunks sit at one place of their heads and
-// share four (cos, sin) pairs.  Two row reads and two row writes (DRAM a third busy, issue slots 60 %, at 32768 tokens x 960
-// channels) where the separate steps (slices made
-// contiguous, normalised, written back, then rotated and split into three tensors) made eighteen: 40 us against 247 us
-// at 16376 tokens x 960 channels.
+// share four (cos, sin) pairs.  Two row reads and two row writes where the separate steps (slices made
+// contiguous, normalised, written back, then rotated and split into three tensors) made eighteen.
+// Bound by issue slots and latency: 31 us at 16376 tokens x 960 channels, 19 at copy bandwidth.  The frequencies (a power per angle)
+// are formed once per warp, so every block is resident and a warp takes several rows; a row's q and k are a warp's each,
+// which halves its registers, and a lane forms one angle of a head of up to 64 channels instead of four.  One token per
+// warp and as many warps as tokens took 41 us (91 at 2048 channels, now 54); resident blocks alone 33 (73).
+constexpr int qkn_ctas(int chunks) { return chunks == 1 ? 6 : chunks == 2 ? 5 : chunks <= 5 ? 3 : 2; }   // per SM, all resident
+
 template <int CHUNKS>
-__global__ void __launch_bounds__(256) qk_norm_rotary_kernel(__nv_bfloat16* __restrict__ qkv,
+__global__ void __launch_bounds__(256, qkn_ctas(CHUNKS)) qk_norm_rotary_kernel(__nv_bfloat16* __restrict__ qkv,
                                                              const int* __restrict__ pos,
                                                              const float* __restrict__ q_gamma,
                                                              const float* __restrict__ k_gamma, long long T, int C,
@@ -795,65 +801,77 @@ __global__ void __launch_bounds__(256) qk_norm_rotary_kernel(__nv_bfloat16* __re
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   const int d0 = (lane * 8) % Dh;          // channel within the head of this lane's chunks
+  // heads of up to 64 channels have no more than 32 angles: each is formed by one lane, the others take it from there
+  const bool shared = Dh <= 64;
   float inv[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e)
-    inv[e] = d0 + 2 * e < rot ? powf(base, -static_cast<float>(d0 + 2 * e) / static_cast<float>(rot)) : 0.f;
-  for (long long t = static_cast<long long>(blockIdx.x) * wpb + (threadIdx.x >> 5); t < T;
-       t += static_cast<long long>(gridDim.x) * wpb) {
-    __nv_bfloat16* row = qkv + t * 3 * C;
-    uint4 raw[2][CHUNKS];
+  for (int e = 0; e < 4; ++e) {
+    const int ch = shared ? 2 * (lane % (Dh / 2)) : d0 + 2 * e;
+    inv[e] = 0.f;                                                         // beyond rot: angle 0, the identity
+    if ((e == 0 || !shared) && ch < rot) inv[e] = powf(base, -static_cast<float>(ch) / static_cast<float>(rot));
+  }
+  for (long long i = static_cast<long long>(blockIdx.x) * wpb + (threadIdx.x >> 5); i < 2 * T;
+       i += static_cast<long long>(gridDim.x) * wpb) {
+    const long long t = i >> 1;
+    const int h = static_cast<int>(i & 1);
+    __nv_bfloat16* row = qkv + t * 3 * C + h * C;
+    uint4 raw[CHUNKS];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int k = 0; k < CHUNKS; ++k) {
-        const int c = k * 256 + lane * 8;
-        raw[h][k] = c < C ? *reinterpret_cast<const uint4*>(row + h * C + c) : make_uint4(0u, 0u, 0u, 0u);
-      }
+    for (int k = 0; k < CHUNKS; ++k) {
+      const int c = k * 256 + lane * 8;
+      raw[k] = c < C ? *reinterpret_cast<const uint4*>(row + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
     float cs[4], sn[4];
     const float ps = static_cast<float>(pos[t]);
+    if (shared) {
+      float s1, c1;
+      sincosf(ps * inv[0], &s1, &c1);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) sincosf(ps * inv[e], &sn[e], &cs[e]);   // beyond rot: angle 0, the identity
+      for (int e = 0; e < 4; ++e) {
+        sn[e] = __shfl_sync(0xffffffffu, s1, d0 / 2 + e);
+        cs[e] = __shfl_sync(0xffffffffu, c1, d0 / 2 + e);
+      }
+    } else {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float sum = 0.f;
+      for (int e = 0; e < 4; ++e) sincosf(ps * inv[e], &sn[e], &cs[e]);
+    }
+    float sum = 0.f;
 #pragma unroll
-      for (int k = 0; k < CHUNKS; ++k) {
+    for (int k = 0; k < CHUNKS; ++k) {
+      float v[8];
+      unpack8(raw[k], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum += v[j];
+    }
+    const float mu = warp_sum(sum) / C;
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < CHUNKS; ++k)
+      if (k * 256 + lane * 8 < C) {
         float v[8];
-        unpack8(raw[h][k], v);
+        unpack8(raw[k], v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sum += v[j];
+        for (int j = 0; j < 8; ++j) ss += (v[j] - mu) * (v[j] - mu);
       }
-      const float mu = warp_sum(sum) / C;
-      float ss = 0.f;
+    const float rs = rsqrtf(warp_sum(ss) / C + eps);
+    const float* gamma = h == 0 ? q_gamma : k_gamma;
 #pragma unroll
-      for (int k = 0; k < CHUNKS; ++k)
-        if (k * 256 + lane * 8 < C) {
-          float v[8];
-          unpack8(raw[h][k], v);
+    for (int k = 0; k < CHUNKS; ++k) {
+      const int c = k * 256 + lane * 8;
+      if (c >= C) continue;
+      const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + c));
+      const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + c + 4));
+      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+      float v[8], o[8];
+      unpack8(raw[k], v);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) ss += (v[j] - mu) * (v[j] - mu);
-        }
-      const float rs = rsqrtf(warp_sum(ss) / C + eps);
-      const float* gamma = h == 0 ? q_gamma : k_gamma;
+      for (int j = 0; j < 8; ++j) v[j] = (v[j] - mu) * rs * g[j];
 #pragma unroll
-      for (int k = 0; k < CHUNKS; ++k) {
-        const int c = k * 256 + lane * 8;
-        if (c >= C) continue;
-        const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + c));
-        const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + c + 4));
-        const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        float v[8], o[8];
-        unpack8(raw[h][k], v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = (v[j] - mu) * rs * g[j];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          o[2 * e] = v[2 * e] * cs[e] - v[2 * e + 1] * sn[e];
-          o[2 * e + 1] = v[2 * e + 1] * cs[e] + v[2 * e] * sn[e];
-        }
-        *reinterpret_cast<uint4*>(row + h * C + c) = pack8(o);
+      for (int e = 0; e < 4; ++e) {
+        o[2 * e] = v[2 * e] * cs[e] - v[2 * e + 1] * sn[e];
+        o[2 * e + 1] = v[2 * e + 1] * cs[e] + v[2 * e] * sn[e];
       }
+      *reinterpret_cast<uint4*>(row + c) = pack8(o);
     }
   }
 }
@@ -1210,12 +1228,11 @@ extern "C" int ubm_qk_norm_rotary(void* qkv, const void* pos, const void* q_gamm
       rot > Dh || (rot & 1) || (reinterpret_cast<uintptr_t>(qkv) & 15) || (reinterpret_cast<uintptr_t>(q_gamma) & 15) ||
       (reinterpret_cast<uintptr_t>(k_gamma) & 15))
     return UBM_ERR_ARGUMENT;
-  const int grid = seq_grid(T, 8);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define UBM_QKN(CH)                                                                                                  \
-  qk_norm_rotary_kernel<CH><<<grid, 256, 0, st>>>(static_cast<__nv_bfloat16*>(qkv), static_cast<const int*>(pos),    \
-                                                  static_cast<const float*>(q_gamma),                                \
-                                                  static_cast<const float*>(k_gamma), T, C, Dh, rot, eps, base)
+  qk_norm_rotary_kernel<CH><<<static_cast<unsigned>(std::min<long long>((2 * T + 7) / 8, sm_count() * qkn_ctas(CH))), 256, 0, st>>>( \
+      static_cast<__nv_bfloat16*>(qkv), static_cast<const int*>(pos), static_cast<const float*>(q_gamma),            \
+      static_cast<const float*>(k_gamma), T, C, Dh, rot, eps, base)
   if (C <= 256) UBM_QKN(1);
   else if (C <= 512) UBM_QKN(2);
   else if (C <= 1024) UBM_QKN(4);
