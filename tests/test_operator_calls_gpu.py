@@ -56,6 +56,25 @@ def test_triangle_attention_masks(N, starting):
         pair.triangle_attention_fused(z[0], m._packed, starting, keep=torch.ones((N - 1, N), device="cuda"))
 
 
+@pytest.mark.parametrize("starting", [True, False])
+@pytest.mark.parametrize("N", [16, 77])
+def test_triangle_attention_outputs_of_other_forms(N, starting):
+    """An fp32 output holds the sums before their rounding, rows of a wider buffer the result itself; the rest of it is left alone."""
+    from uplifting_biomolecular_modeling_b200.ops import pair
+    m = _module(lambda p: p.TriangleAttention(starting=starting))
+    g = torch.Generator(device="cuda").manual_seed(N)
+    z = _rand(g, 1, N, N, 128)
+    keep = (torch.rand((N, N), device="cuda", generator=g) < 0.7) | torch.eye(N, device="cuda", dtype=torch.bool)
+    m(z)                                                                    # packs the weights
+    ref = pair.triangle_attention_fused(z[0], m._packed, starting, keep=keep)
+    wide = torch.full((N, N, 192), 7.0, device="cuda", dtype=BF)
+    pair.triangle_attention_fused(z[0], m._packed, starting, keep=keep, out=wide[:, :, :128])
+    assert torch.equal(wide[:, :, :128], ref) and bool((wide[:, :, 128:] == 7).all())
+    full = torch.empty((N, N, 128), device="cuda")
+    pair.triangle_attention_fused(z[0], m._packed, starting, keep=keep, out=full)
+    assert torch.equal(full.to(BF), ref) and not torch.equal(full, ref.float())
+
+
 @pytest.mark.parametrize("B,N,c,heads", [(1, 5, 384, 16), (2, 137, 384, 16), (3, 200, 768, 16), (1, 64, 128, 4)])
 @pytest.mark.parametrize("epilogue", ["plain", "gate", "slice"])
 @pytest.mark.parametrize("masked", [False, True])

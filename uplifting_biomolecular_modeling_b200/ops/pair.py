@@ -92,13 +92,25 @@ class TransitionPacked:
         return cls(wab, wo, colsum, colbias, hidden)
 
 
+def _result(out: Optional[torch.Tensor], like: torch.Tensor, rows_apart: bool = False) -> torch.Tensor:
+    """A new result in the form of ``like``, or the caller's ``out``: the kernels write it by its address alone, so it has to be bf16 on
+    the same GPU with its elements side by side; with ``rows_apart`` (its rows are addressed block by block) of the same shape, too."""
+    if out is None:
+        return torch.empty_like(like)
+    if out.dtype != torch.bfloat16 or out.device != like.device or not out.is_contiguous() or out.numel() != like.numel() or \
+            (rows_apart and out.shape != like.shape):
+        raise ValueError(f"output of shape {tuple(out.shape)} ({out.dtype}, {out.device}) does not hold a contiguous bf16 result of shape "
+                         f"{tuple(like.shape)} on {like.device}")
+    return out
+
+
 def transition_fused(x: torch.Tensor, w: TransitionPacked, residual: bool = True,
                      out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x: bf16 [..., 128] contiguous.  Returns x + transition(x) (or the update alone)."""
     if x.dtype != torch.bfloat16 or x.shape[-1] != 128 or not x.is_contiguous():
         raise ValueError("transition_fused expects a contiguous bf16 tensor with 128 channels")
     R = x.numel() // 128
-    out = torch.empty_like(x) if out is None else out
+    out = _result(out, x)
     st = native.status_tensor(x.device)
     rc = native.lib().ubm_transition(native.ptr(x), native.ptr(w.wab), native.ptr(w.wo), native.ptr(w.colsum),
                                      native.ptr(w.colbias), 0, 0, native.ptr(out), R, w.hidden,
@@ -170,6 +182,7 @@ def _trimul_blocked(z, m, w: TrimulPacked, outgoing: bool, residual: bool, out, 
     N = z.shape[0]
     Np = ceil_to(N, PLANE_ROW)
     dev = z.device
+    out = _result(out, z, rows_apart=True)
     key = ("trimul_blocked", N, rb, dev)
     if key not in ws:
         ws[key] = (torch.empty((2, 128, N, Np), dtype=torch.bfloat16, device=dev),
@@ -181,7 +194,6 @@ def _trimul_blocked(z, m, w: TrimulPacked, outgoing: bool, residual: bool, out, 
     rc = lib.ubm_trimul_proj(native.ptr(z), native.ptr(w.w_in), native.ptr(w.in_colsum), native.ptr(w.in_colbias),
                              native.ptr(m), native.ptr(planes), 0, N, Np, native.ptr(st), stream)
     native.check(rc, "ubm_trimul_proj")
-    out = torch.empty_like(z) if out is None else out
     for r0 in range(0, N, rb):
         r1 = min(N, r0 + rb)
         xv = xb.view(-1)[: 128 * (r1 - r0) * Np].view(128, r1 - r0, Np)
@@ -221,6 +233,7 @@ def trimul_fused(z: torch.Tensor, mask: Optional[torch.Tensor], w: TrimulPacked,
     if 0 < rb < N:
         m = None if mask is None else mask.to(torch.float32).contiguous()
         return _trimul_blocked(z, m, w, outgoing, residual, out, ws, rb // 8 * 8 or 8)
+    out = _result(out, z)
     planes, x = _trimul_scratch(ws, N, Np, dev)
     kind = 0
     if mask is not None:
@@ -228,7 +241,6 @@ def trimul_fused(z: torch.Tensor, mask: Optional[torch.Tensor], w: TrimulPacked,
         kind = 2 if mask.dtype == torch.bfloat16 and mask.shape == (N, N) and mask.device == dev and mask.is_contiguous() else 1
         if kind == 1:
             mask = mask.to(torch.float32).contiguous()
-    out = torch.empty_like(z) if out is None else out
     rc = native.lib().ubm_trimul(_TRIMUL_ARGS.pack(
         z.data_ptr(), 0 if mask is None else mask.data_ptr(), kind, *w.pointers(), planes.data_ptr(), x.data_ptr(), out.data_ptr(), N, Np,
         1 if outgoing else 0, 1 if residual else 0, native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
@@ -563,6 +575,26 @@ def _triatt_scratch(ws: dict, N: int, Np: int, heads: int, dev) -> tuple:
     return ws[key]
 
 
+def _triatt_into(z, w: TriattPacked, starting: bool, residual: bool, out, ws: dict, mask):
+    """The launches of :func:`triangle_attention_fused` one by one, for an ``out`` that only the output product can write: fp32, or
+    rows of [N * N, 128] in a wider buffer."""
+    N, dev = z.shape[0], z.device
+    Np = ceil_to(N, 8)
+    to = out.view(N * N, 128)
+    if out.dtype not in (torch.bfloat16, torch.float32) or out.device != dev:
+        raise ValueError(f"triangle attention writes bf16 or fp32 on {dev}, not {out.dtype} on {out.device}")
+    qkvgo, hb = _triatt_scratch(ws, N, Np, w.heads, dev)
+    q, k, v, g, og = qkvgo
+    rc = native.lib().ubm_triatt_proj(native.ptr(z), native.ptr(w.w), native.ptr(w.colsum), native.ptr(w.colbias), native.ptr(w.wb),
+                                      native.ptr(w.wb_colsum), native.ptr(w.wb_colbias), native.ptr(q), native.ptr(k), native.ptr(v),
+                                      native.ptr(g), native.ptr(hb), 0, N, Np, w.heads, 0 if starting else 1,
+                                      native.ptr(native.status_tensor(dev)), native.current_stream(dev))
+    native.check(rc, "ubm_triatt_proj")
+    attention_d32(q, k, v, hb, g, og, rows=N, Nq=N, Nk=N, H=w.heads, ldb=Np, transpose_out=not starting, mask=mask)
+    _gemm.gemm(og, w.wo, bias=w.bo, residual=z.view(N * N, 128) if residual else None, out=to)
+    return out
+
+
 def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, residual: bool = True,
                              out: Optional[torch.Tensor] = None, workspace: Optional[dict] = None,
                              mask: Optional[KeyMask] = None, keep: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -582,6 +614,11 @@ def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, r
         if keep is not None:
             mask = KeyMask.lay_out(keep, (N, N), dev)
         return _triatt_blocked(z, w, starting, residual, out, ws, mask, rb)
+    if out is not None and (out.dtype != torch.bfloat16 or not out.is_contiguous()):
+        if keep is not None:
+            mask = KeyMask.lay_out(keep, (N, N), dev)
+        return _triatt_into(z, w, starting, residual, out, ws, mask)
+    out = _result(out, z)
     add = flags = keep_ptr = keep_bytes = keep_row = keep_key = ld_mask = 0
     if keep is not None:
         keep = KeyMask.readable(keep, (N, N), dev)
@@ -599,7 +636,6 @@ def triangle_attention_fused(z: torch.Tensor, w: TriattPacked, starting: bool, r
             raise ValueError(f"key mask of shape {tuple(mask.add.shape)} does not cover [{N}, {N}]")
         add, flags, ld_mask = mask.add.data_ptr(), mask.flags.data_ptr(), mask.add.stride(0)
     qkvgo, hb = _triatt_scratch(ws, N, Np, w.heads, dev)
-    out = torch.empty_like(z) if out is None else out
     rc = native.lib().ubm_triatt(_TRIATT_ARGS.pack(
         z.data_ptr(), keep_ptr, keep_bytes, keep_row, keep_key, add, flags, ld_mask, *w.pointers(), qkvgo.data_ptr(), hb.data_ptr(), out.data_ptr(), N, Np, w.heads,
         1 if starting else 0, 1 if residual else 0, native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
