@@ -102,3 +102,65 @@ def test_outputs_of_row_blocks_keep_their_shape(launches):
     assert not launches
     out = torch.zeros(32, 32, 128, dtype=BF)
     assert _trimul(z, out, {"row_block": 16}) is out
+
+
+class _OnGpu(torch.Tensor):
+    """A tensor of the CPU that says it is on a GPU, so that the forms for one are chosen."""
+    is_cuda = property(lambda self: True)
+
+
+def _gpu(*shape, dtype=BF):
+    return torch.zeros(shape, dtype=dtype).as_subclass(_OnGpu)
+
+
+def _apb_weights(c, heads):
+    r = lambda *s: torch.randn(s)  # noqa: E731
+    return pair.ApbPacked.pack(r(c, c), r(c), r(c, c), r(c, c), r(c, c), r(c, c), heads)
+
+
+@pytest.mark.parametrize("c", [376, 392, 768])
+def test_attention_rows_of_another_width_are_refused(launches, c):
+    planes = torch.zeros(16, 8, 8, dtype=BF)
+    with pytest.raises(ValueError):
+        pair.apb_fused(_gpu(1, 8, c), _apb_weights(384, 16), planes, 8)
+    assert not launches
+    pair.apb_fused(_gpu(1, 8, 384), _apb_weights(384, 16), planes, 8)
+    assert _names(launches) == ["ubm_apb"]
+
+
+def test_an_output_projection_of_another_width_is_refused(launches):
+    w = _apb_weights(384, 16)
+    w.wo = w.wo[:, :-32].contiguous()
+    with pytest.raises(ValueError):
+        pair.apb_fused(_gpu(1, 8, 384), w, torch.zeros(16, 8, 8, dtype=BF), 8)
+    assert "ubm_apb" not in _names(launches)
+
+
+@pytest.mark.parametrize("w12,w3,residual", [((512, 72), (64, 256), True), ((512, 56), (64, 256), True), ((256, 64), (64, 256), True),
+                                             ((576, 64), (64, 256), True), ((512, 64), (32, 256), True)])
+def test_transition_weights_of_another_size_are_refused(launches, w12, w3, residual):
+    x = torch.zeros(9, 64, dtype=BF)
+    with pytest.raises(ValueError):
+        pair.transition_rows(x, None, None, 1e-5, torch.zeros(w12, dtype=BF), torch.zeros(w3, dtype=BF), residual)
+    with pytest.raises(ValueError):
+        pair.transition_rows(x.float(), None, None, 1e-5, torch.zeros(512, 64, dtype=BF), torch.zeros(64, 256, dtype=BF), True)
+    assert not launches
+    pair.transition_rows(x, None, None, 1e-5, torch.zeros(512, 64, dtype=BF), torch.zeros(64, 256, dtype=BF), True)
+    assert _names(launches) == ["ubm_transition_rows"]
+
+
+@pytest.mark.parametrize("c", [64, 256])
+def test_atom_weights_of_another_width_are_refused(launches, c):
+    """Rows of 128 channels with weights packed for others: the projections one by one say so."""
+    from uplifting_biomolecular_modeling_b200.ops import atom
+    r = lambda *s: torch.randn(s)  # noqa: E731
+    a, rows = _gpu(1, 64, 128), _gpu(64, 128)
+    w = pair.ApbPacked.pack(r(128, c), r(128), r(128, c), r(128, c), r(128, c), r(128, 128), 4)
+    with pytest.raises(ValueError):
+        atom.attention(a, rows, rows, w, _gpu(1, 4, 2, 32, 128), rows)
+    with pytest.raises(ValueError):
+        atom.transition(_gpu(1, 256, 128), _gpu(256, 128), _gpu(256, 128), _gpu(256, 128), _gpu(768, c), _gpu(128, 256))
+    assert set(_names(launches)) <= {"ubm_adaln_rows"}
+    atom.attention(a, rows, rows, _apb_weights(128, 4), _gpu(1, 4, 2, 32, 128), rows)
+    atom.transition(_gpu(1, 256, 128), _gpu(256, 128), _gpu(256, 128), _gpu(256, 128), _gpu(768, 128), _gpu(128, 256))
+    assert _names(launches)[-3:] == ["ubm_atom_qkvg", "ubm_window_layer", "ubm_cond_transition"]

@@ -42,7 +42,8 @@ def _plain(t: torch.Tensor) -> bool:
 
 
 def _window_serves(w: pair.ApbPacked, bias: torch.Tensor, B: int, A: int, c: int) -> bool:
-    return (pair.WINDOW_KERNEL == "tc" and c == C and w.H == 4 and w.Dp == 32 and w.wo.shape[0] == C and A % 32 == 0 and A > 0
+    return (pair.WINDOW_KERNEL == "tc" and c == C and w.wqkvg.shape == (4 * C, C) and w.H == 4 and w.Dp == 32 and
+            w.wo.shape == (C, C) and A % 32 == 0 and A > 0
             and (bias is None or (_plain(bias) and bias.shape[0] in (1, B))))
 
 
@@ -82,7 +83,7 @@ def transition(a: torch.Tensor, scale: torch.Tensor, shift: torch.Tensor, gate: 
     :func:`ops.gemm.pack_swiglu3` lays them out."""
     B, A, c = a.shape
     R = B * A
-    if c == C and packed and _plain(a) and w_out.shape[0] == C and w_in.shape[0] == 3 * w_out.shape[1]:
+    if c == C and packed and _plain(a) and w_out.shape[0] == C and w_in.shape == (3 * w_out.shape[1], C):
         sc, sh, gt = _rows_of(scale, R), _rows_of(shift, R), _gate_of(gate, R)
         if (sc is not None and sh is not None and gt is not None and sc.shape == sh.shape == gt.shape
                 and sc.stride(0) == sh.stride(0) and sc.shape[0] >= 128):

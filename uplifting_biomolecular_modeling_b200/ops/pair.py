@@ -124,6 +124,9 @@ def transition_rows(x: torch.Tensor, norm_w, norm_b, eps: float, w12: torch.Tens
     from . import rows as _rows
     R, dim = x.shape
     out_dim, hidden = w3.shape
+    if w12.shape != (2 * hidden, dim) or (residual and out_dim != dim) or x.dtype != torch.bfloat16 or w12.dtype != torch.bfloat16 or \
+            w3.dtype != torch.bfloat16 or not x.is_contiguous() or not w12.is_contiguous() or not w3.is_contiguous():
+        raise ValueError(f"transition_rows: contiguous bf16 rows and weights, {tuple(w12.shape)} and {tuple(w3.shape)} for {tuple(x.shape)}")
     dev = x.device
     g, b = _rows._f32_param(norm_w), _rows._f32_param(norm_b)
     scratch = torch.empty(R * (dim + hidden), dtype=torch.bfloat16, device=dev)      # norm rows, then hidden rows
@@ -451,7 +454,9 @@ def apb_fused(x: torch.Tensor, w: ApbPacked, bias_planes: torch.Tensor, ldb: int
         keep = KeyMask.readable(keep, (B, N), x.device)
         if keep.shape != (B, N):
             keep, mask = None, KeyMask.lay_out(keep, None, x.device)
-    if x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and _one_call(out_gate, out_residual, B * N, c_out):
+    # (the weights' sizes too: the library has only their addresses, one by one the products refuse what does not fit)
+    if x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and w.wqkvg.shape == (4 * HD, c) and w.wo.shape[1] == HD and \
+            _one_call(out_gate, out_residual, B * N, c_out):
         dev = x.device
         rows_bytes = 2 * B * N * HD                     # scratch: q | k | v | gate rows, o, additive mask rows and their flags
         ld_mask = add = flags = mask_bytes = keep_ptr = keep_bytes = keep_row = keep_key = 0
@@ -498,6 +503,9 @@ def single_track(s: torch.Tensor, z: torch.Tensor, keep: Optional[torch.Tensor],
     N, c = s.shape[1:]
     dev = s.device
     hidden = w3.shape[1]
+    if w.wqkvg.shape != (4 * w.H * w.Dp, c) or w.wo.shape != (c, w.H * w.Dp) or w12.shape != (2 * hidden, c) or w3.shape[0] != c or \
+            bias[0].shape != (w.H, 128) or z.shape != (1, N, N, 128):
+        raise ValueError(f"single_track: weights of other sizes than {tuple(s.shape)} and {tuple(z.shape)} take")
     ldb, ld_mask, HD = ceil_to(N, 8), ceil_to(N, MASK_STEP), w.H * w.Dp
     row = 2 * N * c                                         # one [N, c] in bf16
     sizes = (2 * w.H * N * ldb, row, 8 * N * HD, 2 * N * HD, row, 2 * row, row, 2 * N * hidden, 2 * ld_mask, ld_mask // MASK_STEP)
