@@ -76,26 +76,37 @@ def mean_rescale_(o: torch.Tensor, count: torch.Tensor, bias: torch.Tensor, tota
     return o
 
 
-_HB_CACHE = {}
+_HB_CACHE: dict = {}
+
+
+def _kept(t: Optional[torch.Tensor]):
+    """What tells later whether ``t`` is still the tensor, with the contents, that something was made from: the object (weakly), its
+    version, and its storage, held so that no other can have its address (a converted copy swaps ``.data`` and leaves the version)."""
+    return None if t is None else (weakref.ref(t), t._version, t.detach())
+
+
+def _unchanged(kept, t: Optional[torch.Tensor]) -> bool:
+    if kept is None or t is None:
+        return kept is None and t is None
+    return kept[0]() is t and kept[1] == t._version and kept[2].data_ptr() == t.data_ptr() and kept[2].dtype == t.dtype
 
 
 def _head_bias_weights(w: torch.Tensor, ln_w, ln_b, scale: float, device) -> tuple:
-    """(fp32 weights with the norm's scale folded in, their row sums, their products with the norm's shift), kept per weight."""
-    # the cache entry is tied to the live weight tensor object (a freed tensor's address may be reused)
-    key = (id(w), w._version, None if ln_w is None else ln_w._version, float(scale), str(device))
+    """(fp32 weights with the norm's scale folded in, their row sums, their products with the norm's shift), kept until the weight or
+    either parameter of the norm is another one or is written."""
+    key = (id(w), float(scale), str(device))
     entry = _HB_CACHE.get(key)
-    packed = entry[1] if entry is not None and entry[0]() is w else None
-    if packed is None:
-        gam = torch.ones(128, device=device) if ln_w is None else ln_w.detach().float()
-        wf = (w.detach().float() * gam[None, :] * scale).contiguous()
-        colsum = wf.sum(1).contiguous()
-        colbias = torch.zeros(w.shape[0], device=device) if ln_b is None else \
-            ((w.detach().float() @ ln_b.detach().float()) * scale).contiguous()
-        packed = (wf, colsum, colbias)
-        if len(_HB_CACHE) > 4096:
-            _HB_CACHE.clear()
-        _HB_CACHE[key] = (weakref.ref(w), packed)
-    return packed
+    if entry is not None and _unchanged(entry[0], w) and _unchanged(entry[1], ln_w) and _unchanged(entry[2], ln_b):
+        return entry[3]
+    gam = torch.ones(128, device=device) if ln_w is None else ln_w.detach().float()
+    wf = (w.detach().float() * gam[None, :] * scale).contiguous()
+    colsum = wf.sum(1).contiguous()
+    colbias = torch.zeros(w.shape[0], device=device) if ln_b is None else \
+        ((w.detach().float() @ ln_b.detach().float()) * scale).contiguous()
+    if len(_HB_CACHE) > 4096:
+        _HB_CACHE.clear()
+    _HB_CACHE[key] = (_kept(w), _kept(ln_w), _kept(ln_b), (wf, colsum, colbias))
+    return wf, colsum, colbias
 
 
 def pair_head_bias(z: torch.Tensor, ln_w, ln_b, w, scale: float = 1.0, transpose: bool = False,
@@ -119,8 +130,7 @@ def pair_head_bias(z: torch.Tensor, ln_w, ln_b, w, scale: float = 1.0, transpose
         Np = (N + row - 1) // row * row
         make = torch.zeros if Np != N else torch.empty       # the kernel writes no padding
         out = make((H, N, Np), dtype=torch.bfloat16, device=z.device)
-    packed = _head_bias_weights(w, ln_w, ln_b, scale, z.device)
-    wf, colsum, colbias = packed
+    wf, colsum, colbias = _head_bias_weights(w, ln_w, ln_b, scale, z.device)
     rc = native.lib().ubm_pair_head_bias(native.ptr(z), native.ptr(wf), native.ptr(colsum), native.ptr(colbias),
                                          native.ptr(out), N, Np, H, 1 if transpose else 0,
                                          native.current_stream(z.device))
