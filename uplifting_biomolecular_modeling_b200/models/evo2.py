@@ -820,15 +820,25 @@ BYTE_LUT = {c: i for i, c in enumerate("ACGTN")}
 _W_CACHE: dict = {}
 
 
+def _source(t: Optional[torch.Tensor]) -> tuple:
+    """What a form kept of a parameter is compared by: the object, its version and its storage (a converted or sharded copy swaps ``.data``
+    and leaves the version as it is)."""
+    return (None, 0, 0, ()) if t is None else (t, t._version, t.data_ptr(), t.shape)
+
+
+def _is_source(kept: tuple, t: Optional[torch.Tensor]) -> bool:
+    return kept[0] is t and (t is None or (kept[1] == t._version and kept[2] == t.data_ptr() and kept[3] == t.shape))
+
+
 def _bf16_weight(module: nn.Linear):
-    """(contiguous bf16 weight, fp32 bias or None) of a linear layer, kept until the weight is written again."""
-    key = id(module)
-    ent = _W_CACHE.get(key)
-    weight = module.weight               # one look-up: a module's attributes are found through its dictionaries
-    if ent is None or ent[0] is not weight or ent[1] != weight._version:
-        ent = (module.weight, module.weight._version, module.weight.detach().to(torch.bfloat16).contiguous(),
-               None if module.bias is None else module.bias.detach().float().contiguous())
-        _W_CACHE[key] = ent
+    """(contiguous bf16 weight, fp32 bias or None) of a linear layer, kept until either is written again or given other storage."""
+    ent = _W_CACHE.get(id(module))
+    weight, bias = module.weight, module.bias           # one look-up each: a module's attributes are found through its dictionaries
+    if ent is None or not _is_source(ent[0], weight) or not _is_source(ent[1], bias):
+        # (the storages are held along, so that no others can have their addresses)
+        ent = (_source(weight), _source(bias), weight.detach().to(torch.bfloat16).contiguous(),
+               None if bias is None else bias.detach().float().contiguous(), weight.detach(), None if bias is None else bias.detach())
+        _W_CACHE[id(module)] = ent
     return ent[2], ent[3]
 
 
@@ -860,12 +870,12 @@ def fp8_projection(module: nn.Linear, x: torch.Tensor, norm: "RMSNorm") -> torch
 def _e4m3_weight(module: nn.Linear):
     """(e4m3 weight, its dequantisation factor, fp32 bias or None), quantised once per weight version."""
     from ..ops import gemm
-    w = module.weight
+    w, bias = module.weight, module.bias
     ent = _W8_CACHE.get(id(module))
-    ver = (w._version, w.data_ptr(), tuple(w.shape))
-    if ent is None or ent[0] is not w or ent[1] != ver:
+    if ent is None or not _is_source(ent[0], w) or not _is_source(ent[1], bias):
         q, dq = gemm.quantize_e4m3(w)
-        ent = (w, ver, q, dq, None if module.bias is None else module.bias.detach().float().contiguous())
+        # (unlike the storage of a bf16 form, which is the weight's own, that behind these bytes may go)
+        ent = (_source(w), _source(bias), q, dq, None if bias is None else bias.detach().float().contiguous())
         _W8_CACHE[id(module)] = ent
     return ent[2], ent[3], ent[4]
 
