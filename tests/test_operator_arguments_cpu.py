@@ -164,3 +164,33 @@ def test_atom_weights_of_another_width_are_refused(launches, c):
     atom.attention(a, rows, rows, _apb_weights(128, 4), _gpu(1, 4, 2, 32, 128), rows)
     atom.transition(_gpu(1, 256, 128), _gpu(256, 128), _gpu(256, 128), _gpu(256, 128), _gpu(768, 128), _gpu(128, 256))
     assert _names(launches)[-3:] == ["ubm_atom_qkvg", "ubm_window_layer", "ubm_cond_transition"]
+
+
+@pytest.mark.parametrize("workspace", [{}, {"row_block": 16}])
+@pytest.mark.parametrize("shape", [(20, 20), (1, 20), (20, 1), (1, 1), (20,), (400,), (1, 20, 20)])
+def test_masks_of_a_triangle_multiplication_cover_it(monkeypatch, launches, workspace, shape):
+    """What stands where the kernel will read N * N values."""
+    import ctypes
+    N, seen = 20, []
+
+    class Reader:
+        def __getattr__(self, name):
+            def call(*args):
+                if name in ("ubm_trimul", "ubm_trimul_proj"):
+                    at = pair._TRIMUL_ARGS.unpack(args[0])[1] if name == "ubm_trimul" else args[4]
+                    seen.append(torch.frombuffer(bytearray(ctypes.string_at(at, 4 * N * N)), dtype=torch.float32).view(N, N))
+                return 0
+            return call
+
+    monkeypatch.setattr(native, "lib", lambda: Reader())
+    mask = torch.rand(shape)
+    pair.trimul_fused(torch.zeros(N, N, 128, dtype=BF), mask, _trimul_weights(), True, workspace=dict(workspace))
+    assert len(seen) == 1 and torch.equal(seen[0], mask.reshape(N, N) if mask.numel() == N * N else mask.expand(N, N))
+
+
+@pytest.mark.parametrize("workspace", [{}, {"row_block": 16}])
+@pytest.mark.parametrize("shape", [(19, 20), (19, 19), (20, 21), (399,), (2, 20, 20)])
+def test_masks_of_another_size_are_refused(launches, workspace, shape):
+    with pytest.raises(RuntimeError):
+        pair.trimul_fused(torch.zeros(20, 20, 128, dtype=BF), torch.zeros(shape), _trimul_weights(), True, workspace=dict(workspace))
+    assert not launches

@@ -223,7 +223,7 @@ def _trimul_scratch(ws: dict, N: int, Np: int, dev) -> tuple:
 def trimul_fused(z: torch.Tensor, mask: Optional[torch.Tensor], w: TrimulPacked, outgoing: bool,
                  residual: bool = True, out: Optional[torch.Tensor] = None,
                  workspace: Optional[dict] = None) -> torch.Tensor:
-    """z: bf16 [N, N, 128] contiguous; mask: [N, N] or None.  Three launches: projection ->
+    """z: bf16 [N, N, 128] contiguous; mask: [N, N], sizes of one broadcast to it, or None.  Three launches: projection ->
     batched tcgen05 contraction -> output stage.  With ``workspace["row_block"]`` set (the ``chunk_pair_ops`` lever)
     and smaller than N, contraction and output stage run per block of rows (see :func:`_trimul_blocked`)."""
     if z.dtype != torch.bfloat16 or z.dim() != 3 or z.shape[-1] != 128 or not z.is_contiguous():
@@ -233,8 +233,11 @@ def trimul_fused(z: torch.Tensor, mask: Optional[torch.Tensor], w: TrimulPacked,
     dev = z.device
     ws = workspace if workspace is not None else {}
     rb = int(ws.get("row_block", 0) or 0)
+    if mask is not None and mask.shape != (N, N):
+        # the kernel reads N * N values in this order; one row or column stands for all
+        mask = mask.reshape(N, N) if mask.numel() == N * N else mask.expand(N, N)
     if 0 < rb < N:
-        m = None if mask is None else mask.to(torch.float32).contiguous()
+        m = None if mask is None else mask.to(dev, torch.float32).contiguous()
         return _trimul_blocked(z, m, w, outgoing, residual, out, ws, rb // 8 * 8 or 8)
     out = _result(out, z)
     planes, x = _trimul_scratch(ws, N, Np, dev)
@@ -243,7 +246,7 @@ def trimul_fused(z: torch.Tensor, mask: Optional[torch.Tensor], w: TrimulPacked,
         # a bf16 mask of the pair tensor is read as it is; others are converted
         kind = 2 if mask.dtype == torch.bfloat16 and mask.shape == (N, N) and mask.device == dev and mask.is_contiguous() else 1
         if kind == 1:
-            mask = mask.to(torch.float32).contiguous()
+            mask = mask.to(dev, torch.float32).contiguous()
     rc = native.lib().ubm_trimul(_TRIMUL_ARGS.pack(
         z.data_ptr(), 0 if mask is None else mask.data_ptr(), kind, *w.pointers(), planes.data_ptr(), x.data_ptr(), out.data_ptr(), N, Np,
         1 if outgoing else 0, 1 if residual else 0, native.status_tensor(dev).data_ptr(), native.current_stream(dev)))
