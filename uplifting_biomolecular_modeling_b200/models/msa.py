@@ -21,8 +21,9 @@ from .pairformer import PairformerLayer, Transition, _Switchable, plain_linears
 
 
 class OuterProductMean(_Switchable):
-    ROW_BLOCK = 128             # rows of the outer product in one block at least,
-    SCRATCH = 2 << 30           # and as many as these bytes hold where ``row_block`` has been left alone
+    ROW_BLOCK = 128             # rows of the outer product in one block,
+    SCRATCH = 2 << 30           # or as many as these bytes hold, where neither ``row_block`` nor the workspace's row block bounds memory
+    _no_room: Optional[int] = None      # bytes of a block that there was no memory for: no such block is asked for again
 
     def __init__(self, c_in: int = 64, c_hidden: int = 32, c_out: int = 128):
         super().__init__()
@@ -31,7 +32,7 @@ class OuterProductMean(_Switchable):
         self.proj_a = nn.Linear(c_in, c_hidden, bias=False)
         self.proj_b = nn.Linear(c_in, c_hidden, bias=False)
         self.proj_o = nn.Linear(c_hidden * c_hidden, c_out)
-        self.row_block = self.ROW_BLOCK
+        self.row_block: Optional[int] = None      # rows of a block, as asked for
         self.full_mask = False      # set by the caller when the MSA mask is known (on the host) to be all ones
 
     lever = "fused_opm"
@@ -92,7 +93,7 @@ class OuterProductMean(_Switchable):
             else:
                 count = torch.einsum("si,sj->ij", mk.float(), mk.float())
         blocked = c == 32 and (N * c) % 32 == 0
-        rb, t2 = self.row_block, None
+        rb, t2 = self.ROW_BLOCK if self.row_block is None else self.row_block, None
         if blocked:
             rb, t2 = self._block(N, m.device)
         for i0 in range(0, N, rb):
@@ -113,21 +114,23 @@ class OuterProductMean(_Switchable):
             out = (out.float() * (S / count.clamp(min=1.0)).unsqueeze(-1) + bo).to(torch.bfloat16)
         return out.unsqueeze(0)
 
-
     def _block(self, N: int, device) -> tuple:
         """(rows of a block, its scratch): few, equal blocks.  Blocks of 128 rows (0.2 GB at 768 tokens) end in waves that are nearly empty,
         twice each: 1502 us at 1024 sequences x 768 tokens against 1340 in one block (1352 in 16 that stay in L2), 1005 / 936 at 512 x
         768, 638 / 605 at 1024 x 512, 700 / 573 at 64 x 768, 109 / 85 at 1024 x 137."""
-        rows, per_row = self.row_block, N * self.c_hidden ** 2
-        if rows == self.ROW_BLOCK:
-            most = max(rows, self.SCRATCH // (2 * per_row))
-            blocks = -(-N // most)
-            grown = min(N, (-(-N // blocks) + 7) // 8 * 8)         # 8 tokens are a tile of 256 columns
-            if grown > rows:
-                try:
-                    return grown, torch.empty((grown * N, self.c_hidden ** 2), dtype=torch.bfloat16, device=device)
-                except torch.OutOfMemoryError:
-                    pass
+        rows, per_row = self.row_block, 2 * N * self.c_hidden ** 2
+        if rows is None:
+            rows = self.ROW_BLOCK
+            if not (self._workspace or {}).get("row_block"):
+                most = max(rows, self.SCRATCH // per_row // 8 * 8)
+                blocks = -(-N // most)
+                grown = min(N, (-(-N // blocks) + 7) // 8 * 8)         # 8 tokens are a tile of 256 columns
+                if grown > rows and (self._no_room is None or grown * per_row < self._no_room):
+                    try:
+                        return grown, torch.empty((grown * N, self.c_hidden ** 2), dtype=torch.bfloat16, device=device)
+                    except torch.OutOfMemoryError:
+                        # the attempt has emptied the allocator's cache: once, not on every call
+                        self._no_room = grown * per_row
         rows = min(rows, N)
         return rows, torch.empty((rows * N, self.c_hidden ** 2), dtype=torch.bfloat16, device=device)
 
