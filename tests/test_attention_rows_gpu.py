@@ -1,4 +1,4 @@
-"""Two-row forms of the attention kernel: groups that are not full between groups that are (row counts 1 to 7, several items per CTA),
+"""Two-row forms of the attention kernel: groups that are not full (row counts 1 to 7), alone and in front of full ones of the same CTA,
 and head dimension 64 without bias in steps of 128 keys, at key counts around its steps."""
 import pytest
 import torch
@@ -61,3 +61,32 @@ def test_groups_that_are_not_full(rows, D, H, N):
 @pytest.mark.parametrize("Nq,Nk", [(1, 1), (5, 5), (127, 127), (128, 128), (129, 129), (300, 64), (64, 257), (513, 513)])
 def test_no_bias_in_steps_of_128_keys(rows, Nq, Nk):
     assert _case(rows, Nq, Nk, 15, 64, False, False, Nq == Nk, Nq + Nk) < 5e-3
+
+
+def _full_after_partial(rows, N, H):
+    """Whether some CTA (items blockIdx, + grid, ..) takes a full group of two rows behind one with a missing row."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n_qt, n_rp = -(-N // 128), -(-rows // 2)
+    items = n_qt * n_rp * H
+    full = lambda item: item // n_qt % n_rp * 2 + 2 <= rows  # noqa: E731
+    return any(not full(a) and any(full(b) for b in range(a + sms, items, sms)) for a in range(items))
+
+
+# an odd number of key steps (five of 64, three of 128), so that a step counted wrongly is a phase counted wrongly
+@pytest.mark.parametrize("rows,D,H,bias,masked", [(5, 64, 40, True, False), (5, 64, 40, True, True), (5, 64, 40, False, True),
+                                                  (5, 64, 40, False, False), (3, 64, 40, True, True), (3, 32, 40, True, False),
+                                                  (3, 32, 40, True, True), (3, 32, 40, False, True)])
+def test_full_groups_behind_a_missing_row(rows, D, H, bias, masked):
+    N = 300
+    assert _full_after_partial(rows, N, H)
+    assert _case(rows, N, N, H, D, bias, masked, True, rows + H) < 5e-3
+
+
+def test_full_groups_behind_a_missing_row_in_steps_of_128_keys():
+    from uplifting_biomolecular_modeling_b200.ops import pair
+    pair.set_attention_variant(5)
+    try:
+        assert _full_after_partial(5, 300, 40)
+        assert _case(5, 300, 300, 40, 32, True, False, True, 2) < 5e-3
+    finally:
+        pair.set_attention_variant(0)
