@@ -40,3 +40,23 @@ def test_short_of_memory(monkeypatch):
 
     monkeypatch.setattr(msa.torch, "empty", short)
     assert op._block(300, "cuda")[0] == 128 and torch.equal(op(m, mask), ref)
+
+
+@pytest.mark.parametrize("N,scratch,blocks", [(301, 200 * 301 * 2048, [152, 149]), (425, 144 * 425 * 2048, [144, 144, 137]),
+                                              (1100, None, [552, 548])])
+def test_equal_blocks_with_a_shorter_last_one(N, scratch, blocks, monkeypatch):
+    """More than one block, each larger than 128 rows: the last one writes part of the scratch."""
+    from uplifting_biomolecular_modeling_b200.models import msa, pairformer
+    torch.manual_seed(N)
+    op = msa.OuterProductMean().cuda().to(BF).requires_grad_(False)
+    pairformer.set_impl(op, "fused")
+    m = torch.randn(1, 12, N, 64, device="cuda").to(BF)
+    mask = (torch.rand(1, 12, N, device="cuda") < 0.8).to(BF)
+    op.row_block = 128
+    ref = op(m, mask)
+    op.row_block = None
+    if scratch is not None:
+        monkeypatch.setattr(msa.OuterProductMean, "SCRATCH", scratch)
+    rows = op._block(N, "cuda")[0]
+    assert [min(rows, N - i) for i in range(0, N, rows)] == blocks
+    assert torch.equal(op(m, mask), ref)
