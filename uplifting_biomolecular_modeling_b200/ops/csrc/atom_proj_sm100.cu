@@ -129,12 +129,13 @@ atom_qkvg_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  grid_dependency_sync(short_grid(p.num_tiles, 8));
+  grid_dependency_wait();
   for (int i = threadIdx.x; i < 384; i += blockDim.x) sBias[i] = p.bias[i];
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 8));
   const uint32_t my_tiles =
       static_cast<uint32_t>(p.num_tiles) > blockIdx.x ? (p.num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
 
@@ -365,11 +366,12 @@ cond_transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  grid_dependency_sync(short_grid(p.num_tiles, 8));
+  grid_dependency_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 8));
   const uint32_t tY = tmem_base;           // 128 columns
   const uint32_t tAB = tmem_base + 128;    // three buffers of 96
   const uint32_t tH = tmem_base + 416;     // two buffers of 16 (two bf16 a column)

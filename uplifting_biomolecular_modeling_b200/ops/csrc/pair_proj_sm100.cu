@@ -121,7 +121,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  grid_dependency_sync(short_grid(p.num_tiles, 4));
+  grid_dependency_wait();
   // column constants
   for (int i = threadIdx.x; i < 512; i += blockDim.x) {
     sColsum[i] = p.colsum[i];
@@ -131,6 +131,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 4));
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer

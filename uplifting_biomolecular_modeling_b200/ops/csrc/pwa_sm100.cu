@@ -143,11 +143,12 @@ pwa_value_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant_
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
-  grid_dependency_sync(short_grid(p.num_tiles, 4));
+  grid_dependency_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 4));
 
   if (warp == 0) {
     if (lane == 0) {
@@ -360,7 +361,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  grid_dependency_sync(short_grid(p.num_tiles, 4));
+  grid_dependency_wait();
   for (int i = threadIdx.x; i < kPwHC; i += blockDim.x) {
     sConst[i] = p.g_colsum[i];
     sConst[kPwHC + i] = p.g_colbias[i];
@@ -369,6 +370,7 @@ pwa_out_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ 
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 4));
   const bool run = (smem_u32(smem) & 1023u) == 0;
   const int num_tiles = run ? p.num_tiles : 0;
   // local tile n of this CTA (n = 0, 1, ..) belongs to team n & 1 and is that team's (n >> 1)-th

@@ -69,13 +69,20 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
-// Programmatic dependent launch (host_util.h, launch_after): what stands in front of this touches nothing that an earlier kernel of
-// the stream writes and may run while that kernel drains; from here on everything it wrote is there.  With `next` the kernel
+// Programmatic dependent launch (host_util.h, launch_after): what stands in front of the wait touches nothing that an earlier kernel
+// of the stream writes and may run while that kernel drains; from there on everything it wrote is there.  With `next` the kernel
 // behind this one, if it was launched that way, may begin its own set-up as soon as every CTA has passed; without, when this one
-// ends.  The wait does nothing in a launch without the attribute.
-__device__ __forceinline__ void grid_dependency_sync(bool next) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+// ends.  Both do nothing in a launch without the attribute.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel that takes tensor memory lets the next one in behind the __syncthreads() that publishes the address, where every CTA
+// has its columns: one that shared an SM with it and took the columns first would hold them, waiting for this kernel to end, while
+// this kernel waited for them.
+__device__ __forceinline__ void grid_dependency_next(bool next) {
   if (next) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency_sync(bool next) {
+  grid_dependency_wait();
+  grid_dependency_next(next);
 }
 
 // at most `waves` tiles for every CTA of the launch

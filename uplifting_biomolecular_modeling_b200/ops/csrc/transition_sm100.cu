@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kTRThreads, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmWab,
                   const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmOut,
                   TransitionParams p) {
-  grid_dependency_sync(short_grid(p.num_tiles, 8));
+  grid_dependency_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + smem_pad1024(smem_raw);
   uint8_t* sX = smem;                                   // 2 x 32 KB
@@ -170,6 +170,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 8));
   const uint32_t tAB = tmem_base;        // two buffers of 128 columns
   const uint32_t tY = tmem_base + 256;   // 128 columns
   const uint32_t tH = tmem_base + 384;   // two buffers of 32 columns (two bf16 each)

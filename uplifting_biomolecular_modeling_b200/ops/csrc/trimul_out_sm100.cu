@@ -88,7 +88,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  grid_dependency_sync(short_grid(p.num_tiles, 8));
+  grid_dependency_wait();
   for (int i = threadIdx.x; i < 128; i += blockDim.x) {
     sConst[i] = p.o_colsum[i];
     sConst[128 + i] = p.o_colbias[i];
@@ -99,6 +99,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 8));
 
   if (warp == 0) {
     if (lane == 0) {

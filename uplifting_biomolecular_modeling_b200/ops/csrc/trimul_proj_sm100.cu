@@ -105,11 +105,12 @@ trimul_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  grid_dependency_sync(short_grid(p.num_tiles, 8));
+  grid_dependency_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(short_grid(p.num_tiles, 8));
   const bool run = (smem_u32(smem) & 1023u) == 0;
   const int num_tiles = run ? p.num_tiles : 0;
 
