@@ -1672,7 +1672,7 @@ __global__ void __launch_bounds__(kGemvMmaThreads, 2) gemv_mma_kernel(
 template <bool DUAL, bool STAGED>
 int launch_gemv_mma(const __nv_bfloat16* x, const float* gamma, float eps, const __nv_bfloat16* w,
                     const __nv_bfloat16* w2, const float* bias, const __nv_bfloat16* res, __nv_bfloat16* out, int M,
-                    int N, int K, bool pdl, cudaStream_t st) {
+                    int N, int K, cudaStream_t st) {
   auto kern = gemv_mma_kernel<DUAL, STAGED>;
   const size_t smem = STAGED ? static_cast<size_t>(M) * (K * 2 + 16) : 0;
   if (smem > 24 * 1024 &&   // 48 KB with the static part
@@ -1680,17 +1680,9 @@ int launch_gemv_mma(const __nv_bfloat16* x, const float* gamma, float eps, const
     return UBM_ERR_LAUNCH;
   const int tiles = (N + 15) / 16;
   const int slots = sm_count() * (smem > 90 * 1024 ? 1 : 2);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles < slots ? tiles : slots);
-  cfg.blockDim = dim3(kGemvMmaThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, kern, x, gamma, eps, w, w2, bias, res, out, M, N, K) != cudaSuccess) return UBM_ERR_LAUNCH;
+  if (launch_after(true, kern, dim3(tiles < slots ? tiles : slots), kGemvMmaThreads, smem, st, x, gamma, eps, w, w2, bias, res, out, M, N,
+                   K) != cudaSuccess)
+    return UBM_ERR_LAUNCH;
   UBM_CHECK_LAUNCH("gemv_mma_kernel");
   return UBM_OK;
 }
@@ -1707,15 +1699,11 @@ int launch_gemv(const __nv_bfloat16* x, const float* gamma, float eps, const __n
   int grid = (N + wpb - 1) / wpb;
   if (grid > sm_count() * per_sm) grid = sm_count() * per_sm;
   // launched so that its weight prefetch may overlap the tail of the previous kernel in the stream (see the kernel)
-  static const bool pdl = [] {
-    const char* e = getenv("UBM_PDL");
-    return e == nullptr || e[0] != '0';
-  }();
   if constexpr (!W8) {
     const uintptr_t bits = reinterpret_cast<uintptr_t>(w) | (DUAL ? reinterpret_cast<uintptr_t>(w2) : 0);
     if (M >= kGemvMmaMinRows && (K & 63) == 0 && (bits & 31) == 0 && static_cast<size_t>(M) * (K * 2 + 16) <= kGemvMaxSmem) {
-      return gamma != nullptr ? launch_gemv_mma<DUAL, true>(x, gamma, eps, w, w2, bias, res, out, M, N, K, pdl, st)
-                              : launch_gemv_mma<DUAL, false>(x, gamma, eps, w, w2, bias, res, out, M, N, K, pdl, st);
+      return gamma != nullptr ? launch_gemv_mma<DUAL, true>(x, gamma, eps, w, w2, bias, res, out, M, N, K, st)
+                              : launch_gemv_mma<DUAL, false>(x, gamma, eps, w, w2, bias, res, out, M, N, K, st);
     }
   }
 #define UBM_GEMV(MBV)                                                                                          \
@@ -1724,17 +1712,8 @@ int launch_gemv(const __nv_bfloat16* x, const float* gamma, float eps, const __n
     if (smem > 48 * 1024 &&                                                                                    \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvMaxSmem) != cudaSuccess)  \
       return UBM_ERR_LAUNCH;                                                                                   \
-    cudaLaunchConfig_t cfg = {};                                                                               \
-    cfg.gridDim = dim3(grid);                                                                                  \
-    cfg.blockDim = dim3(kGemvThreads);                                                                         \
-    cfg.dynamicSmemBytes = smem;                                                                               \
-    cfg.stream = st;                                                                                           \
-    cudaLaunchAttribute attr[1];                                                                               \
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;                                           \
-    attr[0].val.programmaticStreamSerializationAllowed = 1;                                                    \
-    cfg.attrs = attr;                                                                                          \
-    cfg.numAttrs = pdl ? 1 : 0;                                                                                \
-    if (cudaLaunchKernelEx(&cfg, kern, x, gamma, eps, w, w2, bias, res, out, M, N, K, wscale) != cudaSuccess)  \
+    if (launch_after(true, kern, dim3(grid), kGemvThreads, smem, st, x, gamma, eps, w, w2, bias, res, out, M, N, K, wscale) !=    \
+        cudaSuccess)                                                                                           \
       return UBM_ERR_LAUNCH;                                                                                   \
   } while (0)
   switch (MB) {
