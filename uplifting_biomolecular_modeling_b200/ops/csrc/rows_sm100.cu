@@ -174,8 +174,8 @@ __global__ void __launch_bounds__(256) layernorm_rows_narrow_kernel(const __nv_b
                                                                     const float* __restrict__ beta,
                                                                     __nv_bfloat16* __restrict__ out, long long R,
                                                                     float eps) {
-  grid_dependency_sync(short_rows(R, 256));
   constexpr int C = 8 * LPR;
+  grid_dependency_sync(short_rows(R, C));
   constexpr int RPW = 32 / LPR;
   const int lane = threadIdx.x & 31;
   const int sub = lane / LPR, li = lane % LPR;
