@@ -88,15 +88,20 @@ __device__ __forceinline__ PairA rows_to_a(uint4 lo, uint4 hi, uint32_t zero) {
 
 // The loads and products of a warp are pure functions of their operands, so that the compiler may place them freely (as volatile
 // statements in program order, every load stood in front of the product that waits for it: 4.1 times the time of a
-// unit).  What keeps the V loads behind the barrier is their address, which is redefined there (behind()).
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3) {
+// unit).  What keeps a V load behind the barrier is its address: ldmatrix takes only one that behind() has made, a volatile statement
+// that stays where it stands, in front of it the barrier and behind it everything that uses what it made.
+struct AddressBehind {
+  uint32_t at;
+};
+__device__ __forceinline__ AddressBehind behind(uint32_t addr) {
+  asm volatile("" : "+r"(addr) : : "memory");
+  return {addr};
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(AddressBehind base, uint32_t offset, uint32_t& a0, uint32_t& a1, uint32_t& a2,
+                                                  uint32_t& a3) {
   asm("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
       : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
-      : "r"(addr));
-}
-__device__ __forceinline__ uint32_t behind(uint32_t addr) {
-  asm volatile("" : "+r"(addr) : : "memory");
-  return addr;
+      : "r"(base.at + offset));
 }
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   float d0, d1, d2, d3;
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(kWLThreads, 1) window_layer_kernel(WindowLayer
 #pragma unroll
         for (int n = 0; n < 4; ++n) o[m][n][0] = o[m][n][1] = o[m][n][2] = o[m][n][3] = 0.f;
       }
-      const uint32_t v0a = behind(aV0 + buf), v1a = behind(aV1 + buf);
+      const AddressBehind v0a = behind(aV0 + buf), v1a = behind(aV1 + buf);
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
         uint32_t a[2][4];
@@ -283,8 +288,8 @@ __global__ void __launch_bounds__(kWLThreads, 1) window_layer_kernel(WindowLayer
         // logical keys 16 ks .. + 15: column blocks 2 ks and 2 ks + 1 of the scores
         const uint32_t at = ((ks >> 1) * 32 + 4 * (ks & 1)) * 256;
         uint32_t v[8];
-        ldmatrix_x4_trans(v0a + at, v[0], v[1], v[2], v[3]);
-        ldmatrix_x4_trans(v1a + at, v[4], v[5], v[6], v[7]);
+        ldmatrix_x4_trans(v0a, at, v[0], v[1], v[2], v[3]);
+        ldmatrix_x4_trans(v1a, at, v[4], v[5], v[6], v[7]);
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
