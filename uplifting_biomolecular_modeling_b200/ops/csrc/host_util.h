@@ -110,12 +110,24 @@ inline bool overlap_launches() {
   return on;
 }
 
-// Launch of a kernel that calls grid_dependency_sync() in every thread: with `overlap` its CTAs may be placed, and do their set-up,
-// while the kernel in front of it drains.  Between two kernels of one wave that hides about 3 us of launch, barrier and
+// Launch of a kernel that calls grid_dependency_sync(), or its two parts, in every thread: with `overlap` its CTAs may be placed, and do
+// their set-up, while the kernel in front of it drains.  Between two kernels of one wave that hides about 3 us of launch, barrier and
 // tensor-memory set-up (a Pairformer block of 137 tokens 298 -> 268 us, three atom layers 345 -> 327).  The CTAs then start in the
 // order in which SMs become free, no longer in the order of the tiles that share operands in L2.  So kernels that re-read theirs
 // from L2 for long ask for it, and let the next one begin, only while they are short (attention of 1536 tokens 6064 -> 6122 us, pair
 // averaging 672 -> 678, token layers 635 -> 639 where they did not).
+//
+// Where the lines lie, in captured passes with / without the overlap on either side (spread 0.5 to 1 %; up to 3 at sizes of 50 us):
+//   eight waves (trimul_*, transition, atom_*, window_layer: whether the next one is let in)  triangle multiplication of 230 tokens 46.3 /
+//     48.6 us, 300 (six waves) 77.4 / 79.5, 360 (seven) 97.3 / 99.5, from 460 (twelve) on the same; atom layers of 1 x 12768 125.5 / 129.5
+//   four waves (pwa)  pair averaging of 64 x 256 33.9 / 34.8, 290 x 256 61.2 / 64.1, with its output stage beyond the line 300 x 256 70.3 /
+//     72.6, 600 x 256 107.0 / 107.2, 1024 x 512 382.0 / 372.3
+//   two waves (attention)  triangle attention of 137 tokens 40.6 / 41.0, 200 (1.4 waves) 68.1 / 69.9, a Pairformer block of 137 230.5 / 233.5;
+//     beyond, no difference (170 tokens, 2.3 waves, 52.0 / 51.7; 260 105.8 / 106.1) until the form costs its schedule
+//   rows: see short_rows(); softmax rows of the pair averaging 2048 blocks: 256 x 200 57.4 / 60.4, 16 x 1024 107.5 / 108.4, 2200 and 3000
+//     tokens the same
+//   always (key masks, sums of the single track, decode operators, GEMM): a few us each, or measured to gain at every size
+// The projection of triangle attention is launched without (pair_proj_sm100.cu).
 template <typename... P, typename... A>
 inline cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream,
                                 const A&... args) {
