@@ -122,8 +122,8 @@ inline bool overlap_launches() {
 //     48.6 us, 300 (six waves) 77.4 / 79.5, 360 (seven) 97.3 / 99.5, from 460 (twelve) on the same; atom layers of 1 x 12768 125.5 / 129.5
 //   four waves (pwa)  pair averaging of 64 x 256 33.9 / 34.8, 290 x 256 61.2 / 64.1, with its output stage beyond the line 300 x 256 70.3 /
 //     72.6, 600 x 256 107.0 / 107.2, 1024 x 512 382.0 / 372.3
-//   two waves (attention)  triangle attention of 137 tokens 40.6 / 41.0, 200 (1.4 waves) 68.1 / 69.9, a Pairformer block of 137 230.5 / 233.5;
-//     beyond, no difference (170 tokens, 2.3 waves, 52.0 / 51.7; 260 105.8 / 106.1) until the form costs its schedule
+//   two waves (attention)  triangle attention of 100 tokens 28.2 / 28.7, 137 (1.9 waves) 40.6 / 41.0, a Pairformer block of 137 230.5 /
+//     233.5; beyond, no difference (170 tokens, 2.3 waves, 52.0 / 51.7; 260 105.8 / 106.1) until the form costs its schedule
 //   rows: see short_rows(); softmax rows of the pair averaging 2048 blocks: 256 x 200 57.4 / 60.4, 16 x 1024 107.5 / 108.4, 2200 and 3000
 //     tokens the same
 //   always (key masks, sums of the single track, decode operators, GEMM): a few us each, or measured to gain at every size
