@@ -61,3 +61,9 @@ def test_predictor_plan_names_a_row_for_every_call_class():
     pred.dtype = __import__("torch").bfloat16
     fast = pred.provider_plan(1536, 12768)
     assert fast["triattn|D32H4"].row in ("tcgen05_4row", "stock")              # stock when the table has no cpu cells
+
+
+@pytest.mark.parametrize("heads,c,row", [(4, 128, "mma_window"), (8, 128, "tcgen05_window"), (8, 256, "tcgen05_window")])
+def test_atom_windows_are_recorded_under_the_kernel_that_serves_them(heads, c, row):
+    call = {"head_dim": 32, "heads": heads, "c": c, "window": (32, 128), "dtype": "bf16"}
+    assert pv.select("apb", "sm100", "WIN32x128", 12768, "fast", call).row == row

@@ -147,8 +147,8 @@ class Predictor:
             ("ln", f"C{c.c_m}", n_tokens, {"c": c.c_m, "dtype": dt}),
         ]
         if n_atoms:
-            calls.append(("apb", "WIN32x128", n_atoms, {"head_dim": c.c_atom // c.atom_heads, "window": (32, 128),
-                                                        "dtype": dt}))
+            calls.append(("apb", "WIN32x128", n_atoms, {"head_dim": c.c_atom // c.atom_heads, "heads": c.atom_heads, "c": c.c_atom,
+                                                        "window": (32, 128), "dtype": dt}))
         plan = {}
         for fam, klass, n, call in calls:
             plan[f"{fam}|{klass}"] = provider.select(fam, sm, klass, n, self.mode, call)

@@ -168,9 +168,12 @@ class DiffusionTransformerLayer(_Switchable):
                 or ("window_mask" if (atoms and mask is not None) else None)
             klass = f"WIN{window[0]}x{window[1]}" if window is not None else \
                 f"D{64 if self.pair_bias_attn.head_dim > 32 else 32}H{self.pair_bias_attn.heads}S{a.shape[0]}"
-            if self._decide(why, klass, a.shape[1], {"head_dim": self.pair_bias_attn.head_dim, "dtype": "bf16",
-                                                     **({"window": tuple(window)} if window is not None else {})},
-                            "tcgen05_window" if atoms else "tcgen05_2row"):
+            call = {"head_dim": self.pair_bias_attn.head_dim, "dtype": "bf16"}
+            row = "tcgen05_2row"
+            if window is not None:
+                call.update(window=tuple(window), heads=self.pair_bias_attn.heads, c=a.shape[-1])
+                row = "mma_window" if (call["heads"], call["c"]) == (4, 128) else "tcgen05_window"
+            if self._decide(why, klass, a.shape[1], call, row):
                 return self._fused_token_layer(a, h, bias, mask)
         if isinstance(bias, WindowBias):
             bias = bias.dense()

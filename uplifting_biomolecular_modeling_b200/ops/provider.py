@@ -125,6 +125,7 @@ register(Row("trimul", "tcgen05_3stage", _needs(c_z={128}, c_hidden={128}, dtype
 register(Row("transition", "tcgen05_fused", _needs(c={128}, expansion={4}, dtype={"bf16"})))
 register(Row("transition", "rows_gemm", _needs(dtype={"bf16"})))
 register(Row("apb", "tcgen05_2row", _needs(head_dim={32, 64}, dtype={"bf16"})))
+register(Row("apb", "mma_window", _needs(head_dim={32}, heads={4}, c={128}, window={(32, 128)}, dtype={"bf16"})))
 register(Row("apb", "tcgen05_window", _needs(head_dim={32}, window={(32, 128)}, dtype={"bf16"})))
 register(Row("apb", "simt_window", _needs(head_dim={32}, dtype={"bf16"})))
 register(Row("ln", "rows_narrow", _needs(c={64, 128, 256}, dtype={"bf16"})))
