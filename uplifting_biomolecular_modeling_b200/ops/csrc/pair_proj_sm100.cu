@@ -471,9 +471,11 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
   rc = set_smem(kern, kPPSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  // Not overlapped with the kernel in front (host_util.h, launch_after), nor the attention with it: at up to four tiles a CTA, captured
-  // passes of triangle attention took 26.6 us overlapped and 23.6 so at 64 tokens, 30.5 / 27.7 at 100, 39.2 / 37.4 at 137, 79.4 / 75.4 at
-  // 230, and a Pairformer block the same within half a percent (137 tokens 230.5 / 231.6, 200 323.2 / 322.9); above it lost 1 to 2 %.
+  // Not overlapped with the kernel in front (host_util.h, launch_after), nor the attention with it.  At up to four tiles a CTA, captured
+  // passes, overlapped / so: triangle attention without a mask 26.4 / 24.1 us at 64 tokens, 29.5 / 27.0 at 100, 39.9 / 37.7 at 137, 70.8 /
+  // 67.5 at 220, 110.3 / 106.7 at 271; with one laid out in front, whose launch the overlap hides, 29.7 / 28.7 at 100, 41.0 / 40.4 at 137, but
+  // 54.5 / 55.3 at 180 and 112.0 / 112.9 at 271.  Pairformer blocks without a mask 172.0 / 167.7 at 100 tokens, 466.3 / 461.3 at 271, with
+  // one 174.8 / 172.9 and 478.9 / 480.2.  Beyond four tiles it lost 1 to 2 %.
   kern<<<grid, kPPThreads, kPPSmemBytes, stream>>>(tmX, tmW, maps, outs, p);
   UBM_CHECK_LAUNCH("pair_proj_kernel");
   return UBM_OK;
