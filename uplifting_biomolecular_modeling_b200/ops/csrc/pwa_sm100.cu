@@ -11,8 +11,8 @@
 // GEMM they crossed it eleven times (projections, the transpose into planes, gate, product, transpose back).
 // 1024 sequences x 768 tokens: 0.65 ms (weights 3, softmax 17, values 93, GEMM 277, output stage 165 us, bias planes 34)
 // against 2.54 ms.  Values and output stage move the 0.4 GB of v and o (60 us each at copy bandwidth); neither fills a unit
-// (values at 512 x 512: DRAM 43 %, issue slots 51 %, special-function unit 2 % busy; output stage at 1024 x 768: DRAM 53, issue slots 50,
-// special-function unit 33 %), their warps wait for tensor and shared memory.
+// (values at 512 x 512: DRAM 43 %, issue slots 51 %, special-function unit 2 % busy; output stage at 1024 x 768: DRAM 44, issue slots 52,
+// special-function unit 34 %), their warps wait for tensor and shared memory.
 #include "host_util.h"
 #include "sm100.cuh"
 
