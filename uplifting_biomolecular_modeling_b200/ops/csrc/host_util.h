@@ -127,7 +127,7 @@ inline bool overlap_launches() {
 //   rows: see short_rows(); softmax rows of the pair averaging 2048 blocks: 256 x 200 57.4 / 60.4, 16 x 1024 107.5 / 108.4, 2200 and 3000
 //     tokens the same
 //   always (key masks, sums of the single track, decode operators, GEMM): a few us each, or measured to gain at every size
-// The projection of triangle attention is launched without (pair_proj_sm100.cu).
+//   the projection of triangle attention: four tiles a CTA, and only behind the layout of a mask (pair_proj_sm100.cu)
 template <typename... P, typename... A>
 inline cudaError_t launch_after(bool overlap, void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream,
                                 const A&... args) {

@@ -53,6 +53,7 @@ struct PairProjParams {
   float* stats_out;  // optional [R][2] (mu, rstd) of the input rows, or null
   KernelStatus* status;
   int num_tiles;
+  int overlap;       // launched to overlap the kernel in front, and the next one with it (launch_pair_proj)
   PeerSrc src;       // src.n > 0: the input rows are columns of z fetched from their owners (see host_util.h)
   // q | k | v | gate leave through shared memory: every epilogue warp stages 16 rows x 32 columns (64-byte swizzle) and one
   // lane stores the box with a bulk tensor copy (maps in PairOutMaps).  Under the transposed write, 16 rows that straddle
@@ -121,6 +122,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  grid_dependency_wait();
   // column constants
   for (int i = threadIdx.x; i < 512; i += blockDim.x) {
     sColsum[i] = p.colsum[i];
@@ -130,6 +132,7 @@ pair_proj_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_next(p.overlap != 0);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -417,7 +420,7 @@ static_assert(kPPSmemBytes <= 232448, "shared memory of one CTA");
 
 static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cudaStream_t stream,
                             const void* const* z_ptrs = nullptr, const int* peer_rows = nullptr, int npeers = 0,
-                            int me = 0) {
+                            int me = 0, bool behind_mask = false) {
   CUtensorMap tmX, tmW;
   uint64_t dX[2] = {(uint64_t)kPPC, (uint64_t)p.R};
   uint64_t sX[1] = {(uint64_t)kPPC * 2};
@@ -471,12 +474,13 @@ static int launch_pair_proj(const void* x, const void* w, PairProjParams p, cuda
   rc = set_smem(kern, kPPSmemBytes);
   if (rc) return rc;
   const int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
-  // Not overlapped with the kernel in front (host_util.h, launch_after), nor the attention with it.  At up to four tiles a CTA, captured
-  // passes, overlapped / so: triangle attention without a mask 26.4 / 24.1 us at 64 tokens, 29.5 / 27.0 at 100, 39.9 / 37.7 at 137, 70.8 /
-  // 67.5 at 220, 110.3 / 106.7 at 271; with one laid out in front, whose launch the overlap hides, 29.7 / 28.7 at 100, 41.0 / 40.4 at 137, but
-  // 54.5 / 55.3 at 180 and 112.0 / 112.9 at 271.  Pairformer blocks without a mask 172.0 / 167.7 at 100 tokens, 466.3 / 461.3 at 271, with
-  // one 174.8 / 172.9 and 478.9 / 480.2.  Beyond four tiles it lost 1 to 2 %.
-  kern<<<grid, kPPThreads, kPPSmemBytes, stream>>>(tmX, tmW, maps, outs, p);
+  // Overlapped with the kernel in front (host_util.h, launch_after) only where that lays out the key mask, a few blocks whose time the
+  // set-up hides, and up to four tiles a CTA: passes of triangle attention, overlapped / not, 59.9 / 62.3 us at 180 tokens, 74.1 / 77.0 at
+  // 220, 121.6 / 124.7 at 271, a Pairformer block of 271 494.6 / 499.3; beyond four tiles it loses 1 to 2 %.  Without a mask the kernel in
+  // front is a product, and the attention is let in early: 31.3 / 28.7 us at 100 tokens, 43.5 / 41.2 at 137, 74.9 / 72.2 at 220, 117.0 /
+  // 114.6 at 271.
+  p.overlap = behind_mask && p.num_tiles <= 4 * grid ? 1 : 0;
+  launch_after(p.overlap != 0, kern, grid, kPPThreads, kPPSmemBytes, stream, tmX, tmW, maps, outs, p);
   UBM_CHECK_LAUNCH("pair_proj_kernel");
   return UBM_OK;
 }
@@ -490,7 +494,8 @@ static int triatt_proj_impl(const void* z, const void* w, const void* colsum, co
                                     const void* wb, const void* wb_colsum, const void* wb_colbias, void* q, void* k,
                                     void* v, void* g, void* headbias, void* stats_out, int rows, int plane_rows, int N,
                                     int Np, int H, int transpose_out, void* status, void* stream,
-                                    const void* const* z_ptrs, const int* peer_rows, int npeers, int me) {
+                                    const void* const* z_ptrs, const int* peer_rows, int npeers, int me,
+                                    bool behind_mask = false) {
   using namespace ubm;
   if (N <= 0 || rows <= 0 || plane_rows < rows || Np < N || (Np & 7) || H <= 0 || H > kPPMaxHeads)
     return UBM_ERR_ARGUMENT;
@@ -515,7 +520,7 @@ static int triatt_proj_impl(const void* z, const void* w, const void* colsum, co
   p.transpose_out = transpose_out;
   p.stats_out = static_cast<float*>(stats_out);
   p.status = static_cast<KernelStatus*>(status);
-  return launch_pair_proj(z, w, p, static_cast<cudaStream_t>(stream), z_ptrs, peer_rows, npeers, me);
+  return launch_pair_proj(z, w, p, static_cast<cudaStream_t>(stream), z_ptrs, peer_rows, npeers, me, behind_mask);
 }
 
 extern "C" int ubm_triatt_proj_rows(const void* z, const void* w, const void* colsum, const void* colbias,
@@ -548,4 +553,13 @@ extern "C" int ubm_triatt_proj(const void* z, const void* w, const void* colsum,
                                void* stream) {
   return ubm_triatt_proj_rows(z, w, colsum, colbias, wb, wb_colsum, wb_colbias, q, k, v, g, headbias, stats_out, N, N,
                               N, Np, H, transpose_out, status, stream);
+}
+
+// The same, launched right behind the layout of the key mask.
+extern "C" int ubm_triatt_proj_behind_mask(const void* z, const void* w, const void* colsum, const void* colbias, const void* wb,
+                                           const void* wb_colsum, const void* wb_colbias, void* q, void* k, void* v, void* g,
+                                           void* headbias, void* stats_out, int N, int Np, int H, int transpose_out, void* status,
+                                           void* stream) {
+  return triatt_proj_impl(z, w, colsum, colbias, wb, wb_colsum, wb_colbias, q, k, v, g, headbias, stats_out, N, N, N, Np, H,
+                          transpose_out, status, stream, nullptr, nullptr, 0, 0, true);
 }

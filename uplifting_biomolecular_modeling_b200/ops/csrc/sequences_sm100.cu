@@ -25,6 +25,9 @@ int ubm_key_mask(const void* keep, int elem_bytes, long long s_row, long long s_
 int ubm_triatt_proj(const void* z, const void* w, const void* colsum, const void* colbias, const void* wb, const void* wb_colsum,
                     const void* wb_colbias, void* q, void* k, void* v, void* g, void* headbias, void* stats_out, int N, int Np,
                     int H, int transpose_out, void* status, void* stream);
+int ubm_triatt_proj_behind_mask(const void* z, const void* w, const void* colsum, const void* colbias, const void* wb,
+                                const void* wb_colsum, const void* wb_colbias, void* q, void* k, void* v, void* g, void* headbias,
+                                void* stats_out, int N, int Np, int H, int transpose_out, void* status, void* stream);
 int ubm_attention_d32(const void* q, const void* k, const void* v, const void* bias, const void* gate, void* out,
                       const void* kmask, const void* kflags, int rows, int Nq, int Nk, int H, long long ldb, long long ld_in,
                       long long ld_gate, long long ld_mask, int transpose_out, void* status, void* stream);
@@ -133,8 +136,9 @@ int triatt(const void* z, const Keep& keep, void* add, void* flags, long long ld
   const long long rows = static_cast<long long>(N) * N;
   uint16_t* q = static_cast<uint16_t*>(qkvgo);
   uint16_t *k = q + rows * 128, *v = k + rows * 128, *g = v + rows * 128, *o = g + rows * 128;
-  rc = ubm_triatt_proj(z, w.w, w.colsum, w.colbias, w.wb, w.wb_colsum, w.wb_colbias, q, k, v, g, hb, nullptr, N, Np, H,
-                       starting ? 0 : 1, status, stream);
+  rc = (keep.ptr != nullptr ? ubm_triatt_proj_behind_mask : ubm_triatt_proj)(z, w.w, w.colsum, w.colbias, w.wb, w.wb_colsum, w.wb_colbias,
+                                                                             q, k, v, g, hb, nullptr, N, Np, H, starting ? 0 : 1, status,
+                                                                             stream);
   if (rc) return rc;
   rc = ubm_attention_d32(q, k, v, hb, g, o, add, flags, N, N, N, H, Np, 0, 0, add == nullptr ? 0 : ld_mask, starting ? 0 : 1, status,
                          stream);
