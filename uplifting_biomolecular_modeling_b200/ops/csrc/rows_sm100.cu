@@ -19,12 +19,15 @@
 
 namespace ubm {
 
-// Row kernels of up to 8 MB take a few us each: their launch may overlap the kernel in front.  An encoder layer of 8 x 512 tokens (7.9 MB a
-// norm) takes 149.8 us with it and 151.6 without, one of 2 x 512 71.6 and 73.8; beyond, the CTAs placed early cost more than they
-// hide: 8 x 1024 tokens (15.7 MB) 278.9 with it and 275.0 without, head biases of 256 tokens (16.8 MB) in the pair averaging 52.9 and
-// 51.2.  Conditioned norms, which read two more rows a row, up to 4 MB: two token layers of 5 x 512 (3.9 MB) 252.2 with and 263.0
-// without, of 5 x 1536 (11.8 MB) 639 and 635.
-__host__ __device__ inline bool short_rows(long long R, long long C) { return R * C <= (4ll << 20); }
+// Row kernels of up to 16 MB take a few us each: their launch may overlap the kernel in front.  Without, an outer product of 128 x 700
+// tokens (11.5 MB of rows) takes 613.6 instead of 609.3 us, a pair averaging of 512 x 230 (head biases of 13.5 MB) 106.7 instead of 104.9, a
+// Pairformer block of 220 347.1 instead of 344.3.  (Conditioned norms, which read two more rows a row, up to 4 MB: two token layers of
+// 5 x 512, 3.9 MB a norm, 252 with and 263 without, of 5 x 1536, 11.8 MB, 639 and 635.)
+__host__ __device__ inline bool short_rows(long long R, long long C) { return R * C <= (8ll << 20); }
+// Norms of wide rows, in front of a product, up to 12 MB: encoder layers of 2 x 512 tokens (2 MB a norm) 71.6 with and 73.8 without, 8 x 512
+// (7.9 MB) 149.8 and 151.6, 6 x 900 (10.4 MB) 208.3 and 208.6, but 8 x 1024 (15.7 MB) 292.2 and 287.8: the CTAs placed early then cost more
+// than they hide.
+__host__ __device__ inline bool short_wide_norm(long long R, long long C) { return R * C <= (6ll << 20); }
 
 template <typename T>
 __device__ __forceinline__ float to_f(T v);
@@ -94,7 +97,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_wide_kernel(const __nv_bfl
                                                                   const float* __restrict__ beta,
                                                                   __nv_bfloat16* __restrict__ out, long long R, int C,
                                                                   float eps) {
-  grid_dependency_sync(short_rows(R, C));
+  grid_dependency_sync(short_wide_norm(R, C));
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (long long r = static_cast<long long>(blockIdx.x) * wpb + (threadIdx.x >> 5); r < R;
@@ -508,7 +511,7 @@ __global__ void __launch_bounds__(256) adaln_rows_kernel(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ shift,
                                                          __nv_bfloat16* __restrict__ out, long long R, int C,
                                                          long long cond_rows, long long ld_cond, float eps) {
-  grid_dependency_sync(short_rows(2 * R, C));
+  grid_dependency_sync(short_rows(4 * R, C));
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (long long r = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); r < R;
@@ -545,7 +548,7 @@ __global__ void __launch_bounds__(256) adaln_rows_vec_kernel(const __nv_bfloat16
                                                              const __nv_bfloat16* __restrict__ shift,
                                                              __nv_bfloat16* __restrict__ out, long long R, int C,
                                                              long long cond_rows, long long ld_cond, float eps) {
-  grid_dependency_sync(short_rows(2 * R, C));
+  grid_dependency_sync(short_rows(4 * R, C));
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   for (long long r = static_cast<long long>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); r < R;
@@ -601,7 +604,7 @@ __global__ void __launch_bounds__(256) adaln_rows_c128_kernel(const __nv_bfloat1
                                                               const __nv_bfloat16* __restrict__ shift,
                                                               __nv_bfloat16* __restrict__ out, long long R,
                                                               long long cond_rows, long long ld_cond, float eps) {
-  grid_dependency_sync(short_rows(2 * R, 128));
+  grid_dependency_sync(short_rows(4 * R, 128));
   constexpr int C = 128;
   const int halves_per_block = blockDim.x >> 4;
   const int l16 = threadIdx.x & 15;
@@ -839,8 +842,8 @@ extern "C" int ubm_layernorm_rows(const void* x, const void* gamma, const void* 
     const int gridw = grid_for(R, 8);
     const bool vec = ((reinterpret_cast<uintptr_t>(gg) | reinterpret_cast<uintptr_t>(bb)) & 31) == 0;
 #define UBM_LN_WIDE(CH)                                                                                          \
-  (vec ? launch_after(short_rows(R, C), layernorm_rows_wide_kernel<CH, true>, gridw, 256, 0, st, xx, gg, bb, oo, R, C, eps)                  \
-       : launch_after(short_rows(R, C), layernorm_rows_wide_kernel<CH, false>, gridw, 256, 0, st, xx, gg, bb, oo, R, C, eps))
+  (vec ? launch_after(short_wide_norm(R, C), layernorm_rows_wide_kernel<CH, true>, gridw, 256, 0, st, xx, gg, bb, oo, R, C, eps)                  \
+       : launch_after(short_wide_norm(R, C), layernorm_rows_wide_kernel<CH, false>, gridw, 256, 0, st, xx, gg, bb, oo, R, C, eps))
     if (C <= 512) UBM_LN_WIDE(2);
     else if (C <= 1024) UBM_LN_WIDE(4);
     else if (C <= 1280) UBM_LN_WIDE(5);
@@ -996,17 +999,17 @@ extern "C" int ubm_adaln_rows(const void* a, const void* scale, const void* shif
                      reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   const int grid = grid_for(R, 8);
   if (vec && C == 128) {
-    launch_after(short_rows(2 * R, C), adaln_rows_c128_kernel, grid_for((R + 1) / 2 * 2, 16), 256, 0, st, aa, sc, sh, oo, R, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_c128_kernel, grid_for((R + 1) / 2 * 2, 16), 256, 0, st, aa, sc, sh, oo, R, cond_rows, ld_cond, eps);
   } else if (vec && C <= 256) {
-    launch_after(short_rows(2 * R, C), adaln_rows_vec_kernel<1>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<1>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else if (vec && C <= 512) {
-    launch_after(short_rows(2 * R, C), adaln_rows_vec_kernel<2>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<2>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else if (vec && C <= 768) {
-    launch_after(short_rows(2 * R, C), adaln_rows_vec_kernel<3>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<3>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else if (vec) {
-    launch_after(short_rows(2 * R, C), adaln_rows_vec_kernel<4>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_vec_kernel<4>, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   } else {
-    launch_after(short_rows(2 * R, C), adaln_rows_kernel, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
+    launch_after(short_rows(4 * R, C), adaln_rows_kernel, grid, 256, 0, st, aa, sc, sh, oo, R, C, cond_rows, ld_cond, eps);
   }
   UBM_CHECK_LAUNCH("adaln_rows_kernel");
   return UBM_OK;
