@@ -79,22 +79,20 @@ def mean_rescale_(o: torch.Tensor, count: torch.Tensor, bias: torch.Tensor, tota
 _HB_CACHE: dict = {}
 
 
-def _kept(t: Optional[torch.Tensor]):
+def _kept(t: Optional[torch.Tensor]) -> tuple:
     """What tells later whether ``t`` is still the tensor, with the contents, that something was made from: the object (weakly), its
     version, and its storage, held so that no other can have its address (a converted copy swaps ``.data`` and leaves the version)."""
-    return None if t is None else (weakref.ref(t), t._version, t.detach())
+    return (lambda: None, 0, 0, None) if t is None else (weakref.ref(t), t._version, t.data_ptr(), t.detach())
 
 
-def _unchanged(kept, t: Optional[torch.Tensor]) -> bool:
-    if kept is None or t is None:
-        return kept is None and t is None
-    return kept[0]() is t and kept[1] == t._version and kept[2].data_ptr() == t.data_ptr() and kept[2].dtype == t.dtype
+def _unchanged(kept: tuple, t: Optional[torch.Tensor]) -> bool:
+    return kept[0]() is t and (t is None or (kept[1] == t._version and kept[2] == t.data_ptr()))
 
 
 def _head_bias_weights(w: torch.Tensor, ln_w, ln_b, scale: float, device) -> tuple:
     """(fp32 weights with the norm's scale folded in, their row sums, their products with the norm's shift), kept until the weight or
     either parameter of the norm is another one or is written."""
-    key = (id(w), float(scale), str(device))
+    key = (id(w), scale, device)
     entry = _HB_CACHE.get(key)
     if entry is not None and _unchanged(entry[0], w) and _unchanged(entry[1], ln_w) and _unchanged(entry[2], ln_b):
         return entry[3]
