@@ -820,26 +820,25 @@ BYTE_LUT = {c: i for i, c in enumerate("ACGTN")}
 _W_CACHE: dict = {}
 
 
-def _source(t: Optional[torch.Tensor]) -> tuple:
-    """What a form kept of a parameter is compared by: the object, its version and its storage (a converted or sharded copy swaps ``.data``
-    and leaves the version as it is)."""
-    return (None, 0, 0, ()) if t is None else (t, t._version, t.data_ptr(), t.shape)
-
-
-def _is_source(kept: tuple, t: Optional[torch.Tensor]) -> bool:
-    return kept[0] is t and (t is None or (kept[1] == t._version and kept[2] == t.data_ptr() and kept[3] == t.shape))
-
-
 def _bf16_weight(module: nn.Linear):
-    """(contiguous bf16 weight, fp32 bias or None) of a linear layer, kept until either is written again or given other storage."""
-    ent = _W_CACHE.get(id(module))
+    """(contiguous bf16 weight, fp32 bias or None) of a linear layer, kept until either is written again or given other storage (a
+    converted or sharded copy swaps ``.data`` and leaves the version as it is; the storages are held, so that no others can have
+    their addresses)."""
     weight, bias = module.weight, module.bias           # one look-up each: a module's attributes are found through its dictionaries
-    if ent is None or not _is_source(ent[0], weight) or not _is_source(ent[1], bias):
-        # (the storages are held along, so that no others can have their addresses)
-        ent = (_source(weight), _source(bias), weight.detach().to(torch.bfloat16).contiguous(),
-               None if bias is None else bias.detach().float().contiguous(), weight.detach(), None if bias is None else bias.detach())
-        _W_CACHE[id(module)] = ent
-    return ent[2], ent[3]
+    ent = _W_CACHE.get(id(module))
+    if ent is not None and ent[2] is weight and ent[3] == weight._version and ent[4] == weight.data_ptr() and \
+            ent[5] == weight.numel() and ent[6] is bias and \
+            (bias is None or (ent[7] == bias._version and ent[8] == bias.data_ptr() and ent[9] == bias.numel())):
+        return ent[0], ent[1]
+    form = weight.detach().to(torch.bfloat16).contiguous()
+    of_bias = None if bias is None else bias.detach().float().contiguous()
+    _W_CACHE[id(module)] = (form, of_bias) + _source(weight) + _source(bias) + (weight.detach(), None if bias is None else bias.detach())
+    return form, of_bias
+
+
+def _source(t: Optional[torch.Tensor]) -> tuple:
+    """What a form kept of a parameter is compared by: the object, its version, its storage and size."""
+    return (None, 0, 0, 0) if t is None else (t, t._version, t.data_ptr(), t.numel())
 
 
 def _decode_rows(block: "Block", x: torch.Tensor) -> bool:
@@ -872,7 +871,8 @@ def _e4m3_weight(module: nn.Linear):
     from ..ops import gemm
     w, bias = module.weight, module.bias
     ent = _W8_CACHE.get(id(module))
-    if ent is None or not _is_source(ent[0], w) or not _is_source(ent[1], bias):
+    if ent is None or ent[0][0] is not w or ent[1][0] is not bias or ent[0][1:] != _source(w)[1:] or ent[1][1:] != _source(bias)[1:] or \
+            ent[2].shape != w.shape:
         q, dq = gemm.quantize_e4m3(w)
         # (unlike the storage of a bf16 form, which is the weight's own, that behind these bytes may go)
         ent = (_source(w), _source(bias), q, dq, None if bias is None else bias.detach().float().contiguous())
